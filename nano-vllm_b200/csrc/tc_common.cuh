@@ -1,4 +1,4 @@
-// tcgen05 / TMEM / TMA building blocks shared by the tensor-core kernels (prefill_tc.cu, linear_tc.cu).
+// tcgen05 / TMEM / TMA building blocks shared by the tensor-core kernels (fa_tc.cuh, linear_tc.cu).
 #pragma once
 #include <cuda.h>
 
