@@ -273,25 +273,39 @@ __global__ void __launch_bounds__(128) qknorm_rope_store_tok_kernel(
     }
 }
 
-// store_kvcache_kernel (layers/attention.py:10-30): one warp per (token, kv head).
-__global__ void __launch_bounds__(128) store_kv_kernel(const __nv_bfloat16* __restrict__ k, int64_t k_stride,
+// store_kvcache_kernel (layers/attention.py:10-30): a row of K and of V per (token, kv head).  Bound by HBM.  T = uint4: half a warp per row
+// and U rows per thread group whose loads are all in flight before the first store (U = 4 for prompt steps: 15.7 k tokens of 8 heads, 129 MB,
+// 34.5 us with a warp per row and one 8-byte load each; U = 1 spreads a decode step's few rows).  T = uint2 (a warp per row): projections that
+// are only 8-byte aligned.
+template <typename T, int U>
+__global__ void __launch_bounds__(256) store_kv_kernel(const __nv_bfloat16* __restrict__ k, int64_t k_stride,
                                                        const __nv_bfloat16* __restrict__ v, int64_t v_stride,
                                                        const int32_t* __restrict__ slot_mapping,
                                                        __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, int hkv,
                                                        int block_shift, int n) {
     B200_PDL_SYNC();
-    const int64_t gwarp = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (gwarp >= (int64_t)n * hkv) return;
-    const int tok = (int)(gwarp / hkv);
-    const int kvh = (int)(gwarp - (int64_t)tok * hkv);
-    const int lane = threadIdx.x & 31;
-    const int slot = slot_mapping[tok];
-    if (slot < 0) return;
-    const int64_t row = ((((int64_t)(slot >> block_shift)) * hkv + kvh) << block_shift) + (slot & ((1 << block_shift) - 1));
-    reinterpret_cast<uint2*>(k_cache + row * B200_HEAD_DIM)[lane] =
-        reinterpret_cast<const uint2*>(k + (int64_t)tok * k_stride + kvh * B200_HEAD_DIM)[lane];
-    reinterpret_cast<uint2*>(v_cache + row * B200_HEAD_DIM)[lane] =
-        reinterpret_cast<const uint2*>(v + (int64_t)tok * v_stride + kvh * B200_HEAD_DIM)[lane];
+    constexpr int LANES = B200_HEAD_DIM * 2 / sizeof(T), ROWS = 256 / LANES;
+    const int lane = threadIdx.x % LANES;
+    const int64_t first = (int64_t)blockIdx.x * (ROWS * U) + threadIdx.x / LANES, rows = (int64_t)n * hkv;
+    T kk[U], vv[U];
+    int64_t dst[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int64_t r = first + u * ROWS;
+        dst[u] = -1;
+        if (r >= rows) continue;
+        const int tok = (int)(r / hkv), kvh = (int)(r - (int64_t)tok * hkv);
+        const int slot = slot_mapping[tok];
+        if (slot >= 0) dst[u] = ((((int64_t)(slot >> block_shift)) * hkv + kvh) << block_shift) + (slot & ((1 << block_shift) - 1));
+        kk[u] = reinterpret_cast<const T*>(k + (int64_t)tok * k_stride + kvh * B200_HEAD_DIM)[lane];
+        vv[u] = reinterpret_cast<const T*>(v + (int64_t)tok * v_stride + kvh * B200_HEAD_DIM)[lane];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (dst[u] < 0) continue;
+        reinterpret_cast<T*>(k_cache + dst[u] * B200_HEAD_DIM)[lane] = kk[u];
+        reinterpret_cast<T*>(v_cache + dst[u] * B200_HEAD_DIM)[lane] = vv[u];
+    }
 }
 
 // SiluAndMul.forward (layers/activation.py:8-11)
@@ -412,10 +426,16 @@ extern "C" int b200_store_kv(b200_ctx* ctx, int layer, const void* k, int64_t k_
     if (layer < 0 || layer >= ctx->layers) return B200_EINVAL;
     if (k_stride0 % 4 || v_stride0 % 4 || ((uintptr_t)k & 7) || ((uintptr_t)v & 7)) return B200_EINVAL;
     if (n == 0) return B200_OK;
-    const int64_t warps = (int64_t)n * ctx->num_kv_heads;
-    B200_LAUNCH((store_kv_kernel), (unsigned)((warps + 3) / 4), 128, 0, static_cast<cudaStream_t>(stream), 
-        static_cast<const __nv_bfloat16*>(k), k_stride0, static_cast<const __nv_bfloat16*>(v), v_stride0,
-        slot_mapping, ctx->k_layer(layer), ctx->v_layer(layer), ctx->num_kv_heads, ctx->block_shift, n);
+    const int64_t rows = (int64_t)n * ctx->num_kv_heads;
+    const bool wide = k_stride0 % 8 == 0 && v_stride0 % 8 == 0 && aligned16(k) && aligned16(v);
+    auto go = [&](auto kernel, int rows_per_cta) {
+        B200_LAUNCH((kernel), (unsigned)((rows + rows_per_cta - 1) / rows_per_cta), 256, 0, static_cast<cudaStream_t>(stream),
+            static_cast<const __nv_bfloat16*>(k), k_stride0, static_cast<const __nv_bfloat16*>(v), v_stride0,
+            slot_mapping, ctx->k_layer(layer), ctx->v_layer(layer), ctx->num_kv_heads, ctx->block_shift, n);
+    };
+    if (!wide) go(store_kv_kernel<uint2, 1>, 8);
+    else if (rows >= 148 * 64 * 2) go(store_kv_kernel<uint4, 4>, 64);       // two CTAs of four rows per thread group on every SM
+    else go(store_kv_kernel<uint4, 1>, 16);
     return b200_launch_status(ctx);
 }
 
