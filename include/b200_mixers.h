@@ -128,6 +128,22 @@ int b200m_latent_attention(const void* q_lat, const void* q_raw, int64_t q_tok_s
                            int rot_dim, float scale, int window, int layout, int is32, int flags, int splits, float* part,
                            void* stream);
 
+/* Prompt portions with keys and values formed per head (bf16; B200_EUNSUPPORTED for other sizes than dim 128, rot_dim 64, vdim 128 or operands that
+ * are not 16-byte aligned): one gather, one GEMM of the caller's, one rotation, one attention launch.
+ *   gather: out[cu_k[s] + j] = the cached row of token j of sequence s (rows of row_elems elements; max_k: an upper bound of any sequence's tokens;
+ *           rows from out_rows on are dropped);
+ *   rotate: q[t, h, 0 .. rope_dims) (token stride, head stride) turned by positions[t], in place;
+ *   prompt: q [total_q, heads, dim + rot_dim] (row stride q_stride), rotated; keys and values [total_k, heads * 128] (row stride kv_stride) of the gathered
+ *           rows, whose columns rank .. rank + rot_dim are the key part all heads share; causal at the end of each sequence's keys, sink and window as
+ *           above; out [total_q, heads * vdim]. */
+int b200m_latent_gather(const void* cache, int row_elems, const int32_t* block_tables, int bt_stride, int block_size, const int32_t* cu_k, int num_seqs,
+                        int max_k, void* out, int out_rows, void* stream);
+int b200m_latent_rotate(void* q, int64_t tok_stride, int head_stride, const float* cos_sin, int rope_dims, const int64_t* positions, int n, int heads,
+                        int layout, void* stream);
+int b200m_latent_prompt(const void* q, int64_t q_stride, const void* keys, const void* values, int64_t kv_stride, const void* rows, int row_elems, int rank,
+                        int total_k, const int32_t* cu_q, const int32_t* cu_k, const float* sink, void* out, int total_q, int num_seqs, int max_q,
+                        int heads, int dim, int rot_dim, int vdim, float scale, int window, void* stream);
+
 /* ---- windowed grouped-query attention ------------------------------------------------------------------------------ */
 
 /* Per token of qkv = [q (q_cols) | k (k_cols) | v (v_cols)] (row stride `stride`): q <- q / rms(q) * q_norm_w over ALL q_cols

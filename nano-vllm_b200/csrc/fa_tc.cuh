@@ -25,7 +25,14 @@
 #pragma once
 #include "tc_common.cuh"
 
+// Each library that includes this names its copy: kernels, and the record of their shared-memory opt-in, must not be merged across libraries
+// of one process (a template's static is one object for all of them).
+#ifndef B200FA_COPY
+#define B200FA_COPY attn
+#endif
+
 namespace b200fa {
+inline namespace B200FA_COPY {
 
 using namespace b200tc;
 
@@ -47,6 +54,7 @@ struct FaParams {
     int hq, hkv, hp;                    // query heads, kv heads, head items (hq / 2 or hq)
     int q_col_step;                     // columns from one head of Q to the next
     int k_col_step, v_col0, v_col_step; // columns of kv head h: h * step (+ v_col0)
+    int k2_col;                         // 192-wide heads: first column of the last 64 key elements, shared by the heads, in their own map
     int block_size, box_rows;           // paged: rows of a page, rows per TMA box
     int64_t row0, page_rows, head_rows; // paged row = row0 + page * page_rows + kvh * head_rows + row in page
     float scale_log2;
@@ -248,7 +256,7 @@ struct FaSlot {
 template <int DQK, bool PAIR_HEADS, bool GENERAL>
 __global__ void __launch_bounds__(THREADS, 1)
 fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-          const __grid_constant__ FaParams p) {
+          const __grid_constant__ CUtensorMap tm_k2, const __grid_constant__ FaParams p) {
     using L = FaSmem<DQK>;
     constexpr uint32_t IDESC_QK = make_idesc(BM, BN, false), IDESC_PV = make_idesc(BM, DV, true);
     constexpr int RT = PAIR_HEADS ? BM : 2 * BM;
@@ -640,8 +648,11 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 if (lane == 0) mbar_expect_tx(bar(B_KFULL + sl.i), L::kKBytes);
                 __syncwarp();
                 if (lane < boxes)
-                    for (int h = 0; h < DQK / 64; ++h)
-                        tma_load_2d(base + L::kOffK + sl.i * L::kKBytes + lane * p.box_rows * 128 + h * L::kKSub, &tm_k, bar(B_KFULL + sl.i), it.kvh * p.k_col_step + h * 64, row);
+                    for (int h = 0; h < DQK / 64; ++h) {
+                        const uint32_t dst = base + L::kOffK + sl.i * L::kKBytes + lane * p.box_rows * 128 + h * L::kKSub;
+                        if (h < 2) tma_load_2d(dst, &tm_k, bar(B_KFULL + sl.i), it.kvh * p.k_col_step + h * 64, row);
+                        else tma_load_2d(dst, &tm_k2, bar(B_KFULL + sl.i), p.k2_col, row);         // the key part all heads share
+                    }
                 if (!fa_wait(bar(B_VEMPTY + sl.i), sl.ph ^ 1, dead)) goto leave;
                 if (lane == 0) mbar_expect_tx(bar(B_VFULL + sl.i), L::kVBytes);
                 __syncwarp();
@@ -663,9 +674,11 @@ leave:
     if (warp == 12) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
-// Launch; the caller has filled everything but hp / max_rb and built the maps (box of Q: 64 x 128, of K and V: 64 x box_rows or 64 x BN).
+// Launch; the caller has filled everything but hp / max_rb and built the maps (box of Q: 64 x 128, of K and V: 64 x box_rows or 64 x BN;
+// tk2 is only read with 192-wide heads).
 template <int DQK, bool PAIR_HEADS, bool GENERAL>
-int fa_launch(FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, int total_q, int max_seqlen_q, cudaStream_t stream) {
+int fa_launch(FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tk2, int total_q, int max_seqlen_q,
+              cudaStream_t stream) {
     constexpr int RT = PAIR_HEADS ? BM : 2 * BM;
     p.hp = PAIR_HEADS ? p.hq / 2 : p.hq;
     p.max_rb = (max_seqlen_q + RT - 1) / RT;
@@ -679,8 +692,9 @@ int fa_launch(FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const C
     if (bound > (1ll << 30)) return B200_EUNSUPPORTED;
     int64_t grid = bound < sms ? bound : sms;
     if ((bound + grid - 1) / grid > ITEM_CAP) grid = (bound + ITEM_CAP - 1) / ITEM_CAP;
-    B200_LAUNCH((fa_kernel<DQK, PAIR_HEADS, GENERAL>), dim3((unsigned)grid), THREADS, (FaSmem<DQK>::kTotal), stream, tq, tk, tv, p);
+    B200_LAUNCH((fa_kernel<DQK, PAIR_HEADS, GENERAL>), dim3((unsigned)grid), THREADS, (FaSmem<DQK>::kTotal), stream, tq, tk, tv, tk2, p);
     return b200_launch_status(nullptr);
 }
 
+}  // inline namespace
 }  // namespace b200fa

@@ -45,6 +45,6 @@ int b200_prefill_fa_launch(b200_ctx* ctx, int layer, const void* q, int64_t q_st
     // An even head group: the item's two tiles are two heads that share every K and V tile.  Else (groups of 1, 3, ..): 256 rows of one head.
     const bool pair = (num_q_heads / num_kv_heads) % 2 == 0;
     if (scale > 0.f)
-        return pair ? fa_launch<D, true, false>(p, tq, tk, tv, total_q, max_seqlen_q, stream) : fa_launch<D, false, false>(p, tq, tk, tv, total_q, max_seqlen_q, stream);
-    return pair ? fa_launch<D, true, true>(p, tq, tk, tv, total_q, max_seqlen_q, stream) : fa_launch<D, false, true>(p, tq, tk, tv, total_q, max_seqlen_q, stream);
+        return pair ? fa_launch<D, true, false>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream) : fa_launch<D, false, false>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream);
+    return pair ? fa_launch<D, true, true>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream) : fa_launch<D, false, true>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream);
 }

@@ -1,0 +1,146 @@
+// Prompt portions of the hybrid decoders' attention layers on the persistent tcgen05 kernel (fa_tc.cuh).
+//
+//   windowed grouped-query attention : queries from the projection, keys and values from token-major cache rows through the page table
+//   latent attention                 : keys and values of every head formed from the cached latents first.  Per (head, query, key) the
+//                                      products are then 192 + 128 wide instead of the 576 + 512 of attention over the latents themselves
+//                                      (rank 512), which pays from a few tens of queries per sequence on.
+#define B200FA_COPY mix
+#include "mix_common.cuh"
+#include "fa_tc.cuh"
+
+using namespace b200fa;
+
+namespace {
+
+// Rows of a cache are read by page: the map covers every row a page id can name.
+constexpr uint64_t ANY_ROWS = (1ull << 31) - 1;
+
+// Pages the kernel's boxes can follow: a block of 64 keys is whole pages, or lies inside one.
+bool pages_ok(int block_size) { return block_size % BN == 0 || (block_size >= 8 && BN % block_size == 0); }
+
+// The cached rows of every sequence, one after the other: out[cu_k[s] + j] = cache row of token j of sequence s.  A warp per row, 16-byte pieces.
+__global__ void __launch_bounds__(256) latent_gather_kernel(const uint4* __restrict__ cache, int pieces, const int32_t* __restrict__ block_tables, int bt_stride,
+                                                            int block_size, const int32_t* __restrict__ cu_k, uint4* __restrict__ out, int out_rows) {
+    B200_PDL_SYNC();
+    const int s = blockIdx.y, j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int k0 = cu_k[s], len = cu_k[s + 1] - k0;
+    if (j >= len || k0 + j >= out_rows) return;
+    int page = block_tables[(int64_t)s * bt_stride + j / block_size];
+    page = page < 0 ? 0 : page;
+    const uint4* src = cache + ((int64_t)page * block_size + j % block_size) * pieces;
+    uint4* dst = out + (int64_t)(k0 + j) * pieces;
+    for (int c = lane; c < pieces; c += 32) dst[c] = src[c];
+}
+
+// The rotated part of every head's query, in place: a thread per pair.  layout 0: pairs (2i, 2i + 1), 1: (i, i + dims / 2).
+__global__ void __launch_bounds__(256) latent_rotate_kernel(__nv_bfloat16* q, int64_t tok_stride, int head_stride, const float* __restrict__ cos_sin, int dims,
+                                                            const int64_t* __restrict__ positions, int n, int heads, int layout) {
+    B200_PDL_SYNC();
+    const int half = dims / 2;
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= (int64_t)n * heads * half) return;
+    const int c = (int)(i % half), h = (int)(i / half % heads), t = (int)(i / half / heads);
+    __nv_bfloat16* x = q + t * tok_stride + (int64_t)h * head_stride;
+    const float* cs = cos_sin + positions[t] * dims;
+    const int e0 = layout ? c : 2 * c, e1 = layout ? c + half : 2 * c + 1;
+    const float u = __bfloat162float(x[e0]), v = __bfloat162float(x[e1]);
+    x[e0] = __float2bfloat16_rn(u * cs[c] - v * cs[half + c]);
+    x[e1] = __float2bfloat16_rn(v * cs[c] + u * cs[half + c]);
+}
+
+}  // namespace
+
+// Called from b200m_window_attention, which has validated the arguments.
+int b200m_window_prompt(const void* q, int64_t q_stride, const void* cache, int row_elems, int v_off, const int32_t* block_tables, int bt_stride, int block_size,
+                        const int32_t* cu_q, const int32_t* cu_k, const float* slopes, int window, int chunk, const float* sinks, const void* gate,
+                        int64_t gate_stride, int gate_elems, float out_scale, void* out, int64_t out_stride, bool out_f32, int total_q, int num_seqs, int max_q,
+                        int heads, int kv_heads, float scale, cudaStream_t stream) {
+    constexpr int D = 128;
+    const uintptr_t bases = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out) |
+                            (gate && gate_elems ? reinterpret_cast<uintptr_t>(gate) : 0);
+    if (bases % 16 || q_stride % 8 || row_elems % 8 || v_off % 8 || out_stride % (out_f32 ? 4 : 8) || (gate && gate_elems && gate_stride % 8) || !pages_ok(block_size))
+        return B200_EUNSUPPORTED;
+    const int box = block_size < BN ? block_size : BN;
+    CUtensorMap tq, tk;
+    if (!make_map(&tq, q, (uint64_t)heads * D, (uint64_t)total_q, (uint64_t)q_stride, BM) ||
+        !make_map(&tk, cache, (uint64_t)row_elems, ANY_ROWS, (uint64_t)row_elems, box))
+        return B200_EUNSUPPORTED;
+    FaParams p = {};
+    p.cu_q = cu_q;
+    p.cu_k = cu_k;
+    p.block_tables = block_tables;
+    p.bt_stride = bt_stride;
+    p.num_seqs = num_seqs;
+    p.hq = heads;
+    p.hkv = kv_heads;
+    p.q_col_step = p.k_col_step = p.v_col_step = D;
+    p.v_col0 = v_off;
+    p.block_size = block_size;
+    p.box_rows = box;
+    p.page_rows = block_size;
+    p.scale_log2 = scale * LOG2E;
+    p.slopes = slopes;
+    p.sinks = sinks;
+    p.window = window;
+    p.chunk = chunk;
+    p.out = out;
+    p.out_stride = out_stride;
+    p.out_f32 = out_f32;
+    p.out_scale = out_scale;
+    p.gate = static_cast<const __nv_bfloat16*>(gate);
+    p.gate_stride = gate_stride;
+    p.gate_elems = gate_elems;
+    const bool pair = heads / kv_heads % 2 == 0, plain = !slopes && scale > 0.f;
+    if (pair) return plain ? fa_launch<D, true, false>(p, tq, tk, tk, tk, total_q, max_q, stream) : fa_launch<D, true, true>(p, tq, tk, tk, tk, total_q, max_q, stream);
+    return plain ? fa_launch<D, false, false>(p, tq, tk, tk, tk, total_q, max_q, stream) : fa_launch<D, false, true>(p, tq, tk, tk, tk, total_q, max_q, stream);
+}
+
+extern "C" int b200m_latent_gather(const void* cache, int row_elems, const int32_t* block_tables, int bt_stride, int block_size, const int32_t* cu_k, int num_seqs,
+                                   int max_k, void* out, int out_rows, void* stream) {
+    if (!cache || !block_tables || !cu_k || !out || row_elems <= 0 || block_size <= 0 || num_seqs < 0 || out_rows < 0) return B200_EINVAL;
+    if (row_elems % 8 || (reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) % 16 || num_seqs > 65535) return B200_EUNSUPPORTED;
+    if (num_seqs == 0 || max_k <= 0 || out_rows == 0) return B200_OK;
+    B200_LAUNCH((latent_gather_kernel), dim3((max_k + 7) / 8, num_seqs), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(cache), row_elems / 8,
+                block_tables, bt_stride, block_size, cu_k, static_cast<uint4*>(out), out_rows);
+    return b200_launch_status(nullptr);
+}
+
+extern "C" int b200m_latent_rotate(void* q, int64_t tok_stride, int head_stride, const float* cos_sin, int rope_dims, const int64_t* positions, int n, int heads,
+                                   int layout, void* stream) {
+    if (!q || !cos_sin || !positions || n < 0 || heads <= 0 || rope_dims < 0 || rope_dims % 2) return B200_EINVAL;
+    const int64_t total = (int64_t)n * heads * (rope_dims / 2);
+    if (total == 0) return B200_OK;
+    B200_LAUNCH((latent_rotate_kernel), dim3((unsigned)((total + 255) / 256)), 256, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(q), tok_stride,
+                head_stride, cos_sin, rope_dims, positions, n, heads, layout);
+    return b200_launch_status(nullptr);
+}
+
+extern "C" int b200m_latent_prompt(const void* q, int64_t q_stride, const void* keys, const void* values, int64_t kv_stride, const void* rows, int row_elems, int rank,
+                                   int total_k, const int32_t* cu_q, const int32_t* cu_k, const float* sink, void* out, int total_q, int num_seqs, int max_q,
+                                   int heads, int dim, int rot_dim, int vdim, float scale, int window, void* stream) {
+    if (!q || !keys || !values || !rows || !cu_q || !cu_k || !out || total_q < 0 || num_seqs < 0 || heads <= 0 || rank <= 0 || total_k < 0) return B200_EINVAL;
+    const uintptr_t bases = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(values) |
+                            reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out);
+    if (dim != 128 || rot_dim != 64 || vdim != 128 || scale <= 0.f || bases % 16 || q_stride % 8 || kv_stride % 8 || row_elems % 8 || rank % 8) return B200_EUNSUPPORTED;
+    if (total_q == 0 || num_seqs == 0 || max_q <= 0) return B200_OK;
+    CUtensorMap tq, tk, tv, tr;
+    if (!make_map(&tq, q, (uint64_t)heads * 192, (uint64_t)total_q, (uint64_t)q_stride, BM) || !make_map(&tk, keys, (uint64_t)heads * 128, (uint64_t)total_k, (uint64_t)kv_stride, BN) ||
+        !make_map(&tv, values, (uint64_t)heads * 128, (uint64_t)total_k, (uint64_t)kv_stride, BN) || !make_map(&tr, rows, (uint64_t)row_elems, (uint64_t)total_k, (uint64_t)row_elems, BN))
+        return B200_EUNSUPPORTED;
+    FaParams p = {};
+    p.cu_q = cu_q;
+    p.cu_k = cu_k;
+    p.num_seqs = num_seqs;
+    p.hq = p.hkv = heads;
+    p.q_col_step = 192;
+    p.k_col_step = p.v_col_step = 128;
+    p.k2_col = rank;
+    p.block_size = p.box_rows = BN;
+    p.scale_log2 = scale * LOG2E;
+    p.sinks = sink;
+    p.window = window;
+    p.out = out;
+    p.out_stride = (int64_t)heads * vdim;
+    p.out_scale = 1.0f;
+    return fa_launch<192, false, false>(p, tq, tk, tv, tr, total_q, max_q, static_cast<cudaStream_t>(stream));
+}

@@ -20,6 +20,12 @@
 //                          than 32 / 64 / 128 (multiples of eight up to 128) run as 64, 96 or 128 with zero columns
 #include "mma_common.cuh"
 
+// prompt_attn.cu: prompt portions on the tcgen05 kernel; B200_EUNSUPPORTED for forms it does not take
+int b200m_window_prompt(const void* q, int64_t q_stride, const void* cache, int row_elems, int v_off, const int32_t* block_tables, int bt_stride, int block_size,
+                        const int32_t* cu_q, const int32_t* cu_k, const float* slopes, int window, int chunk, const float* sinks, const void* gate,
+                        int64_t gate_stride, int gate_elems, float out_scale, void* out, int64_t out_stride, bool out_f32, int total_q, int num_seqs, int max_q,
+                        int heads, int kv_heads, float scale, cudaStream_t stream);
+
 namespace {
 
 constexpr int WA_WARPS = 8;
@@ -765,6 +771,12 @@ extern "C" int b200m_window_attention(const void* q, int64_t q_stride, const voi
     if (total_q == 0 || num_seqs == 0 || max_q <= 0) return B200_OK;
     if (vdim > 512) return B200_EUNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (!is32 && !(flags & 1) && cu_q != nullptr && dim == 128 && vdim == 128 && vsets == 1 && rule.keep_first == 0 && softcap == 0.f) {
+        const int rc = b200m_window_prompt(q, q_stride, cache, row_elems, v_off, block_tables, bt_stride, block_size, cu_q, cu_k, slopes, window, chunk, sinks, gate,
+                                           gate_stride, gate_elems, out_scale, out, out_stride, out_f32, total_q, num_seqs, max_q, num_heads, num_kv_heads,
+                                           scale, st);
+        if (rc != B200_EUNSUPPORTED) return rc;                          // page sizes or alignments that kernel does not take: on to the next one
+    }
     const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(cache)) % 16 == 0) && q_stride % 8 == 0 &&
                          row_elems % 8 == 0 && v_off % 8 == 0 && out_stride % 2 == 0 && reinterpret_cast<uintptr_t>(out) % 8 == 0;
     if (!is32 && !(flags & 1) && aligned && dim % 8 == 0 && vdim % 8 == 0 && dim <= 128 && vdim <= 128) {
