@@ -7,9 +7,10 @@ key part shared by all heads are cached, and the softmax denominator carries a l
     p = exp(s) / (sum_j exp(s_j) + exp(sink[h]))
     out = W_o concat_h ( W_uv[h] sum_j p_j c_j )
 
-The product path never materialises per-head keys or values: ``q_nope . W_uk c = (W_uk^T q_nope) . c`` moves W_uk to the
+Single tokens never materialise per-head keys or values: ``q_nope . W_uk c = (W_uk^T q_nope) . c`` moves W_uk to the
 query side (one batched GEMM over the step's tokens) and W_uv is applied to the attention output, so the attention kernel
-runs multi-query over the cached rows.  A layer with ``kv_from`` reads another layer's cache (it has no W_dkv) with its own
+runs multi-query over the cached rows.  Prompt portions form keys and values first (``mixops.latent_prompt``): 192 + 128 columns per
+head, query and key instead of twice the latent's.  A layer with ``kv_from`` reads another layer's cache (it has no W_dkv) with its own
 W_uk / W_uv, queries and sink.
 """
 from __future__ import annotations
@@ -44,8 +45,9 @@ class LatentAttention:
         self.q_norm = e(self.q_rank)
         self.kv_norm = e(self.kv_rank) if self.kv_from is None else None
         self.w_uq = e(H * qd, self.q_rank)
-        self.w_uk = e(H, self.dim, self.kv_rank)          # q_lat[h] = q_nope[h] @ w_uk[h]
-        self.w_uv = e(H, self.vdim, self.kv_rank)
+        self.w_ukv = e(H * (self.dim + self.vdim), self.kv_rank)      # [W_uk ; W_uv]: one GEMM forms every head's keys and values
+        self.w_uk = self.w_ukv[:H * self.dim].view(H, self.dim, self.kv_rank)          # q_lat[h] = q_nope[h] @ w_uk[h]
+        self.w_uv = self.w_ukv[H * self.dim:].view(H, self.vdim, self.kv_rank)
         self.w_o = e(width, H * self.vdim)
         self.sink = torch.zeros(H, dtype=torch.float32, device=device)
         self.cache = None                                 # [num_blocks * block_size, kv_rank + rot_dim]; the source layer's when kv_from
@@ -86,6 +88,9 @@ class LatentAttention:
         if self.kv_from is None:
             mixops.latent_store(down[:, self.q_rank:], self.kv_norm, self.cos_sin, positions, ctx.slot_mapping, self.cache,
                                 R, rd, self.eps)
+        if mixops.latent_expands(q, d, rd, self.vdim, R, self.scale, self.cache, ctx.block_tables, self.block_size, spans):
+            return F.linear(mixops.latent_prompt(q, self.w_ukv, d, self.vdim, self.cache, ctx.block_tables, self.block_size, spans, self.sink, self.cos_sin,
+                                                 positions, self.scale), self.w_o)
         q_lat = torch.bmm(q[:, :, :d].transpose(0, 1), self.w_uk)                       # [H, n, R]
         o_lat = mixops.latent_attention(q_lat, q, d, self.cache, ctx.block_tables, self.block_size, spans, self.sink,
                                         self.cos_sin, self.scale)
@@ -102,7 +107,7 @@ class GatedWindowLatentAttention:
         out = W_o ( concat_h ( W_uv[h] sum_j softmax(s)_j c_j ) * sigmoid(W_g h) )
 
     The rotation pairs element i of the rotated part with element i + rot.dims / 2 (banded frequencies).  As in ``LatentAttention``
-    per-head keys and values are never formed: W_uk moves to the query side, W_uv to the output, and the attention kernel runs
+    single tokens never form per-head keys and values: W_uk moves to the query side, W_uv to the output, and the attention kernel runs
     multi-query over the cached rows ``[c | k_rot]``, one per token, layer instance and page slot.  ``[W_q ; W_dkv ; W_g]`` and
     ``extra_rows`` more rows (with a bias) that read the same input are one GEMM; ``forward`` returns the extra columns as a view.
     """
@@ -132,8 +137,9 @@ class GatedWindowLatentAttention:
         self.w_extra = self.w_in[self.in_cols:] if extra_rows else None
         self.b_extra = self.b_in[self.in_cols:] if extra_rows else None
         self.kv_norm = e(R)
-        self.w_uk = e(H, self.dim, R)                                      # q_lat[h] = q_nope[h] @ w_uk[h]
-        self.w_uv = e(H, self.vdim, R)
+        self.w_ukv = e(H * (self.dim + self.vdim), R)                      # [W_uk ; W_uv]
+        self.w_uk = self.w_ukv[:H * self.dim].view(H, self.dim, R)         # q_lat[h] = q_nope[h] @ w_uk[h]
+        self.w_uv = self.w_ukv[H * self.dim:].view(H, self.vdim, R)
         self.w_o = e(width, H * self.vdim)
         self.cache: list = []                                              # per instance [num_blocks * block_size, kv_rank + rot_dim]
         self.block_size = 0
@@ -184,9 +190,13 @@ class GatedWindowLatentAttention:
         cache = self.cache[inst]
         mixops.latent_store(proj[:, self.q_cols:], self.kv_norm, self.cos_sin, positions, ctx.slot_mapping, cache, R, rd, self.eps,
                             layout=mixops.ROT_HALVES)
-        q_lat = torch.bmm(q[:, :, :d].transpose(0, 1), self.w_uk)                       # [H, n, R]
-        o_lat = mixops.latent_attention(q_lat, q, d, cache, ctx.block_tables, self.block_size, spans, None, self.cos_sin, self.scale,
-                                        window=self.window, layout=mixops.ROT_HALVES)
-        o = torch.bmm(o_lat, self.w_uv.transpose(1, 2))                                 # [H, n, vdim]
-        gated = mixops.head_rotate_gate(o.permute(1, 0, 2), self.dtype, gate=proj[:, self.q_cols + self.kv_cols:self.in_cols])
+        if mixops.latent_expands(q, d, rd, self.vdim, R, self.scale, cache, ctx.block_tables, self.block_size, spans):
+            o = mixops.latent_prompt(q, self.w_ukv, d, self.vdim, cache, ctx.block_tables, self.block_size, spans, None, self.cos_sin, positions, self.scale,
+                                     window=self.window, layout=mixops.ROT_HALVES).view(n, H, self.vdim)
+        else:
+            q_lat = torch.bmm(q[:, :, :d].transpose(0, 1), self.w_uk)                   # [H, n, R]
+            o_lat = mixops.latent_attention(q_lat, q, d, cache, ctx.block_tables, self.block_size, spans, None, self.cos_sin, self.scale,
+                                            window=self.window, layout=mixops.ROT_HALVES)
+            o = torch.bmm(o_lat, self.w_uv.transpose(1, 2)).permute(1, 0, 2)            # [n, H, vdim]
+        gated = mixops.head_rotate_gate(o, self.dtype, gate=proj[:, self.q_cols + self.kv_cols:self.in_cols])
         return F.linear(gated, self.w_o), (proj[:, self.in_cols:] if self.extra else None)

@@ -317,6 +317,48 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, q_rot_off: int, c
     return out
 
 
+# Keys and values formed per head pay from a few queries per sequence on: forming them costs 2 * 2 * rank * 128 operations per head and cached row on the
+# library's GEMM, and saves attention over the latents at 87 TFLOP/s.  Measured (width 2048, 16 heads, layer, us, formed against latents): 1 x 4 queries over
+# 2048 rows 127 / 301, 8 x 4 over 2048 149 / 327, 16 x 4 over 4000 460 / 518, 8 x 64 over 2048 160 / 416, 4 x 2048 354 / 3627.
+LATENT_EXPAND_QUERIES = 4
+LATENT_EXPAND_ROWS = 1 << 17          # most rows whose keys and values are held at once (16 heads: 1 GiB)
+
+
+def latent_expands(q: torch.Tensor, dim: int, rot_dim: int, vdim: int, rank: int, scale: float, cache: torch.Tensor, block_tables: torch.Tensor,
+                   block_size: int, spans: StepSpans) -> bool:
+    """Whether a step's latent attention forms keys and values per head (``latent_prompt``): prompt portions of the sizes that kernel takes."""
+    n = q.shape[0]
+    return (spans.cu_q is not None and q.dtype == torch.bfloat16 and (dim, rot_dim, vdim) == (128, 64, 128) and scale > 0 and rank % 8 == 0
+            and n >= LATENT_EXPAND_QUERIES * spans.num_seqs and spans.num_seqs * block_tables.shape[1] * block_size <= LATENT_EXPAND_ROWS
+            and spans.num_seqs < 65536 and q.stride(0) % 8 == 0 and q.stride(2) == 1 and q.stride(1) == dim + rot_dim
+            and (q.data_ptr() | cache.data_ptr()) % 16 == 0)
+
+
+def latent_prompt(q: torch.Tensor, w_ukv: torch.Tensor, dim: int, vdim: int, cache: torch.Tensor, block_tables: torch.Tensor, block_size: int,
+                  spans: StepSpans, sink: torch.Tensor | None, cos_sin: torch.Tensor, positions: torch.Tensor, scale: float, window: int = 0,
+                  layout: int = ROT_PAIRS) -> torch.Tensor:
+    """q [n, H, dim + rot_dim] (its rotated part is turned in place), w_ukv [H * dim + H * vdim, rank] -> [n, H * vdim]: the cached rows of the step's
+    sequences are gathered, every head's keys and values formed from their latents by one GEMM, and attention runs over those."""
+    n, H, qd = q.shape
+    row = cache.shape[-1]
+    rank = row - (qd - dim)
+    assert cache.is_contiguous() and w_ukv.is_contiguous() and w_ukv.shape == (H * (dim + vdim), rank) and block_tables.stride(1) == 1
+    assert positions.dtype == torch.int64 and cos_sin.dtype == torch.float32 and block_tables.dtype == torch.int32
+    max_k = block_tables.shape[1] * block_size
+    total = spans.num_seqs * max_k                    # an upper bound known without asking the device
+    rows = torch.empty(total, row, dtype=cache.dtype, device=cache.device)
+    _call("b200m_latent_gather", cache.data_ptr(), row, block_tables.data_ptr(), block_tables.stride(0), block_size, spans.cu_k.data_ptr(), spans.num_seqs,
+          max_k, rows.data_ptr(), total, _stream())
+    _call("b200m_latent_rotate", q.data_ptr() + 2 * dim, q.stride(0), q.stride(1), cos_sin.data_ptr(), cos_sin.shape[1], positions.data_ptr(), n, H, int(layout),
+          _stream())
+    kv = torch.nn.functional.linear(rows[:, :rank], w_ukv)
+    out = torch.empty(n, H * vdim, dtype=q.dtype, device=q.device)
+    _call("b200m_latent_prompt", q.data_ptr(), q.stride(0), kv.data_ptr(), kv.data_ptr() + 2 * H * dim, kv.stride(0), rows.data_ptr(), row, rank, total,
+          spans.cu_q.data_ptr(), spans.cu_k.data_ptr(), _p(sink), out.data_ptr(), n, spans.num_seqs, spans.max_q, H, dim, qd - dim, vdim, scale, int(window),
+          _stream())
+    return out
+
+
 # ---- windowed grouped-query attention --------------------------------------------------------------------------------------
 def qk_norm_store(qkv: torch.Tensor, q_cols: int, k_cols: int, v_cols: int, q_norm: torch.Tensor | None, k_norm: torch.Tensor | None,
                   slots: torch.Tensor | None, cache: torch.Tensor | None, eps: float) -> None:

@@ -98,3 +98,76 @@ def test_pages_under_a_prefix(ops):
         got = ops.paged_prefill(0, q.cuda(), None, None, cu(len_q).cuda(), cu(len_k).cuda(), max(len_q), max(len_k), 128 ** -0.5,
                                 block_tables=tables.cuda(), num_kv_heads=1)
         assert_close_bf16(got, want, f"prefix, pages of {bs}")
+
+
+# ---- the same kernel over token-major cache rows (windowed attention) and over formed keys and values (latent attention) --------------------
+@pytest.fixture(scope="module")
+def mx():
+    from nanovllm import mixops as _mx
+    return _mx
+
+
+def paged_rows(len_k, bs, cols, seed):
+    nblk = sum(-(-c // bs) for c in len_k) + 1
+    tables = make_tables(len_k, bs, nblk, seed=seed)
+    return bf(nblk * bs, cols, seed=seed + 1).cuda(), tables.cuda()
+
+
+def spans_of(mx, len_q, len_k):
+    return mx.StepSpans(len(len_q), max(len_q), cu(len_q).cuda(), cu(len_k).cuda(), None)
+
+
+WINDOW_FORMS = {
+    "bias and window": dict(slopes=True, window=100),
+    "bias alone": dict(slopes=True),
+    "window below a block": dict(window=7),
+    "chunks and sinks": dict(chunk=96, sinks=True),
+    "head gate": dict(gate="heads", out_scale=0.5),
+    "element gate, fp32 result": dict(gate="elems", out_f32=True, window=64),
+    "negative scale": dict(scale=-0.06),
+}
+
+
+@pytest.mark.parametrize("form", WINDOW_FORMS)
+@pytest.mark.parametrize("heads,kv_heads,bs", [(4, 2, 256), (3, 1, 16), (2, 2, 64), (4, 1, 24)])        # pages of 24: the route falls through
+def test_windowed_prompts_against_the_fp32_pipe(mx, form, heads, kv_heads, bs):
+    """Against the general fp32 path of the same entry point on the same bf16 inputs (test_gpu_tipetar.py and others hold that one to float64): P and
+    the result are rounded to bf16, 2^-9 relative each."""
+    f = dict(WINDOW_FORMS[form])
+    len_q, len_k = [1, 130, 63, 200], [150, 130, 191, 329]
+    n, H = sum(len_q), heads
+    cache, tables = paged_rows(len_k, bs, kv_heads * 256, 30)
+    q = bf(n, H * 128 + 16, seed=31).cuda()
+    gate = None
+    if f.get("gate"):
+        gate = bf(n, (H if f["gate"] == "heads" else H * 128) + 8, seed=32).cuda()[:, :H if f["gate"] == "heads" else H * 128]
+    kw = dict(slopes=torch.exp2(-torch.arange(1, H + 1, dtype=torch.float32)).cuda() if f.get("slopes") else None, window=f.get("window", 0), chunk=f.get("chunk", 0),
+              sinks=torch.linspace(-1, 2, H).cuda() if f.get("sinks") else None, gate=gate, out_scale=f.get("out_scale", 1.0), out_f32=f.get("out_f32", False))
+    args = (q, cache, tables, bs, spans_of(mx, len_q, len_k), H, kv_heads, 128, 128, f.get("scale", 128 ** -0.5))
+    got, want = mx.window_attention(*args, **kw), mx.window_attention(*args, fma=True, **kw)
+    assert got.dtype == want.dtype
+    assert_close_bf16(got, want, form)
+
+
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("len_q,len_k,window,bs", [([64, 129, 1], [64, 129, 300], 0, 256), ([255, 257], [600, 257], 0, 16), ([40, 200], [333, 200], 50, 256)])
+def test_latent_prompts_against_attention_over_the_latents(mx, layout, len_q, len_k, window, bs):
+    """Keys and values formed per head against the products with the latents themselves, fp32 throughout (the general path on the same values): what
+    differs are the bf16 roundings of keys, values and P on one side, 2^-9 relative each, none on the other."""
+    from nanovllm.layers.rotary_embedding import build_banded_cos_sin
+    H, d, rd, R, n = 4, 128, 64, 64, sum(len_q)
+    cache, tables = paged_rows(len_k, bs, R + rd, 40)
+    q = bf(n, H, d + rd, seed=41).cuda()
+    w = bf(H * (d + 128), R, scale=R ** -0.5, seed=42).cuda()
+    sink = torch.linspace(-1, 1, H).cuda() if window == 0 else None
+    cs = build_banded_cos_sin(rd, 1024, 1e4, None, "cuda")
+    pos = torch.cat([torch.arange(b - a, b) for a, b in zip(len_q, len_k)]).cuda()
+    spans = spans_of(mx, len_q, len_k)
+    assert mx.latent_expands(q, d, rd, 128, R, 192 ** -0.5, cache, tables, bs, spans)
+    assert not mx.latent_expands(q, d, rd, 64, R, 192 ** -0.5, cache, tables, bs, spans)
+    uk, uv = w[:H * d].view(H, d, R).float(), w[H * d:].view(H, 128, R).float()
+    q_lat = torch.bmm(q[:, :, :d].transpose(0, 1).float(), uk)
+    o_lat = mx.latent_attention(q_lat, q.float(), d, cache.float(), tables, bs, spans, sink, cs, 192 ** -0.5, window=window, layout=layout)
+    want = torch.bmm(o_lat, uv.transpose(1, 2)).transpose(0, 1).reshape(n, H * 128)
+    got = mx.latent_prompt(q, w, d, 128, cache, tables, bs, spans, sink, cs, pos, 192 ** -0.5, window=window, layout=layout)
+    assert_close_bf16(got, want, "latent prompts", rel_l2=8e-3, ulps=3.0)
