@@ -312,9 +312,15 @@ int b200m_moe_route_grouped(const float* logits, int64_t ld, int n, int num_outp
 int b200m_moe_align(const int32_t* idx, int pairs, int num_experts, int32_t* sorted_rows, int cap, int32_t* pos_of,
                     int32_t* tile_expert, int32_t* num_tiles, int32_t* counts, void* stream);
 
+/* The experts' inputs in grouped order (bf16): out[i] = A[pair / top] (* wgt[pair], rounded) for every grouped row i that has a pair; out [max_tiles * tile, K]. */
+int b200m_moe_gather(const void* A, int64_t a_stride, const int32_t* sorted_rows, const float* wgt, int top, const int32_t* num_tiles, int max_tiles, int K,
+                     void* out, void* stream);
+
 /* C[i, :] = act(A_i . W[expert of i]^T) for every grouped row i.  gather: A_i = A[pair / top] * wgt[pair] (the expert's
  * weighted input; wgt NULL: unweighted); else A_i = A[i].  W [experts, N, K].  act 1 = relu^2; act 2 = gated: W holds N/2
- * gate rows, then N/2 up rows, and C[i, o] = silu(gate_o) * up_o has N/2 columns.  C is T, or fp32 when out_f32. */
+ * gate rows, then N/2 up rows, and C[i, o] = silu(gate_o) * up_o has N/2 columns.  C is T, or fp32 when out_f32.
+ * Bits 8 and up of act: about how many rows an expert has, which picks between a form that streams weights and one for many
+ * rows (bf16, not gathered; tcgen05); A and C then hold max_tiles * tile rows.  0: the general form. */
 int b200m_moe_gemm(const void* A, int64_t a_stride, const int32_t* sorted_rows, const float* wgt, int top, int gather,
                    const int32_t* tile_expert, const int32_t* num_tiles, int max_tiles, const void* W, int N, int K, void* C,
                    int out_f32, int act, int is32, void* stream);
@@ -324,6 +330,14 @@ int b200m_moe_gemm(const void* A, int64_t a_stride, const int32_t* sorted_rows, 
 int b200m_moe_combine(const float* rows, const int32_t* pos_of, int top, const void* shared, const float* gate_logit,
                       int64_t gate_ld, const float* wgt, const float* ident, float* out, int n, int width, int is32,
                       void* stream);
+
+/* Everything between the router's choice and the routed block's result (bf16), as one call: align, gather, the two grouped GEMMs (W_in [experts, N, K] with act,
+ * W_out [experts, width, N or N / 2]; fp32 results), combine.  wgt [n, top] weights the experts' inputs (weigh_inputs) or their results; the other
+ * arguments as for b200m_moe_combine.  workspace: b200m_moe_experts_workspace_bytes(n * top, ...) bytes, 256-byte aligned. */
+size_t b200m_moe_experts_workspace_bytes(int64_t pairs, int num_experts, int K, int inter, int width);
+int b200m_moe_experts(const void* A, int64_t a_stride, const int32_t* idx, const float* wgt, int weigh_inputs, int n, int top, int num_experts,
+                      const void* W_in, int N, int K, int act, const void* W_out, int width, const void* shared, const float* gate_logit, int64_t gate_ld,
+                      const float* ident, float* out, void* workspace, size_t workspace_bytes, void* stream);
 
 #ifdef __cplusplus
 }

@@ -100,27 +100,7 @@ static_assert(BAR_DEAD + 4 <= 320, "barrier area");
 
 __device__ __forceinline__ void fa_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
-__device__ __forceinline__ uint32_t fa_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok;
-}
-// Bounded wait; false: some wait of this CTA gave up and every role leaves.
-__device__ __forceinline__ bool fa_wait(uint32_t bar, uint32_t parity, uint32_t dead) {
-    if (fa_try(bar, parity)) return true;
-    uint64_t t0, t1;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-    do {
-        uint32_t d;
-        if (fa_try(bar, parity)) return true;
-        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(d) : "r"(dead) : "memory");
-        if (d) return false;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-    } while (t1 - t0 < 2000000000ull);                                   // two seconds: far beyond any wait of a healthy launch
-    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
-    atomicAdd(&fa_wait_timeouts, 1u);
-    return false;
-}
+__device__ __forceinline__ bool fa_wait(uint32_t bar, uint32_t parity, uint32_t dead) { return bounded_wait(bar, parity, dead, &fa_wait_timeouts); }
 
 __device__ __forceinline__ void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -129,27 +109,25 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint
         : "memory");
 }
 
-#define FA_R8(v, o) "=r"(v[o]), "=r"(v[o + 1]), "=r"(v[o + 2]), "=r"(v[o + 3]), "=r"(v[o + 4]), "=r"(v[o + 5]), "=r"(v[o + 6]), "=r"(v[o + 7])
-#define FA_I8(v, o) "r"(v[o]), "r"(v[o + 1]), "r"(v[o + 2]), "r"(v[o + 3]), "r"(v[o + 4]), "r"(v[o + 5]), "r"(v[o + 6]), "r"(v[o + 7])
 // 32 consecutive columns of this thread's lane, without the wait
 __device__ __forceinline__ void tmem_ld32n(uint32_t taddr, float* v) {
     uint32_t* r = reinterpret_cast<uint32_t*>(v);
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,"
         "%28,%29,%30,%31}, [%32];\n\t"
-        : FA_R8(r, 0), FA_R8(r, 8), FA_R8(r, 16), FA_R8(r, 24)
+        : TC_R8(r, 0), TC_R8(r, 8), TC_R8(r, 16), TC_R8(r, 24)
         : "r"(taddr));
 }
 // 16 columns times f, in place (without the wait for the store)
 __device__ __forceinline__ void tmem_scale16(uint32_t taddr, float f) {
     uint32_t r[16];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
-                 : FA_R8(r, 0), FA_R8(r, 8)
+                 : TC_R8(r, 0), TC_R8(r, 8)
                  : "r"(taddr)
                  : "memory");
 #pragma unroll
     for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * f);
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), FA_I8(r, 0), FA_I8(r, 8)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), TC_I8(r, 0), TC_I8(r, 8)
                  : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -158,7 +136,7 @@ __device__ __forceinline__ void tmem_st32u(uint32_t taddr, const uint32_t* v) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,"
         "%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
-        FA_I8(v, 0), FA_I8(v, 8), FA_I8(v, 16), FA_I8(v, 24)
+        TC_I8(v, 0), TC_I8(v, 8), TC_I8(v, 16), TC_I8(v, 24)
         : "memory");
 }
 
@@ -181,15 +159,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-__device__ __forceinline__ void st_256(void* p, const uint32_t* v) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), FA_I8(v, 0) : "memory");
-}
-__device__ __forceinline__ bool elect_one() {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok));
-    return ok != 0;
-}
-
 // One work item.  Its list entry: (sequence, row block | head item << 20, key blocks of tile 0 | of tile 1 << 16, first block | "the last
 // block reaches past the keys" << 31).
 struct FaItem {
@@ -504,6 +473,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 }
 #pragma unroll 1
                 for (int q4 = 0; q4 < DV / 32; ++q4) {
+                    __syncwarp();
                     float o[32];
                     tmem_ld32(tmem_o + t * 128 + lane_base + q4 * 32, o);
                     if (!valid) continue;

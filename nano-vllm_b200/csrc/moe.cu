@@ -11,6 +11,10 @@
 //   moe_combine_kernel: per token, the sum of its choices' rows (fixed order) plus the gated shared expert
 #include "mix_common.cuh"
 
+// moe_tc.cu: the grouped GEMM on tcgen05; B200_EUNSUPPORTED for shapes it does not take
+int b200m_moe_gemm_tc(const void* A, int64_t a_stride, const int32_t* sorted_rows, const int32_t* tile_expert, const int32_t* num_tiles, int max_tiles, const void* W, int N, int K,
+                      void* C, int out_f32, int act, int rows_per_expert, cudaStream_t stream);
+
 namespace {
 
 // One warp per token: lane l looks at experts l, l + 32, ...; the chosen ones are struck from a per-lane bit mask (so the kernel
@@ -69,14 +73,14 @@ __global__ void __launch_bounds__(RG_WARPS * 32) moe_route_grouped_kernel(const 
                                                                           int num_real, int score_kind, int renorm, float scale,
                                                                           int32_t* __restrict__ idx, float* __restrict__ wgt) {
     B200_PDL_SYNC();
-    __shared__ float sh_s[RG_WARPS][RG_MAX];          // plain scores
-    __shared__ float sh_g[RG_WARPS][RG_MAX];          // group scores; after the group choice: 1 = open, 0 = closed
+    extern __shared__ float sh_route[];               // per warp: E plain scores, then E (at least as many as groups) group scores; after the group
+                                                      // choice 1 = open, 0 = closed.  Sized to E: 32 KB for the most experts left 28 warps on an SM
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * RG_WARPS + warp;
     if (t >= n) return;
     const float* z = logits + (int64_t)t * ld;
-    float* sc = sh_s[warp];
-    float* gs = sh_g[warp];
+    float* sc = sh_route + warp * 2 * E;
+    float* gs = sc + E;
     constexpr int NONE = 0x7fffffff;
     if (score_kind == 0) {
         float mx = -INFINITY;
@@ -174,22 +178,99 @@ __global__ void __launch_bounds__(RG_WARPS * 32) moe_route_grouped_kernel(const 
     for (int k = lane; k < top; k += 32) wgt[(int64_t)t * top + k] *= f;
 }
 
-// One CTA.  pairs = n * top entries of idx.  Outputs: sorted_rows[cap] (pair index, or -1 for padding), pos_of[pairs]
-// (where each pair went), tile_expert[max_tiles], num_tiles[0].  counts: scratch of 2 * E ints.
-__global__ void __launch_bounds__(1024) moe_align_kernel(const int32_t* __restrict__ idx, int pairs, int E, int bm,
-                                                         int32_t* __restrict__ sorted_rows, int cap, int32_t* __restrict__ pos_of,
-                                                         int32_t* __restrict__ tile_expert, int32_t* __restrict__ num_tiles,
-                                                         int32_t* __restrict__ counts) {
+// One cluster.  pairs = n * top entries of idx.  Outputs: sorted_rows[cap] (pair index, or -1 for padding), pos_of[pairs] (where each pair
+// went), tile_expert[max_tiles], num_tiles[0].  Each CTA counts its share of the pairs per expert, reads the others' counts from their shared
+// memory, and so knows where its pairs of every expert go; only padding is filled with -1.  Latency-bound: 32 k pairs of 32 experts took 41 us in one
+// CTA that also walked the experts serially.  The order inside an expert changes nothing in the results (rows are independent), so
+// an atomic cursor is enough.
+constexpr int AL_E = 1024;         // experts whose counters fit
+__global__ void __launch_bounds__(1024) moe_align_kernel(const int32_t* __restrict__ idx, int pairs, int E, int bm, int32_t* __restrict__ sorted_rows, int cap,
+                                                         int32_t* __restrict__ pos_of, int32_t* __restrict__ tile_expert, int32_t* __restrict__ num_tiles) {
     B200_PDL_SYNC();
-    __shared__ int32_t sh_counts[2048];
-    const bool in_shared = E <= 1024;                            // the usual case: counters in shared memory, `counts` unused
-    int32_t* cnt = in_shared ? sh_counts : counts;               // [E] pairs per expert
-    int32_t* start = in_shared ? sh_counts + 1024 : counts + E;  // [E] first sorted row of the expert
+    __shared__ int32_t mine[AL_E], start[AL_E], total[AL_E], warp_sum_[33];
+    uint32_t rank, ctas;
+    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %cluster_nctarank;" : "=r"(ctas));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int share = (pairs + (int)ctas - 1) / (int)ctas, p0 = min(pairs, (int)rank * share), p1 = min(pairs, p0 + share);
+    for (int e = tid; e < E; e += 1024) mine[e] = 0;
+    __syncthreads();
+    for (int i = p0 + tid; i < p1; i += 1024) {
+        const int e = idx[i];
+        if (e >= 0) atomicAdd(&mine[min(e, E - 1)], 1);                  // a negative index is a pair without an expert GEMM; one too large is counted at the edge, never written through
+    }
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    int before = 0, all = 0;                                             // expert tid: pairs of the CTAs before this one, of all
+    if (tid < E) {
+        const uint32_t at = smem_u32(&mine[tid]);
+        for (uint32_t c = 0; c < ctas; ++c) {
+            uint32_t remote;
+            int v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(c));
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+            if (c < rank) before += v;
+            all += v;
+        }
+    }
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");      // nobody reads `mine` of another CTA any more
+    // exclusive prefix of the experts' tiles
+    const int tiles = (all + bm - 1) / bm;
+    int inc = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    if (lane == 31) warp_sum_[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        int v = warp_sum_[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        warp_sum_[lane] = v;
+    }
+    __syncthreads();
+    const int t0 = inc - tiles + (warp ? warp_sum_[warp - 1] : 0), used = warp_sum_[31];
+    if (tid < E) {
+        start[tid] = t0 * bm;
+        total[tid] = all;
+        mine[tid] = t0 * bm + before;                                    // now this CTA's cursor
+        for (int k = rank; k < tiles; k += ctas) tile_expert[t0 + k] = tid;
+    }
+    if (rank == 0 && tid == 0) num_tiles[0] = used;
+    __syncthreads();
+    for (int i = p0 + tid; i < p1; i += 1024) {
+        int e = idx[i], p = -1;
+        if (e >= 0) {
+            e = min(e, E - 1);
+            p = atomicAdd(&mine[e], 1);
+            sorted_rows[p] = i;
+        }
+        pos_of[i] = p;
+    }
+    for (int e = (int)rank * 32 + warp; e < E; e += (int)ctas * 32) {    // a warp per expert: the padding behind its run
+        const int end = (total[e] + bm - 1) / bm * bm;
+        for (int k = total[e] + lane; k < end; k += 32) sorted_rows[start[e] + k] = -1;
+    }
+    for (int i = used * bm + (int)rank * 1024 + tid; i < cap; i += (int)ctas * 1024) sorted_rows[i] = -1;
+}
+
+// More experts than AL_E: one CTA, counters in global memory (counts: scratch of 2 * E ints).
+__global__ void __launch_bounds__(1024) moe_align_wide_kernel(const int32_t* __restrict__ idx, int pairs, int E, int bm,
+                                                              int32_t* __restrict__ sorted_rows, int cap, int32_t* __restrict__ pos_of,
+                                                              int32_t* __restrict__ tile_expert, int32_t* __restrict__ num_tiles,
+                                                              int32_t* __restrict__ counts) {
+    B200_PDL_SYNC();
+    int32_t* cnt = counts;                                       // [E] pairs per expert
+    int32_t* start = counts + E;                                 // [E] first sorted row of the expert
     for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
     for (int i = threadIdx.x; i < cap; i += blockDim.x) sorted_rows[i] = -1;
     __syncthreads();
     for (int i = threadIdx.x; i < pairs; i += blockDim.x)
-        if (idx[i] >= 0) atomicAdd(&cnt[min(idx[i], E - 1)], 1);      // a negative index is a pair without an expert GEMM; one too large is counted at the edge, never written through
+        if (idx[i] >= 0) atomicAdd(&cnt[min(idx[i], E - 1)], 1);
     __syncthreads();
     if (threadIdx.x == 0) {
         int at = 0;
@@ -203,8 +284,6 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int32_t* __restri
         num_tiles[0] = at / bm;
     }
     __syncthreads();
-    // rows of one expert in ascending pair order would need a stable sort; the order inside an expert changes nothing in
-    // the results (rows are independent), so an atomic cursor is enough
     for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
         if (idx[i] < 0) {
             pos_of[i] = -1;
@@ -482,6 +561,50 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const int32_t
     }
 }
 
+// The same with four columns per thread and the rows of up to eight choices in flight at once (width a multiple of four, 16-byte aligned rows).
+// HBM-bound: 8192 tokens x 4 choices x 2048 columns read 215 MB of rows; one column per thread with its choices in turn took 114 us.
+template <typename T>
+__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const float* __restrict__ rows, const int32_t* __restrict__ pos_of, int top,
+                                                              const T* __restrict__ shared, const float* __restrict__ gate_logit, int64_t gate_ld,
+                                                              const float* __restrict__ wgt, const float* __restrict__ ident, float* __restrict__ out, int width) {
+    B200_PDL_SYNC();
+    const int64_t t = blockIdx.x;
+    const int c = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (c >= width) return;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = 0; k0 < top; k0 += 8) {
+        float4 v[8];
+        float w[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            w[k] = 0.f;
+            v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k0 + k >= top) continue;
+            const int p = pos_of[t * top + k0 + k];
+            const float* src = p >= 0 ? rows + (int64_t)p * width : ident ? ident + t * width : nullptr;
+            if (!src) continue;
+            w[k] = wgt ? wgt[t * top + k0 + k] : 1.0f;
+            v[k] = *reinterpret_cast<const float4*>(src + c);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            a.x = fmaf(w[k], v[k].x, a.x);
+            a.y = fmaf(w[k], v[k].y, a.y);
+            a.z = fmaf(w[k], v[k].z, a.z);
+            a.w = fmaf(w[k], v[k].w, a.w);
+        }
+    }
+    if (shared) {
+        const float g = gate_logit ? sigmoidf_(gate_logit[t * gate_ld]) : 1.0f;
+        const T* s = shared + t * width + c;
+        a.x = fmaf(g, ldf(s), a.x);
+        a.y = fmaf(g, ldf(s + 1), a.y);
+        a.z = fmaf(g, ldf(s + 2), a.z);
+        a.w = fmaf(g, ldf(s + 3), a.w);
+    }
+    *reinterpret_cast<float4*>(out + t * width + c) = a;
+}
+
 }  // namespace
 
 extern "C" int b200m_moe_tile_rows(void) { return MG_BM; }
@@ -504,7 +627,7 @@ extern "C" int b200m_moe_route_grouped(const float* logits, int64_t ld, int n, i
     if (score_kind < 0 || score_kind > 1) return B200_EINVAL;
     if (num_outputs > RG_MAX) return B200_EUNSUPPORTED;
     if (n == 0) return B200_OK;
-    B200_LAUNCH((moe_route_grouped_kernel), (n + RG_WARPS - 1) / RG_WARPS, RG_WARPS * 32, 0, static_cast<cudaStream_t>(stream), logits, ld,
+    B200_LAUNCH((moe_route_grouped_kernel), (n + RG_WARPS - 1) / RG_WARPS, RG_WARPS * 32, (size_t)RG_WARPS * 2 * num_outputs * sizeof(float), static_cast<cudaStream_t>(stream), logits, ld,
                 n, num_outputs, top, correction, n_groups, keep, num_real, score_kind, renorm, scale, idx, wgt);
     return b200_launch_status(nullptr);
 }
@@ -513,8 +636,29 @@ extern "C" int b200m_moe_align(const int32_t* idx, int pairs, int num_experts, i
                                int32_t* tile_expert, int32_t* num_tiles, int32_t* counts, void* stream) {
     if (!idx || !sorted_rows || !pos_of || !tile_expert || !num_tiles || !counts || pairs < 0 || num_experts <= 0) return B200_EINVAL;
     if (cap % MG_BM || cap < ((pairs + num_experts * (MG_BM - 1)) / MG_BM) * MG_BM) return B200_EWORKSPACE;
-    B200_LAUNCH((moe_align_kernel), 1, 1024, 0, static_cast<cudaStream_t>(stream), idx, pairs, num_experts, (int)MG_BM, sorted_rows, cap,
-                pos_of, tile_expert, num_tiles, counts);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (num_experts > AL_E) {
+        B200_LAUNCH((moe_align_wide_kernel), 1, 1024, 0, st, idx, pairs, num_experts, (int)MG_BM, sorted_rows, cap, pos_of, tile_expert, num_tiles, counts);
+        return b200_launch_status(nullptr);
+    }
+    // a CTA per 2048 pairs up to a portable cluster: two passes of a CTA's threads
+    int ctas = 1;
+    while (ctas < 8 && ctas * 2048 < pairs) ctas *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {(unsigned)ctas, 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+#ifdef B200_PDL
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = b200_tls_pdl_off() ? 1 : 2;
+#endif
+    cudaLaunchKernelEx(&cfg, moe_align_kernel, idx, pairs, num_experts, (int)MG_BM, sorted_rows, cap, pos_of, tile_expert, num_tiles);
     return b200_launch_status(nullptr);
 }
 
@@ -523,12 +667,17 @@ extern "C" int b200m_moe_gemm(const void* A, int64_t a_stride, const int32_t* so
                               void* C, int out_f32, int act, int is32, void* stream) {
     if (!A || !sorted_rows || !tile_expert || !num_tiles || !W || !C || N <= 0 || K <= 0 || max_tiles < 0) return B200_EINVAL;
     if (gather && top <= 0) return B200_EINVAL;
+    const int rows_per_expert = act > 0 ? act >> 8 : 0;
+    if (act > 0) act &= 255;
     if (act < 0 || act > 2 || (act == 2 && (N & 1))) return B200_EINVAL;
     if (max_tiles == 0) return B200_OK;
     const int n_out = act == 2 ? N / 2 : N;                // output columns
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool tc = !is32 && (K % 8 == 0) && (a_stride % 8 == 0) && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) % 16 == 0);
     if (tc) {
+        const int rc = gather ? B200_EUNSUPPORTED
+                              : b200m_moe_gemm_tc(A, a_stride, sorted_rows, tile_expert, num_tiles, max_tiles, W, N, K, C, out_f32, act, rows_per_expert, st);
+        if (rc != B200_EUNSUPPORTED) return rc;
         dim3 g2(act == 2 ? (n_out + MM_BN / 2 - 1) / (MM_BN / 2) : (N + MM_BN - 1) / MM_BN, max_tiles);
         using bf = __nv_bfloat16;
         const size_t smem = 2 * (size_t)(MG_BM + MM_BN) * MM_LD * sizeof(bf);
@@ -564,6 +713,12 @@ extern "C" int b200m_moe_combine(const float* rows, const int32_t* pos_of, int t
                                  void* stream) {
     if (!rows || !pos_of || !out || n < 0 || width <= 0 || top <= 0) return B200_EINVAL;
     if (n == 0) return B200_OK;
+    const uintptr_t bases = reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ident);
+    if (width % 4 == 0 && bases % 16 == 0 && width <= 65535 * 1024) {
+        B200M_DISPATCH(is32, B200_LAUNCH((moe_combine_vec_kernel<T>), dim3(n, (width + 1023) / 1024), 256, 0, static_cast<cudaStream_t>(stream), rows, pos_of, top,
+                                         static_cast<const T*>(shared), gate_logit, gate_ld, wgt, ident, out, width));
+        return b200_launch_status(nullptr);
+    }
     B200M_DISPATCH(is32, B200_LAUNCH((moe_combine_kernel<T>), n, 256, 0, static_cast<cudaStream_t>(stream), rows, pos_of, top,
                                      static_cast<const T*>(shared), gate_logit, gate_ld, wgt, ident, out, n, width));
     return b200_launch_status(nullptr);

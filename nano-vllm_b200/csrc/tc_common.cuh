@@ -57,6 +57,40 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) 
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+#define TC_R8(v, o) "=r"(v[o]), "=r"(v[o + 1]), "=r"(v[o + 2]), "=r"(v[o + 3]), "=r"(v[o + 4]), "=r"(v[o + 5]), "=r"(v[o + 6]), "=r"(v[o + 7])
+#define TC_I8(v, o) "r"(v[o]), "r"(v[o + 1]), "r"(v[o + 2]), "r"(v[o + 3]), "r"(v[o + 4]), "r"(v[o + 5]), "r"(v[o + 6]), "r"(v[o + 7])
+// 32 bytes: a whole sector (32-byte aligned)
+__device__ __forceinline__ void st_256(void* p, const uint32_t* v) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), TC_I8(v, 0) : "memory");
+}
+// The same lane of a converged warp every time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
+__device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok;
+}
+// Bounded wait; false: some wait of this CTA gave up (`dead`, a shared word) and every role leaves.
+__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, uint32_t dead, uint32_t* timeouts) {
+    if (mbar_try(bar, parity)) return true;
+    uint64_t t0, t1;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    do {
+        uint32_t d;
+        if (mbar_try(bar, parity)) return true;
+        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(d) : "r"(dead) : "memory");
+        if (d) return false;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+    } while (t1 - t0 < 2000000000ull);                                   // two seconds: far beyond any wait of a healthy launch
+    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
+    atomicAdd(timeouts, 1u);
+    return false;
+}
+
 // Shared-memory matrix descriptor (cute::UMMA::SmemDescriptor): 128-byte swizzle, version 1.
 //   K-major operand  : rows of 128 B, 8-row groups 1024 B apart (SBO); LBO unused.
 //   MN-major operand : 64-element (128 B) runs along MN, 8 k-rows per 1024 B group (SBO), next 64-element

@@ -131,13 +131,15 @@ class RoutedExpertsFF:
         n = h.shape[0]
         logits = F.linear(h.float(), self.w_router)
         idx, wgt = mixops.moe_route(logits, self.experts, self.top)
-        sorted_rows, pos_of, tile_expert, num_tiles = mixops.moe_align(idx, self.experts)
-        inter = mixops.moe_gemm(h, sorted_rows, tile_expert, num_tiles, self.w_up, wgt=wgt, top=self.top, act=1)
-        rows = mixops.moe_gemm(inter, sorted_rows, tile_expert, num_tiles, self.w_down, out_f32=True)
         shared = gate = None
         if self.shared_ff:
             shared = F.linear(mixops.ff_act(F.linear(h, self.sh_up), mixops.FF_RELU2), self.sh_down)
             gate = logits[:, self.experts]
+        if h.dtype == torch.bfloat16:
+            return None, mixops.moe_experts(h, idx, wgt, self.w_up, self.w_down, 1, True, shared, gate)
+        sorted_rows, pos_of, tile_expert, num_tiles = mixops.moe_align(idx, self.experts)
+        inter = mixops.moe_gemm(h, sorted_rows, tile_expert, num_tiles, self.w_up, wgt=wgt, top=self.top, act=1)
+        rows = mixops.moe_gemm(inter, sorted_rows, tile_expert, num_tiles, self.w_down, out_f32=True)
         return None, mixops.moe_combine(rows, pos_of, self.top, n, shared, gate)
 
 
@@ -204,12 +206,14 @@ class GroupRoutedExpertsFF:
         logits = F.linear(x32, self.w_router, self.router_bias)
         idx, wgt = mixops.moe_route_grouped(logits, self.outputs, self.top, self.correction, self.groups, self.keep, self.experts,
                                             scale=self.route_scale)
-        sorted_rows, pos_of, tile_expert, num_tiles = mixops.moe_align(idx, max(self.experts, 1))
-        inter = mixops.moe_gemm(h, sorted_rows, tile_expert, num_tiles, self.w_gate_up, top=self.top, act=2, gather=True)
-        rows = mixops.moe_gemm(inter, sorted_rows, tile_expert, num_tiles, self.w_down, out_f32=True)
         shared = None
         if self.shared_ff:
             shared = F.linear(mixops.ff_act(F.linear(h, self.sh_gate_up), mixops.FF_SILU_MUL), self.sh_down)
+        if h.dtype == torch.bfloat16:
+            return mixops.moe_experts(h, idx, wgt, self.w_gate_up, self.w_down, 2, False, shared, ident=x32 if self.identity else None)
+        sorted_rows, pos_of, tile_expert, num_tiles = mixops.moe_align(idx, max(self.experts, 1))
+        inter = mixops.moe_gemm(h, sorted_rows, tile_expert, num_tiles, self.w_gate_up, top=self.top, act=2, gather=True)
+        rows = mixops.moe_gemm(inter, sorted_rows, tile_expert, num_tiles, self.w_down, out_f32=True)
         return mixops.moe_combine(rows, pos_of, self.top, n, shared, None, wgt=wgt, ident=x32 if self.identity else None)
 
 

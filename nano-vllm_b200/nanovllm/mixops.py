@@ -731,9 +731,17 @@ def moe_gemm(A: torch.Tensor, sorted_rows, tile_expert, num_tiles, W: torch.Tens
     _same(is32, W)
     cap = sorted_rows.numel()
     out = torch.empty(cap, W.shape[1] // 2 if act == 2 else W.shape[1], dtype=torch.float32 if out_f32 else A.dtype, device=A.device)
+    N, K = W.shape[1], W.shape[2]
+    if (wgt is not None or gather) and not is32 and K % 8 == 0 and N % 256 == 0 and A.stride(0) % 8 == 0 and (A.data_ptr() | W.data_ptr()) % 16 == 0:
+        grouped = torch.empty(cap, K, dtype=A.dtype, device=A.device)              # the tcgen05 forms read grouped rows
+        _call("b200m_moe_gather", A.data_ptr(), A.stride(0), sorted_rows.data_ptr(), _p(wgt), top, num_tiles.data_ptr(), tile_expert.numel(), K,
+              grouped.data_ptr(), _stream())
+        A, wgt, gather = grouped, None, False
+    # about how many rows an expert has: the grouped buffer's rows less its padding (0, the general form, when A is shorter than the buffer)
+    per_expert = max(1, (cap - W.shape[0] * (moe_tile_rows() - 1)) // W.shape[0]) if A.shape[0] >= cap else 0
     _call("b200m_moe_gemm", A.data_ptr(), A.stride(0), sorted_rows.data_ptr(), _p(wgt), top, int(wgt is not None or gather),
           tile_expert.data_ptr(), num_tiles.data_ptr(), tile_expert.numel(), W.data_ptr(), W.shape[1], W.shape[2], out.data_ptr(),
-          int(out_f32), act, is32, _stream())
+          int(out_f32), act | min(per_expert, 1 << 22) << 8, is32, _stream())
     return out
 
 
@@ -751,4 +759,27 @@ def moe_combine(rows: torch.Tensor, pos_of: torch.Tensor, top: int, n: int, shar
     assert ident is None or (ident.dtype == torch.float32 and ident.is_contiguous() and ident.shape == out.shape)
     _call("b200m_moe_combine", rows.data_ptr(), pos_of.data_ptr(), top, _p(shared), _p(gate_logit), gld, _p(wgt), _p(ident),
           out.data_ptr(), n, width, is32, _stream())
+    return out
+
+
+def moe_experts(A: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor, act: int, weigh_inputs: bool,
+                shared: torch.Tensor | None = None, gate_logit: torch.Tensor | None = None, ident: torch.Tensor | None = None) -> torch.Tensor:
+    """The routed block after the router's choice (idx, wgt [n, top]), bf16, as one call of six launches: grouping, gathered inputs (weighted with
+    ``weigh_inputs``), act(x W_in^T), (.) W_out^T, and each token's sum -> fp32 [n, width].  The other arguments as for ``moe_combine``."""
+    n, top = idx.shape
+    E, N, K = w_in.shape
+    width = w_out.shape[1]
+    assert A.dim() == 2 and A.stride(1) == 1 and A.shape == (n, K) and w_in.is_contiguous() and w_out.is_contiguous() and w_out.shape[0] == E
+    assert w_out.shape[2] == (N // 2 if act == 2 else N) and A.dtype == w_in.dtype == w_out.dtype == torch.bfloat16
+    assert idx.dtype == torch.int32 and idx.is_contiguous() and wgt.dtype == torch.float32 and wgt.is_contiguous() and wgt.shape == idx.shape
+    assert shared is None or (shared.dtype == A.dtype and shared.is_contiguous() and shared.shape == (n, width))
+    assert gate_logit is None or gate_logit.dtype == torch.float32
+    assert ident is None or (ident.dtype == torch.float32 and ident.is_contiguous() and ident.shape == (n, width))
+    out = torch.empty(n, width, dtype=torch.float32, device=A.device)
+    size = nat.load_mix().b200m_moe_experts_workspace_bytes(n * top, E, K, w_out.shape[2], width)
+    space = torch.empty(size, dtype=torch.uint8, device=A.device)
+    _call("b200m_moe_experts", A.data_ptr(), A.stride(0), idx.data_ptr(), wgt.data_ptr(), int(weigh_inputs), n, top, E, w_in.data_ptr(), N, K, act,
+          w_out.data_ptr(), width, _p(shared), _p(gate_logit), gate_logit.stride(0) if gate_logit is not None else 0, _p(ident), out.data_ptr(),
+          space.data_ptr(), size, _stream())
+    ops.LAUNCHES[0] += 4 + int(N % 256 == 0)
     return out

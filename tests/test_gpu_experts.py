@@ -1,0 +1,115 @@
+"""The grouped expert GEMMs on tcgen05 (csrc/moe_tc.cu) at the sizes where their tiling can go wrong: experts with no rows, one, a tile less
+one, a tile, a tile and one, odd numbers of tiles; K that is no multiple of a stage; one and several blocks of weight rows; both forms, every
+activation and result type, gathered rows with and without weights.
+
+Reference: the same bf16 operands multiplied in fp32 by torch.  Both sides accumulate in fp32 in another order (1e-5 relative); bf16 results
+carry one more rounding (2^-9)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def mx():
+    from nanovllm import mixops as _mx
+    return _mx
+
+
+def routing(counts, top, seed):
+    """idx [n, top] in which expert e is chosen counts[e] times, in a shuffled order (-1 fills up)."""
+    g = torch.Generator().manual_seed(seed)
+    flat = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)])
+    flat = torch.cat([flat, torch.full((-flat.numel() % top,), -1)])
+    return flat[torch.randperm(flat.numel(), generator=g)].view(-1, top).to(torch.int32).cuda()
+
+
+COUNTS = {"few": [0, 1, 5, 63, 64, 0, 2], "edges": [65, 128, 0, 129, 127, 1, 192], "many": [700, 64, 257], "one expert": [0, 0, 333]}
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("act,gather,weighted,out_f32", [(0, False, False, True), (1, True, True, False), (2, True, False, False), (2, True, True, True)])
+@pytest.mark.parametrize("N,K", [(256, 64), (512, 200), (768, 1024)])
+@pytest.mark.parametrize("form", ["stream", "rows"])
+def test_grouped_gemm(mx, counts, act, gather, weighted, out_f32, N, K, form, monkeypatch):
+    counts, top = COUNTS[counts], 3
+    E = len(counts)
+    idx = routing(counts, top, 1)
+    n = idx.shape[0]
+    g = torch.Generator(device="cuda").manual_seed(2)
+    rows, pos_of, tile_expert, num_tiles = mx.moe_align(idx, E)
+    cap = rows.numel()
+    A = torch.randn(n if gather else cap, K + 8, generator=g, device="cuda").to(torch.bfloat16)[:, :K]
+    W = (torch.randn(E, N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    wgt = torch.rand(n, top, generator=g, device="cuda") if weighted else None
+    if not gather:
+        A = A.clone()
+        A[rows < 0] = float("nan")                   # padding rows of the grouped buffer hold anything: nothing may come of them
+    lib = mx.nat.load_mix()
+    real = lib.b200m_moe_gemm
+    hint = 1 if form == "stream" else 1 << 20
+
+    class Lib:
+        def __getattr__(self, name):
+            if name != "b200m_moe_gemm":
+                return getattr(lib, name)
+            return lambda *a: real(*a[:-3], (a[-3] & 255) | hint << 8, *a[-2:])
+
+    monkeypatch.setattr(mx.nat, "load_mix", lambda: Lib())
+    got = mx.moe_gemm(A, rows, tile_expert, num_tiles, W, wgt=wgt, top=top, act=act, out_f32=out_f32, gather=gather)
+    live = (rows >= 0).nonzero().view(-1)
+    pair = rows[live].long()
+    e = idx.view(-1)[pair].long()
+    x = A[pair // top].float() if gather else A[live].float()
+    if weighted:
+        x = (x * wgt.view(-1)[pair, None]).to(torch.bfloat16).float()       # the expert's input is a bf16 tensor
+    y = torch.empty(live.numel(), N, device="cuda")
+    for k in range(E):
+        y[e == k] = x[e == k] @ W[k].float().T
+    if act == 1:
+        y = torch.relu(y).square()
+    elif act == 2:
+        y = torch.nn.functional.silu(y[:, :N // 2]) * y[:, N // 2:]
+    have = got[live].float()
+    assert torch.isfinite(have).all()
+    err = ((have - y).norm() / y.norm()).item()
+    assert err < (2e-5 if out_f32 else 4e-3), err
+    assert (have - y).abs().max().item() <= (1e-4 if out_f32 else 2 ** -7) * max(1.0, y.abs().max().item())
+
+
+@pytest.mark.parametrize("n,E,top", [(1, 5, 2), (300, 40, 3), (3000, 7, 4), (700, 1500, 2)])
+def test_grouping(mx, n, E, top):
+    """Every pair lands in its expert's run once, runs start on tiles, the rest is padding; one CTA, clusters, and more experts than counters."""
+    g = torch.Generator().manual_seed(3)
+    idx = torch.randint(-1, E, (n, top), generator=g).to(torch.int32)
+    if E == 7:
+        idx[idx == 2] = 5                            # an expert without rows, one with most
+    rows, pos_of, tile_expert, num_tiles = (t.cpu() for t in mx.moe_align(idx.cuda(), E))
+    flat, used = idx.view(-1), int(num_tiles)
+    assert torch.equal(pos_of < 0, flat < 0)
+    live = (flat >= 0).nonzero().view(-1)
+    assert torch.equal(rows[pos_of[live].long()], live.to(torch.int32))
+    assert int((rows >= 0).sum()) == live.numel() and bool((rows[used * 64:] < 0).all())
+    assert torch.equal(tile_expert[pos_of[live].long() // 64], flat[live])
+    counts = torch.bincount(flat[live].long(), minlength=E)
+    assert used == int(((counts + 63) // 64).sum()) and torch.equal(torch.bincount(tile_expert[:used].long(), minlength=E), (counts + 63) // 64)
+
+
+@pytest.mark.parametrize("n", [1, 200, 2600])
+@pytest.mark.parametrize("act,N,weigh_inputs,shared,ident", [(1, 256, True, True, False), (2, 512, False, True, True), (2, 192, False, False, True)])
+def test_one_call_against_its_parts(mx, n, act, N, weigh_inputs, shared, ident):
+    """The one-call form against the single entry points on the same inputs: the same operations, so only the order of fp32 sums may differ."""
+    E, top, K, width = 9, 3, 136, 260 if N == 192 else 512
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    idx = torch.randint(-1 if ident else 0, E, (n, top), generator=g, device="cuda").to(torch.int32)
+    wgt, h = torch.rand(n, top, generator=g, device="cuda"), rn(n, K).to(torch.bfloat16)
+    w_in, w_out = (rn(E, N, K) * K ** -0.5).to(torch.bfloat16), (rn(E, width, N // act) * 0.1).to(torch.bfloat16)
+    sh, gate = (rn(n, width).to(torch.bfloat16), rn(n, 3)[:, 1]) if shared else (None, None)
+    x = rn(n, width) if ident else None
+    got = mx.moe_experts(h, idx, wgt, w_in, w_out, act, weigh_inputs, sh, gate, x)
+    rows, pos_of, tile_expert, num_tiles = mx.moe_align(idx, E)
+    inter = mx.moe_gemm(h, rows, tile_expert, num_tiles, w_in, wgt=wgt if weigh_inputs else None, top=top, act=act, gather=True)
+    res = mx.moe_gemm(inter, rows, tile_expert, num_tiles, w_out, out_f32=True)
+    want = mx.moe_combine(res, pos_of, top, n, sh, gate, wgt=None if weigh_inputs else wgt, ident=x)
+    assert ((got - want).norm() / want.norm()).item() < 1e-5
