@@ -566,6 +566,7 @@ extern "C" size_t b200_decode_workspace_bytes(const b200_ctx* ctx, int max_batch
 }
 
 int b200_decode_mma_launch(b200_ctx* ctx, int layer, const DecodeParams& prm, int G, cudaStream_t stream);
+int b200_decode_small_launch(b200_ctx* ctx, const DecodeParams& prm, int G, bool fused, cudaStream_t stream);
 
 static bool use_mma_decode() {
     static int v = -1;
@@ -629,10 +630,12 @@ static int decode_common(b200_ctx* ctx, int layer, const void* q, int64_t q_stri
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // Kernel choice by head-group size (measured on the benchmark's batch-256 step, same KV bytes):
     //   G = 2: FMA 97.6 us, MMA 99.4 us      G = 4: FMA 121.6, MMA 101.9      G = 8: FMA 215.7, MMA 104.2
-    if (fused) {
-        if (G > 2) return B200_EUNSUPPORTED;
-        return G == 1 ? launch_decode<1, true>(ctx, prm, st) : launch_decode<2, true>(ctx, prm, st);
+    if (fused && G > 2) return B200_EUNSUPPORTED;
+    if (!use_mma_decode()) {                     // small steps (decode_small.cu has the rule)
+        const int rc = b200_decode_small_launch(ctx, prm, G, fused, st);
+        if (rc != B200_EUNSUPPORTED) return rc;
     }
+    if (fused) return G == 1 ? launch_decode<1, true>(ctx, prm, st) : launch_decode<2, true>(ctx, prm, st);
     if (G > 2 || use_mma_decode()) return b200_decode_mma_launch(ctx, layer, prm, G, st);
     return G == 1 ? launch_decode<1, false>(ctx, prm, st) : launch_decode<2, false>(ctx, prm, st);
 }

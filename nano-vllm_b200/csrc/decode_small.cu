@@ -1,0 +1,313 @@
+// Single-token paged decode attention of small steps (reference nanovllm/layers/attention.py:71-74).
+//
+// A step of a few sequences is bound by latency, not by HBM: the stream-K kernel (decode_attn.cu) prefixes the whole batch, gives each warp
+// eight chunks that pass through a two-deep ring one after the other, and merges through global memory with a counter (15-20 us whatever the
+// bytes).  Here a CTA belongs to one (sequence, kv head): its eight warps take 16-token chunks in turn, straight from global memory into
+// registers (16 loads of 16 bytes per lane in flight, the next chunk's already asked for), meet in shared memory, and the CTAs of a cluster that
+// share a long context exchange their partials through distributed shared memory.  No workspace, no atomics, one launch; the order of every
+// sum is fixed by the shape.
+//
+// Arithmetic as in decode_attn.cu: fp32 on the FMA pipe, half a warp per token, 16 lanes x 8 dims; FUSED takes the raw qkv projection
+// (q/k-norm, RoPE and the KV append happen here).  Wider head groups than GW heads take several CTAs per kv head (K and V then come from L2).
+#include "decode_common.cuh"
+
+using namespace b200dec;
+
+namespace {
+
+constexpr int SW = 8;                              // warps per CTA
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory"); }
+__device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
+    uint32_t remote;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+
+// GW: query heads of this CTA.  grid = (splits of a context, hkv * (G / GW), batch), cluster = (splits, 1, 1).
+template <int GW, bool FUSED>
+__global__ void __launch_bounds__(SW * 32, 1) paged_decode_small_kernel(const DecodeParams p, int G) {
+    B200_PDL_TRIGGER();
+    constexpr int D = B200_HEAD_DIM;
+    __shared__ float sh_o[SW][GW][D];              // each warp's unnormalised result
+    __shared__ float sh_ml[SW][GW][2];
+    __shared__ float red_o[GW][D];                 // this CTA's
+    __shared__ float red_ml[GW][2];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, hw = lane >> 4, j = lane & 15;
+    const int splits = gridDim.x, rank = blockIdx.x, subs = G / GW;
+    const int kvh = blockIdx.y / subs, head0 = kvh * G + (blockIdx.y % subs) * GW, b = blockIdx.z;
+    const bool writer = blockIdx.y % subs == 0;    // of the CTAs that share a kv head, the one that appends
+    // metadata is uploaded before the step: read while the kernels in front drain
+    const int ctx = max(p.context_lens[b], 0);
+    const int old = FUSED ? max(ctx - 1, 0) : ctx; // tokens that are in the cache
+    const int n = (old + CHUNK - 1) / CHUNK, c0 = (int)((int64_t)n * rank / splits), c1 = (int)((int64_t)n * (rank + 1) / splits);
+    const int32_t* bt = p.block_tables + (int64_t)b * p.bt_stride;
+    const int mask = (1 << p.block_shift) - 1;
+    auto row_of = [&](int ck) -> int64_t {         // first cache row of a chunk (a chunk lies inside one page)
+        const int tok = ck * CHUNK;
+        return (((int64_t)bt[tok >> p.block_shift] * p.hkv + kvh) << p.block_shift) + (tok & mask);
+    };
+    int64_t row = c0 + warp < c1 ? row_of(c0 + warp) : 0;
+    B200_PDL_WAIT();
+
+    auto load = [&](int ck, int64_t at, uint4 (&k)[8], uint4 (&v)[8]) {      // rows past the context: zeros, nothing is read
+        const int valid = old - ck * CHUNK;
+        const uint4* ks = reinterpret_cast<const uint4*>(p.k_layer + at * D) + j;
+        const uint4* vs = reinterpret_cast<const uint4*>(p.v_layer + at * D) + j;
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            const int t = 2 * it + hw;
+            k[it] = t < valid ? ks[t * (D / 8)] : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            const int t = 2 * it + hw;
+            v[it] = t < valid ? vs[t * (D / 8)] : make_uint4(0, 0, 0, 0);
+        }
+    };
+    uint4 kr[8], vr[8];
+    if (c0 + warp < c1) load(c0 + warp, row, kr, vr);
+
+    // ---- queries ----
+    float qf[GW][8], qw[8], kw[8], cosr[8], sinr[8];
+    auto norm_rope = [&](float (&x)[8], const float (&w)[8]) {               // RMS norm -> bf16 -> NeoX rotation -> bf16, as qknorm_rope_store_kernel
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss = fmaf(x[e], x[e], ss);
+#pragma unroll
+        for (int o2 = 8; o2 > 0; o2 >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o2);
+        const float rstd = 1.0f / sqrtf(ss / (float)D + p.eps);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float y = round_bf16(__fmul_rn(__fmul_rn(x[e], rstd), w[e]));
+            const float other = __shfl_xor_sync(0xffffffffu, y, 8);          // element d +- 64
+            const float r = (j < 8) ? __fsub_rn(__fmul_rn(y, cosr[e]), __fmul_rn(other, sinr[e]))
+                                    : __fadd_rn(__fmul_rn(y, cosr[e]), __fmul_rn(other, sinr[e]));
+            x[e] = round_bf16(r);
+        }
+    };
+    const __nv_bfloat16* qrow = p.q + (int64_t)b * p.q_stride + j * 8;
+    if (FUSED) {
+        unpack8(*reinterpret_cast<const uint4*>(p.q_norm_w + j * 8), qw);
+        unpack8(*reinterpret_cast<const uint4*>(p.k_norm_w + j * 8), kw);
+        const float* cs = p.cos_sin + (int64_t)old * D + (j & 7) * 8;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            cosr[e] = cs[e];
+            sinr[e] = cs[64 + e];
+        }
+    }
+    float o[GW][8], m[GW], l[GW];
+#pragma unroll
+    for (int g = 0; g < GW; ++g) {
+        unpack8(*reinterpret_cast<const uint4*>(qrow + (head0 + g) * D), qf[g]);
+        if (FUSED) norm_rope(qf[g], qw);
+        m[g] = -INFINITY;
+        l[g] = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            qf[g][e] *= p.scale_log2;
+            o[g][e] = 0.f;
+        }
+    }
+    // the score of token 2 * my_it + hw ends up in this lane (and its neighbour j ^ 1)
+    const int my_it = ((j >> 3) & 1) * 4 + ((j >> 2) & 1) * 2 + ((j >> 1) & 1);
+
+#pragma unroll 1
+    for (int ck = c0 + warp; ck < c1; ck += SW) {
+        uint4 kn[8], vn[8];
+        if (ck + SW < c1) load(ck + SW, row_of(ck + SW), kn, vn);
+        float acc[GW][8];
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            float kf[8];
+            unpack8(kr[it], kf);
+#pragma unroll
+            for (int g = 0; g < GW; ++g) {
+                float a = qf[g][0] * kf[0];
+#pragma unroll
+                for (int e = 1; e < 8; ++e) a = fmaf(qf[g][e], kf[e], a);
+                acc[g][it] = a;
+            }
+        }
+        const bool ok = ck * CHUNK + 2 * my_it + hw < old;
+#pragma unroll
+        for (int g = 0; g < GW; ++g) {             // sum over the 16 dim slices, scattering tokens over lanes: 8 -> 4 -> 2 -> 1 values
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const float send = (j & 8) ? acc[g][x] : acc[g][x + 4], keep = (j & 8) ? acc[g][x + 4] : acc[g][x];
+                acc[g][x] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const float send = (j & 4) ? acc[g][x] : acc[g][x + 2], keep = (j & 4) ? acc[g][x + 2] : acc[g][x];
+                acc[g][x] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+            }
+            const float send = (j & 2) ? acc[g][0] : acc[g][1], keep = (j & 2) ? acc[g][1] : acc[g][0];
+            float s = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s = ok ? s : -INFINITY;
+            const float m_new = fmaxf(m[g], warp_max(s));                    // a chunk holds at least one token
+            const float alpha = fast_exp2(m[g] - m_new), pv = fast_exp2(s - m_new);
+            m[g] = m_new;
+            l[g] = l[g] * alpha + ((j & 1) ? 0.f : pv);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[g][e] *= alpha;
+            // token 2 it + hw sits in lanes whose bits (8, 4, 2) spell it: fetch each weight from there
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+                const float w = __shfl_sync(0xffffffffu, pv, (lane & 16) | ((it & 4) << 1) | ((it & 2) << 1) | ((it & 1) << 1));
+                float vf[8];
+                unpack8(vr[it], vf);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) o[g][e] = fmaf(w, vf[e], o[g][e]);
+            }
+        }
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            kr[it] = kn[it];
+            vr[it] = vn[it];
+        }
+    }
+    if (FUSED && ctx > 0 && rank == splits - 1 && warp == SW - 1) {          // the step's own token
+        float kn[8], vn[8];
+        const uint4 v_raw = *reinterpret_cast<const uint4*>(qrow + (p.hkv * G + p.hkv + kvh) * D);
+        unpack8(*reinterpret_cast<const uint4*>(qrow + (p.hkv * G + kvh) * D), kn);
+        unpack8(v_raw, vn);
+        norm_rope(kn, kw);
+        if (hw == 0 && writer) {
+            const int64_t at = (((int64_t)bt[old >> p.block_shift] * p.hkv + kvh) << p.block_shift) + (old & mask);
+            *reinterpret_cast<uint4*>(p.k_layer_w + at * D + j * 8) = pack8(kn);
+            *reinterpret_cast<uint4*>(p.v_layer_w + at * D + j * 8) = v_raw;
+        }
+#pragma unroll
+        for (int g = 0; g < GW; ++g) {
+            float s = qf[g][0] * kn[0];
+#pragma unroll
+            for (int e = 1; e < 8; ++e) s = fmaf(qf[g][e], kn[e], s);
+#pragma unroll
+            for (int o2 = 8; o2 > 0; o2 >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o2);
+            const float m_new = fmaxf(m[g], s), alpha = fast_exp2(m[g] - m_new), pn = fast_exp2(s - m_new);
+            m[g] = m_new;
+            l[g] = l[g] * alpha + (lane == 0 ? pn : 0.f);
+            const float w = hw == 0 ? pn : 0.f;    // the halves' results are summed below
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[g][e] = fmaf(w, vn[e], o[g][e] * alpha);
+        }
+    }
+    // ---- the warps of this CTA meet ----
+#pragma unroll
+    for (int g = 0; g < GW; ++g) {
+        l[g] = warp_sum(l[g]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[g][e] += __shfl_xor_sync(0xffffffffu, o[g][e], 16);
+        if (hw == 0) {
+            *reinterpret_cast<float4*>(&sh_o[warp][g][j * 8]) = make_float4(o[g][0], o[g][1], o[g][2], o[g][3]);
+            *reinterpret_cast<float4*>(&sh_o[warp][g][j * 8 + 4]) = make_float4(o[g][4], o[g][5], o[g][6], o[g][7]);
+        }
+        if (lane == 0) {
+            sh_ml[warp][g][0] = m[g];
+            sh_ml[warp][g][1] = l[g];
+        }
+    }
+    __syncthreads();
+    auto store = [&](int g, int d, float v) { p.out[(int64_t)b * p.out_stride + (head0 + g) * D + d] = __float2bfloat16_rn(v); };
+    for (int i = tid; i < GW * D; i += SW * 32) {
+        const int g = i / D, d = i % D;
+        float M = -INFINITY, L = 0.f, a = 0.f;
+#pragma unroll
+        for (int w = 0; w < SW; ++w) M = fmaxf(M, sh_ml[w][g][0]);
+#pragma unroll
+        for (int w = 0; w < SW; ++w) {
+            const float f = sh_ml[w][g][0] == -INFINITY ? 0.f : fast_exp2(sh_ml[w][g][0] - M);
+            L = fmaf(f, sh_ml[w][g][1], L);
+            a = fmaf(f, sh_o[w][g][d], a);
+        }
+        if (splits == 1) {
+            store(g, d, L > 0.f ? a / L : 0.f);
+        } else {
+            red_o[g][d] = a;
+            if (d == 0) {
+                red_ml[g][0] = M;
+                red_ml[g][1] = L;
+            }
+        }
+    }
+    if (splits == 1) return;
+    // ---- the CTAs of the cluster meet: each writes its share of the columns ----
+    cluster_sync();
+    for (int i = rank * (SW * 32) + tid; i < GW * D; i += splits * SW * 32) {
+        const int g = i / D, d = i % D;
+        float ms[8], M = -INFINITY, L = 0.f, a = 0.f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            ms[c] = c < splits ? ld_cluster(&red_ml[g][0], c) : -INFINITY;
+            M = fmaxf(M, ms[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            if (c >= splits || ms[c] == -INFINITY) continue;
+            const float f = fast_exp2(ms[c] - M);
+            L = fmaf(f, ld_cluster(&red_ml[g][1], c), L);
+            a = fmaf(f, ld_cluster(&red_o[g][d], c), a);
+        }
+        store(g, d, L > 0.f ? a / L : 0.f);
+    }
+    cluster_sync();                                // nobody leaves while its partials are being read
+}
+
+template <int GW, bool FUSED>
+int launch_small(b200_ctx* ctx, const DecodeParams& prm, int G, int splits, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, prm.hkv * (G / GW), prm.batch);
+    cfg.blockDim = dim3(SW * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (splits > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim = {(unsigned)splits, 1, 1};
+        ++na;
+    }
+#ifdef B200_PDL
+    if (!b200_tls_pdl_off()) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na].val.programmaticStreamSerializationAllowed = 1;
+        ++na;
+    }
+#endif
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
+    cudaLaunchKernelEx(&cfg, paged_decode_small_kernel<GW, FUSED>, prm, G);
+    return b200_launch_status(ctx);
+}
+
+}  // namespace
+
+// Called from decode_common() in decode_attn.cu; B200_EUNSUPPORTED: a step for the stream-K kernels.
+//
+// Taken while every (sequence, kv head) has a CTA of its own in one wave and no warp can get more than MAX_CHUNKS chunks, whatever the contexts
+// are (bounded by the table's width; the lengths are on the device).  A chunk takes a warp about 0.75 us (twice that with four heads), so the
+// longest context allowed ends no later than the stream-K kernels do on the smallest step.  Measured (one layer of the captured Qwen3-0.6B step, us,
+// here / stream-K): 1 row 9 / 22, 4 rows 12 / 22, 16 rows of up to 1024 tokens 17 / 23; beyond the bound 16 rows of 600-8192 tokens 74 / 47.
+int b200_decode_small_launch(b200_ctx* ctx, const DecodeParams& prm, int G, bool fused, cudaStream_t stream) {
+    const int GW = G >= 4 ? 4 : G, ctas = prm.batch * prm.hkv * (G / GW), MAX_CHUNKS = GW == 4 ? 4 : 16;
+    if (ctas > ctx->sm_count) return B200_EUNSUPPORTED;
+    int splits = 1;
+    while (splits < 8 && ctas * splits * 2 <= ctx->sm_count) splits *= 2;
+    const int64_t chunks = ((int64_t)prm.bt_stride << prm.block_shift) / CHUNK;
+    if (chunks > (int64_t)MAX_CHUNKS * SW * splits) return B200_EUNSUPPORTED;
+    if (fused) return GW == 1 ? launch_small<1, true>(ctx, prm, G, splits, stream) : launch_small<2, true>(ctx, prm, G, splits, stream);
+    switch (GW) {
+        case 1: return launch_small<1, false>(ctx, prm, G, splits, stream);
+        case 2: return launch_small<2, false>(ctx, prm, G, splits, stream);
+        default: return launch_small<4, false>(ctx, prm, G, splits, stream);
+    }
+}
