@@ -128,6 +128,14 @@ int b200m_latent_attention(const void* q_lat, const void* q_raw, int64_t q_tok_s
                            int rot_dim, float scale, int window, int layout, int is32, int flags, int splits, float* part,
                            void* stream);
 
+/* Single-token steps of the sizes the tcgen05 form takes (bf16; rank 256 or 512, rot_dim 64, at most 16 heads and 1024 rows, scale > 0, pages that are
+ * multiples or divisors of 128 rows and at least 8; else B200_EUNSUPPORTED): arguments as for b200m_latent_attention, n rows with ctx_lens.  workspace:
+ * b200m_latent_decode_workspace_bytes(...) bytes of the current device, nothing is kept in it. */
+size_t b200m_latent_decode_workspace_bytes(int n, int num_heads, int rank);
+int b200m_latent_decode(const void* q_lat, const void* q_raw, int64_t q_tok_stride, int q_head_stride, int q_rot_off, const void* cache, const int32_t* block_tables,
+                        int bt_stride, int block_size, const int32_t* ctx_lens, const float* sink, const float* cos_sin, int rope_dims, void* out, int n,
+                        int num_heads, int rank, int rot_dim, float scale, int window, int layout, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Prompt portions with keys and values formed per head (bf16; B200_EUNSUPPORTED for other sizes than dim 128, rot_dim 64, vdim 128 or operands that
  * are not 16-byte aligned): one gather, one GEMM of the caller's, one rotation, one attention launch.
  *   gather: out[cu_k[s] + j] = the cached row of token j of sequence s (rows of row_elems elements; max_k: an upper bound of any sequence's tokens;

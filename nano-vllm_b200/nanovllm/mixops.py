@@ -299,6 +299,15 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, q_rot_off: int, c
     _same(is32, q_raw, cache)
     if out is None:
         out = torch.empty_like(q_lat)
+    if not is32 and not fma and spans.cu_q is None and H <= 16 and rank in (256, 512) and rot_dim == 64 and n <= 1024 and scale > 0 \
+            and (block_size % 128 == 0 or (block_size >= 8 and 128 % block_size == 0)) and (q_lat.data_ptr() | cache.data_ptr() | out.data_ptr()) % 16 == 0:
+        size = nat.load_mix().b200m_latent_decode_workspace_bytes(n, H, rank)
+        space = torch.empty(size, dtype=torch.uint8, device=q_lat.device)
+        _call("b200m_latent_decode", q_lat.data_ptr(), q_raw.data_ptr(), q_raw.stride(0), q_raw.stride(1), q_rot_off, cache.data_ptr(), block_tables.data_ptr(),
+              block_tables.stride(0), block_size, spans.ctx_lens.data_ptr(), _p(sink), cos_sin.data_ptr(), cos_sin.shape[1], out.data_ptr(), n, H, rank, rot_dim,
+              scale, int(window), int(layout), space.data_ptr(), size, _stream())
+        ops.LAUNCHES[0] += 1
+        return out
     # single-token steps: few (sequence) CTAs would each walk a whole context; share the key tiles out so that about two
     # CTAs per SM are in flight.  The bound comes from the block-table width (static, so it also holds inside a CUDA graph).
     splits, part = 1, None

@@ -1,0 +1,51 @@
+"""Single-token latent attention on tcgen05 (csrc/latent_decode.cu): contexts around the 128-key tiles, steps with fewer and more tiles than CTAs,
+empty rows, stale cache rows that hold NaN, windows, sinks, both rotation layouts, fewer heads than columns, page sizes on both sides of a tile.
+
+Reference: the general path of the same entry point in fp32 on the same values (held to float64 by test_gpu_tafopel.py).  P is rounded to bf16
+(2^-9 relative) and so is the result."""
+import pytest
+import torch
+
+from test_gpu_kernels import assert_close_bf16, bf, make_tables
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rank,H", [(512, 16), (256, 16), (512, 5)])
+@pytest.mark.parametrize("lens,bs,window,layout", [([1], 256, 0, 0), ([127, 128, 129, 0, 400], 16, 0, 1), ([300, 5, 1000], 128, 200, 0), ([3000, 1, 2500], 256, 0, 1),
+                                                   ([17 * i + 1 for i in range(200)], 32, 0, 0)])
+def test_against_the_general_path(rank, H, lens, bs, window, layout):
+    from nanovllm import mixops as mx
+    from nanovllm.layers.rotary_embedding import build_banded_cos_sin
+    n, rd = len(lens), 64
+    nblk = sum(-(-c // bs) for c in lens) + 1
+    tables = make_tables(lens, bs, nblk, seed=50)
+    cache = bf(nblk * bs, rank + rd, seed=51).cuda()
+    q_lat, q_raw = bf(H, n, rank, seed=52).cuda(), bf(n, H, 128 + rd, seed=53).cuda()
+    sink = torch.linspace(-1, 1, H).cuda() if layout == 0 else None
+    cs = build_banded_cos_sin(rd, 4096, 1e4, None, "cuda")
+    spans = mx.StepSpans(n, 1, None, None, torch.tensor(lens, dtype=torch.int32).cuda())
+    args = (tables.cuda(), bs, spans, sink, cs, 0.03)
+    live = torch.tensor(lens) > 0
+    want = mx.latent_attention(q_lat.float(), q_raw.float(), 128, cache.float(), *args, window=window, layout=layout)
+    dead = torch.ones(nblk * bs, dtype=torch.bool)
+    for i, c in enumerate(lens):
+        p = torch.arange(c)
+        dead[tables[i][p // bs].long() * bs + p % bs] = False
+    cache[dead.cuda()] = float("nan")
+    got = mx.latent_attention(q_lat, q_raw, 128, cache, *args, window=window, layout=layout)
+    assert_close_bf16(got[:, live.cuda()], want[:, live.cuda()], f"{rank} {H} {bs}", rel_l2=6e-3, ulps=3.0)
+
+
+@pytest.mark.parametrize("H,rank,rd,bs", [(17, 256, 64, 256), (4, 128, 64, 256), (4, 256, 32, 256), (4, 256, 64, 24)])
+def test_other_sizes_take_the_general_form(H, rank, rd, bs):
+    from nanovllm import mixops as mx
+    from nanovllm.layers.rotary_embedding import build_banded_cos_sin
+    lens = [70, 200]
+    nblk = sum(-(-c // bs) for c in lens) + 1
+    tables, cache = make_tables(lens, bs, nblk, seed=54), bf(nblk * bs, rank + rd, seed=55).cuda()
+    q_lat, q_raw = bf(H, 2, rank, seed=56).cuda(), bf(2, H, 128 + rd, seed=57).cuda()
+    cs = build_banded_cos_sin(rd, 4096, 1e4, None, "cuda")
+    args = (tables.cuda(), bs, mx.StepSpans(2, 1, None, None, torch.tensor(lens, dtype=torch.int32).cuda()), None, cs, 0.03)
+    want = mx.latent_attention(q_lat.float(), q_raw.float(), 128, cache.float(), *args)
+    assert_close_bf16(mx.latent_attention(q_lat, q_raw, 128, cache, *args), want, "general form", rel_l2=6e-3, ulps=3.0)
