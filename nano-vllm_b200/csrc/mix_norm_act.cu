@@ -359,6 +359,45 @@ __global__ void __launch_bounds__(ROW_THREADS) rmsnorm_any_kernel(const T* __res
     for (int c = threadIdx.x; c < cols; c += blockDim.x) stf(o + c, ldf(xr + c) * rstd * ldf(w + c));
 }
 
+// The same for bf16 rows of whole 16-byte pieces, a warp per row and the row in registers (VPL pieces per lane): one pass over memory with every load in
+// flight.  Bound by HBM; a CTA per row with scalar loads and a block reduction took 21.6 us for 8192 rows of 768 columns (25 MB).
+template <int VPL>
+__global__ void __launch_bounds__(128) rmsnorm_vec_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_stride, const __nv_bfloat16* __restrict__ w,
+                                                          __nv_bfloat16* __restrict__ out, int64_t out_stride, int rows, int cols, float eps) {
+    B200_PDL_SYNC();
+    const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= rows) return;
+    const uint4 *xr = reinterpret_cast<const uint4*>(x + r * x_stride), *wr = reinterpret_cast<const uint4*>(w);
+    const int pieces = cols / 8;
+    uint4 raw[VPL], wv[VPL];
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        const int c = lane + 32 * k;
+        raw[k] = c < pieces ? xr[c] : make_uint4(0, 0, 0, 0);
+        wv[k] = c < pieces ? wr[c] : make_uint4(0, 0, 0, 0);
+    }
+    float q = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        float f[8];
+        unpack8(raw[k], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q = fmaf(f[e], f[e], q);
+    }
+    const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)cols + eps);
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+        const int c = lane + 32 * k;
+        if (c >= pieces) continue;
+        float f[8], g[8];
+        unpack8(raw[k], f);
+        unpack8(wv[k], g);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = f[e] * rstd * g[e];
+        reinterpret_cast<uint4*>(out + r * out_stride)[c] = pack8(f);
+    }
+}
+
 __device__ __forceinline__ float gelu_tanh_(float z) {
     return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
@@ -674,6 +713,19 @@ extern "C" int b200m_rmsnorm(const void* x, int64_t x_stride, const void* w, voi
                              float eps, int is32, void* stream) {
     if (!x || !w || !out || rows < 0 || cols <= 0) return B200_EINVAL;
     if (rows == 0) return B200_OK;
+    const uintptr_t bases = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out);
+    if (!is32 && cols % 8 == 0 && cols <= 2048 && x_stride % 8 == 0 && out_stride % 8 == 0 && bases % 16 == 0) {
+        using bf = __nv_bfloat16;
+        auto go = [&](auto kernel) {
+            B200_LAUNCH((kernel), (rows + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream), static_cast<const bf*>(x), x_stride, static_cast<const bf*>(w), static_cast<bf*>(out),
+                        out_stride, rows, cols, eps);
+        };
+        if (cols <= 256) go(rmsnorm_vec_kernel<1>);
+        else if (cols <= 512) go(rmsnorm_vec_kernel<2>);
+        else if (cols <= 1024) go(rmsnorm_vec_kernel<4>);
+        else go(rmsnorm_vec_kernel<8>);
+        return b200_launch_status(nullptr);
+    }
     B200M_DISPATCH(is32, B200_LAUNCH((rmsnorm_any_kernel<T>), rows, ROW_THREADS, 0, static_cast<cudaStream_t>(stream),
                                      static_cast<const T*>(x), x_stride, static_cast<const T*>(w), static_cast<T*>(out),
                                      out_stride, cols, eps));

@@ -32,20 +32,52 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(const uint4* __restr
     for (int c = lane; c < pieces; c += 32) dst[c] = src[c];
 }
 
-// The rotated part of every head's query, in place: a thread per pair.  layout 0: pairs (2i, 2i + 1), 1: (i, i + dims / 2).
+// The rotated part of every head's query, in place: a thread per V pairs (V = 4: 16-byte (layout 0) or 8-byte (layout 1) accesses; a pair per thread
+// took 24.6 us for 8192 tokens x 16 heads of 64 columns, 17 MB read and written).  layout 0: pairs (2i, 2i + 1), 1: (i, i + dims / 2).
+template <int V>
 __global__ void __launch_bounds__(256) latent_rotate_kernel(__nv_bfloat16* q, int64_t tok_stride, int head_stride, const float* __restrict__ cos_sin, int dims,
                                                             const int64_t* __restrict__ positions, int n, int heads, int layout) {
     B200_PDL_SYNC();
-    const int half = dims / 2;
+    const int half = dims / 2, per = half / V;
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (i >= (int64_t)n * heads * half) return;
-    const int c = (int)(i % half), h = (int)(i / half % heads), t = (int)(i / half / heads);
+    if (i >= (int64_t)n * heads * per) return;
+    const int c = (int)(i % per) * V, h = (int)(i / per % heads), t = (int)(i / per / heads);
     __nv_bfloat16* x = q + t * tok_stride + (int64_t)h * head_stride;
     const float* cs = cos_sin + positions[t] * dims;
-    const int e0 = layout ? c : 2 * c, e1 = layout ? c + half : 2 * c + 1;
-    const float u = __bfloat162float(x[e0]), v = __bfloat162float(x[e1]);
-    x[e0] = __float2bfloat16_rn(u * cs[c] - v * cs[half + c]);
-    x[e1] = __float2bfloat16_rn(v * cs[c] + u * cs[half + c]);
+    float u[V], v[V];
+    if constexpr (V == 4) {
+        const float4 co = *reinterpret_cast<const float4*>(cs + c), si = *reinterpret_cast<const float4*>(cs + half + c);
+        const float cc[4] = {co.x, co.y, co.z, co.w}, ss[4] = {si.x, si.y, si.z, si.w};
+        if (layout) {
+            uint2 *lo = reinterpret_cast<uint2*>(x + c), *hi = reinterpret_cast<uint2*>(x + c + half);
+            const uint2 a = *lo, b = *hi;
+            const float fa[4] = {bf16lo(a.x), bf16hi(a.x), bf16lo(a.y), bf16hi(a.y)}, fb[4] = {bf16lo(b.x), bf16hi(b.x), bf16lo(b.y), bf16hi(b.y)};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                u[k] = fa[k] * cc[k] - fb[k] * ss[k];
+                v[k] = fb[k] * cc[k] + fa[k] * ss[k];
+            }
+            *lo = make_uint2(pack_bf16x2(u[0], u[1]), pack_bf16x2(u[2], u[3]));
+            *hi = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+        } else {
+            uint4* at = reinterpret_cast<uint4*>(x + 2 * c);
+            float f[8];
+            unpack8(*at, f);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float a = f[2 * k], b = f[2 * k + 1];
+                f[2 * k] = a * cc[k] - b * ss[k];
+                f[2 * k + 1] = b * cc[k] + a * ss[k];
+            }
+            *at = pack8(f);
+        }
+    } else {
+        const int e0 = layout ? c : 2 * c, e1 = layout ? c + half : 2 * c + 1;
+        u[0] = __bfloat162float(x[e0]);
+        v[0] = __bfloat162float(x[e1]);
+        x[e0] = __float2bfloat16_rn(u[0] * cs[c] - v[0] * cs[half + c]);
+        x[e1] = __float2bfloat16_rn(v[0] * cs[c] + u[0] * cs[half + c]);
+    }
 }
 
 }  // namespace
@@ -108,10 +140,16 @@ extern "C" int b200m_latent_gather(const void* cache, int row_elems, const int32
 extern "C" int b200m_latent_rotate(void* q, int64_t tok_stride, int head_stride, const float* cos_sin, int rope_dims, const int64_t* positions, int n, int heads,
                                    int layout, void* stream) {
     if (!q || !cos_sin || !positions || n < 0 || heads <= 0 || rope_dims < 0 || rope_dims % 2) return B200_EINVAL;
-    const int64_t total = (int64_t)n * heads * (rope_dims / 2);
-    if (total == 0) return B200_OK;
-    B200_LAUNCH((latent_rotate_kernel), dim3((unsigned)((total + 255) / 256)), 256, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(q), tok_stride,
-                head_stride, cos_sin, rope_dims, positions, n, heads, layout);
+    if (n == 0 || rope_dims == 0) return B200_OK;
+    auto go = [&](auto kernel, int per) {
+        const int64_t total = (int64_t)n * heads * (rope_dims / 2 / per);
+        B200_LAUNCH((kernel), dim3((unsigned)((total + 255) / 256)), 256, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(q), tok_stride, head_stride, cos_sin,
+                    rope_dims, positions, n, heads, layout);
+    };
+    if (rope_dims % 8 == 0 && tok_stride % 8 == 0 && head_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(cos_sin)) % 16 == 0)
+        go(latent_rotate_kernel<4>, 4);
+    else
+        go(latent_rotate_kernel<1>, 1);
     return b200_launch_status(nullptr);
 }
 

@@ -171,3 +171,25 @@ def test_latent_prompts_against_attention_over_the_latents(mx, layout, len_q, le
     want = torch.bmm(o_lat, uv.transpose(1, 2)).transpose(0, 1).reshape(n, H * 128)
     got = mx.latent_prompt(q, w, d, 128, cache, tables, bs, spans, sink, cs, pos, 192 ** -0.5, window=window, layout=layout)
     assert_close_bf16(got, want, "latent prompts", rel_l2=8e-3, ulps=3.0)
+
+
+@pytest.mark.parametrize("dims,off", [(64, 128), (16, 128), (6, 128), (64, 124)])
+@pytest.mark.parametrize("layout", [0, 1])
+def test_rotation_in_place(mx, dims, off, layout):
+    """Wide and pair-by-pair accesses (odd sizes, 8-byte aligned starts) against float64; nothing beside the rotated columns changes."""
+    from nanovllm.layers.rotary_embedding import build_banded_cos_sin
+    n, H = 37, 3
+    q = bf(n, H, 192, seed=60).cuda()
+    want = q.double()
+    pos = torch.arange(n).flip(0).cuda() * 7
+    cs = build_banded_cos_sin(dims, 512, 1e4, None, "cuda")
+    c, s = cs[pos, :dims // 2].double()[:, None], cs[pos, dims // 2:].double()[:, None]
+    lo = slice(off, off + dims, 2) if layout == 0 else slice(off, off + dims // 2)
+    hi = slice(off + 1, off + dims, 2) if layout == 0 else slice(off + dims // 2, off + dims)
+    u, v = want[..., lo].clone(), want[..., hi].clone()
+    want[..., lo], want[..., hi] = u * c - v * s, v * c + u * s
+    mx._call("b200m_latent_rotate", q.data_ptr() + 2 * off, q.stride(0), q.stride(1), cs.data_ptr(), dims, pos.data_ptr(), n, H, layout, mx._stream())
+    assert (q.double() - want).abs().max().item() <= 2 ** -8 * want.abs().max().item()
+    keep = torch.ones(192, dtype=torch.bool)
+    keep[off:off + dims] = False
+    assert torch.equal(q[..., keep.cuda()].double(), want[..., keep.cuda()])
