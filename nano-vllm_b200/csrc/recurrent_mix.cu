@@ -491,8 +491,8 @@ struct BlockShape {
 // coefficient places of a block: key normalisers, query normalisers (* scale), A (t, s < t), B (t, s <= t), write strengths * key normaliser
 constexpr int CF_RK = 0, CF_RQ = 4, CF_A = 8, CF_B = 14, CF_W = 24;
 
-template <typename T, int DPL, int COLS, bool CH, bool DELTA>
-__global__ void __launch_bounds__(MB_THREADS, DPL <= 16 ? 2 : 1) matrix_state_block_kernel(
+template <typename T, int DPL, int COLS, int PER_SM, bool CH, bool DELTA>
+__global__ void __launch_bounds__(MB_THREADS, PER_SM) matrix_state_block_kernel(
     const T* __restrict__ x, int64_t stride, int q_off, int k_off, int v_off, const float* __restrict__ write_in,
     const T* __restrict__ write_t, int64_t write_stride, DecayIn dec, ScalarGate<T> sg, float* __restrict__ state,
     const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q, const int32_t* __restrict__ cu_k,
@@ -943,26 +943,31 @@ int launch_matrix_state(const void* x, int64_t stride, int q_off, int k_off, int
                         int vdim, float q_scale, cudaStream_t st, const ScalarGate<T>& sg = {}, int ones = 0) {
     if (dim > 256) return B200_EUNSUPPORTED;
     const int vcols = vdim + ones;
-#define MB_GO(DPL, COLS)                                                                                                           \
+#define MB_GO(DPL, COLS, PER_SM)                                                                                                   \
     do {                                                                                                                           \
         using SH = BlockShape<DPL, COLS>;                                                                                          \
         constexpr int CPL = SH::DP / 32;                                                                                           \
         const size_t smem = sizeof(float) * 2 * SH::FLOATS;                                                                        \
         static B200SmemOptIn opt;                                                                                                  \
-        if (opt.ensure(matrix_state_block_kernel<T, DPL, COLS, CH, DELTA>, smem) != cudaSuccess) return B200_ECUDA;                \
+        if (opt.ensure(matrix_state_block_kernel<T, DPL, COLS, PER_SM, CH, DELTA>, smem) != cudaSuccess) return B200_ECUDA;                \
         const int vx = dim % CPL == 0 && stride % CPL == 0 && q_off % CPL == 0 && k_off % CPL == 0 &&                              \
                        reinterpret_cast<uintptr_t>(x) % 16 == 0;                                                                   \
         const int vg = CH && dim % CPL == 0 && dec.stride % (CPL < 4 ? CPL : 4) == 0 && reinterpret_cast<uintptr_t>(dec.in) % 16 == 0;  \
-        B200_LAUNCH((matrix_state_block_kernel<T, DPL, COLS, CH, DELTA>), dim3(H, num_seqs, (vcols + SH::GC - 1) / SH::GC), MB_THREADS, \
+        B200_LAUNCH((matrix_state_block_kernel<T, DPL, COLS, PER_SM, CH, DELTA>), dim3(H, num_seqs, (vcols + SH::GC - 1) / SH::GC), MB_THREADS, \
                     smem, st, static_cast<const T*>(x), stride, q_off, k_off, v_off, write_in, static_cast<const T*>(write_t),     \
                     write_stride, dec, sg, state, state_slots, cu_q, cu_k, ctx_lens, out, H, G, dim, vdim, ones, q_scale, vx, vg); \
         return b200_launch_status(nullptr);                                                                                        \
     } while (0)
     if (cu_q != nullptr && max_q > MB_T) {                  // prompt portions: four tokens at a time
-        if (dim <= 32) MB_GO(4, 4);
-        if (dim <= 64) MB_GO(8, 4);
-        if (dim <= 128) MB_GO(16, 4);
-        MB_GO(32, 2);
+        if (dim <= 32) MB_GO(4, 4, 2);
+        if (dim <= 64) MB_GO(8, 4, 2);
+        if (dim <= 128) {
+            // the step's CTAs fit the SMs at one each: all the registers for it (128 spill the products; layer of 4 x 2048 tokens 995 -> 898 us).  More
+            // CTAs than that: two per SM hide each other's shuffles.
+            if ((int64_t)H * num_seqs * ((vcols + 63) / 64) <= 148) MB_GO(16, 4, 1);
+            MB_GO(16, 4, 2);
+        }
+        MB_GO(32, 2, 1);
     }
 #undef MB_GO
     if constexpr (!CH && !DELTA) {
