@@ -17,11 +17,6 @@ namespace {
 
 constexpr int SW = 8;                              // warps per CTA
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory"); }
 __device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
     uint32_t remote;
@@ -295,8 +290,9 @@ int launch_small(b200_ctx* ctx, const DecodeParams& prm, int G, int splits, cuda
 //
 // Taken while every (sequence, kv head) has a CTA of its own in one wave and no warp can get more than MAX_CHUNKS chunks, whatever the contexts
 // are (bounded by the table's width; the lengths are on the device).  A chunk takes a warp about 0.75 us (twice that with four heads), so the
-// longest context allowed ends no later than the stream-K kernels do on the smallest step.  Measured (one layer of the captured Qwen3-0.6B step, us,
-// here / stream-K): 1 row 9 / 22, 4 rows 12 / 22, 16 rows of up to 1024 tokens 17 / 23; beyond the bound 16 rows of 600-8192 tokens 74 / 47.
+// longest context allowed ends no later than the stream-K kernels do on the smallest step.  Measured (whole captured Qwen3-0.6B
+// step, us, here / stream-K): 1 row 980 / 1323, 4 rows 1040 / 1330, 16 rows of up to 1024 tokens 1195 / 1362; beyond the bound (the operator alone) 16 rows of
+// 600-8192 tokens 78 / 52, with 32 heads 112 / 56.
 int b200_decode_small_launch(b200_ctx* ctx, const DecodeParams& prm, int G, bool fused, cudaStream_t stream) {
     const int GW = G >= 4 ? 4 : G, ctas = prm.batch * prm.hkv * (G / GW), MAX_CHUNKS = GW == 4 ? 4 : 16;
     if (ctas > ctx->sm_count) return B200_EUNSUPPORTED;

@@ -12,7 +12,7 @@
 //                      tile of 64 rows (N), three CTAs per SM so that all items are in flight and share the memory bandwidth evenly.
 //
 // Both read grouped rows: the experts' inputs are gathered (and weighted) by a copy in front.  Gathering them inside, four rows per TMA
-// gather instruction, took 383 us where the copy and the box loads take 230 (8192 tokens, width 2048, gate | up), and 89 us against 50 on 64 tokens.
+// gather instruction, took 383 us where the copy and the box loads take 23 + 158 (8192 tokens, width 2048, gate | up), and 89 us against 4.5 + 42 on 64 tokens.
 // Padding rows (-1) hold anything and are never written: a result row depends on its own input row alone.
 #include "mix_common.cuh"
 #include "tc_common.cuh"
