@@ -258,7 +258,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_BF16, block_n: 
            stages: int = 0) -> torch.Tensor:
     """x [rows, k] @ w[n, k]^T on tcgen05.  EPI_SILU: w = [gate; up] rows, returns silu(gate) * up [rows, n/2];
     EPI_PARTIAL: returns fp32 [k_splits, rows, n] partial sums for ``add_rmsnorm_partials``.
-    ``stages`` (0 = default): ring depth in slots of 16 KB + block_n * 128 B."""
+    ``stages`` (0 = default): ring depth in slots of 16 KB + block_n * 128 B.  ``cluster`` (1, 2 or 4) has to divide the column blocks and
+    has no other effect: every CTA loads its own x tile."""
     _need(x, torch.bfloat16, "x"); _need(w, torch.bfloat16, "w")
     assert x.dim() == 2 and w.dim() == 2 and x.stride(1) == 1 and w.is_contiguous() and x.shape[1] == w.shape[1]
     rows, k = x.shape
@@ -296,7 +297,8 @@ def lm_head_sample(hidden: torch.Tensor, lm_head: torch.Tensor, temperatures: to
                    out_keys: torch.Tensor | None = None, step_dev: torch.Tensor | None = None, block_n: int = 128,
                    pdl: bool = False, shallow: bool = True, cluster: int = 1) -> torch.Tensor:
     """Fused LM head + sampling: hidden [rows, k] x lm_head [vocab, k] -> token ids, without materialising the logits.
-    ``key_workspace``: int64/uint64 [>= rows], zero before the call, zero again after it."""
+    ``key_workspace``: int64/uint64 [>= rows], zero before the call, zero again after it.  ``cluster``: as in ``linear``, and 2 or 4 take the
+    deep ring."""
     _need(hidden, torch.bfloat16, "hidden"); _need(lm_head, torch.bfloat16, "lm_head")
     assert hidden.dim() == 2 and hidden.stride(1) == 1 and lm_head.is_contiguous() and hidden.shape[1] == lm_head.shape[1]
     assert key_workspace.is_cuda and key_workspace.element_size() == 8 and key_workspace.numel() >= hidden.shape[0]

@@ -65,15 +65,9 @@ for M in (256, 128, 64, 16, 1):
         r[f"qkv_tc_bn{bn}{'_pdl' if pdl else ''}{'_shallow' if sh else ''}"] = timed(
             lambda i: ops.linear(x_h, w_qkv[i], ops.EPI_BF16, bn, pdl=pdl, shallow=sh))
 
-    for bn, cl in itertools.product((32, 64), (2, 4)):
-        r[f"qkv_tc_bn{bn}_cluster{cl}_pdl"] = timed(lambda i: ops.linear(x_h, w_qkv[i], ops.EPI_BF16, bn, pdl=True, cluster=cl))
-
     r["gate_up+silu_cublas"] = timed(lambda i: ops.silu_mul(F.linear(x_h, w_gu[i])))
     for bn, pdl in itertools.product((32, 64), (False, True)):
         r[f"gate_up+silu_tc_bn{bn}{'_pdl' if pdl else ''}"] = timed(lambda i: ops.linear(x_h, w_gu[i], ops.EPI_SILU, bn, pdl=pdl))
-
-    for bn, cl in itertools.product((32, 64), (2, 4)):
-        r[f"gate_up+silu_tc_bn{bn}_cluster{cl}_pdl"] = timed(lambda i: ops.linear(x_h, w_gu[i], ops.EPI_SILU, bn, pdl=True, cluster=cl))
 
     for name, xin, ws, k in (("o", x_o, w_o, OIN), ("down", x_i, w_dn, INTER)):
         r[f"{name}+addnorm_cublas"] = timed(lambda i: ops.add_rmsnorm(F.linear(xin, ws[i]), resid, wn, 1e-6))
@@ -100,9 +94,9 @@ for M in (256, 128, 64, 16, 1):
     temps = torch.full((M,), 0.6, device="cuda")
     kws = torch.zeros(M, dtype=torch.int64, device="cuda")
     r["lm_head+sample_cublas"] = timed(lambda i: ops.sample(F.linear(x_h, heads[i]), temps, 1, 0), nsets=2)
-    for sh, cl in ((True, 1), (False, 1), (False, 2), (False, 4)):
-        r[f"lm_head+sample_fused_{'shallow' if sh else 'deep'}_cluster{cl}"] = timed(
-            lambda i: ops.lm_head_sample(x_h, heads[i], temps, 1, 0, kws, shallow=sh, cluster=cl), nsets=2)
+    for sh in (True, False):
+        r[f"lm_head+sample_fused_{'shallow' if sh else 'deep'}"] = timed(
+            lambda i: ops.lm_head_sample(x_h, heads[i], temps, 1, 0, kws, shallow=sh), nsets=2)
     del heads
     res[f"M{M}"] = r
     print(f"M={M} done " + json.dumps(r), file=sys.stderr, flush=True)

@@ -86,3 +86,15 @@ def test_public_api_matches_reference_surface(golden_dir):
         assert mine[:len(params)] == params, f"{method}: {mine} vs reference {params}"
         for extra in mine[len(params):]:
             assert extra[1] != "<required>" or extra[2] == "VAR_KEYWORD", f"{method}: extra required parameter {extra}"
+
+
+def test_loads_of_the_libraries_write_their_own_cta_only():
+    """The libraries are loaded by tensor-parallel ranks: no TMA or bulk load in them spreads its data over the CTAs of a cluster."""
+    import glob
+    import re
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nano-vllm_b200", "csrc")
+    files = glob.glob(os.path.join(csrc, "*.cu")) + glob.glob(os.path.join(csrc, "*.cuh"))
+    assert len(files) > 20
+    for f in files:
+        for line in open(f):
+            assert not re.search(r"cp\.async\.bulk.*multicast", line), (f, line)
