@@ -33,6 +33,9 @@ extern "C" {
 
 int b200m_abi_version(void);
 
+/* As b200_wait_timeouts, for this library's kernels. */
+int b200m_wait_timeouts(void);
+
 /* out[i, :] = table[ids[i], :] as fp32 (the residual stream); copy (optional) receives the same rows in the table's type. */
 int b200m_embed(const int64_t* ids, const void* table, float* out, void* copy, int n, int width, int64_t vocab, int is32,
                 void* stream);

@@ -45,7 +45,8 @@ enum {
     B200_ECUDA = -3,        /* a CUDA runtime call failed; b200_last_cuda_error() has the text */
     B200_ENOTBOUND = -4,    /* KV cache not bound (b200_kv_bind) */
     B200_EWORKSPACE = -5,   /* workspace too small */
-    B200_EARCH = -6         /* device is not compute capability 10.x */
+    B200_EARCH = -6,        /* device is not compute capability 10.x */
+    B200_EWAIT = -7         /* nothing was launched: waits inside an earlier launch gave up, whose results are undefined (said once) */
 };
 
 /* ---- lifetime ------------------------------------------------------------------------- */
@@ -64,6 +65,10 @@ int b200_sm_count(const b200_ctx* ctx);
 int b200_set_pdl(int enabled);
 /* ABI version of this header; bumped on any signature change. */
 int b200_abi_version(void);
+
+/* Waits inside this library's kernels that gave up since the process began (0 in a healthy one; the results of such a launch are undefined).  Reads
+ * host memory: current for work that the caller has waited for.  A program that replays graphs asks here; a launch says B200_EWAIT once by itself. */
+int b200_wait_timeouts(void);
 
 /* Replaces the per-module k_cache / v_cache binding of ModelRunner.allocate_kv_cache
  * (engine/model_runner.py:103-121).  The caller allocates 2 * layers * num_blocks * num_kv_heads *

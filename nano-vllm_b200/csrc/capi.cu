@@ -1,7 +1,10 @@
 // Context lifetime and KV binding behind include/b200_paged_attn.h.
 #include "common.cuh"
+#include "wait_report.cuh"
 
 extern "C" int b200_abi_version(void) { return 2; }
+
+extern "C" int b200_wait_timeouts(void) { return (int)b200wait::timeouts(); }
 
 extern "C" const char* b200_strerror(int code) {
     switch (code) {
@@ -12,6 +15,7 @@ extern "C" const char* b200_strerror(int code) {
         case B200_ENOTBOUND: return "KV cache not bound (call b200_kv_bind)";
         case B200_EWORKSPACE: return "workspace too small (see b200_decode_workspace_bytes)";
         case B200_EARCH: return "device is not compute capability 10.x (this library is sm_100a only)";
+        case B200_EWAIT: return "waits inside an earlier launch gave up: its results are undefined";
         default: return "unknown error";
     }
 }

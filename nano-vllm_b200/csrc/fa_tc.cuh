@@ -25,14 +25,10 @@
 #pragma once
 #include "tc_common.cuh"
 
-// Each library that includes this names its copy: kernels, and the record of their shared-memory opt-in, must not be merged across libraries
-// of one process (a template's static is one object for all of them).
-#ifndef B200FA_COPY
-#define B200FA_COPY attn
-#endif
-
+// A copy per library (B200_LIB): kernels, and the record of their shared-memory opt-in, must not be merged across libraries of one process (a
+// template's static is one object for all of them).
 namespace b200fa {
-inline namespace B200FA_COPY {
+inline namespace B200_LIB {
 
 using namespace b200tc;
 
@@ -68,9 +64,8 @@ struct FaParams {
     const __nv_bfloat16* gate;          // or null: result times sigmoid(gate), one per head or one per element
     int64_t gate_stride;
     int gate_elems;
+    uint32_t* report;                   // host word for waits that gave up: results of such a launch are undefined
 };
-
-static __device__ uint32_t fa_wait_timeouts;   // waits that gave up (a kernel bug or a lost copy): results of such a launch are undefined
 
 template <int DQK>
 struct FaSmem {
@@ -99,8 +94,6 @@ constexpr uint32_t BAR_TMEM = B_COUNT * 8, BAR_DEAD = BAR_TMEM + 4;      // tcge
 static_assert(BAR_DEAD + 4 <= 320, "barrier area");
 
 __device__ __forceinline__ void fa_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-
-__device__ __forceinline__ bool fa_wait(uint32_t bar, uint32_t parity, uint32_t dead) { return bounded_wait(bar, parity, dead, &fa_wait_timeouts); }
 
 __device__ __forceinline__ void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -233,6 +226,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
     const uint32_t base = smem_u32(smem);
     const uint32_t bars = base + L::kOffBar, dead = bars + BAR_DEAD;
     auto bar = [&](uint32_t i) { return bars + i * 8; };
+    auto fa_wait = [&](uint32_t b, uint32_t parity) { return bounded_wait(b, parity, dead, p.report); };
     int4* list = reinterpret_cast<int4*>(smem + L::kOffList);
     float* lbuf = reinterpret_cast<float*>(smem + L::kOffL);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -327,7 +321,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
             for (int j = 0; j < n; ++j, ++blk) {
                 const int key0 = (it.j_lo + j) * BN;
                 const uint32_t b = blk & 1, ts = ts0 + b * BN;
-                if (!fa_wait(bar(B_S + t * 2 + b), (blk >> 1) & 1, dead)) goto leave;
+                if (!fa_wait(bar(B_S + t * 2 + b), (blk >> 1) & 1)) goto leave;
                 tc_fence_after();
                 float s[BN];
                 tmem_ld32n(ts, s);
@@ -371,7 +365,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                     m_ref = m_upd;
                     l_sum *= f;
                     if (j > 0) {                                         // O holds the blocks before this one once their products are done
-                        if (!fa_wait(bar(B_PV + t), (blk - 1) & 1, dead)) goto leave;
+                        if (!fa_wait(bar(B_PV + t), (blk - 1) & 1)) goto leave;
                         tc_fence_after();
 #pragma unroll 1
                         for (int c = 0; c < DV; c += 16) tmem_scale16(to + c, f);
@@ -401,7 +395,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 tc_fence_before();
                 fa_arrive(bar(B_P + t * 2 + b));
             }
-            if (!fa_wait(bar(B_OFREE + t), (items & 1) ^ 1, dead)) goto leave;     // the sums of the item before have been read
+            if (!fa_wait(bar(B_OFREE + t), (items & 1) ^ 1)) goto leave;     // the sums of the item before have been read
             lbuf[t * BM + r] = l_sum;
             fa_arrive(bar(B_L + t));
             ++items;
@@ -421,7 +415,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 // The last block reaches past the sequence's keys: those V rows are not its own (stale page rows, the next sequence of a
                 // packed batch, perhaps NaN).  Their P is exactly 0, but 0 * NaN would poison the sum: zero the staged rows (a whole
                 // 128-byte row is swizzle-agnostic).
-                if (!fa_wait(bar(B_VRAW), fixes & 1, dead)) goto leave;  // an MMA warp has seen it land
+                if (!fa_wait(bar(B_VRAW), fixes & 1)) goto leave;  // an MMA warp has seen it land
                 ++fixes;
                 int first = it.len_k - (last - BN);
                 first = first > 0 ? first : 0;
@@ -440,11 +434,11 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 const int head = it.head0 + (PAIR_HEADS ? t : 0), row = it.r0[t] + r;
                 const bool valid = row < it.len_q;
                 const int64_t grow = it.q0 + (valid ? row : 0);
-                if (!fa_wait(bar(B_L + t), items[t] & 1, dead)) goto leave;
+                if (!fa_wait(bar(B_L + t), items[t] & 1)) goto leave;
                 const float l = lbuf[t * BM + r];
                 float f = l > 0.f ? p.out_scale / l : 0.f;
                 if (p.gate && !p.gate_elems && valid) f *= 1.0f / (1.0f + expf(-__bfloat162float(p.gate[grow * p.gate_stride + head])));
-                if (!fa_wait(bar(B_O + t), items[t] & 1, dead)) goto leave;
+                if (!fa_wait(bar(B_O + t), items[t] & 1)) goto leave;
                 tc_fence_after();
                 if (!p.out_f32 && !(p.gate && p.gate_elems)) {
                     // the usual result: all of O into registers, so that the next item's products can start, then the stores
@@ -521,8 +515,8 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
         if (n_items > 0) la_load();
         auto qk = [&]() -> bool {                                        // S = Q K^T into the buffer whose P went two blocks ago
             const uint32_t qb = la_e % L::kQBufs;
-            if (la_j == 0 && !fa_wait(bar(B_QFULL + qb), (la_e / L::kQBufs) & 1, dead)) return false;
-            if (!fa_wait(bar(B_KFULL + ks.i), ks.ph, dead)) return false;
+            if (la_j == 0 && !fa_wait(bar(B_QFULL + qb), (la_e / L::kQBufs) & 1)) return false;
+            if (!fa_wait(bar(B_KFULL + ks.i), ks.ph)) return false;
             tc_fence_after();
             const bool mine = la_j < la_n;
             if (leader) {
@@ -551,16 +545,16 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 for (int k = 0; k < 2 && la_e < n_items && (L::kQBufs > 1 || la_e == e); ++k)
                     if (!qk()) goto leave;
             for (int j = 0; j < nmax; ++j) {
-                if (!fa_wait(bar(B_VFULL + vs.i), vs.ph, dead)) goto leave;
+                if (!fa_wait(bar(B_VFULL + vs.i), vs.ph)) goto leave;
                 if (w.w < 0 && j + 1 == nmax) {
                     if (t == 0 && leader) fa_arrive(bar(B_VRAW));
-                    if (!fa_wait(bar(B_VFIX), fixes & 1, dead)) goto leave;
+                    if (!fa_wait(bar(B_VFIX), fixes & 1)) goto leave;
                     ++fixes;
                 }
                 if (j < n) {
-                    if (!fa_wait(bar(B_P + t * 2 + pbuf), pph, dead)) goto leave;
+                    if (!fa_wait(bar(B_P + t * 2 + pbuf), pph)) goto leave;
                     if (j == 0) {                                        // the results of the item before have been read out
-                        if (!fa_wait(bar(B_OFREE + t), oph, dead)) goto leave;
+                        if (!fa_wait(bar(B_OFREE + t), oph)) goto leave;
                         oph ^= 1;
                     }
                     tc_fence_after();
@@ -586,7 +580,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
         auto load_q = [&](int e) -> bool {
             const FaItem it = fa_item<PAIR_HEADS>(p, list, e);
             const uint32_t qb = e % L::kQBufs;
-            if (!fa_wait(bar(B_QEMPTY + qb), ((e / L::kQBufs) & 1) ^ 1, dead)) return false;
+            if (!fa_wait(bar(B_QEMPTY + qb), ((e / L::kQBufs) & 1) ^ 1)) return false;
             if (lane == 0) {
                 mbar_expect_tx(bar(B_QFULL + qb), ((it.n[0] > 0) + (it.n[1] > 0)) * L::kQTile);
                 for (int t = 0; t < 2; ++t)
@@ -614,7 +608,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                     page = page < 0 ? 0 : page;
                     row = (int)(p.row0 + page * p.page_rows + it.kvh * p.head_rows + key % p.block_size);
                 }
-                if (!fa_wait(bar(B_KEMPTY + sl.i), sl.ph ^ 1, dead)) goto leave;
+                if (!fa_wait(bar(B_KEMPTY + sl.i), sl.ph ^ 1)) goto leave;
                 if (lane == 0) mbar_expect_tx(bar(B_KFULL + sl.i), L::kKBytes);
                 __syncwarp();
                 if (lane < boxes)
@@ -623,7 +617,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                         if (h < 2) tma_load_2d(dst, &tm_k, bar(B_KFULL + sl.i), it.kvh * p.k_col_step + h * 64, row);
                         else tma_load_2d(dst, &tm_k2, bar(B_KFULL + sl.i), p.k2_col, row);         // the key part all heads share
                     }
-                if (!fa_wait(bar(B_VEMPTY + sl.i), sl.ph ^ 1, dead)) goto leave;
+                if (!fa_wait(bar(B_VEMPTY + sl.i), sl.ph ^ 1)) goto leave;
                 if (lane == 0) mbar_expect_tx(bar(B_VFULL + sl.i), L::kVBytes);
                 __syncwarp();
                 if (lane < boxes)
@@ -652,6 +646,7 @@ int fa_launch(FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const C
     constexpr int RT = PAIR_HEADS ? BM : 2 * BM;
     p.hp = PAIR_HEADS ? p.hq / 2 : p.hq;
     p.max_rb = (max_seqlen_q + RT - 1) / RT;
+    if (const int rc = b200wait::launch_word(&p.report); rc != B200_OK) return rc;
     if (p.hp >= 2048 || p.max_rb >= (1 << 20)) return B200_EUNSUPPORTED;
     static B200SmemOptIn optin;
     B200_CUDA_CHECK((b200_ctx*)nullptr, optin.ensure(fa_kernel<DQK, PAIR_HEADS, GENERAL>, FaSmem<DQK>::kTotal));

@@ -31,7 +31,6 @@ constexpr uint32_t OFF_BAR = (OFF_CUM + (SEQ_CAP + 1) * 4 + 7) / 8 * 8;
 constexpr uint32_t SMEM = OFF_BAR + 192;
 constexpr uint32_t B_FULL = 0, B_EMPTY = UNITS, B_S = 2 * UNITS, B_PV = B_S + 1, B_P = B_PV + 1, B_Q = B_P + 1, B_COUNT = B_Q + 1;
 constexpr float THRESHOLD = 8.0f, LOG2E = 1.4426950408889634f;
-static __device__ uint32_t latent_wait_timeouts;                      // waits that gave up: results of such a launch are undefined
 
 struct LatentParams {
     const __nv_bfloat16* q_lat;                                       // [H, n, rank]
@@ -48,6 +47,7 @@ struct LatentParams {
     float* part;                                                      // slot (CTA + sequence): [H][rank] results, then [H][2] (maximum, sum)
     int64_t slot;                                                     // floats per slot, a multiple of four (the results are read 16 bytes at a time)
     __nv_bfloat16* out;                                               // [H, n, rank]
+    uint32_t* report;                                                 // host word for waits that gave up: results of such a launch are undefined
 };
 
 // Key tiles of a sequence: from the one that holds the first visible key.
@@ -72,10 +72,12 @@ __device__ __forceinline__ int prefix_tiles(const LatentParams& p, int* cum, int
     return at;
 }
 
-// A share walks (sequence, tile) pairs.
-struct Walk {
-    int s, end;                                                       // sequence, tile index (over all sequences) past its part of the share
-};
+// Whether v holds for any of the 128 softmax threads (a meeting of theirs).
+__device__ __forceinline__ bool any_of_128(bool v) {
+    int any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 2, 128, p;\n\tselp.b32 %0, 1, 0, q;\n\t}" : "=r"(any) : "r"((int)v) : "memory");
+    return any != 0;
+}
 __device__ __forceinline__ int find_seq(const int* cum, int n, int tile) {       // the sequence that owns a tile
     int lo = 0, hi = n;
     while (hi - lo > 1) {
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t base = smem_u32(smem), bars = base + OFF_BAR, dead = bars + B_COUNT * 8 + 4;
     auto bar = [&](uint32_t i) { return bars + i * 8; };
-    volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem + OFF_BAR + B_COUNT * 8);        // TMEM, dead
+    volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem + OFF_BAR + B_COUNT * 8);        // TMEM, dead, warps 0-3 leave
     int* cum = reinterpret_cast<int*>(smem + OFF_CUM);
     float* red = reinterpret_cast<float*>(smem + OFF_RED);
     float *m_ref = red + 4 * NH, *factor = m_ref + NH;
@@ -100,7 +102,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
     if (tid == 0) {
         for (uint32_t i = 0; i < B_COUNT; ++i) mbar_init(bar(i), i >= B_P ? 128 : 1);
         mbar_fence_init();
-        words[1] = 0;
+        words[1] = words[2] = 0;
     }
     if (warp == 5) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars + B_COUNT * 8), "r"(128u) : "memory");
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
         // ---- softmax, queries, partial results ----
         const uint32_t lanes = (uint32_t)(warp * 32) << 16;
         uint32_t g = 0;                                               // tiles so far
+        bool alive = true;                                            // of this warp: no wait of its own gave up
         for (int t = t_begin; t < t_end;) {
             const int s = find_seq(cum, p.n, t), seg_end = min(t_end, cum[s + 1]), seg_begin = t, ctx = p.ctx_lens[s];
             const int tile0 = first_tile(p, ctx) - cum[s], lo = p.window > 0 ? ctx - p.window : 0;
@@ -162,7 +165,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
             for (int h = 0; h < NH; ++h) l[h] = 0.f;
             for (; t < seg_end; ++t, ++g) {
                 const int key = (t + tile0) * KEYS + tid;
-                if (!bounded_wait(bar(B_S), g & 1, dead, &latent_wait_timeouts)) goto leave;
+                alive = alive && bounded_wait(bar(B_S), g & 1, dead, p.report);
                 tc_fence_after();
                 float sc[NH];
                 {
@@ -175,12 +178,12 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
 #pragma unroll
                     for (int h = 0; h < NH; ++h) sc[h] = seen ? __uint_as_float(r[h]) * p.scale_log2 : -INFINITY;
                 }
-                bool grow = false;
+                bool grow = !alive;
 #pragma unroll
                 for (int h = 0; h < NH; ++h) grow |= sc[h] > m_ref[h] + THRESHOLD;
-                int any;
-                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 2, 128, p;\n\tselp.b32 %0, 1, 0, q;\n\t}" : "=r"(any) : "r"((int)grow) : "memory");
-                if (any) {
+                if (!alive) words[2] = 1;
+                if (any_of_128(grow)) {
+                    if (words[2]) goto leave;                         // all four warps or none: they meet at barriers
 #pragma unroll
                     for (int h = 0; h < NH; ++h) {
                         const float m = warp_max(sc[h]);
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
 #pragma unroll
                     for (int h = 0; h < NH; ++h) l[h] *= factor[h];
                     if (t > seg_begin) {                              // O^T holds the share's tiles before this one once their products are done
-                        if (!bounded_wait(bar(B_PV), (g - 1) & 1, dead, &latent_wait_timeouts)) goto leave;
+                        alive = bounded_wait(bar(B_PV), (g - 1) & 1, dead, p.report);
                         tc_fence_after();
                         for (int b = 0; b < pairs; ++b) {
                             uint32_t r[NH];
@@ -214,7 +217,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
                         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     }
                 }
-                if (g > 0 && !bounded_wait(bar(B_PV), (g - 1) & 1, dead, &latent_wait_timeouts)) goto leave;          // P has been read
+                if (g > 0) alive = alive && bounded_wait(bar(B_PV), (g - 1) & 1, dead, p.report);          // P has been read
+                if (!alive) continue;                                 // leaves at the next meeting
                 uint8_t* pp = smem + OFF_P + (tid >> 6) * QPIECE + (tid & 7) * 2;
 #pragma unroll
                 for (int h = 0; h < NH; ++h) {
@@ -235,7 +239,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar(B_P)) : "memory");
             }
             // ---- this share's part of the sequence ----
-            if (!bounded_wait(bar(B_PV), (g - 1) & 1, dead, &latent_wait_timeouts)) goto leave;
+            alive = alive && bounded_wait(bar(B_PV), (g - 1) & 1, dead, p.report);
+            if (any_of_128(!alive)) goto leave;
             tc_fence_after();
             float* dst = p.part + (int64_t)(blockIdx.x + s) * p.slot;
             for (int b = 0; b < pairs; ++b) {
@@ -277,7 +282,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
                 }
                 for (int k = 0; k < units; ++k, ++u) {
                     const uint32_t slot = u % UNITS;
-                    if (!bounded_wait(bar(B_EMPTY + slot), ((u / UNITS) & 1) ^ 1, dead, &latent_wait_timeouts)) goto leave;
+                    if (!bounded_wait(bar(B_EMPTY + slot), ((u / UNITS) & 1) ^ 1, dead, p.report)) goto leave;
                     if (lane == 0) mbar_expect_tx(bar(B_FULL + slot), k < pairs ? UNIT : PIECE);
                     __syncwarp();
                     if (lane < boxes)
@@ -295,11 +300,11 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
         uint32_t g = 0, u = 0, segs = 0;
         for (int t = t_begin; t < t_end; ++segs) {
             const int s = find_seq(cum, p.n, t), seg_end = min(t_end, cum[s + 1]), seg_begin = t;
-            if (!bounded_wait(bar(B_Q), segs & 1, dead, &latent_wait_timeouts)) goto leave;
+            if (!bounded_wait(bar(B_Q), segs & 1, dead, p.report)) goto leave;
             for (; t < seg_end; ++t, ++g, u += units) {
                 for (int k = 0; k < units; ++k) {
                     const uint32_t slot = (u + k) % UNITS;
-                    if (!bounded_wait(bar(B_FULL + slot), ((u + k) / UNITS) & 1, dead, &latent_wait_timeouts)) goto leave;
+                    if (!bounded_wait(bar(B_FULL + slot), ((u + k) / UNITS) & 1, dead, p.report)) goto leave;
                     tc_fence_after();
                     if (leader) {
                         const uint64_t kd = kd0 + slot * (UNIT / 16), qd = qd0 + k * (2 * QPIECE / 16);
@@ -314,7 +319,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
                         }
                     }
                 }
-                if (!bounded_wait(bar(B_P), g & 1, dead, &latent_wait_timeouts)) goto leave;
+                if (!bounded_wait(bar(B_P), g & 1, dead, p.report)) goto leave;
                 tc_fence_after();
                 if (leader) {
                     for (int b = 0; b < pairs; ++b) {
@@ -425,7 +430,8 @@ extern "C" int b200m_latent_decode(const void* q_lat, const void* q_raw, int64_t
     if (!make_map(&tm, cache, (uint64_t)(rank + rot_dim), (1ull << 31) - 1, (uint64_t)(rank + rot_dim), box)) return B200_EUNSUPPORTED;       // rows are named by page
     LatentParams p = {static_cast<const __nv_bfloat16*>(q_lat), static_cast<const __nv_bfloat16*>(q_raw), q_tok_stride, q_head_stride, q_rot_off, block_tables, bt_stride,
                       block_size, box, ctx_lens, sink, cos_sin, rope_dims, layout, n, num_heads, rank, window, scale * LOG2E, static_cast<float*>(workspace), slot_floats(num_heads, rank),
-                      static_cast<__nv_bfloat16*>(out)};
+                      static_cast<__nv_bfloat16*>(out), nullptr};
+    if (const int rc = b200wait::launch_word(&p.report); rc != B200_OK) return rc;
     static B200SmemOptIn opt;
     B200_CUDA_CHECK((b200_ctx*)nullptr, opt.ensure(latent_decode_kernel, SMEM));
     cudaStream_t st = static_cast<cudaStream_t>(stream);

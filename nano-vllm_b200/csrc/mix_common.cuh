@@ -5,8 +5,10 @@
 // path, the float instance keeps every tensor in 32 bits.  What the kernels accumulate (norm statistics, softmax, the
 // residual stream, recurrent state, router scores) is fp32 in both.
 #pragma once
+#define B200_LIB mix
 #include "common.cuh"
 #include "b200_mixers.h"
+#include "wait_report.cuh"
 
 template <typename T>
 __device__ __forceinline__ float ldf(const T* p);

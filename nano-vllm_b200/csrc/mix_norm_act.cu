@@ -554,6 +554,8 @@ __global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ x, int
 
 extern "C" int b200m_abi_version(void) { return 6; }
 
+extern "C" int b200m_wait_timeouts(void) { return (int)b200wait::timeouts(); }
+
 extern "C" int b200m_ff_glu_clamped(const void* x, int64_t x_stride, void* out, int64_t rows, int n, float limit, float alpha, int is32,
                                     void* stream) {
     if (!x || !out || rows < 0 || n <= 0 || x_stride < 2 * (int64_t)n) return B200_EINVAL;

@@ -23,7 +23,6 @@ using namespace b200tc;
 
 constexpr int TILE = 64;                          // rows per tile of moe_align
 constexpr uint32_t ROW_B = 128;                   // bytes of a staged row: 64 bf16
-static __device__ uint32_t moe_wait_timeouts;     // waits that gave up: results of such a launch are undefined
 
 struct MoeParams {
     const int32_t* sorted_rows;                   // [max_tiles * 64] pair index or -1
@@ -33,6 +32,7 @@ struct MoeParams {
     int N, K, n_out, act;                         // weight rows per expert, output columns; act 0 none, 1 relu^2, 2 gated SiLU
     void* C;
     int out_f32;
+    uint32_t* report;                             // host word for waits that gave up: results of such a launch are undefined
 };
 
 __device__ __forceinline__ float moe_act1(float v) {
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) moe_rows_kernel(const __grid_con
             const int c0 = i % nblk * cols;
             const int64_t row = (int64_t)(ent & 0x7fffffffu) * TILE + tid;
             const int pair = tid < TILE || (ent >> 31) ? p.sorted_rows[row] : -1;
-            if (!bounded_wait(acc_full + b * 8, (n >> 1) & 1, dead, &moe_wait_timeouts)) goto leave;
+            if (!bounded_wait(acc_full + b * 8, (n >> 1) & 1, dead, p.report)) goto leave;
             tc_fence_after();
             const uint32_t acc = tmem + b * 256 + ((uint32_t)(warp * 32) << 16);
 #pragma unroll 1
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) moe_rows_kernel(const __grid_con
         for (int i = blockIdx.x; i < items; i += gridDim.x) {
             const int tile = list[i / nblk] & 0x7fffffffu, w0 = p.tile_expert[tile] * p.N + i % nblk * cols;
             for (int k = 0; k < ksteps; ++k) {
-                if (!bounded_wait(empty + s * 8, ph, dead, &moe_wait_timeouts)) goto leave;
+                if (!bounded_wait(empty + s * 8, ph, dead, p.report)) goto leave;
                 if (lane == 0) {
                     const uint32_t dst = base + s * R_STAGE, bar = full + s * 8;
                     mbar_expect_tx(bar, R_STAGE);
@@ -167,10 +167,10 @@ __global__ void __launch_bounds__(R_THREADS, 1) moe_rows_kernel(const __grid_con
         uint32_t s = 0, ph = 0, n = 0;
         for (int i = blockIdx.x; i < items; i += gridDim.x, ++n) {
             const uint32_t b = n & 1;
-            if (!bounded_wait(acc_empty + b * 8, ((n >> 1) & 1) ^ 1, dead, &moe_wait_timeouts)) goto leave;
+            if (!bounded_wait(acc_empty + b * 8, ((n >> 1) & 1) ^ 1, dead, p.report)) goto leave;
             tc_fence_after();
             for (int k = 0; k < ksteps; ++k) {
-                if (!bounded_wait(full + s * 8, ph, dead, &moe_wait_timeouts)) goto leave;
+                if (!bounded_wait(full + s * 8, ph, dead, p.report)) goto leave;
                 tc_fence_after();
                 if (leader) {
                     const uint64_t ad = ad0 + s * (R_STAGE / 16), wd = wd0 + s * (R_STAGE / 16);
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(S_THREADS, 3) moe_stream_kernel(const __grid_c
         const int w0 = p.tile_expert[tile] * p.N + c0;
         for (int k = 0; k < ksteps && ok; ++k) {
             const uint32_t s = k % S_STAGES, dst = base + s * S_STAGE, bar = full + s * 8;
-            if (!bounded_wait(empty + s * 8, ((k / S_STAGES) & 1) ^ 1, dead, &moe_wait_timeouts)) {
+            if (!bounded_wait(empty + s * 8, ((k / S_STAGES) & 1) ^ 1, dead, p.report)) {
                 ok = false;
                 break;
             }
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(S_THREADS, 3) moe_stream_kernel(const __grid_c
         constexpr uint32_t IDESC = make_idesc(128, TILE, false);
         for (int k = 0; k < ksteps && ok; ++k) {
             const uint32_t s = k % S_STAGES;
-            if (!bounded_wait(full + s * 8, (k / S_STAGES) & 1, dead, &moe_wait_timeouts)) {
+            if (!bounded_wait(full + s * 8, (k / S_STAGES) & 1, dead, p.report)) {
                 ok = false;
                 break;
             }
@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(S_THREADS, 3) moe_stream_kernel(const __grid_c
         }
     }
     __syncwarp();
-    if (ok) ok = bounded_wait(done, 0, dead, &moe_wait_timeouts);
-    if (!ok || words[1]) {                        // gave up: let copies that are still in flight land first
+    if (ok) ok = bounded_wait(done, 0, dead, p.report);
+    if (__any_sync(0xffffffffu, !ok || words[1])) {      // gave up: let copies that are still in flight land first
         for (int i = 0; i < 1000; ++i) __nanosleep(1000);
         ok = false;
     }
@@ -359,7 +359,8 @@ int b200m_moe_gemm_tc(const void* A, int64_t a_stride, const int32_t* sorted_row
     const int n_out = act == 2 ? N / 2 : N, cols = (act == 2 ? 64 : 128) * (stream_form ? 1 : 2);
     const uintptr_t bases = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W);
     if (rows_per_expert <= 0 || K % 8 || a_stride % 8 || bases % 16 || reinterpret_cast<uintptr_t>(C) % 32 || n_out % cols || max_tiles > (stream_form ? 65535 : R_TILES)) return B200_EUNSUPPORTED;
-    MoeParams p = {sorted_rows, tile_expert, num_tiles, max_tiles, N, K, n_out, act, C, out_f32};
+    MoeParams p = {sorted_rows, tile_expert, num_tiles, max_tiles, N, K, n_out, act, C, out_f32, nullptr};
+    if (const int rc = b200wait::launch_word(&p.report); rc != B200_OK) return rc;
     CUtensorMap ta, tw;
     if (!make_map(&ta, A, (uint64_t)K, (uint64_t)max_tiles * TILE, (uint64_t)a_stride, stream_form ? TILE : 128) ||
         !make_map(&tw, W, (uint64_t)K, ANY_ROWS, (uint64_t)K, stream_form ? 64 : 128))

@@ -4,7 +4,6 @@
 //   latent attention                 : keys and values of every head formed from the cached latents first.  Per (head, query, key) the
 //                                      products are then 192 + 128 wide instead of the 576 + 512 of attention over the latents themselves
 //                                      (rank 512), which pays from a few tens of queries per sequence on.
-#define B200FA_COPY mix
 #include "mix_common.cuh"
 #include "fa_tc.cuh"
 

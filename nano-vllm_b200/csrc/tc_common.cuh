@@ -3,6 +3,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "wait_report.cuh"
 
 namespace b200tc {
 
@@ -74,20 +75,28 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-// Bounded wait; false: some wait of this CTA gave up (`dead`, a shared word) and every role leaves.
-__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, uint32_t dead, uint32_t* timeouts) {
-    if (mbar_try(bar, parity)) return true;
+// Bounded wait of a whole, converged warp: one answer for all its lanes, since what follows is often a collective of the warp.  false: some wait
+// of this CTA gave up (`dead`, a shared word) and every role leaves; `report` is the host's word for it (wait_report.cuh).
+__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, uint32_t dead, uint32_t* report) {
+    uint32_t ok = mbar_try(bar, parity);
+    if (__all_sync(0xffffffffu, ok)) return true;
     uint64_t t0, t1;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
     do {
         uint32_t d;
-        if (mbar_try(bar, parity)) return true;
+        if (!ok) ok = mbar_try(bar, parity);
+        if (__all_sync(0xffffffffu, ok)) return true;
         asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(d) : "r"(dead) : "memory");
-        if (d) return false;
+        if (__any_sync(0xffffffffu, d)) return false;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-    } while (t1 - t0 < 2000000000ull);                                   // two seconds: far beyond any wait of a healthy launch
-    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
-    atomicAdd(timeouts, 1u);
+    } while (!__any_sync(0xffffffffu, t1 - t0 >= 2000000000ull));        // two seconds: far beyond any wait of a healthy launch
+    if ((threadIdx.x & 31) == 0) {
+        asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
+        volatile uint32_t* w = report;
+        *w = *w + 1;                                                     // two CTAs at once may count as one: the word has moved all the same
+        __threadfence_system();
+    }
+    __syncwarp();
     return false;
 }
 

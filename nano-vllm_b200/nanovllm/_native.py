@@ -20,6 +20,7 @@ SIGNATURES = {
     "b200_last_cuda_error": (C.c_char_p, [_vp]),
     "b200_sm_count": (_i, [_vp]),
     "b200_abi_version": (_i, []),
+    "b200_wait_timeouts": (_i, []),
     "b200_set_pdl": (_i, [_i]),
     "b200_kv_bind": (_i, [_vp, _vp, _vp, _i, _i64, _i, _i, _i]),
     "b200_decode_workspace_bytes": (_sz, [_vp, _i, _i]),
@@ -49,6 +50,7 @@ SIGNATURES = {
 _f32p = _vp
 MIX_SIGNATURES = {
     "b200m_abi_version": (_i, []),
+    "b200m_wait_timeouts": (_i, []),
     "b200m_embed": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i64, _i, _vp]),
     "b200m_add_normed": (_i, [_vp, _vp, _vp, _vp, _f, _f, _vp, _i, _i, _f, _i, _vp]),
     "b200m_rmsnorm_rows": (_i, [_vp, _vp, _vp, _f, _vp, _i, _i, _f, _i, _vp]),
@@ -107,6 +109,10 @@ class B200Error(RuntimeError):
     pass
 
 
+class WaitTimeout(B200Error):
+    """A wait inside a kernel gave up (seconds, where microseconds are usual): the results of that launch are undefined."""
+
+
 def lib_path() -> Path:
     return Path(os.environ.get("B200ATTN_LIB", _LIB_PATH))
 
@@ -163,12 +169,18 @@ def load_mix():
 
 
 _CODES = {0: "ok", -1: "invalid argument", -2: "unsupported shape", -3: "CUDA runtime error", -4: "cache not bound",
-          -5: "workspace too small", -6: "device is not compute capability 10.x"}
+          -5: "workspace too small", -6: "device is not compute capability 10.x",
+          -7: "waits inside an earlier launch gave up: its results are undefined"}
+
+
+def wait_timeouts() -> int:
+    """Waits inside kernels that gave up since the process began, over the libraries that are loaded (host memory, no synchronisation)."""
+    return (_lib.b200_wait_timeouts() if _lib is not None else 0) + (_mix.b200m_wait_timeouts() if _mix is not None else 0)
 
 
 def check_mix(code: int):
     if code != 0:
-        raise B200Error(f"libb200mix: {_CODES.get(code, 'unknown error')} (code {code})")
+        raise (WaitTimeout if code == -7 else B200Error)(f"libb200mix: {_CODES.get(code, 'unknown error')} (code {code})")
 
 
 def check(code: int, ctx=None):
@@ -178,7 +190,7 @@ def check(code: int, ctx=None):
     msg = lib.b200_strerror(code).decode()
     if code == -3:                        # ctx None: the text of this thread's last context-less call
         msg += ": " + lib.b200_last_cuda_error(ctx).decode()
-    raise B200Error(f"libb200attn: {msg} (code {code})")
+    raise (WaitTimeout if code == -7 else B200Error)(f"libb200attn: {msg} (code {code})")
 
 
 class Handle:

@@ -227,6 +227,7 @@ class ModelRunner:
         self.d2h_bytes_last = 0
         self._done = [torch.cuda.Event(), torch.cuda.Event()]
         self._launches = 0
+        self._waits_seen = nat.wait_timeouts()
         self._pending: deque = deque()            # (read-back buffer, rows) of steps launched but not collected
 
     # ---- init-time passes -----------------------------------------------------------------------
@@ -550,6 +551,10 @@ class ModelRunner:
             from .peer_reduce import PeerExchangeTimeout
             raise PeerExchangeTimeout("tensor-parallel peer exchange timed out in this step (a rank stopped or fell >10 s "
                                       "behind); its tokens are invalid -- rerun with B200_TP_ALLREDUCE=nccl to bypass")
+        gave_up = nat.wait_timeouts()
+        if gave_up != self._waits_seen:
+            self._waits_seen = gave_up
+            raise nat.WaitTimeout("a wait inside a kernel gave up in this step or the one behind it; their tokens are invalid")
         return self.h_tokens_np[kk][:n].tolist()
 
     def drain(self) -> None:
