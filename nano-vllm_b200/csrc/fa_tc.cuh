@@ -227,6 +227,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
     const uint32_t bars = base + L::kOffBar, dead = bars + BAR_DEAD;
     auto bar = [&](uint32_t i) { return bars + i * 8; };
     auto fa_wait = [&](uint32_t b, uint32_t parity) { return bounded_wait(b, parity, dead, p.report); };
+    auto lane_wait = [&](uint32_t b, uint32_t parity) { return bounded_wait_as<false>(b, parity, dead, p.report); };
     int4* list = reinterpret_cast<int4*>(smem + L::kOffList);
     float* lbuf = reinterpret_cast<float*>(smem + L::kOffL);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -515,8 +516,8 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
         if (n_items > 0) la_load();
         auto qk = [&]() -> bool {                                        // S = Q K^T into the buffer whose P went two blocks ago
             const uint32_t qb = la_e % L::kQBufs;
-            if (la_j == 0 && !fa_wait(bar(B_QFULL + qb), (la_e / L::kQBufs) & 1)) return false;
-            if (!fa_wait(bar(B_KFULL + ks.i), ks.ph)) return false;
+            if (la_j == 0 && !lane_wait(bar(B_QFULL + qb), (la_e / L::kQBufs) & 1)) return false;
+            if (!lane_wait(bar(B_KFULL + ks.i), ks.ph)) return false;
             tc_fence_after();
             const bool mine = la_j < la_n;
             if (leader) {
@@ -545,16 +546,16 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 for (int k = 0; k < 2 && la_e < n_items && (L::kQBufs > 1 || la_e == e); ++k)
                     if (!qk()) goto leave;
             for (int j = 0; j < nmax; ++j) {
-                if (!fa_wait(bar(B_VFULL + vs.i), vs.ph)) goto leave;
+                if (!lane_wait(bar(B_VFULL + vs.i), vs.ph)) goto leave;
                 if (w.w < 0 && j + 1 == nmax) {
                     if (t == 0 && leader) fa_arrive(bar(B_VRAW));
-                    if (!fa_wait(bar(B_VFIX), fixes & 1)) goto leave;
+                    if (!lane_wait(bar(B_VFIX), fixes & 1)) goto leave;
                     ++fixes;
                 }
                 if (j < n) {
-                    if (!fa_wait(bar(B_P + t * 2 + pbuf), pph)) goto leave;
+                    if (!lane_wait(bar(B_P + t * 2 + pbuf), pph)) goto leave;
                     if (j == 0) {                                        // the results of the item before have been read out
-                        if (!fa_wait(bar(B_OFREE + t), oph)) goto leave;
+                        if (!lane_wait(bar(B_OFREE + t), oph)) goto leave;
                         oph ^= 1;
                     }
                     tc_fence_after();

@@ -75,30 +75,36 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-// Bounded wait of a whole, converged warp: one answer for all its lanes, since what follows is often a collective of the warp.  false: some wait
-// of this CTA gave up (`dead`, a shared word) and every role leaves; `report` is the host's word for it (wait_report.cuh).
-__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, uint32_t dead, uint32_t* report) {
+// Bounded waits.  false: some wait of this CTA gave up (`dead`, a shared word) and every role leaves; `report` is the host's word for it
+// (wait_report.cuh).  WHOLE: a converged warp waits and all its lanes get one answer, for warps that go on to collectives of the warp.  Else a lane
+// answers for itself: enough where nothing but one lane's products follows, and a vote less in warps bound by the instructions around them.
+template <bool WHOLE>
+__device__ __forceinline__ bool bounded_wait_as(uint32_t bar, uint32_t parity, uint32_t dead, uint32_t* report) {
     uint32_t ok = mbar_try(bar, parity);
-    if (__all_sync(0xffffffffu, ok)) return true;
+    if (WHOLE ? __all_sync(0xffffffffu, ok) : ok) return true;
     uint64_t t0, t1;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    bool late;
     do {
         uint32_t d;
         if (!ok) ok = mbar_try(bar, parity);
-        if (__all_sync(0xffffffffu, ok)) return true;
+        if (WHOLE ? __all_sync(0xffffffffu, ok) : ok) return true;
         asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(d) : "r"(dead) : "memory");
-        if (__any_sync(0xffffffffu, d)) return false;
+        if (WHOLE ? __any_sync(0xffffffffu, d) : d) return false;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-    } while (!__any_sync(0xffffffffu, t1 - t0 >= 2000000000ull));        // two seconds: far beyond any wait of a healthy launch
-    if ((threadIdx.x & 31) == 0) {
+        late = t1 - t0 >= 2000000000ull;                                 // two seconds: far beyond any wait of a healthy launch
+        if (WHOLE) late = __any_sync(0xffffffffu, late);
+    } while (!late);
+    if (!WHOLE || (threadIdx.x & 31) == 0) {
         asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
         volatile uint32_t* w = report;
-        *w = *w + 1;                                                     // two CTAs at once may count as one: the word has moved all the same
+        *w = *w + 1;                                                     // two at once may count as one: the word has moved all the same
         __threadfence_system();
     }
-    __syncwarp();
+    if (WHOLE) __syncwarp();
     return false;
 }
+__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, uint32_t dead, uint32_t* report) { return bounded_wait_as<true>(bar, parity, dead, report); }
 
 // Shared-memory matrix descriptor (cute::UMMA::SmemDescriptor): 128-byte swizzle, version 1.
 //   K-major operand  : rows of 128 B, 8-row groups 1024 B apart (SBO); LBO unused.

@@ -69,15 +69,17 @@ def test_collect_raises_once_per_news(monkeypatch):
 
 
 def test_every_bounded_wait_reports_and_is_the_whole_warps():
-    """A bounded wait has no other sink than the launch's host word, and the warp votes before it answers."""
+    """A bounded wait has no other sink than the launch's host word, and the warp votes before it answers; lanes answer for themselves in the prompt
+    kernel's product warps alone."""
     text = open(os.path.join(CSRC, "tc_common.cuh")).read()
-    body = text[text.index("bool bounded_wait("):]
+    body = text[text.index("bool bounded_wait_as("):]
     body = body[:body.index("\n}\n")]
-    assert body.count("return true") == body.count("if (__all_sync(0xffffffffu, ok)) return true") == 2
+    assert body.count("return true") == body.count("if (WHOLE ? __all_sync(0xffffffffu, ok) : ok) return true") == 2
     calls = 0
     for name in sorted(os.listdir(CSRC)):
         if name.endswith((".cu", ".cuh")) and name != "tc_common.cuh":
             source = open(os.path.join(CSRC, name)).read()
             calls += source.count("bounded_wait(")
+            assert source.count("bounded_wait_as<false>(") == (name == "fa_tc.cuh"), name
             assert source.count("bounded_wait(") == len(re.findall(r"bounded_wait\([^;]*?, dead, p\.report\)", source)), name
     assert calls >= 10
