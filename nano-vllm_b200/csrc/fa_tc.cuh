@@ -5,7 +5,7 @@
 // kv head (PAIR_HEADS), or 256 consecutive rows of one head.  Keys come in blocks of 64.  Roles (512 threads):
 //
 //   warps 0-3, 4-7   softmax of tile 0 / tile 1: thread = query row; S row from TMEM, scale / bias / mask, running maximum, exp2, P (bf16)
-//                    back into the TMEM columns of S; O is rescaled in TMEM only when a row's maximum grows by more than 2^8
+//                    back into the TMEM columns of S; O is rescaled in TMEM when a row's maximum grows by more than FaParams::lag (log2)
 //   warps 8-11       results: O / l from TMEM to memory while the softmax warps are at the next item; zeroes V rows past the last key
 //   warps 12, 13     tcgen05.mma of tile 0 / tile 1: S_t = Q_t K^T (both operands in shared memory), O_t += P_t V (P from TMEM, V an MN-major
 //                    operand); one warp for both tiles was bound by the instructions around its products (2490 cycles per 64 keys)
@@ -38,7 +38,6 @@ constexpr int DV = 128;                 // columns of a value row
 constexpr int THREADS = 512;
 constexpr int ITEM_CAP = 96;            // items per CTA (more items: more CTAs)
 constexpr int LEVELS_CAP = 8192;        // row blocks per sequence that the longest-first order covers (its counters lie where Q will be)
-constexpr float RESCALE_THRESHOLD = 8.0f;
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct FaParams {
@@ -54,6 +53,10 @@ struct FaParams {
     int block_size, box_rows;           // paged: rows of a page, rows per TMA box
     int64_t row0, page_rows, head_rows; // paged row = row0 + page * page_rows + kvh * head_rows + row in page
     float scale_log2;
+    // How far (log2) a row's maximum may pass the reference its weights are formed against.  Above 0 spares most rescaling of O, but the row's largest
+    // weights are then rounded to bf16 where 2^0 is exact, which peaked rows feel: scores of deviation 1 / 2 / 5 over 2048 keys are 0.0016 / 0.0016 /
+    // 0.0012 from 64 bits at 8, and 0.0015 / 0.0009 / 0.0004 at 0.
+    float lag;
     const float* slopes;                // per head, or null: score -= slope * (query position - key position)
     const float* sinks;                 // per head, or null: score of an extra term without a value
     int window, chunk;                  // visible keys: the last `window`, or those of the query's own chunk (0: all)
@@ -110,18 +113,6 @@ __device__ __forceinline__ void tmem_ld32n(uint32_t taddr, float* v) {
         "%28,%29,%30,%31}, [%32];\n\t"
         : TC_R8(r, 0), TC_R8(r, 8), TC_R8(r, 16), TC_R8(r, 24)
         : "r"(taddr));
-}
-// 16 columns times f, in place (without the wait for the store)
-__device__ __forceinline__ void tmem_scale16(uint32_t taddr, float f) {
-    uint32_t r[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
-                 : TC_R8(r, 0), TC_R8(r, 8)
-                 : "r"(taddr)
-                 : "memory");
-#pragma unroll
-    for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * f);
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), TC_I8(r, 0), TC_I8(r, 8)
-                 : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -359,7 +350,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 mx[1] = max3(mx[1], s[BN - 2], s[BN - 1]);
                 float m_new = max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]);
                 if (!GENERAL) m_new *= p.scale_log2;
-                const bool grow = m_new > m_ref + RESCALE_THRESHOLD;     // m_ref = -inf: the first block with a visible key
+                const bool grow = m_new > m_ref + p.lag;                 // m_ref = -inf: the first block with a visible key
                 if (__any_sync(0xffffffffu, grow)) {
                     const float m_upd = grow ? m_new : m_ref;
                     const float f = m_ref == m_upd ? 1.0f : fast_exp2(m_ref - m_upd);
@@ -369,7 +360,14 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                         if (!fa_wait(bar(B_PV + t), (blk - 1) & 1)) goto leave;
                         tc_fence_after();
 #pragma unroll 1
-                        for (int c = 0; c < DV; c += 16) tmem_scale16(to + c, f);
+                        for (int c = 0; c < DV; c += 32) {
+                            float o[32];
+                            tmem_ld32n(to + c, o);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int k = 0; k < 32; ++k) o[k] *= f;
+                            tmem_st32u(to + c, reinterpret_cast<const uint32_t*>(o));
+                        }
                         tmem_wait_st();
                     }
                 }

@@ -23,6 +23,7 @@ int b200_prefill_fa_launch(b200_ctx* ctx, int layer, const void* q, int64_t q_st
     p.hkv = num_kv_heads;
     p.q_col_step = D;
     p.scale_log2 = scale * LOG2E;
+    p.lag = 8.0f;
     p.out = out;
     p.out_stride = out_stride0;
     p.out_scale = 1.0f;

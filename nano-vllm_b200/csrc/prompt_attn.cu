@@ -110,6 +110,7 @@ int b200m_window_prompt(const void* q, int64_t q_stride, const void* cache, int 
     p.box_rows = box;
     p.page_rows = block_size;
     p.scale_log2 = scale * LOG2E;
+    p.lag = 0.f;                         // as the mma.sync forms of these layers
     p.slopes = slopes;
     p.sinks = sinks;
     p.window = window;
@@ -174,6 +175,7 @@ extern "C" int b200m_latent_prompt(const void* q, int64_t q_stride, const void* 
     p.k2_col = rank;
     p.block_size = p.box_rows = BN;
     p.scale_log2 = scale * LOG2E;
+    p.lag = 0.f;                         // as the mma.sync forms of these layers
     p.sinks = sink;
     p.window = window;
     p.out = out;
