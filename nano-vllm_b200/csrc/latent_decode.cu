@@ -7,9 +7,13 @@
 //
 //   warp 4       TMA: a tile as units of 128 columns (two swizzled [128 keys][64] pieces, 32 KB) and the rotated part (16 KB), six slots in flight
 //   warp 5       tcgen05.mma with the KEYS as rows (M = 128) and the heads as columns (N = 16): S^T = K Q^T, then O^T (128 latent columns at a time)
-//                += C^T P with the same staged rows as MN-major operand; both results are a few TMEM columns, so nothing is padded to 128 heads
+//                += C^T P (N = 32) with the same staged rows as MN-major operand; both results are a few TMEM columns, so nothing is padded to 128 heads
 //   warps 0-3    thread = key: 16 scores from TMEM, exp2 against a reference maximum per head that moves only when a score passes it by 2^8 (then
 //                O^T's columns are scaled), P to shared memory; row sums stay per thread until the end of a share
+//
+// P goes in as two bf16 terms, the rounded weight and what it left, side by side as 32 columns: the product is bound by its 128 rows, and a reference
+// that lags behind the maximum would otherwise have a row's largest weights rounded where 2^0 is exact (one term: 0.00453 from 64 bits on 64 rows of
+// 2048-4096 tokens, the former kernel 0.00447).
 //
 // The mma.sync form this replaces for these sizes staged 64-key tiles with one tile in flight and read every row twice (output columns in two halves):
 // 224 us + 14 us merge at the size above.
@@ -24,8 +28,9 @@ constexpr int KEYS = 128, NH = 16, UNITS = 6, THREADS = 192, SEQ_CAP = 1024, SHA
 constexpr uint32_t PIECE = KEYS * 128, UNIT = 2 * PIECE;              // [128 keys][64 columns]
 constexpr uint32_t QPIECE = NH * 128;                                 // [16 heads][64 columns]
 constexpr uint32_t OFF_Q = UNITS * UNIT;                              // up to 9 pieces
-constexpr uint32_t OFF_P = OFF_Q + 9 * QPIECE;                        // two pieces [16 heads][64 keys]
-constexpr uint32_t OFF_RED = OFF_P + 2 * QPIECE;                      // float[4][16] per-warp maxima / sums, float[16] reference maxima, float[16] factors
+constexpr uint32_t OFF_P = OFF_Q + 9 * QPIECE;                        // two PPIECEs
+constexpr uint32_t PPIECE = 2 * QPIECE;                               // [16 heads: weights, 16 heads: what they left][64 keys]
+constexpr uint32_t OFF_RED = OFF_P + 2 * PPIECE;                      // float[4][16] per-warp maxima / sums, float[16] reference maxima, float[16] factors
 constexpr uint32_t OFF_CUM = OFF_RED + 6 * NH * 4;                    // int[SEQ_CAP + 1] tiles before each sequence
 constexpr uint32_t OFF_BAR = (OFF_CUM + (SEQ_CAP + 1) * 4 + 7) / 8 * 8;
 constexpr uint32_t SMEM = OFF_BAR + 192;
@@ -105,7 +110,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
         words[1] = words[2] = 0;
     }
     if (warp == 5) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars + B_COUNT * 8), "r"(128u) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars + B_COUNT * 8), "r"(256u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 128) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm) : "memory");
@@ -115,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = words[0], tmem_o = tmem + 32;               // S^T at 0, O^T block b at 32 + 16 b
+    const uint32_t tmem = words[0], tmem_o = tmem + 32;               // S^T at 0, O^T block b at 32 + 32 b
     const int total = cum[p.n];
     const int t_begin = (int)((int64_t)total * blockIdx.x / gridDim.x), t_end = (int)((int64_t)total * (blockIdx.x + 1) / gridDim.x);
 
@@ -203,28 +208,25 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
                         alive = bounded_wait(bar(B_PV), (g - 1) & 1, dead, p.report);
                         tc_fence_after();
                         for (int b = 0; b < pairs; ++b) {
-                            uint32_t r[NH];
-                            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
-                                         : TC_R8(r, 0), TC_R8(r, 8)
-                                         : "r"(tmem_o + lanes + b * NH)
-                                         : "memory");
+                            float r[2 * NH];
+                            tmem_ld32(tmem_o + lanes + b * 2 * NH, r);
 #pragma unroll
-                            for (int h = 0; h < NH; ++h) r[h] = __float_as_uint(__uint_as_float(r[h]) * factor[h]);
-                            asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(tmem_o + lanes + b * NH), TC_I8(r, 0),
-                                         TC_I8(r, 8)
-                                         : "memory");
+                            for (int h = 0; h < 2 * NH; ++h) r[h] *= factor[h % NH];
+                            tmem_st32(tmem_o + lanes + b * 2 * NH, r);
                         }
-                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     }
                 }
                 if (g > 0) alive = alive && bounded_wait(bar(B_PV), (g - 1) & 1, dead, p.report);          // P has been read
                 if (!alive) continue;                                 // leaves at the next meeting
-                uint8_t* pp = smem + OFF_P + (tid >> 6) * QPIECE + (tid & 7) * 2;
+                uint8_t* pp = smem + OFF_P + (tid >> 6) * PPIECE + (tid & 7) * 2;
 #pragma unroll
                 for (int h = 0; h < NH; ++h) {
                     const float pv = m_ref[h] == -INFINITY ? 0.f : fast_exp2(sc[h] - m_ref[h]);
                     l[h] += pv;
-                    *reinterpret_cast<__nv_bfloat16*>(pp + h * 128 + ((((tid & 63) >> 3) ^ (h & 7)) << 4)) = __float2bfloat16_rn(pv);
+                    const __nv_bfloat16 hi = __float2bfloat16_rn(pv);
+                    uint8_t* at = pp + h * 128 + ((((tid & 63) >> 3) ^ (h & 7)) << 4);
+                    *reinterpret_cast<__nv_bfloat16*>(at) = hi;
+                    *reinterpret_cast<__nv_bfloat16*>(at + QPIECE) = __float2bfloat16_rn(pv - __bfloat162float(hi));
                 }
                 if (key >= ctx) {                                     // a row past the context may hold anything, and 0 * NaN would poison the sum
                     const uint32_t u0 = g * units;
@@ -244,14 +246,11 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
             tc_fence_after();
             float* dst = p.part + (int64_t)(blockIdx.x + s) * p.slot;
             for (int b = 0; b < pairs; ++b) {
-                uint32_t r[NH];
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
-                             : TC_R8(r, 0), TC_R8(r, 8)
-                             : "r"(tmem_o + lanes + b * NH)
-                             : "memory");
+                float r[2 * NH];
+                tmem_ld32(tmem_o + lanes + b * 2 * NH, r);
 #pragma unroll
                 for (int h = 0; h < NH; ++h)
-                    if (h < p.H) dst[(int64_t)h * p.rank + b * 128 + tid] = __uint_as_float(r[h]);
+                    if (h < p.H) dst[(int64_t)h * p.rank + b * 128 + tid] = r[h] + r[NH + h];
             }
             tc_fence_before();
 #pragma unroll
@@ -295,7 +294,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
     } else {
         // ---- products ----
         const bool leader = elect_one();
-        constexpr uint32_t IDESC_S = make_idesc(KEYS, NH, false), IDESC_O = make_idesc(128, NH, false) | (1u << 15);      // A of the second: MN-major
+        constexpr uint32_t IDESC_S = make_idesc(KEYS, NH, false), IDESC_O = make_idesc(128, 2 * NH, false) | (1u << 15);      // A of the second: MN-major
         const uint64_t kd0 = make_desc(base, 16, 1024), qd0 = make_desc(base + OFF_Q, 16, 1024), vd0 = make_desc(base, PIECE, 1024), pd0 = make_desc(base + OFF_P, 16, 1024);
         uint32_t g = 0, u = 0, segs = 0;
         for (int t = t_begin; t < t_end; ++segs) {
@@ -327,7 +326,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
                         const uint64_t vd = vd0 + slot * (UNIT / 16);
 #pragma unroll
                         for (int q = 0; q < KEYS / 16; ++q)
-                            tc_mma(tmem_o + b * NH, vd + q * (2048 / 16), pd0 + (q >> 2) * (QPIECE / 16) + (q & 3) * 2, IDESC_O, t > seg_begin || q > 0);
+                            tc_mma(tmem_o + b * 2 * NH, vd + q * (2048 / 16), pd0 + (q >> 2) * (PPIECE / 16) + (q & 3) * 2, IDESC_O, t > seg_begin || q > 0);
                         tc_commit(bar(B_EMPTY + slot));
                     }
                     tc_commit(bar(B_PV));
@@ -341,7 +340,7 @@ leave:
         for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     tc_fence_before();
     __syncthreads();
-    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128u) : "memory");
+    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
 // out[h, s, :] = sum over the shares that hold part of sequence s, in their order; the sink counts once.  grid (n, H), a thread per four columns.  The

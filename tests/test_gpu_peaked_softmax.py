@@ -106,3 +106,23 @@ def test_latent_prompts(deviation):
     cut = lambda parts: torch.cat([torch.cat(parts[:H], 1), torch.cat(parts[H:], 1)])
     want, sim = cut(want), cut(sim)
     assert relative(got, want) <= 1.1 * relative(sim, want), (relative(got, want), relative(sim, want))
+
+
+@pytest.mark.parametrize("deviation", [1.0, 5.0])
+@pytest.mark.parametrize("lens", [[3000, 700, 129], [8000]])
+def test_latent_decode(deviation, lens):
+    """Two bf16 terms hold the weights here: what is left is the rounding of the result."""
+    from nanovllm import mixops as mx
+    H, rd, R, n = 16, 64, 512, len(lens)
+    rows, scale = bf(sum(lens), R + rd, seed=8).cuda(), deviation / (R + rd) ** 0.5
+    cache, tables = paged(rows, lens, 128, 9)
+    q_lat, q_raw = bf(H, n, R, seed=10).cuda(), bf(n, H, rd, seed=11).cuda()
+    cs = torch.cat((torch.ones(1, rd // 2), torch.zeros(1, rd // 2)), 1).expand(max(lens), -1).contiguous().cuda()
+    spans = mx.StepSpans(n, 1, None, None, torch.tensor(lens, dtype=torch.int32).cuda())
+    got = mx.latent_attention(q_lat, q_raw, 0, cache, tables, 128, spans, None, cs, scale)
+    want, at = torch.empty(H, n, R, dtype=torch.float64, device="cuda"), 0
+    for i, l in enumerate(lens):
+        c = rows[at:at + l].double()
+        want[:, i] = torch.softmax(torch.cat((q_lat[:, i], q_raw[i]), -1).double() @ c.T * scale, -1) @ c[:, :R]
+        at += l
+    assert relative(got, want) <= 1.1 * relative(rounded(want), want), (relative(got, want), relative(rounded(want), want))
