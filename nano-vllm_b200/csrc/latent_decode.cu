@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
     }
     if (tid == 128) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm) : "memory");
     B200_PDL_TRIGGER();
-    if (warp == 0) prefix_tiles(p, cum, lane);                        // lengths are uploaded before the step
-    B200_PDL_WAIT();
+    B200_PDL_WAIT();                                                  // a kernel in front may have written the lengths
+    if (warp == 0) prefix_tiles(p, cum, lane);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -350,9 +350,9 @@ __global__ void __launch_bounds__(128) latent_fold_kernel(const LatentParams p, 
     __shared__ int cum[SEQ_CAP + 1];
     __shared__ float fac[SHARES], red[4];
     const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    B200_PDL_WAIT();
     if (tid < 32) prefix_tiles(p, cum, tid);
     __syncthreads();
-    B200_PDL_WAIT();
     const int64_t total = cum[p.n];
     const int t0 = cum[s], t1 = cum[s + 1];
     if (t0 == t1) return;

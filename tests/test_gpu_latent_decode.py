@@ -49,3 +49,28 @@ def test_other_sizes_take_the_general_form(H, rank, rd, bs):
     args = (tables.cuda(), bs, mx.StepSpans(2, 1, None, None, torch.tensor(lens, dtype=torch.int32).cuda()), None, cs, 0.03)
     want = mx.latent_attention(q_lat.float(), q_raw.float(), 128, cache.float(), *args)
     assert_close_bf16(mx.latent_attention(q_lat, q_raw, 128, cache, *args), want, "general form", rel_l2=6e-3, ulps=3.0)
+
+
+@pytest.mark.parametrize("n", [1, 200])
+def test_lengths_written_by_the_kernel_in_front(n):
+    """The lengths come out of this library's own gather of rows, whose launch lets the next one begin before it has written them."""
+    from nanovllm import mixops as mx, ops
+    from nanovllm.layers.rotary_embedding import build_banded_cos_sin
+    rank, rd, H, bs, most = 256, 64, 4, 128, 2048
+    tables = torch.arange(n * most // bs, dtype=torch.int32).view(n, -1).cuda()
+    cache, q_lat, q_raw = bf(most * n, rank + rd, seed=58).cuda(), bf(H, n, rank, seed=59).cuda(), bf(n, H, rd, seed=60).cuda()
+    cs = build_banded_cos_sin(rd, most, 1e4, None, "cuda")
+    g = torch.Generator().manual_seed(61)
+    rows = 1 << 18                                                       # the step's lengths are the last of many rows: they are written late
+    for turn in range(3):
+        lens = torch.randint(1, most, (n,), generator=g, dtype=torch.int32).cuda()
+        held = torch.zeros(rows * 8 + (n + 7) // 8 * 8, dtype=torch.int32, device="cuda")
+        source = torch.zeros_like(held)
+        source[rows * 8:rows * 8 + n] = lens
+        ids = torch.arange(held.numel() // 8, device="cuda")
+        spans = lambda t: mx.StepSpans(n, 1, None, None, t)
+        want = mx.latent_attention(q_lat, q_raw, 0, cache, tables, bs, spans(lens), None, cs, 0.03)
+        torch.cuda.synchronize()
+        ops.embedding(ids, source.view(torch.bfloat16).view(-1, 16), out=held.view(torch.bfloat16).view(-1, 16))
+        got = mx.latent_attention(q_lat, q_raw, 0, cache, tables, bs, spans(held[rows * 8:rows * 8 + n]), None, cs, 0.03)
+        assert torch.equal(got, want)

@@ -98,3 +98,12 @@ def test_loads_of_the_libraries_write_their_own_cta_only():
     for f in files:
         for line in open(f):
             assert not re.search(r"cp\.async\.bulk.*multicast", line), (f, line)
+
+
+def test_latent_decode_reads_lengths_after_the_kernel_in_front():
+    """A launch may begin before the kernel in front has written: whatever walks the lengths stands behind the dependency wait."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nano-vllm_b200", "csrc")
+    kernels = open(os.path.join(csrc, "latent_decode.cu")).read().split("__global__")[1:]
+    assert len(kernels) == 2
+    for k in kernels:
+        assert 0 < k.index("B200_PDL_WAIT()") < k.index("prefix_tiles(p")
