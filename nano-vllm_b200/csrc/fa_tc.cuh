@@ -603,9 +603,9 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 int row = it.k0 + key0;
                 if (p.block_tables && lane < boxes) {
                     const int key = key0 + lane * p.box_rows;
-                    int page = key < it.len_k ? p.block_tables[(int64_t)it.seq * p.bt_stride + key / p.block_size] : 0;
-                    page = page < 0 ? 0 : page;
-                    row = (int)(p.row0 + page * p.page_rows + it.kvh * p.head_rows + key % p.block_size);
+                    const int page = key < it.len_k ? p.block_tables[(int64_t)it.seq * p.bt_stride + key / p.block_size] : -1;
+                    // no page (below a window, past the keys): a box outside the map, which reads as zeros
+                    row = page < 0 ? -p.box_rows : (int)(p.row0 + page * p.page_rows + it.kvh * p.head_rows + key % p.block_size);
                 }
                 if (!fa_wait(bar(B_KEMPTY + sl.i), sl.ph ^ 1)) goto leave;
                 if (lane == 0) mbar_expect_tx(bar(B_KFULL + sl.i), L::kKBytes);

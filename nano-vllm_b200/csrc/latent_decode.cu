@@ -275,9 +275,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_decode_kernel(const __grid_
                 int row = 0;
                 if (lane < boxes) {
                     const int key = (t + tile0) * KEYS + lane * p.box_rows;
-                    int page = key < ctx ? p.block_tables[(int64_t)s * p.bt_stride + key / p.block_size] : 0;
-                    page = page < 0 ? 0 : page;
-                    row = page * p.block_size + key % p.block_size;
+                    const int page = key < ctx ? p.block_tables[(int64_t)s * p.bt_stride + key / p.block_size] : -1;
+                    row = page < 0 ? -p.box_rows : page * p.block_size + key % p.block_size;      // no page: outside the map, zeros
                 }
                 for (int k = 0; k < units; ++k, ++u) {
                     const uint32_t slot = u % UNITS;

@@ -74,3 +74,22 @@ def test_lengths_written_by_the_kernel_in_front(n):
         ops.embedding(ids, source.view(torch.bfloat16).view(-1, 16), out=held.view(torch.bfloat16).view(-1, 16))
         got = mx.latent_attention(q_lat, q_raw, 0, cache, tables, bs, spans(held[rows * 8:rows * 8 + n]), None, cs, 0.03)
         assert torch.equal(got, want)
+
+
+def test_pages_below_the_window_may_be_absent():
+    from nanovllm import mixops as mx
+    from nanovllm.layers.rotary_embedding import build_banded_cos_sin
+    H, rank, rd, bs, window, lens = 4, 256, 64, 16, 100, [700, 391, 60]
+    nblk = sum(-(-c // bs) for c in lens)
+    cache = bf((nblk + 1) * bs, rank + rd, seed=62).cuda()
+    cache[:bs] = float("nan")
+    tables = make_tables(lens, bs, nblk, seed=63)
+    tables[tables >= 0] += 1
+    q_lat, q_raw = bf(H, 3, rank, seed=64).cuda(), bf(3, H, rd, seed=65).cuda()
+    cs = build_banded_cos_sin(rd, 1024, 1e4, None, "cuda")
+    spans = mx.StepSpans(3, 1, None, None, torch.tensor(lens, dtype=torch.int32).cuda())
+    call = lambda t: mx.latent_attention(q_lat, q_raw, 0, cache, t.cuda(), bs, spans, None, cs, 0.03, window=window)
+    want = call(tables)
+    for i, l in enumerate(lens):
+        tables[i, :max(l - window, 0) // bs] = -1
+    assert torch.equal(call(tables), want) and torch.isfinite(want).all()

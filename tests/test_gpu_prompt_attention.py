@@ -193,3 +193,21 @@ def test_rotation_in_place(mx, dims, off, layout):
     keep = torch.ones(192, dtype=torch.bool)
     keep[off:off + dims] = False
     assert torch.equal(q[..., keep.cuda()].double(), want[..., keep.cuda()])
+
+
+@pytest.mark.parametrize("bs,window", [(16, 100), (32, 7)])
+def test_pages_below_the_window_may_be_absent(mx, bs, window):
+    """Table entries of pages that no query sees are -1 and whatever page 0 holds (NaN here) stays out: bit for bit the result with all pages there."""
+    heads, kv_heads, len_q, len_k = 4, 2, [40, 130], [700, 391]
+    nblk = sum(-(-c // bs) for c in len_k)
+    cache = bf((nblk + 1) * bs, kv_heads * 256, seed=70).cuda()
+    cache[:bs] = float("nan")
+    tables = make_tables(len_k, bs, nblk, seed=71)
+    tables[tables >= 0] += 1                                             # page 0 belongs to nobody
+    q = bf(sum(len_q), heads * 128, seed=72).cuda()
+    call = lambda t: mx.window_attention(q, cache, t.cuda(), bs, spans_of(mx, len_q, len_k), heads, kv_heads, 128, 128, 128 ** -0.5, window=window)
+    want = call(tables)
+    assert torch.isfinite(want).all()
+    for i, (n, l) in enumerate(zip(len_q, len_k)):
+        tables[i, :(l - n - window + 1) // bs] = -1
+    assert torch.equal(call(tables), want)
