@@ -101,6 +101,10 @@ int b200_paged_decode(b200_ctx* ctx, int layer, const void* q, int64_t q_stride0
                       void* out, int64_t out_stride0, int batch, int num_q_heads, float scale,
                       void* workspace, size_t workspace_bytes, void* stream);
 
+/* How b200_paged_decode(_fused) would run a step of `batch` rows with block tables of bt_stride columns: the CTAs that share a context in the kernel
+ * for small steps (1, 2, 4 or 8), 0 for the other kernels, or a negative code.  Depends on these numbers, the bound cache and the device alone. */
+int b200_decode_small_splits(const b200_ctx* ctx, int batch, int num_q_heads, int bt_stride);
+
 /* One-launch decode layer front end: what Qwen3Attention.forward does between the qkv GEMM and o_proj for a decode
  * step (models/qwen3.py:77-86 + layers/attention.py:62-63,71-74): q_norm / k_norm (RMSNorm over head_dim, rounded
  * to bf16), NeoX RoPE at position context_lens[b]-1 (cos_sin: fp32 [max_pos, head_dim] = cat(cos, sin)), the step's

@@ -286,20 +286,35 @@ int launch_small(b200_ctx* ctx, const DecodeParams& prm, int G, int splits, cuda
 
 }  // namespace
 
-// Called from decode_common() in decode_attn.cu; B200_EUNSUPPORTED: a step for the stream-K kernels.
+// CTAs along a context (1, 2, 4 or 8: the cluster), or 0: a step for the stream-K kernels.
 //
 // Taken while every (sequence, kv head) has a CTA of its own in one wave and no warp can get more than MAX_CHUNKS chunks, whatever the contexts
 // are (bounded by the table's width; the lengths are on the device).  A chunk takes a warp about 0.75 us (twice that with four heads), so the
-// longest context allowed ends no later than the stream-K kernels do on the smallest step.  Measured (whole captured Qwen3-0.6B
-// step, us, here / stream-K): 1 row 980 / 1323, 4 rows 1040 / 1330, 16 rows of up to 1024 tokens 1195 / 1362; beyond the bound (the operator alone) 16 rows of
-// 600-8192 tokens 78 / 52, with 32 heads 112 / 56.
-int b200_decode_small_launch(b200_ctx* ctx, const DecodeParams& prm, int G, bool fused, cudaStream_t stream) {
-    const int GW = G >= 4 ? 4 : G, ctas = prm.batch * prm.hkv * (G / GW), MAX_CHUNKS = GW == 4 ? 4 : 16;
-    if (ctas > ctx->sm_count) return B200_EUNSUPPORTED;
+// longest context allowed ends no later than the stream-K kernels do on the smallest step.  A captured step's tables are as wide as the longest
+// sequence the engine may hold, so that length decides there: with 8 kv heads in groups of two, 1 and 2 rows take this kernel up to 16384 tokens, 4 rows
+// up to 8192, 8 up to 4096, 9-18 up to 2048.  Measured (whole captured Qwen3-0.6B step, us, here / stream-K): 1 row 980 / 1323, 4 rows 1040 / 1330, 16
+// rows with tables of 1024 tokens 1195 / 1362; beyond the bound (the operator alone) 16 rows of 600-8192 tokens 78 / 52, with 32 heads 112 / 56.
+static int small_splits(const b200_ctx* ctx, int batch, int G, int bt_stride) {
+    const int GW = G >= 4 ? 4 : G, ctas = batch * ctx->num_kv_heads * (G / GW), MAX_CHUNKS = GW == 4 ? 4 : 16;
+    if (ctas > ctx->sm_count) return 0;
     int splits = 1;
     while (splits < 8 && ctas * splits * 2 <= ctx->sm_count) splits *= 2;
-    const int64_t chunks = ((int64_t)prm.bt_stride << prm.block_shift) / CHUNK;
-    if (chunks > (int64_t)MAX_CHUNKS * SW * splits) return B200_EUNSUPPORTED;
+    const int64_t chunks = ((int64_t)bt_stride << ctx->block_shift) / CHUNK;
+    return chunks > (int64_t)MAX_CHUNKS * SW * splits ? 0 : splits;
+}
+
+extern "C" int b200_decode_small_splits(const b200_ctx* ctx, int batch, int num_q_heads, int bt_stride) {
+    if (!ctx || batch <= 0 || bt_stride < 0 || num_q_heads <= 0) return B200_EINVAL;
+    if (!ctx->k_base) return B200_ENOTBOUND;
+    const int G = num_q_heads % ctx->num_kv_heads ? 0 : num_q_heads / ctx->num_kv_heads;
+    if (G != 1 && G != 2 && G != 4 && G != 8) return B200_EUNSUPPORTED;
+    return small_splits(ctx, batch, G, bt_stride);
+}
+
+// Called from decode_common() in decode_attn.cu; B200_EUNSUPPORTED: a step for the stream-K kernels.
+int b200_decode_small_launch(b200_ctx* ctx, const DecodeParams& prm, int G, bool fused, cudaStream_t stream) {
+    const int GW = G >= 4 ? 4 : G, splits = small_splits(ctx, prm.batch, G, prm.bt_stride);
+    if (splits == 0) return B200_EUNSUPPORTED;
     if (fused) return GW == 1 ? launch_small<1, true>(ctx, prm, G, splits, stream) : launch_small<2, true>(ctx, prm, G, splits, stream);
     switch (GW) {
         case 1: return launch_small<1, false>(ctx, prm, G, splits, stream);
