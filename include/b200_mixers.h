@@ -141,19 +141,22 @@ int b200m_latent_decode(const void* q_lat, const void* q_raw, int64_t q_tok_stri
 
 /* Prompt portions with keys and values formed per head (bf16; B200_EUNSUPPORTED for other sizes than dim 128, rot_dim 64, vdim 128 or operands that
  * are not 16-byte aligned): one gather, one GEMM of the caller's, one rotation, one attention launch.
- *   gather: out[cu_k[s] + j] = the cached row of token j of sequence s (rows of row_elems elements; max_k: an upper bound of any sequence's tokens;
- *           rows from out_rows on are dropped);
+ *   visible: with a window, cu_rows[s] (num_seqs + 1) = the keys of the sequences before s that some query of theirs sees (those from window - 1 before
+ *           the first query on); without one all are seen and cu_rows is cu_k;
+ *   gather: out rows [cu_rows[s], cu_rows[s + 1]) = the cached rows of that many tokens at the end of sequence s (rows of row_elems elements; a
+ *           page that is absent, -1, gives zeros; rows from out_rows on are dropped);
  *   rotate: q[t, h, 0 .. rope_dims) (token stride, head stride) turned by positions[t], in place;
- *   prompt: q [total_q, heads, dim + rot_dim] (row stride q_stride), rotated; keys and values [total_k, heads * 128] (row stride kv_stride) of the gathered
+ *   prompt (any consecutive heads): q [total_q, heads, dim + rot_dim] (row stride q_stride), rotated; keys and values [total_k, heads * 128] (row stride kv_stride) of the gathered
  *           rows, whose columns rank .. rank + rot_dim are the key part all heads share; causal at the end of each sequence's keys, sink and window as
- *           above; out [total_q, heads * vdim]. */
-int b200m_latent_gather(const void* cache, int row_elems, const int32_t* block_tables, int bt_stride, int block_size, const int32_t* cu_k, int num_seqs,
-                        int max_k, void* out, int out_rows, void* stream);
+ *           above, with cu_rows for cu_k; out [total_q, heads * vdim] (row stride out_stride). */
+int b200m_latent_visible(const int32_t* cu_q, const int32_t* cu_k, int num_seqs, int window, int32_t* cu_rows, void* stream);
+int b200m_latent_gather(const void* cache, int row_elems, const int32_t* block_tables, int bt_stride, int block_size, const int32_t* cu_k, const int32_t* cu_rows,
+                        int num_seqs, void* out, int out_rows, void* stream);
 int b200m_latent_rotate(void* q, int64_t tok_stride, int head_stride, const float* cos_sin, int rope_dims, const int64_t* positions, int n, int heads,
                         int layout, void* stream);
 int b200m_latent_prompt(const void* q, int64_t q_stride, const void* keys, const void* values, int64_t kv_stride, const void* rows, int row_elems, int rank,
-                        int total_k, const int32_t* cu_q, const int32_t* cu_k, const float* sink, void* out, int total_q, int num_seqs, int max_q,
-                        int heads, int dim, int rot_dim, int vdim, float scale, int window, void* stream);
+                        int total_k, const int32_t* cu_q, const int32_t* cu_k, const float* sink, void* out, int64_t out_stride, int total_q, int num_seqs,
+                        int max_q, int heads, int dim, int rot_dim, int vdim, float scale, int window, void* stream);
 
 /* ---- windowed grouped-query attention ------------------------------------------------------------------------------ */
 

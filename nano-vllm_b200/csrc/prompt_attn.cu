@@ -17,18 +17,64 @@ constexpr uint64_t ANY_ROWS = (1ull << 31) - 1;
 // Pages the kernel's boxes can follow: a block of 64 keys is whole pages, or lies inside one.
 bool pages_ok(int block_size) { return block_size % BN == 0 || (block_size >= 8 && BN % block_size == 0); }
 
-// The cached rows of every sequence, one after the other: out[cu_k[s] + j] = cache row of token j of sequence s.  A warp per row, 16-byte pieces.
+// The last rows of every sequence, one sequence after the other: out[i] for i in [cu_rows[s], cu_rows[s + 1]) are the cached rows of that many tokens at the
+// end of sequence s.  A warp per row, 16-byte pieces.
 __global__ void __launch_bounds__(256) latent_gather_kernel(const uint4* __restrict__ cache, int pieces, const int32_t* __restrict__ block_tables, int bt_stride,
-                                                            int block_size, const int32_t* __restrict__ cu_k, uint4* __restrict__ out, int out_rows) {
+                                                            int block_size, const int32_t* __restrict__ cu_k, const int32_t* __restrict__ cu_rows, int num_seqs,
+                                                            uint4* __restrict__ out, int out_rows) {
     B200_PDL_SYNC();
-    const int s = blockIdx.y, j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int k0 = cu_k[s], len = cu_k[s + 1] - k0;
-    if (j >= len || k0 + j >= out_rows) return;
-    int page = block_tables[(int64_t)s * bt_stride + j / block_size];
-    page = page < 0 ? 0 : page;
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= out_rows || i >= cu_rows[num_seqs]) return;
+    int s = 0;                                                           // the last sequence that begins at or before row i
+    for (int hi = num_seqs; hi - s > 1;) {
+        const int mid = (s + hi) >> 1;
+        if (cu_rows[mid] <= i) s = mid;
+        else hi = mid;
+    }
+    const int j = cu_k[s + 1] - cu_k[s] - (cu_rows[s + 1] - i);          // token of the sequence
+    const int page = block_tables[(int64_t)s * bt_stride + j / block_size];
     const uint4* src = cache + ((int64_t)page * block_size + j % block_size) * pieces;
-    uint4* dst = out + (int64_t)(k0 + j) * pieces;
-    for (int c = lane; c < pieces; c += 32) dst[c] = src[c];
+    uint4* dst = out + (int64_t)i * pieces;
+    for (int c = lane; c < pieces; c += 32) dst[c] = page < 0 ? make_uint4(0, 0, 0, 0) : src[c];
+}
+
+// cu_rows[s] = sum over the sequences before s of the keys that some query of theirs sees: all up to `window` - 1 before the first query.  One CTA.
+__global__ void __launch_bounds__(1024) latent_visible_kernel(const int32_t* __restrict__ cu_q, const int32_t* __restrict__ cu_k, int num_seqs, int window,
+                                                              int32_t* __restrict__ cu_rows) {
+    B200_PDL_SYNC();
+    __shared__ int sums[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int at = 0;
+    for (int s0 = 0; s0 < num_seqs; s0 += 1024) {
+        const int s = s0 + tid;
+        int len = 0;
+        if (s < num_seqs) {
+            const int n = cu_q[s + 1] - cu_q[s];
+            len = n > 0 ? min(cu_k[s + 1] - cu_k[s], n + window - 1) : 0;
+        }
+        int inc = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        if (lane == 31) sums[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            int v = sums[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += u;
+            }
+            sums[lane] = v;
+        }
+        __syncthreads();
+        if (s < num_seqs) cu_rows[s] = at + inc - len + (warp ? sums[warp - 1] : 0);
+        at += sums[31];
+        __syncthreads();
+    }
+    if (tid == 0) cu_rows[num_seqs] = at;
 }
 
 // The rotated part of every head's query, in place: a thread per V pairs (V = 4: 16-byte (layout 0) or 8-byte (layout 1) accesses; a pair per thread
@@ -127,13 +173,19 @@ int b200m_window_prompt(const void* q, int64_t q_stride, const void* cache, int 
     return plain ? fa_launch<D, false, false>(p, tq, tk, tk, tk, total_q, max_q, stream) : fa_launch<D, false, true>(p, tq, tk, tk, tk, total_q, max_q, stream);
 }
 
-extern "C" int b200m_latent_gather(const void* cache, int row_elems, const int32_t* block_tables, int bt_stride, int block_size, const int32_t* cu_k, int num_seqs,
-                                   int max_k, void* out, int out_rows, void* stream) {
-    if (!cache || !block_tables || !cu_k || !out || row_elems <= 0 || block_size <= 0 || num_seqs < 0 || out_rows < 0) return B200_EINVAL;
-    if (row_elems % 8 || (reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) % 16 || num_seqs > 65535) return B200_EUNSUPPORTED;
-    if (num_seqs == 0 || max_k <= 0 || out_rows == 0) return B200_OK;
-    B200_LAUNCH((latent_gather_kernel), dim3((max_k + 7) / 8, num_seqs), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(cache), row_elems / 8,
-                block_tables, bt_stride, block_size, cu_k, static_cast<uint4*>(out), out_rows);
+extern "C" int b200m_latent_visible(const int32_t* cu_q, const int32_t* cu_k, int num_seqs, int window, int32_t* cu_rows, void* stream) {
+    if (!cu_q || !cu_k || !cu_rows || num_seqs < 0 || window <= 0) return B200_EINVAL;
+    B200_LAUNCH((latent_visible_kernel), 1, 1024, 0, static_cast<cudaStream_t>(stream), cu_q, cu_k, num_seqs, window, cu_rows);
+    return b200_launch_status(nullptr);
+}
+
+extern "C" int b200m_latent_gather(const void* cache, int row_elems, const int32_t* block_tables, int bt_stride, int block_size, const int32_t* cu_k, const int32_t* cu_rows,
+                                   int num_seqs, void* out, int out_rows, void* stream) {
+    if (!cache || !block_tables || !cu_k || !cu_rows || !out || row_elems <= 0 || block_size <= 0 || num_seqs < 0 || out_rows < 0) return B200_EINVAL;
+    if (row_elems % 8 || (reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) % 16) return B200_EUNSUPPORTED;
+    if (num_seqs == 0 || out_rows == 0) return B200_OK;
+    B200_LAUNCH((latent_gather_kernel), (out_rows + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(cache), row_elems / 8, block_tables,
+                bt_stride, block_size, cu_k, cu_rows, num_seqs, static_cast<uint4*>(out), out_rows);
     return b200_launch_status(nullptr);
 }
 
@@ -154,12 +206,12 @@ extern "C" int b200m_latent_rotate(void* q, int64_t tok_stride, int head_stride,
 }
 
 extern "C" int b200m_latent_prompt(const void* q, int64_t q_stride, const void* keys, const void* values, int64_t kv_stride, const void* rows, int row_elems, int rank,
-                                   int total_k, const int32_t* cu_q, const int32_t* cu_k, const float* sink, void* out, int total_q, int num_seqs, int max_q,
+                                   int total_k, const int32_t* cu_q, const int32_t* cu_k, const float* sink, void* out, int64_t out_stride, int total_q, int num_seqs, int max_q,
                                    int heads, int dim, int rot_dim, int vdim, float scale, int window, void* stream) {
     if (!q || !keys || !values || !rows || !cu_q || !cu_k || !out || total_q < 0 || num_seqs < 0 || heads <= 0 || rank <= 0 || total_k < 0) return B200_EINVAL;
     const uintptr_t bases = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(values) |
                             reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out);
-    if (dim != 128 || rot_dim != 64 || vdim != 128 || scale <= 0.f || bases % 16 || q_stride % 8 || kv_stride % 8 || row_elems % 8 || rank % 8) return B200_EUNSUPPORTED;
+    if (dim != 128 || rot_dim != 64 || vdim != 128 || scale <= 0.f || bases % 16 || q_stride % 8 || out_stride % 8 || kv_stride % 8 || row_elems % 8 || rank % 8) return B200_EUNSUPPORTED;
     if (total_q == 0 || num_seqs == 0 || max_q <= 0) return B200_OK;
     CUtensorMap tq, tk, tv, tr;
     if (!make_map(&tq, q, (uint64_t)heads * 192, (uint64_t)total_q, (uint64_t)q_stride, BM) || !make_map(&tk, keys, (uint64_t)heads * 128, (uint64_t)total_k, (uint64_t)kv_stride, BN) ||
@@ -179,7 +231,7 @@ extern "C" int b200m_latent_prompt(const void* q, int64_t q_stride, const void* 
     p.sinks = sink;
     p.window = window;
     p.out = out;
-    p.out_stride = (int64_t)heads * vdim;
+    p.out_stride = out_stride;
     p.out_scale = 1.0f;
     return fa_launch<192, false, false>(p, tq, tk, tv, tr, total_q, max_q, static_cast<cudaStream_t>(stream));
 }

@@ -84,9 +84,10 @@ MIX_SIGNATURES = {
     "b200m_latent_store": (_i, [_vp, _i64, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _vp]),
     "b200m_latent_decode_workspace_bytes": (_sz, [_i, _i, _i]),
     "b200m_latent_decode": (_i, [_vp, _vp, _i64, _i, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _vp, _sz, _vp]),
-    "b200m_latent_gather": (_i, [_vp, _i, _vp, _i, _i, _vp, _i, _i, _vp, _i, _vp]),
+    "b200m_latent_visible": (_i, [_vp, _vp, _i, _i, _vp, _vp]),
+    "b200m_latent_gather": (_i, [_vp, _i, _vp, _i, _i, _vp, _vp, _i, _vp, _i, _vp]),
     "b200m_latent_rotate": (_i, [_vp, _i64, _i, _vp, _i, _vp, _i, _i, _i, _vp]),
-    "b200m_latent_prompt": (_i, [_vp, _i64, _vp, _vp, _i64, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp]),
+    "b200m_latent_prompt": (_i, [_vp, _i64, _vp, _vp, _i64, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp]),
     "b200m_latent_attention": (_i, [_vp, _vp, _i64, _i, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i,
                                     _f, _i, _i, _i, _i, _i, _vp, _vp]),
     "b200m_causal_conv": (_i, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]),

@@ -248,7 +248,11 @@ class ModelRunner:
             for i, s in enumerate(seqs):
                 s.block_table = list(range(i * per, (i + 1) * per))
                 s.state_slot = i
+        # what a prompt step over long cached prefixes holds beside these activations counts as peak too
+        scratch = getattr(self.model, "prompt_scratch_bytes", lambda rows: 0)(cfg.max_num_seqs * cfg.max_model_len)
+        held = torch.empty(scratch, dtype=torch.uint8, device=self.device)
         self.run(seqs, True)
+        del held
         if self.owns_cache:
             self.model.unbind_cache()
         torch.cuda.empty_cache()
@@ -380,7 +384,7 @@ class ModelRunner:
             bt = bt.view(len(seqs), -1)
         slot = views["slot_mapping"] if a["slot_mapping"].size else None
         set_context(True, views["cu_seqlens_q"], views["cu_seqlens_k"], a["max_seqlen_q"], a["max_seqlen_k"],
-                    slot, None, bt, views.get("state_slots"), views.get("logit_rows"))
+                    slot, None, bt, views.get("state_slots"), views.get("logit_rows"), int(a["cu_seqlens_k"][-1]))
         return views["input_ids"], views["positions"], views["temps"], views["step"]
 
     def _padded_rows(self, n: int) -> int:

@@ -76,6 +76,10 @@ class LatentAttention:
             return False
         return True
 
+    def prompt_scratch_bytes(self, rows: int) -> int:
+        """Most bytes a prompt step of at most ``rows`` cached tokens holds beside its activations."""
+        return mixops.latent_scratch_bytes(self.heads, self.dim, self.vdim, self.kv_rank + self.rot_dim, rows) if self.dtype == torch.bfloat16 else 0
+
     def cache_row_elems(self) -> int:
         """Cached elements per token (0 for a layer that borrows another layer's cache)."""
         return 0 if self.kv_from is not None else self.kv_rank + self.rot_dim
@@ -169,6 +173,9 @@ class GatedWindowLatentAttention:
         return {"q": (self.q_cols, width), "dkv": (self.kv_cols, width), "dkv.norm": (R,), "uk": (H * self.dim, R), "uv": (H * self.vdim, R),
                 "g": (self.g_cols, width), "o": (width, H * self.vdim)}
 
+    def prompt_scratch_bytes(self, rows: int) -> int:
+        return mixops.latent_scratch_bytes(self.heads, self.dim, self.vdim, self.kv_cols, rows) if self.dtype == torch.bfloat16 else 0
+
     def cache_row_elems(self) -> int:
         return self.kv_cols
 
@@ -190,7 +197,7 @@ class GatedWindowLatentAttention:
         cache = self.cache[inst]
         mixops.latent_store(proj[:, self.q_cols:], self.kv_norm, self.cos_sin, positions, ctx.slot_mapping, cache, R, rd, self.eps,
                             layout=mixops.ROT_HALVES)
-        if mixops.latent_expands(q, d, rd, self.vdim, R, self.scale, cache, ctx.block_tables, self.block_size, spans):
+        if mixops.latent_expands(q, d, rd, self.vdim, R, self.scale, cache, ctx.block_tables, self.block_size, spans, self.window):
             o = mixops.latent_prompt(q, self.w_ukv, d, self.vdim, cache, ctx.block_tables, self.block_size, spans, None, self.cos_sin, positions, self.scale,
                                      window=self.window, layout=mixops.ROT_HALVES).view(n, H, self.vdim)
         else:

@@ -19,7 +19,8 @@ from . import ops
 class StepSpans:
     """Which tokens of a step belong to which sequence, in the two forms the kernels take.
 
-    varlen step:  cu_q, cu_k int32 [S + 1] (cumulative tokens of this step / tokens held after it), max_q on the host
+    varlen step:  cu_q, cu_k int32 [S + 1] (cumulative tokens of this step / tokens held after it), max_q on the host; max_k and total_k, the
+                  longest and the sum of the tokens held after it, where the host knows them (0: it does not, and table widths bound them)
     decode step:  ctx_lens int32 [S] (tokens held after the step, 0 = padding row), one token per row
     """
     num_seqs: int
@@ -27,6 +28,8 @@ class StepSpans:
     cu_q: torch.Tensor | None = None
     cu_k: torch.Tensor | None = None
     ctx_lens: torch.Tensor | None = None
+    max_k: int = 0
+    total_k: int = 0
 
 
 def _is32(t: torch.Tensor) -> int:
@@ -326,45 +329,93 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, q_rot_off: int, c
     return out
 
 
-# Keys and values formed per head pay from a few queries per sequence on: forming them costs 2 * 2 * rank * 128 operations per head and cached row on the
-# library's GEMM, and saves attention over the latents at 87 TFLOP/s.  Measured (width 2048, 16 heads, layer, us, formed against latents): 1 x 4 queries over
-# 2048 rows 127 / 301, 8 x 4 over 2048 149 / 327, 16 x 4 over 4000 460 / 518, 8 x 64 over 2048 160 / 416, 4 x 2048 354 / 3627.
-LATENT_EXPAND_QUERIES = 4
-LATENT_EXPAND_ROWS = 1 << 17          # most rows whose keys and values are held at once (16 heads: 1 GiB)
+# Prompt portions of latent attention have two forms: keys and values formed per head for every key that some query sees (latent_prompt), or attention over
+# the latents themselves (latent_attention).  ``latent_costs`` estimates both and the
+# cheaper one runs; only numbers that the host has enter, so a step whose lengths it does not know is taken at the width of its tables.
+LATENT_ROWS_BYTES = 1 << 29          # most bytes of gathered rows; longer steps take the latents
+LATENT_KV_BYTES = 1 << 29            # most bytes of formed keys and values held at once: more of them are formed a few heads at a time
+
+
+def _latent_rows(n: int, block_tables: torch.Tensor, block_size: int, spans: StepSpans, window: int) -> tuple[int, int]:
+    """Keys that the queries of a step see, over all sequences and for the longest one: exact where the host knows the lengths and no window cuts them, else
+    upper bounds."""
+    width = block_tables.shape[1] * block_size
+    most = min(spans.max_k, width) if spans.max_k else width
+    total = min(spans.total_k, spans.num_seqs * most) if spans.total_k else spans.num_seqs * most
+    if window > 0:
+        most, total = min(most, spans.max_q + window - 1), min(total, n + spans.num_seqs * (window - 1))
+    return total, most
 
 
 def latent_expands(q: torch.Tensor, dim: int, rot_dim: int, vdim: int, rank: int, scale: float, cache: torch.Tensor, block_tables: torch.Tensor,
-                   block_size: int, spans: StepSpans) -> bool:
-    """Whether a step's latent attention forms keys and values per head (``latent_prompt``): prompt portions of the sizes that kernel takes."""
-    n = q.shape[0]
-    return (spans.cu_q is not None and q.dtype == torch.bfloat16 and (dim, rot_dim, vdim) == (128, 64, 128) and scale > 0 and rank % 8 == 0
-            and n >= LATENT_EXPAND_QUERIES * spans.num_seqs and spans.num_seqs * block_tables.shape[1] * block_size <= LATENT_EXPAND_ROWS
-            and spans.num_seqs < 65536 and q.stride(0) % 8 == 0 and q.stride(2) == 1 and q.stride(1) == dim + rot_dim
-            and (q.data_ptr() | cache.data_ptr()) % 16 == 0)
+                   block_size: int, spans: StepSpans, window: int = 0) -> bool:
+    """Whether a step's latent attention forms keys and values per head (``latent_prompt``): prompt portions of the sizes that kernel takes, where that
+    is the smaller work."""
+    n, H = q.shape[:2]
+    if not (spans.cu_q is not None and q.dtype == torch.bfloat16 and (dim, rot_dim, vdim) == (128, 64, 128) and scale > 0 and rank % 8 == 0 and n > 0
+            and q.stride(0) % 8 == 0 and q.stride(2) == 1 and q.stride(1) == dim + rot_dim and (q.data_ptr() | cache.data_ptr()) % 16 == 0):
+        return False
+    rows, most = _latent_rows(n, block_tables, block_size, spans, window)
+    if rows * (rank + rot_dim) * 2 > LATENT_ROWS_BYTES:
+        return False
+    formed, latents = latent_costs(n, H, rank, spans.num_seqs, rows, most)
+    return formed < latents
+
+
+def latent_costs(n: int, heads: int, rank: int, seqs: int, rows: int, most: int) -> tuple[float, float]:
+    """Microseconds of the two forms of a prompt step of ``n`` tokens in ``seqs`` sequences that see ``rows`` keys, the longest ``most`` (a B200).
+
+    Formed: per key the GEMM's 512 * heads * rank operations at 1.4 PFLOP/s and 512 bytes per head written and read again, and the longest sequence's blocks of
+    64 keys one after the other.  Over the latents: CTAs of 64 (token, head) rows per 256 latent columns, each a chain over its keys; many of them share
+    the chip.  Measured, formed / latents, 16 heads at rank 512: 1 x 4 queries over 2048 keys 57 / 269, 16 x 4 over 2048 201 / 267, 32 x 4 over 2048 378 / 296,
+    64 x 4 over 2048 728 / 305, 64 x 32 over 2048 734 / 1602, 64 x 8 over 512 205 / 175, 64 x 16 over 512 205 / 346; rank 256: 64 x 16 over 512 166 / 123,
+    64 x 32 over 512 166 / 239, 16 x 4 over 8192 558 / 514; 4 heads at rank 512: 64 x 4 over 2048 242 / 234, 64 x 16 over 2048 244 / 305."""
+    formed = 30.0 + rows * (heads * rank * 3.75e-7 + heads * 1.25e-4 + 2e-4) + most / 64 * 0.7
+    wide, chunks = (rank + 64) / 320, -(-rank // 256)
+    tiles, mean = max(seqs, n * heads / 64), rows / max(seqs, 1)
+    return formed, max(40.0 + wide * (33.0 + 0.05 * most), chunks * wide * tiles * (0.2 + 3.4e-4 * mean))
+
+
+def latent_scratch_bytes(heads: int, dim: int, vdim: int, row: int, rows: int) -> int:
+    """Most bytes that ``latent_prompt`` holds beside its inputs and result, in a step of at most ``rows`` keys."""
+    return min(rows * row * 2, LATENT_ROWS_BYTES) + min(rows * heads * (dim + vdim) * 2, max(LATENT_KV_BYTES, min(rows * row * 2, LATENT_ROWS_BYTES) // row * (dim + vdim)))
 
 
 def latent_prompt(q: torch.Tensor, w_ukv: torch.Tensor, dim: int, vdim: int, cache: torch.Tensor, block_tables: torch.Tensor, block_size: int,
                   spans: StepSpans, sink: torch.Tensor | None, cos_sin: torch.Tensor, positions: torch.Tensor, scale: float, window: int = 0,
                   layout: int = ROT_PAIRS) -> torch.Tensor:
-    """q [n, H, dim + rot_dim] (its rotated part is turned in place), w_ukv [H * dim + H * vdim, rank] -> [n, H * vdim]: the cached rows of the step's
-    sequences are gathered, every head's keys and values formed from their latents by one GEMM, and attention runs over those."""
+    """q [n, H, dim + rot_dim] (its rotated part is turned in place), w_ukv [H * dim + H * vdim, rank] -> [n, H * vdim]: the cached rows that the step's
+    queries see are gathered, every head's keys and values formed from their latents by a GEMM, and attention runs over those."""
     n, H, qd = q.shape
     row = cache.shape[-1]
     rank = row - (qd - dim)
     assert cache.is_contiguous() and w_ukv.is_contiguous() and w_ukv.shape == (H * (dim + vdim), rank) and block_tables.stride(1) == 1
     assert positions.dtype == torch.int64 and cos_sin.dtype == torch.float32 and block_tables.dtype == torch.int32
-    max_k = block_tables.shape[1] * block_size
-    total = spans.num_seqs * max_k                    # an upper bound known without asking the device
+    S = spans.num_seqs
+    total, _ = _latent_rows(n, block_tables, block_size, spans, window)
+    cu_rows = spans.cu_k
+    if window > 0:
+        cu_rows = torch.empty(S + 1, dtype=torch.int32, device=q.device)
+        _call("b200m_latent_visible", spans.cu_q.data_ptr(), spans.cu_k.data_ptr(), S, int(window), cu_rows.data_ptr(), _stream())
     rows = torch.empty(total, row, dtype=cache.dtype, device=cache.device)
-    _call("b200m_latent_gather", cache.data_ptr(), row, block_tables.data_ptr(), block_tables.stride(0), block_size, spans.cu_k.data_ptr(), spans.num_seqs,
-          max_k, rows.data_ptr(), total, _stream())
+    _call("b200m_latent_gather", cache.data_ptr(), row, block_tables.data_ptr(), block_tables.stride(0), block_size, spans.cu_k.data_ptr(), cu_rows.data_ptr(), S,
+          rows.data_ptr(), total, _stream())
     _call("b200m_latent_rotate", q.data_ptr() + 2 * dim, q.stride(0), q.stride(1), cos_sin.data_ptr(), cos_sin.shape[1], positions.data_ptr(), n, H, int(layout),
           _stream())
-    kv = torch.nn.functional.linear(rows[:, :rank], w_ukv)
     out = torch.empty(n, H * vdim, dtype=q.dtype, device=q.device)
-    _call("b200m_latent_prompt", q.data_ptr(), q.stride(0), kv.data_ptr(), kv.data_ptr() + 2 * H * dim, kv.stride(0), rows.data_ptr(), row, rank, total,
-          spans.cu_q.data_ptr(), spans.cu_k.data_ptr(), _p(sink), out.data_ptr(), n, spans.num_seqs, spans.max_q, H, dim, qd - dim, vdim, scale, int(window),
-          _stream())
+    latents, group = rows[:, :rank], max(1, min(H, LATENT_KV_BYTES // max(total * (dim + vdim) * 2, 1)))
+    for h in range(0, H, group):
+        g = min(group, H - h)
+        if g == H:
+            kv = torch.nn.functional.linear(latents, w_ukv)
+            keys, values = kv[:, :H * dim], kv[:, H * dim:]
+        else:
+            keys = values = None                      # the former heads' are given back first
+            keys = torch.nn.functional.linear(latents, w_ukv[h * dim:(h + g) * dim])
+            values = torch.nn.functional.linear(latents, w_ukv[H * dim + h * vdim:H * dim + (h + g) * vdim])
+        _call("b200m_latent_prompt", q.data_ptr() + 2 * h * qd, q.stride(0), keys.data_ptr(), values.data_ptr(), keys.stride(0), rows.data_ptr(), row, rank, total,
+              spans.cu_q.data_ptr(), cu_rows.data_ptr(), sink.data_ptr() + 4 * h if sink is not None else None, out.data_ptr() + 2 * h * vdim, out.stride(0), n, S,
+              spans.max_q, g, dim, qd - dim, vdim, scale, int(window), _stream())
     return out
 
 

@@ -175,6 +175,9 @@ class FegolornForCausalLM:
         elem = 4 if self.dtype == torch.float32 else 2
         return sum(b.mixer.cache_row_elems() * self.cfg.copies[i] for i, b in self.blocks.items()) * block_size * elem
 
+    def prompt_scratch_bytes(self, rows: int) -> int:
+        return max((b.mixer.prompt_scratch_bytes(rows) for b in self.blocks.values() if isinstance(b.mixer, GatedWindowLatentAttention)), default=0)
+
     def state_slot_bytes(self) -> int:
         return 8
 
@@ -199,7 +202,8 @@ class FegolornForCausalLM:
     @staticmethod
     def _spans(ctx, n: int) -> mixops.StepSpans:
         if ctx.is_prefill:
-            return mixops.StepSpans(ctx.cu_seqlens_q.numel() - 1, int(ctx.max_seqlen_q), ctx.cu_seqlens_q, ctx.cu_seqlens_k, None)
+            return mixops.StepSpans(ctx.cu_seqlens_q.numel() - 1, int(ctx.max_seqlen_q), ctx.cu_seqlens_q, ctx.cu_seqlens_k, None,
+                                    int(ctx.max_seqlen_k), int(ctx.total_seqlen_k))
         return mixops.StepSpans(n, 1, None, None, ctx.context_lens)
 
     @torch.inference_mode()

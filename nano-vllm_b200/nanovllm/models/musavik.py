@@ -185,7 +185,8 @@ class MusavikForCausalLM:
     @staticmethod
     def _spans(ctx, n: int) -> mixops.StepSpans:
         if ctx.is_prefill:
-            return mixops.StepSpans(ctx.cu_seqlens_q.numel() - 1, int(ctx.max_seqlen_q), ctx.cu_seqlens_q, ctx.cu_seqlens_k, None)
+            return mixops.StepSpans(ctx.cu_seqlens_q.numel() - 1, int(ctx.max_seqlen_q), ctx.cu_seqlens_q, ctx.cu_seqlens_k, None,
+                                    int(ctx.max_seqlen_k), int(ctx.total_seqlen_k))
         return mixops.StepSpans(n, 1, None, None, ctx.context_lens)
 
     def _open_pass(self, x_act: torch.Tensor, x0_act: torch.Tensor) -> torch.Tensor:

@@ -184,7 +184,8 @@ class PekunexForCausalLM:
     @staticmethod
     def _spans(ctx, n: int) -> mixops.StepSpans:
         if ctx.is_prefill:
-            return mixops.StepSpans(ctx.cu_seqlens_q.numel() - 1, int(ctx.max_seqlen_q), ctx.cu_seqlens_q, ctx.cu_seqlens_k, None)
+            return mixops.StepSpans(ctx.cu_seqlens_q.numel() - 1, int(ctx.max_seqlen_q), ctx.cu_seqlens_q, ctx.cu_seqlens_k, None,
+                                    int(ctx.max_seqlen_k), int(ctx.total_seqlen_k))
         return mixops.StepSpans(n, 1, None, None, ctx.context_lens)
 
     @torch.inference_mode()

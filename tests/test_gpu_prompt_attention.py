@@ -211,3 +211,76 @@ def test_pages_below_the_window_may_be_absent(mx, bs, window):
     for i, (n, l) in enumerate(zip(len_q, len_k)):
         tables[i, :(l - n - window + 1) // bs] = -1
     assert torch.equal(call(tables), want)
+
+
+def latent_case(mx, H, R, len_q, len_k, bs, seed, known=True):
+    from nanovllm.layers.rotary_embedding import build_banded_cos_sin
+    n = sum(len_q)
+    cache, tables = paged_rows(len_k, bs, R + 64, seed)
+    q, w = bf(n, H, 192, seed=seed + 2).cuda(), bf(H * 256, R, scale=R ** -0.5, seed=seed + 3).cuda()
+    cs = build_banded_cos_sin(64, max(len_k), 1e4, None, "cuda")
+    pos = torch.cat([torch.arange(b - a, b) for a, b in zip(len_q, len_k)]).cuda()
+    extra = (max(len_k), sum(len_k)) if known else ()
+    spans = mx.StepSpans(len(len_q), max(len_q), cu(len_q).cuda(), cu(len_k).cuda(), None, *extra)
+    return q, w, cache, tables, spans, cs, pos
+
+
+def over_the_latents(mx, case, bs, sink, window):
+    q, w, cache, tables, spans, cs, pos = case
+    n, H = q.shape[:2]
+    R = w.shape[1]
+    uk, uv = w[:H * 128].view(H, 128, R).float(), w[H * 128:].view(H, 128, R).float()
+    o = mx.latent_attention(torch.bmm(q[:, :, :128].transpose(0, 1).float(), uk), q.float(), 128, cache.float(), tables, bs, spans, sink, cs, 192 ** -0.5, window=window)
+    return torch.bmm(o, uv.transpose(1, 2)).transpose(0, 1).reshape(n, H * 128)
+
+
+@pytest.mark.parametrize("window", [0, 90])
+@pytest.mark.parametrize("known", [True, False])
+@pytest.mark.parametrize("group", [1, 2, 3, 4])
+def test_latent_prompts_of_ragged_steps(mx, window, known, group, monkeypatch):
+    """Sequences of very different lengths, with and without lengths on the host, a window that cuts most keys, and keys and values formed for a few heads at a
+    time: as attention over the latents."""
+    H, R, len_q, len_k, bs = 4, 64, [64, 1, 129, 30], [1200, 5, 129, 700], 16
+    case = latent_case(mx, H, R, len_q, len_k, bs, 80, known)
+    q, w, cache, tables, spans, cs, pos = case
+    total, most = mx._latent_rows(q.shape[0], tables, bs, spans, window)
+    seen = [min(k, a + window - 1) if window else k for a, k in zip(len_q, len_k)]
+    assert sum(seen) <= total and max(seen) <= most
+    if known and not window:
+        assert (total, most) == (sum(len_k), max(len_k))
+    sink = torch.linspace(-1, 1, H).cuda()
+    want = over_the_latents(mx, case, bs, sink, window)
+    monkeypatch.setattr(mx, "LATENT_KV_BYTES", total * 512 * group)
+    got = mx.latent_prompt(q, w, 128, 128, cache, tables, bs, spans, sink, cs, pos, 192 ** -0.5, window=window)
+    assert_close_bf16(got, want, "ragged", rel_l2=8e-3, ulps=3.0)
+
+
+@pytest.mark.parametrize("len_q,len_k,window,rows", [([100] * 31 + [4096], [100] * 31 + [4096], 0, 31 * 100 + 4096), ([16, 16], [30000, 12000], 1024, 2 * 1039)])
+def test_latent_prompts_hold_the_rows_that_are_seen(mx, len_q, len_k, window, rows):
+    """A long sequence beside short ones, and a short portion behind a long context under a window: memory for the real rows alone."""
+    H, R, bs = 4, 64, 256
+    q, w, cache, tables, spans, cs, pos = latent_case(mx, H, R, len_q, len_k, bs, 85)
+    args = (q, w, 128, 128, cache, tables, bs, spans, None, cs, pos, 192 ** -0.5)
+    assert mx.latent_expands(q, 128, 64, 128, R, 192 ** -0.5, cache, tables, bs, spans, window)
+    mx.latent_prompt(*args, window=window)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    out = mx.latent_prompt(*args, window=window)
+    used = torch.cuda.max_memory_allocated() - held - out.numel() * 2
+    spare = 3 << 20                                                      # the allocator hands out a larger free block when less than 1 MiB of it would be left
+    assert used <= rows * (H * 512 + (R + 64) * 2) + spare               # the padded rows would be 302 and 138 MB
+    assert used <= mx.latent_scratch_bytes(H, 128, 128, R + 64, rows) + spare
+
+
+def test_rows_seen_through_a_window(mx):
+    """The prefix over sequences, at sizes around the block of 1024 that forms it; sequences without queries count nothing."""
+    for S in (1, 31, 1024, 1025, 2500):
+        g = torch.Generator().manual_seed(S)
+        q = torch.randint(0, 50, (S,), generator=g)
+        k = q + torch.randint(0, 300, (S,), generator=g)
+        out = torch.empty(S + 1, dtype=torch.int32, device="cuda")
+        a, b = cu(q.tolist()).cuda(), cu(k.tolist()).cuda()
+        mx._call("b200m_latent_visible", a.data_ptr(), b.data_ptr(), S, 64, out.data_ptr(), mx._stream())
+        want = torch.where(q > 0, torch.minimum(k, q + 63), torch.zeros_like(q))
+        assert torch.equal(out.cpu(), cu(want.tolist()))
