@@ -75,7 +75,7 @@ def ensure_model_dir(local_rank: int) -> str:
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons while the timed region runs (B200_PROFILING.md)."""
+    """nvidia-smi clocks / throttle reasons while the timed region runs."""
     Q = ("clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
          "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
 
@@ -117,7 +117,7 @@ def load_peaks() -> dict:
         p = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
         return {"hbm_gbs": p["hbm_gbs"], "source": "MEASURED_PEAKS.json (measured copy)"}
     except Exception:
-        return {"hbm_gbs": 6650.0, "source": "fallback (B200_PROFILING.md)"}
+        return {"hbm_gbs": 6650.0, "source": "fallback (an earlier copy measurement)"}
 
 
 WORKLOAD = ("Qwen3-0.6B random-init bf16, 256 seqs, in/out U[100,1024] (reference bench.py shape), temperature 0.6, "

@@ -1,6 +1,6 @@
-"""INTEGRATION.md option B, executable: the binding a maintainer of the reference adds to put libb200attn.so behind
+"""Option B of the integration notes, executable: the binding a maintainer of the reference adds to put libb200attn.so behind
 ``nanovllm.layers.attention.Attention`` -- and nothing else.  This file imports NOTHING from this repository's
-``nano-vllm_b200`` package: it is the ctypes stub of INTEGRATION.md verbatim plus ``patch()``, which applies the two
+``nano-vllm_b200`` package: it is the ctypes stub of those notes verbatim plus ``patch()``, which applies the two
 edits the document describes (Attention.forward body; head-major cache allocation + bind) to an imported reference
 package.  tests/test_gpu_reference_forward.py runs the otherwise unmodified reference through it on the GPU and
 compares logits and greedy tokens with the unmodified reference (flash-attn) on the same weights and script.

@@ -1,8 +1,8 @@
 """CPU oracle for the paged-attention hot path.  TEST INFRASTRUCTURE ONLY.
 
 Everything under ``oracle/`` is a checker: a CPU restatement of what the
-reference (GeeeekExplorer/nano-vllm @ bb823b3e) computes on the path named by
-BASELINE.json's north_star.  Only ``tests/``, ``__graft_entry__.smoke()`` and
+reference (GeeeekExplorer/nano-vllm @ bb823b3e) computes on its attention and
+serving path.  Only ``tests/``, ``__graft_entry__.smoke()`` and
 ``bench.py``'s cpu_baseline / ``--impl reference`` legs may import it.  The
 product package (``nano-vllm_b200/nanovllm``) never does, and fails loudly if
 its CUDA library is missing.

@@ -1,4 +1,4 @@
-"""BASELINE.json configs[2] sanity + timing: Qwen3-8B dims (random init), block_size=16, prefix cache on, one B200.
+"""Sanity + timing at Qwen3-8B dims (random init), block_size=16, prefix cache on, one B200.
 
     NANOVLLM_ALLOW_RANDOM_INIT=1 python profiles/config3_8b.py [num_seqs] [max_tokens]
 

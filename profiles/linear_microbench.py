@@ -1,6 +1,6 @@
 """Staged tcgen05 linear (csrc/linear_tc.cu) against the library path it would replace, at Qwen3-0.6B decode shapes.
 
-    timeout 600 python profiles/linear_microbench.py > gpurun_out/linear_microbench.json
+    python profiles/linear_microbench.py > linear_microbench.json
 
 A configuration the library refuses (unsupported shape) is recorded as null; results are flushed per batch size.
 

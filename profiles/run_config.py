@@ -1,4 +1,4 @@
-"""BASELINE.json configs[2..4] end to end through the public API, one process per GPU.
+"""Three larger workloads (numbers 3 to 5 below) end to end through the public API, one process per GPU.
 
     python profiles/run_config.py 3                                   # Qwen3-8B, 512 seqs, block 16, prefix cache, 1 GPU
     python -m torch.distributed.run --nnodes=1 --nproc-per-node 4 --master-addr 127.0.0.1 --master-port 29640 profiles/run_config.py 4
@@ -16,7 +16,7 @@ throughput (wall clock around generate(), after a warm-up generate), the decode 
 shapes (CUDA events, rank 0's shard), KV sizing, and a parity leg: greedy requests whose tokens must agree (a) between
 all ranks, (b) between twin prompts served in different batches / through the prefix cache, and (c) -- configs 3 and 4 use
 the same model and the same greedy prompts -- between the 1-GPU run and the TP4 run (tokens of config 3 are saved to
-gpurun_out/r02_config3_greedy_tokens.json, committed as profiles/r02_config3_greedy_tokens.json and compared by config 4).
+profiles/r02_config3_greedy_tokens.json and compared by config 4).
 """
 import json
 import os
@@ -27,8 +27,7 @@ import time
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path[:0] = [ROOT, os.path.join(ROOT, "nano-vllm_b200")]
 os.environ.setdefault("NANOVLLM_ALLOW_RANDOM_INIT", "1")
-GREEDY_FILE = os.path.join(ROOT, "profiles", "r02_config3_greedy_tokens.json")          # committed copy, read by config 4
-GREEDY_OUT = os.path.join(ROOT, "gpurun_out", "r02_config3_greedy_tokens.json")          # written by config 3 (gpurun merges gpurun_out/ back)
+GREEDY_FILE = GREEDY_OUT = os.path.join(ROOT, "profiles", "r02_config3_greedy_tokens.json")          # written by config 3, read by config 4
 
 
 def requests_for(cfg: int):

@@ -1,6 +1,6 @@
 """Turn an `ncu --metrics gpu__time_duration.sum --csv` launch list into the per-kernel share table kept in profiles/README.md.
 
-    python profiles/summarize_launches.py gpurun_out/c6_launches_decode.csv [more.csv ...]
+    python profiles/summarize_launches.py launches_decode.csv [more.csv ...]
 
 Times under ncu are serialised and cold-cache: only the SHARES are comparable with bench.py's CUDA-event numbers.
 """

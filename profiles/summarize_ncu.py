@@ -1,6 +1,6 @@
 """Turn an .ncu-rep into the short text summary committed under profiles/ (run here, no GPU needed).
 
-    python profiles/summarize_ncu.py gpurun_out/decode_full.ncu-rep > profiles/r01_decode_kernel_ncu.txt
+    python profiles/summarize_ncu.py capture.ncu-rep > profiles/decode_kernel_ncu.txt
 """
 import csv
 import io
