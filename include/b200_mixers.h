@@ -347,11 +347,12 @@ int b200m_moe_combine(const float* rows, const int32_t* pos_of, int top, const v
 
 /* Everything between the router's choice and the routed block's result (bf16), as one call: align, gather, the two grouped GEMMs (W_in [experts, N, K] with act,
  * W_out [experts, width, N or N / 2]; fp32 results), combine.  wgt [n, top] weights the experts' inputs (weigh_inputs) or their results; the other
- * arguments as for b200m_moe_combine.  workspace: b200m_moe_experts_workspace_bytes(n * top, ...) bytes, 256-byte aligned. */
-size_t b200m_moe_experts_workspace_bytes(int64_t pairs, int num_experts, int K, int inter, int width);
+ * arguments as for b200m_moe_combine.  rows [rows_cap, width] takes the second GEMM's results (as many rows as b200m_moe_align's cap at least); workspace:
+ * b200m_moe_experts_workspace_bytes(n * top, ..., inter = N or N / 2) bytes; both 256-byte aligned. */
+size_t b200m_moe_experts_workspace_bytes(int64_t pairs, int num_experts, int K, int inter);
 int b200m_moe_experts(const void* A, int64_t a_stride, const int32_t* idx, const float* wgt, int weigh_inputs, int n, int top, int num_experts,
                       const void* W_in, int N, int K, int act, const void* W_out, int width, const void* shared, const float* gate_logit, int64_t gate_ld,
-                      const float* ident, float* out, void* workspace, size_t workspace_bytes, void* stream);
+                      const float* ident, float* out, float* rows, int rows_cap, void* workspace, size_t workspace_bytes, void* stream);
 
 #ifdef __cplusplus
 }

@@ -385,9 +385,9 @@ namespace {
 
 struct ExpertsSpace {
     int cap;                                      // rows of the grouped buffers
-    size_t sorted, pos, tile, num, counts, grouped, inter, rows, bytes;
+    size_t sorted, pos, tile, num, counts, grouped, inter, bytes;
 };
-ExpertsSpace experts_space(int64_t pairs, int experts, int K, int inter, int width) {
+ExpertsSpace experts_space(int64_t pairs, int experts, int K, int inter) {
     ExpertsSpace s;
     const int64_t cap = (pairs + (int64_t)experts * (TILE - 1) + TILE - 1) / TILE * TILE;
     s.cap = cap < (1ll << 31) ? (int)cap : 0;
@@ -404,30 +404,29 @@ ExpertsSpace experts_space(int64_t pairs, int experts, int K, int inter, int wid
     s.counts = take(8 * (size_t)experts);
     s.grouped = take(2 * (size_t)cap * K);
     s.inter = take(2 * (size_t)cap * inter);
-    s.rows = take(4 * (size_t)cap * width);
     s.bytes = at;
     return s;
 }
 
 }  // namespace
 
-extern "C" size_t b200m_moe_experts_workspace_bytes(int64_t pairs, int num_experts, int K, int inter, int width) {
-    if (pairs < 0 || num_experts <= 0 || K <= 0 || inter <= 0 || width <= 0) return 0;
-    return experts_space(pairs, num_experts, K, inter, width).bytes;
+extern "C" size_t b200m_moe_experts_workspace_bytes(int64_t pairs, int num_experts, int K, int inter) {
+    if (pairs < 0 || num_experts <= 0 || K <= 0 || inter <= 0) return 0;
+    return experts_space(pairs, num_experts, K, inter).bytes;
 }
 
 extern "C" int b200m_moe_experts(const void* A, int64_t a_stride, const int32_t* idx, const float* wgt, int weigh_inputs, int n, int top, int num_experts,
                                  const void* W_in, int N, int K, int act, const void* W_out, int width, const void* shared, const float* gate_logit, int64_t gate_ld,
-                                 const float* ident, float* out, void* workspace, size_t workspace_bytes, void* stream) {
-    if (!A || !idx || !wgt || !W_in || !W_out || !out || !workspace || n < 0 || top <= 0 || num_experts <= 0 || N <= 0 || K <= 0 || width <= 0 || act < 0 || act > 2 ||
+                                 const float* ident, float* out, float* rows, int rows_cap, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!A || !idx || !wgt || !W_in || !W_out || !out || !rows || !workspace || n < 0 || top <= 0 || num_experts <= 0 || N <= 0 || K <= 0 || width <= 0 || act < 0 || act > 2 ||
         (act == 2 && N % 2))
         return B200_EINVAL;
     if (n == 0) return B200_OK;
     const int inter = act == 2 ? N / 2 : N;
     const int64_t pairs = (int64_t)n * top;
-    const ExpertsSpace s = experts_space(pairs, num_experts, K, inter, width);
+    const ExpertsSpace s = experts_space(pairs, num_experts, K, inter);
     if (s.cap == 0 || pairs >= (1ll << 31)) return B200_EUNSUPPORTED;
-    if (workspace_bytes < s.bytes || reinterpret_cast<uintptr_t>(workspace) % 256) return B200_EWORKSPACE;
+    if (workspace_bytes < s.bytes || reinterpret_cast<uintptr_t>(workspace) % 256 || rows_cap < s.cap || reinterpret_cast<uintptr_t>(rows) % 256) return B200_EWORKSPACE;
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     int32_t *sorted = reinterpret_cast<int32_t*>(ws + s.sorted), *pos = reinterpret_cast<int32_t*>(ws + s.pos), *tile = reinterpret_cast<int32_t*>(ws + s.tile),
             *num = reinterpret_cast<int32_t*>(ws + s.num), *counts = reinterpret_cast<int32_t*>(ws + s.counts);
@@ -444,7 +443,7 @@ extern "C" int b200m_moe_experts(const void* A, int64_t a_stride, const int32_t*
     else if (rc == B200_EUNSUPPORTED)
         rc = b200m_moe_gemm(A, a_stride, sorted, in_wgt, top, 1, tile, num, tiles, W_in, N, K, ws + s.inter, 0, act, 0, stream);
     if (rc != B200_OK) return rc;
-    rc = b200m_moe_gemm(ws + s.inter, inter, sorted, nullptr, top, 0, tile, num, tiles, W_out, width, inter, ws + s.rows, 1, hint, 0, stream);
+    rc = b200m_moe_gemm(ws + s.inter, inter, sorted, nullptr, top, 0, tile, num, tiles, W_out, width, inter, rows, 1, hint, 0, stream);
     if (rc != B200_OK) return rc;
-    return b200m_moe_combine(reinterpret_cast<float*>(ws + s.rows), pos, top, shared, gate_logit, gate_ld, weigh_inputs ? nullptr : wgt, ident, out, n, width, 0, stream);
+    return b200m_moe_combine(rows, pos, top, shared, gate_logit, gate_ld, weigh_inputs ? nullptr : wgt, ident, out, n, width, 0, stream);
 }

@@ -824,8 +824,8 @@ def moe_combine(rows: torch.Tensor, pos_of: torch.Tensor, top: int, n: int, shar
 
 def moe_experts(A: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor, act: int, weigh_inputs: bool,
                 shared: torch.Tensor | None = None, gate_logit: torch.Tensor | None = None, ident: torch.Tensor | None = None) -> torch.Tensor:
-    """The routed block after the router's choice (idx, wgt [n, top]), bf16, as one call of six launches: grouping, gathered inputs (weighted with
-    ``weigh_inputs``), act(x W_in^T), (.) W_out^T, and each token's sum -> fp32 [n, width].  The other arguments as for ``moe_combine``."""
+    """The routed block after the router's choice (idx, wgt [n, top]), bf16, as one call of five launches: grouping, gathered inputs (weighted with
+    ``weigh_inputs``; four where the first GEMM gathers by itself), act(x W_in^T), (.) W_out^T, and each token's sum -> fp32 [n, width].  The other arguments as for ``moe_combine``."""
     n, top = idx.shape
     E, N, K = w_in.shape
     width = w_out.shape[1]
@@ -836,10 +836,13 @@ def moe_experts(A: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, w_in: tor
     assert gate_logit is None or gate_logit.dtype == torch.float32
     assert ident is None or (ident.dtype == torch.float32 and ident.is_contiguous() and ident.shape == (n, width))
     out = torch.empty(n, width, dtype=torch.float32, device=A.device)
-    size = nat.load_mix().b200m_moe_experts_workspace_bytes(n * top, E, K, w_out.shape[2], width)
+    # the fp32 results apart from the rest: one block of all together is rarely free in the allocator's cache, and a first pass then waits for the driver
+    rows = torch.empty(moe_capacity(n * top, E), width, dtype=torch.float32, device=A.device)
+    size = nat.load_mix().b200m_moe_experts_workspace_bytes(n * top, E, K, w_out.shape[2])
     space = torch.empty(size, dtype=torch.uint8, device=A.device)
     _call("b200m_moe_experts", A.data_ptr(), A.stride(0), idx.data_ptr(), wgt.data_ptr(), int(weigh_inputs), n, top, E, w_in.data_ptr(), N, K, act,
           w_out.data_ptr(), width, _p(shared), _p(gate_logit), gate_logit.stride(0) if gate_logit is not None else 0, _p(ident), out.data_ptr(),
-          space.data_ptr(), size, _stream())
-    ops.LAUNCHES[0] += 4 + int(N % 256 == 0)
+          rows.data_ptr(), rows.shape[0], space.data_ptr(), size, _stream())
+    gathered = N % 256 == 0 and K % 8 == 0 and A.stride(0) % 8 == 0 and A.data_ptr() % 16 == 0          # as the library decides
+    ops.LAUNCHES[0] += 3 + int(gathered)
     return out

@@ -113,3 +113,28 @@ def test_one_call_against_its_parts(mx, n, act, N, weigh_inputs, shared, ident):
     res = mx.moe_gemm(inter, rows, tile_expert, num_tiles, w_out, out_f32=True)
     want = mx.moe_combine(res, pos_of, top, n, sh, gate, wgt=None if weigh_inputs else wgt, ident=x)
     assert ((got - want).norm() / want.norm()).item() < 1e-5
+
+
+@pytest.mark.parametrize("N", [512, 640])
+def test_one_call_counts_as_its_steps_do(mx, N):
+    """The launches of the one call are those of grouping, copy (where the first GEMM reads grouped rows), GEMMs and sum called one by one, with the same result; the
+    fp32 rows are no part of its workspace."""
+    from nanovllm import ops
+    n, top, E, width = 3000, 4, 16, 512
+    idx = routing([n * top // E] * E, top, 5)
+    g = torch.Generator(device="cuda").manual_seed(6)
+    A = torch.randn(n, width, generator=g, device="cuda").to(torch.bfloat16)
+    w_in = (torch.randn(E, N, width, generator=g, device="cuda") * width ** -0.5).to(torch.bfloat16)
+    w_out = (torch.randn(E, width, N // 2, generator=g, device="cuda") * width ** -0.5).to(torch.bfloat16)
+    wgt = torch.rand(n, top, generator=g, device="cuda")
+    at = [ops.LAUNCHES[0]]
+    got = mx.moe_experts(A, idx, wgt, w_in, w_out, 2, False)
+    at.append(ops.LAUNCHES[0])
+    rows, pos_of, tile_expert, num_tiles = mx.moe_align(idx, E)
+    inter = mx.moe_gemm(A, rows, tile_expert, num_tiles, w_in, top=top, act=2, gather=True)
+    want = mx.moe_combine(mx.moe_gemm(inter, rows, tile_expert, num_tiles, w_out, out_f32=True), pos_of, top, n, None, None, wgt=wgt)
+    at.append(ops.LAUNCHES[0])
+    assert at[1] - at[0] == at[2] - at[1] == (5 if N % 256 == 0 else 4)
+    assert (got - want).norm() <= 2e-5 * want.norm()
+    cap = mx.moe_capacity(n * top, E)
+    assert mx.nat.load_mix().b200m_moe_experts_workspace_bytes(n * top, E, width, N // 2) <= cap * 2 * (width + N // 2) + 12 * cap + 4096
