@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(1024) latent_visible_kernel(const int32_t* __r
         int len = 0;
         if (s < num_seqs) {
             const int n = cu_q[s + 1] - cu_q[s];
-            len = n > 0 ? min(cu_k[s + 1] - cu_k[s], n + window - 1) : 0;
+            len = n > 0 ? (int)min((int64_t)(cu_k[s + 1] - cu_k[s]), (int64_t)n + window - 1) : 0;      // any window, up to the largest int
         }
         int inc = len;
 #pragma unroll

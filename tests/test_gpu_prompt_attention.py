@@ -281,6 +281,7 @@ def test_rows_seen_through_a_window(mx):
         k = q + torch.randint(0, 300, (S,), generator=g)
         out = torch.empty(S + 1, dtype=torch.int32, device="cuda")
         a, b = cu(q.tolist()).cuda(), cu(k.tolist()).cuda()
-        mx._call("b200m_latent_visible", a.data_ptr(), b.data_ptr(), S, 64, out.data_ptr(), mx._stream())
-        want = torch.where(q > 0, torch.minimum(k, q + 63), torch.zeros_like(q))
-        assert torch.equal(out.cpu(), cu(want.tolist()))
+        for window in (1, 64, 2 ** 31 - 1):
+            mx._call("b200m_latent_visible", a.data_ptr(), b.data_ptr(), S, window, out.data_ptr(), mx._stream())
+            want = torch.where(q > 0, torch.minimum(k, q + window - 1), torch.zeros_like(q))
+            assert torch.equal(out.cpu(), cu(want.tolist()))
