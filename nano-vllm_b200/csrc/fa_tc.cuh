@@ -12,12 +12,12 @@
 //   warp 14          TMA: Q of the next items, K and V blocks through two rings of slots
 //
 // TMEM (512 columns): S / P of each tile twice (4 x 64), O of each tile (2 x 128).  A tile's products come in the order PV(j) QK(j+2):
-// scores are two blocks ahead, so a softmax warp finds its next block's scores ready and never waits for the products of the block it just
-// left.  The walk does not stop at the end of an item: with two Q buffers the next items' first scores follow the last blocks of the
+// scores are two blocks ahead, so a softmax warp finds its next block's scores ready and waits for the products of the block it just left only
+// to rescale O.  The walk does not stop at the end of an item: with two Q buffers the next items' first scores follow the last blocks of the
 // present one.
 //
 // What bounds it: per step (64 keys, both tiles) the products take 2 x (384 + 256) cycles (QK^T reads 48 KB of shared memory at 128 B per
-// cycle, PV 4 M multiply-adds) and 16384 exponentials 1024 on the special-function unit (16 per cycle); a step measures 1700-1800 cycles,
+// cycle, PV 2 M multiply-adds) and 16384 exponentials 1024 on the special-function unit (16 per cycle); a step measures 1700-1800 cycles,
 // most of it the softmax warps' instructions.  128-key blocks with one S per tile read less but put softmax, PV and QK of a tile in one
 // chain: 1950 cycles per 64 keys.  A quarter to a half of the exponentials by a polynomial on the multiply-add pipe shortened the step to
 // 1650 cycles and the time by nothing (the clock gave way).  Items are dealt out longest first (causal tiles late in a sequence see the

@@ -6,7 +6,7 @@
 //                      256 rows of its weights (N = 256; with the gated activation 128 gate rows and the 128 matching up rows), K in
 //                      stages of 64 through a 4-deep TMA ring, two accumulators in TMEM so that an item's results are written while the
 //                      next one multiplies.
-//                      Bound by the L2 -> shared-memory path: 48 KB per 4 M multiply-adds, 94 B per cycle and SM at the tensor cores' full
+//                      Bound by the L2 -> shared-memory path: 48 KB per 2 M multiply-adds, 94 B per cycle and SM at the tensor cores' full
 //                      rate.  128 x 256 tiles rather than 64 x 128 (the mma.sync form) halve that traffic.
 //   moe_stream_kernel  few rows: HBM-bound, every weight is read once.  A CTA takes 128 weight rows (M; gated: 64 gate + 64 up) times one
 //                      tile of 64 rows (N), three CTAs per SM so that all items are in flight and share the memory bandwidth evenly.
