@@ -59,7 +59,7 @@ def test_linear_explicit_ring_depth(stages, block_n):
 @pytest.mark.parametrize("cluster", [2, 4])
 @pytest.mark.parametrize("rows", [1, 100, 256])
 def test_linear_multicast_cluster(cluster, rows):
-    """x tiles fetched once per cluster and multicast to its CTAs: bit-identical to the unclustered kernel."""
+    """``cluster`` has to divide the column blocks and changes nothing else (every CTA loads its own x tile): bit-identical to the call without it."""
     from nanovllm import ops
     x, w = _inputs(rows, 4096, 1024, seed=rows + cluster)
     base = ops.linear(x, w, ops.EPI_BF16, 32)
