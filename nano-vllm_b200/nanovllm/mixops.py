@@ -704,7 +704,7 @@ def causal_conv(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None
     _call("b200m_causal_conv", x.data_ptr(), x.stride(0), weight.data_ptr(), _p(bias), conv_state.data_ptr(), state_slots.data_ptr(),
           _p(spans.cu_q), _p(spans.cu_k), _p(spans.ctx_lens), out.data_ptr(), spans.num_seqs, spans.max_q, channels, taps, int(silu),
           is32, _stream())
-    if taps > 1 and not (spans.cu_q is None and taps <= 8):       # single-token steps update the history in the same launch
+    if taps > 8:                                            # up to eight taps the history moves on in the same launch
         ops.LAUNCHES[0] += 1
     return out
 
