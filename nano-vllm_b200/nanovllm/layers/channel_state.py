@@ -87,6 +87,7 @@ class _ChannelStateMixer:
         self.in_cols = _pad8(at)
         self.w_in = torch.zeros(self.in_cols, self.width, dtype=self.dtype, device=self.device)
         self.second = {leaf[:-1] + "2": torch.zeros(cols, _pad8(new[leaf]), dtype=self.dtype, device=self.device) for leaf, cols in self.low_rank()}
+        self._second_t = {leaf: w.t() for leaf, w in self.second.items()}           # views
 
     def _cols(self, proj: torch.Tensor, leaf: str) -> torch.Tensor:
         a, rows = self.at[leaf]
@@ -99,7 +100,7 @@ class _ChannelStateMixer:
         t = proj[:, a:a + w.shape[1]]
         if f32 and self._mm_f32_out:
             try:
-                return torch.mm(t, w.t(), out_dtype=torch.float32)
+                return torch.mm(t, self._second_t[leaf[:-1] + "2"], out_dtype=torch.float32)
             except (RuntimeError, TypeError):
                 self._mm_f32_out = False
         y = F.linear(t, w)
@@ -195,7 +196,7 @@ class ChannelDeltaMixer(_ChannelStateMixer):
         qkv = mixops.causal_conv(proj[:, :self.conv_cols], self.conv_w, None, self.conv_state[inst], ctx.state_slots, spans)
         o = mixops.channel_state(qkv, 0, Q, 2 * Q, self._cols(proj, "b"), self._second(proj, "a1", True), self.rate, self.decay_bias,
                                  self.decay_sign, self.state[inst], ctx.state_slots, spans, self.heads, self.kv_heads, self.dim, self.vdim,
-                                 self.dim ** -0.5)
+                                 self.dim ** -0.5, forgetting=True)          # rate = -exp(A_log)
         return mixops.head_rmsnorm_gate(o, self.norm_w, self._second(proj, "g1", False), self.eps, self.dtype, silu=False, out=out)
 
 

@@ -586,13 +586,25 @@ def gated_delta(x: torch.Tensor, q_off: int, k_off: int, v_off: int, ba: torch.T
     return out
 
 
+_DELTA_WS = [0, 0]             # workspace bytes of a chunk of one sequence and head, and the most that a step takes beyond one chunk
+
+
+def delta_chunks(max_q: int, dim: int) -> bool:
+    """Whether a step's portions take the chunked form of the channel delta rule.  Its rows are 128 channels wide; a chunk is sixteen tokens: one
+    16-token portion 15 us against 16 (16 heads), sixteen of them 29 against 35 (8 heads 21 against 21), of 6 tokens 28 against 27 (8 heads 19
+    against 16); longer ones 1.2 to 3 times faster."""
+    return max_q >= 16 and 64 < dim <= 128
+
+
 def channel_state(x: torch.Tensor, q_off: int, k_off: int, v_off: int, write: torch.Tensor | None, decay_in: torch.Tensor, rate: torch.Tensor,
                   decay_bias: torch.Tensor, decay_sign: float, state: torch.Tensor, state_slots: torch.Tensor, spans: StepSpans, heads: int,
-                  kv_heads: int, dim: int, vdim: int, q_scale: float) -> torch.Tensor:
+                  kv_heads: int, dim: int, vdim: int, q_scale: float, forgetting: bool = False) -> torch.Tensor:
     """Matrix state with one decay per head and key channel, exp(rate[h] * softplus(sign * (decay_in + decay_bias))).
     x [n, cols]: q, k ([kv_heads, dim] at q_off / k_off) and v ([heads, vdim] at v_off); ``write`` [n, heads] (a row-strided view): delta rule
     with unit-norm q and k; None: gated linear attention.  decay_in fp32 [n, heads * dim] is scratch (single-token steps
-    form the decays in place first); state fp32 [slots, heads, vdim, dim] -> fp32 [n, heads, vdim]."""
+    form the decays in place first); state fp32 [slots, heads, vdim, dim] -> fp32 [n, heads, vdim].
+    ``forgetting``: the caller's rates are never above zero, so that no decay is above one; bf16 portions under the delta rule then run on the
+    tensor cores (``delta_chunks``)."""
     n = x.shape[0]
     is32 = _is32(x)
     assert x.dim() == 2 and x.stride(1) == 1 and decay_in.dtype == torch.float32 and decay_in.stride(1) == 1 and decay_in.shape == (n, heads * dim)
@@ -601,6 +613,23 @@ def channel_state(x: torch.Tensor, q_off: int, k_off: int, v_off: int, write: to
     assert write is None or (write.shape == (n, heads) and write.stride(1) == 1)
     _same(is32, write)
     out = torch.empty(n, heads, vdim, dtype=torch.float32, device=x.device)
+    if forgetting and write is not None and not is32 and spans.cu_q is not None and delta_chunks(spans.max_q, dim):
+        lib = nat.load_mix()
+        if not _DELTA_WS[0]:
+            _DELTA_WS[:] = lib.b200m_channel_delta_workspace_bytes(1, 1, 1), lib.b200m_channel_delta_workspace_bytes(0, 0, 0)
+        chunks, one = (spans.max_q + 15) >> 4, _DELTA_WS[0] * spans.num_seqs * heads
+        fit = max(1, min(chunks, _DELTA_WS[1] // one))      # chunks that a pair of launches takes
+        size = fit * one
+        ws = torch.empty(size, dtype=torch.uint8, device=x.device)
+        rc = lib.b200m_channel_delta_prompts(
+            x.data_ptr(), x.stride(0), q_off, k_off, v_off, write.data_ptr(), write.stride(0), decay_in.data_ptr(), decay_in.stride(0), rate.data_ptr(),
+            decay_bias.data_ptr(), decay_sign, state.data_ptr(), state_slots.data_ptr(), spans.cu_q.data_ptr(), spans.cu_k.data_ptr(), out.data_ptr(), n,
+            spans.num_seqs, spans.max_q, heads, kv_heads, dim, vdim, q_scale, ws.data_ptr(), size, _stream())
+        if rc != -2:                                        # B200_EUNSUPPORTED: other alignments and odd sizes, below
+            nat.check_mix(rc)
+            ops.LAUNCHES[0] += 2 * -(-chunks // fit) - 1
+            return out
+        ops.LAUNCHES[0] -= 1
     if spans.cu_q is None or spans.max_q <= 4:
         ops.LAUNCHES[0] += 1
     _call("b200m_channel_state", x.data_ptr(), x.stride(0), q_off, k_off, v_off, _p(write), write.stride(0) if write is not None else 0,
