@@ -253,6 +253,17 @@ int b200_lm_head_sample(const void* hidden, int64_t hidden_stride0, const void* 
 int b200_add_rmsnorm_partials(const float* partials, int splits, void* residual, const void* weight, void* out,
                               int rows, int cols, float eps, int flags, void* stream);
 
+/* Linear layers of at most 16 rows with the ops around them (csrc/linear_rows.cu): out[rows, n] = bf16(z w^T), with
+ *   norm_w NULL: z = x, the sum over k as `splits` (at most 8) equal parts added in order, as b200_linear's partials;
+ *   else z = rmsnorm(x) * norm_w, or with add: rmsnorm(x + add) * norm_w and residual_out = bf16(x + add) ([rows, k] contiguous, neither x nor add), rounded
+ *   as b200_add_rmsnorm rounds; splits must be 1.
+ *   silu: w is [2 * n, k], gate rows then up rows, out = SiluAndMul(bf16(z w^T)); needs norm_w.
+ * k a multiple of 64 * splits, n of 16 (silu: 8), k within what shared memory holds (at least 3072), row strides of x and add multiples of 8 elements,
+ * pointers 16-byte aligned; else B200_EUNSUPPORTED.
+ * flags bit 0: programmatic stream serialization; the weights are then asked for before the kernel in front has ended. */
+int b200_linear_rows(const void* x, int64_t x_stride0, const void* add, int64_t add_stride0, void* residual_out, const void* norm_w, float eps,
+                     const void* w, void* out, int64_t out_stride0, int rows, int n, int k, int splits, int silu, int flags, void* stream);
+
 /* The tail of a decoder layer for a decode-size batch on one GPU, as ONE persistent kernel (csrc/layer_tail.cu):
  *   o_proj -> residual add + RMSNorm -> gate_up_proj + SiluAndMul -> down_proj -> residual add + RMSNorm [-> next qkv_proj]
  * i.e. RowParallelLinear o_proj + RMSNorm.add_rms_forward + Qwen3MLP + the next layer's input_layernorm and

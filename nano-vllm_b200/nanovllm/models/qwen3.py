@@ -103,6 +103,11 @@ class Qwen3ForCausalLM:
         else:
             tcc[3], tcc[5] = fit(self.q_size, tcc[3]), fit(self.inter, tcc[5])
             self.tc_big = (fit(self.q_size, min(tcc[3], self.tc_big_splits)), fit(self.inter, min(tcc[5], self.tc_big_splits)))
+        # Steps of at most 16 rows: four launches a layer around attention, norms and SiluAndMul inside the products (csrc/linear_rows.cu), with the results of
+        # the launches they replace, bit for bit
+        fits = all(k % 512 == 0 and k <= 3072 and n % 16 == 0 for n, k in ((self.q_size + 2 * self.kv_size, self.hidden), (self.hidden, self.q_size),
+                                                                           (self.inter, self.hidden), (self.hidden, self.inter)))
+        self.few_rows = 16 if mode == "auto" and self.tc_linear and tp_size == 1 and fits and max(tcc[3], tcc[5]) <= 8 else 0
         # B200_TAIL=mega: in decode steps of up to 256 rows on one GPU, everything between two attention kernels
         # (o_proj, add+norm, gate_up+SiluAndMul, down_proj, add+norm, the next layer's qkv_proj) is ONE persistent launch
         # (csrc/layer_tail.cu) instead of seven.  Measured 58-70 us per layer against 30 us for the chain (r02_layer_tail_microbench.json):
@@ -343,6 +348,21 @@ class Qwen3ForCausalLM:
             main.wait_event(ev_join)
         return out
 
+    def _forward_few_rows(self, residual: torch.Tensor, positions: torch.Tensor, ctx) -> torch.Tensor:
+        """A decode step of at most ``few_rows`` rows."""
+        cfg, add = self.tc_cfg, None
+        pdl, last = bool(cfg[6]), len(self.layers) - 1
+        for li, L in enumerate(self.layers):
+            qkv, residual = ops.linear_rows(residual, L.qkv, L.ln1, self.eps, add, pdl=pdl)
+            # attention starts when qkv_proj has ended: blocks of it that come early sit on the few SMs which that leaves free, two thirds of the others' time
+            # longer (16 rows of 100-1024 tokens: 19.2 us a layer against 14.1)
+            o, _ = ops.linear_rows(self._attention(li, qkv, positions, ctx, no_pdl=True), L.o, splits=cfg[3], pdl=pdl)
+            act, residual = ops.linear_rows(residual, L.gate_up, L.ln2, self.eps, o, silu=True, pdl=pdl)
+            if li < last:
+                add, _ = ops.linear_rows(act, L.down, splits=cfg[5], pdl=pdl)
+        parts = ops.linear(act, L.down, ops.EPI_PARTIAL, cfg[4], cfg[5], pdl=pdl)
+        return ops.add_rmsnorm_partials(parts, residual, self.norm, self.eps, pdl=pdl)[0]
+
     @torch.inference_mode()
     def forward(self, input_ids: torch.Tensor, positions: torch.Tensor) -> torch.Tensor:
         ctx = get_context()
@@ -352,6 +372,8 @@ class Qwen3ForCausalLM:
         if self.mega_tail and not ctx.is_prefill and input_ids.shape[0] <= self.mega_rows and self.attn[0].k_cache.numel() > 0:
             return self._forward_mega(input_ids, positions, ctx)
         h = ops.embedding(input_ids, self.embed)
+        if not ctx.is_prefill and 0 < h.shape[0] <= self.few_rows and self.attn[0].k_cache.numel() > 0:
+            return self._forward_few_rows(h, positions, ctx)
         residual, in_peer = None, False
         cfg = self.tc_cfg
         tc = self.tc_linear and h.shape[0] <= self.tc_max_rows and (

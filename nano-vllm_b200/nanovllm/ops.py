@@ -292,6 +292,22 @@ def add_rmsnorm_partials(partials: torch.Tensor, residual: torch.Tensor, weight:
     return out, residual
 
 
+def linear_rows(x: torch.Tensor, w: torch.Tensor, norm_w: torch.Tensor | None = None, eps: float = 0.0, add: torch.Tensor | None = None,
+                silu: bool = False, splits: int = 1, pdl: bool = False):
+    """At most 16 rows: x @ w^T (the sum over k in ``splits`` parts), of rmsnorm(x [+ add]) * norm_w where ``norm_w`` is given, through SiluAndMul with
+    ``silu`` (w = [gate; up] rows).  Returns (out, residual): residual is x, or x + add in a tensor of its own."""
+    _need(x, torch.bfloat16, "x"); _need(w, torch.bfloat16, "w")
+    assert x.dim() == 2 and w.dim() == 2 and x.stride(1) == 1 and w.is_contiguous() and x.shape[1] == w.shape[1]
+    assert add is None or (add.dtype == torch.bfloat16 and add.shape == x.shape and add.stride(1) == 1 and norm_w is not None)
+    rows, k = x.shape
+    n = w.shape[0] // 2 if silu else w.shape[0]
+    out = torch.empty(rows, n, dtype=torch.bfloat16, device=x.device)
+    residual = x if add is None else torch.empty(rows, k, dtype=torch.bfloat16, device=x.device)
+    nat.check(nat.load().b200_linear_rows(x.data_ptr(), x.stride(0), _ptr(add), 0 if add is None else add.stride(0), None if add is None else residual.data_ptr(),
+                                          _ptr(norm_w), eps, w.data_ptr(), out.data_ptr(), out.stride(0), rows, n, k, splits, int(silu), int(pdl), _stream()))
+    return out, residual
+
+
 def lm_head_sample(hidden: torch.Tensor, lm_head: torch.Tensor, temperatures: torch.Tensor | None, seed: int, step: int,
                    key_workspace: torch.Tensor, out: torch.Tensor | None = None, index_offset: int = 0,
                    out_keys: torch.Tensor | None = None, step_dev: torch.Tensor | None = None, block_n: int = 128,
