@@ -321,6 +321,11 @@ int b200m_head_rmsnorm_gate(const float* x, const float* floor, const void* w, i
 
 int b200m_moe_tile_rows(void);
 
+/* Router logits: out[n, num_outputs] = x w^T (+ bias) in fp32; x [n, K] in the activation type (row stride x_stride), w [num_outputs, K] and bias fp32.
+ * K and x_stride multiples of 8, x and w 16-byte aligned, at most 1024 outputs; else B200_EUNSUPPORTED. */
+int b200m_moe_logits(const void* x, int64_t x_stride, const float* w, const float* bias, float* out, int n, int num_outputs, int K, int is32,
+                     void* stream);
+
 /* idx / wgt [n, top]: the experts with the largest logits and sigmoid(logit) of each. */
 int b200m_moe_route(const float* logits, int64_t ld, int n, int num_experts, int top, int32_t* idx, float* wgt, void* stream);
 

@@ -102,6 +102,7 @@ MIX_SIGNATURES = {
     "b200m_moe_align": (_i, [_vp, _i, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp]),
     "b200m_moe_gather": (_i, [_vp, _i64, _vp, _vp, _i, _vp, _i, _i, _vp, _vp]),
     "b200m_moe_gemm": (_i, [_vp, _i64, _vp, _vp, _i, _i, _vp, _vp, _i, _vp, _i, _i, _vp, _i, _i, _i, _vp]),
+    "b200m_moe_logits": (_i, [_vp, _i64, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "b200m_moe_experts_workspace_bytes": (_sz, [_i64, _i, _i, _i]),
     "b200m_moe_experts": (_i, [_vp, _i64, _vp, _vp, _i, _i, _i, _i, _vp, _i, _i, _i, _vp, _i, _vp, _vp, _i64, _vp, _vp, _vp, _i, _vp, _sz, _vp]),
     "b200m_moe_combine": (_i, [_vp, _vp, _i, _vp, _vp, _i64, _vp, _vp, _vp, _i, _i, _i, _vp]),

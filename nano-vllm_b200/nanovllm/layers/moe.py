@@ -129,7 +129,7 @@ class RoutedExpertsFF:
     def forward(self, h: torch.Tensor):
         """-> (None, fp32 tensor)"""
         n = h.shape[0]
-        logits = F.linear(h.float(), self.w_router)
+        logits = mixops.moe_logits(h, self.w_router)
         idx, wgt = mixops.moe_route(logits, self.experts, self.top)
         shared = gate = None
         if self.shared_ff:
@@ -201,9 +201,9 @@ class GroupRoutedExpertsFF:
         return out
 
     def forward(self, h: torch.Tensor, x32: torch.Tensor) -> torch.Tensor:
-        """h: the block's input in the activation type, x32: the same rows in fp32 (router input, identity experts) -> fp32."""
+        """h: the block's input in the activation type, x32: the same rows in fp32 (router input, identity experts; without those h will do) -> fp32."""
         n = h.shape[0]
-        logits = F.linear(x32, self.w_router, self.router_bias)
+        logits = mixops.moe_logits(x32, self.w_router, self.router_bias)
         idx, wgt = mixops.moe_route_grouped(logits, self.outputs, self.top, self.correction, self.groups, self.keep, self.experts,
                                             scale=self.route_scale)
         shared = None
@@ -248,7 +248,7 @@ class BiasedTopKExpertsFF(GroupRoutedExpertsFF):
 
     def forward(self, h: torch.Tensor):
         """-> (fp32 [n, width], the extra rows' projection of h or None)."""
-        y = super().forward(h, h if h.dtype == torch.float32 else h.float())
+        y = super().forward(h, h)                                           # (no identity experts here: the rows are the router's input alone)
         return y, (F.linear(h, self.w_extra, self.b_extra) if self.w_extra is not None else None)
 
 

@@ -771,6 +771,20 @@ def moe_capacity(pairs: int, num_experts: int) -> int:
     return (pairs + num_experts * (bm - 1) + bm - 1) // bm * bm
 
 
+def moe_logits(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    """Router logits fp32 [n, outputs] = x w^T (+ bias); x [n, K] in the activation type, w [outputs, K] and bias fp32."""
+    n, K = x.shape
+    assert x.stride(1) == 1 and w.dtype == torch.float32 and w.is_contiguous() and w.shape[1] == K
+    assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.shape == w.shape[:1])
+    out = torch.empty(n, w.shape[0], dtype=torch.float32, device=x.device)
+    rc = nat.load_mix().b200m_moe_logits(x.data_ptr(), x.stride(0), w.data_ptr(), _p(bias), out.data_ptr(), n, w.shape[0], K, _is32(x), _stream())
+    if rc == -2:                                            # B200_EUNSUPPORTED: odd sizes and alignments
+        ops.LAUNCHES[0] -= 1
+        return torch.nn.functional.linear(x.float(), w, bias)
+    nat.check_mix(rc)
+    return out
+
+
 def moe_route(logits: torch.Tensor, num_experts: int, top: int):
     """logits fp32 [n, >= num_experts] -> (idx int32 [n, top], weights fp32 [n, top])."""
     assert logits.dtype == torch.float32 and logits.dim() == 2 and logits.stride(1) == 1

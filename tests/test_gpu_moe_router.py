@@ -1,0 +1,26 @@
+"""Router logits (csrc/moe_router.cu) against float64: token and output tiles full and not, one CTA and clusters along k, a last step of k that is short.  An fp32
+sum of K products in any order is within K 2^-24 of the sum of their magnitudes; sqrt(K) of the 2-norms is what random signs leave: 2e-6 of the result."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,E,K", [(1, 16, 1024), (64, 33, 2048), (33, 40, 2048), (31, 17, 136), (300, 20, 1024), (5000, 40, 512), (6500, 40, 2048), (6401, 17, 264), (2, 41, 264), (70, 100, 768), (3, 1, 8)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_against_float64(dtype, n, E, K, bias):
+    from nanovllm import mixops as mx
+    g = torch.Generator(device="cuda").manual_seed(n + E)
+    x = torch.randn(n, K + 8, device="cuda", generator=g).to(dtype)[:, :K]
+    w = torch.randn(E, K, device="cuda", generator=g)
+    b = torch.randn(E, device="cuda", generator=g) if bias else None
+    want = x.double() @ w.double().t() + (b.double() if bias else 0)
+    got = mx.moe_logits(x, w, b)
+    assert got.shape == (n, E) and (got - want).norm() <= 2e-6 * want.norm()
+
+
+def test_other_sizes_go_to_the_library():
+    from nanovllm import mixops as mx
+    x, w = torch.randn(5, 20, device="cuda"), torch.randn(3, 20, device="cuda")
+    assert torch.allclose(mx.moe_logits(x, w), x @ w.t(), atol=1e-5)
