@@ -146,7 +146,8 @@ int launch_router(const void* x, int64_t x_stride, const float* w, const float* 
     // k over a cluster while the tiles leave SMs idle
     int ctas = 1;
     while (ctas < 8 && (int64_t)tok * outs * ctas * 2 <= 148 && steps >= ctas * 2) ctas *= 2;
-    const int kc = (steps + ctas - 1) / ctas * RO_K;
+    const int per = (steps + ctas - 1) / ctas, kc = per * RO_K;
+    ctas = (steps + per - 1) / per;                         // nobody without columns: such a CTA would not wait for its first copies before its sums take their place
     static B200SmemOptIn opt;
     if (opt.ensure(moe_router_kernel<T, NT, NE>, SM::BYTES) != cudaSuccess) return B200_ECUDA;
     cudaLaunchConfig_t cfg = {};

@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("n,E,K", [(1, 16, 1024), (64, 33, 2048), (33, 40, 2048), (31, 17, 136), (300, 20, 1024), (5000, 40, 512), (6500, 40, 2048), (6401, 17, 264), (2, 41, 264), (70, 100, 768), (3, 1, 8)])
+@pytest.mark.parametrize("n,E,K", [(1, 16, 1024), (64, 33, 2048), (33, 40, 2048), (31, 17, 136), (300, 20, 1024), (5000, 40, 512), (6500, 40, 2048), (6401, 17, 264), (2, 41, 264), (70, 100, 768), (4, 16, 640), (2, 40, 1152), (3, 1, 8)])
 @pytest.mark.parametrize("bias", [False, True])
 def test_against_float64(dtype, n, E, K, bias):
     from nanovllm import mixops as mx
