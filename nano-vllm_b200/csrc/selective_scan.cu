@@ -75,8 +75,10 @@ __global__ void __launch_bounds__(256) causal_conv_kernel(const T* __restrict__ 
     }
 }
 
-// The same for bf16 rows in 8-byte steps: four channels per thread, TB tokens' inputs in flight at once, at most four taps.
-constexpr int CONV_TB = 8;
+// The same for bf16 rows in 8-byte steps: four channels per thread, TB tokens' inputs in flight, at most four taps.
+// Bound by HBM and by the instructions: 8192 tokens of 3072 channels move 100 MB (16 us) and take 28, with batches of eight inputs that were asked for together 39;
+// eight or sixteen in flight 30, tiles of 16 or 64 tokens 30-33 (fewer registers and more warps count for more than more loads a thread).
+constexpr int CONV_TB = 4;
 __global__ void __launch_bounds__(128) causal_conv_vec_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_stride, const __nv_bfloat16* __restrict__ w,
                                                               const __nv_bfloat16* __restrict__ bias, float* conv_state,
                                                               const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q,
@@ -111,14 +113,18 @@ __global__ void __launch_bounds__(128) causal_conv_vec_kernel(const __nv_bfloat1
             win[k][0] = f.x, win[k][1] = f.y, win[k][2] = f.z, win[k][3] = f.w;
         }
     }
+    // a token's place in `in` takes the input CONV_TB tokens on as soon as it is read: that many loads are in flight all along
+    const __nv_bfloat16* next = xs + (int64_t)i0 * x_stride;
+    __nv_bfloat16* to = os + (int64_t)i0 * channels;
+    uint2 in[CONV_TB];
+#pragma unroll
+    for (int j = 0; j < CONV_TB; ++j, next += x_stride) in[j] = i0 + j < i1 ? *reinterpret_cast<const uint2*>(next) : make_uint2(0, 0);
     for (int i = i0; i < i1; i += CONV_TB) {
-        uint2 in[CONV_TB];
 #pragma unroll
-        for (int j = 0; j < CONV_TB; ++j) in[j] = i + j < i1 ? *reinterpret_cast<const uint2*>(xs + (int64_t)(i + j) * x_stride) : make_uint2(0, 0);
-#pragma unroll
-        for (int j = 0; j < CONV_TB; ++j) {
+        for (int j = 0; j < CONV_TB; ++j, next += x_stride, to += channels) {
             if (i + j >= i1) break;
             widen(in[j], win[0]);
+            if (i + j + CONV_TB < i1) in[j] = *reinterpret_cast<const uint2*>(next);
             float a[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -129,7 +135,7 @@ __global__ void __launch_bounds__(128) causal_conv_vec_kernel(const __nv_bfloat1
 #pragma unroll
                 for (int k = 3; k >= 1; --k) win[k][e] = win[k - 1][e];
             }
-            *reinterpret_cast<uint2*>(os + (int64_t)(i + j) * channels) = make_uint2(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]));
+            *reinterpret_cast<uint2*>(to) = make_uint2(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]));
         }
     }
     if (i0 == 0) {                                          // the one thread that reads these channels' history moves it on: what the window holds
