@@ -135,6 +135,14 @@ int b200_paged_prefill(b200_ctx* ctx, int layer, const void* q, int64_t q_stride
                        int total_q, int num_seqs, int max_seqlen_q, int max_seqlen_k,
                        int num_q_heads, int num_kv_heads, float scale, void* stream);
 
+/* b200_store_kv of num_slots rows and b200_paged_prefill of packed prompts in one launch.  B200_EUNSUPPORTED
+ * (nothing launched) for alignments, scales and rows inside the cache that it does not take: call the two instead. */
+int b200_paged_prefill_store(b200_ctx* ctx, int layer, const void* q, int64_t q_stride0, const void* k,
+                             int64_t k_stride0, const void* v, int64_t v_stride0, const int32_t* slot_mapping,
+                             int num_slots, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, void* out,
+                             int64_t out_stride0, int total_q, int num_seqs, int max_seqlen_q, int num_q_heads,
+                             int num_kv_heads, float scale, void* stream);
+
 /* ---- the fused ops around it (the reference's five @torch.compile sites) ---------------- */
 
 /* RMSNorm.rms_forward (layers/layernorm.py:16-26): out = x * rsqrt(mean(x^2)+eps) * w, fp32

@@ -39,6 +39,9 @@ constexpr int THREADS = 512;
 constexpr int ITEM_CAP = 96;            // items per CTA (more items: more CTAs)
 constexpr int LEVELS_CAP = 8192;        // row blocks per sequence that the longest-first order covers (its counters lie where Q will be)
 constexpr float LOG2E = 1.4426950408889634f;
+#ifndef FA_COPY_PAIRS
+#define FA_COPY_PAIRS 8
+#endif
 
 struct FaParams {
     const int32_t* cu_q;
@@ -68,6 +71,57 @@ struct FaParams {
     int64_t gate_stride;
     int gate_elems;
     uint32_t* report;                   // host word for waits that gave up: results of such a launch are undefined
+    // or null: rows of K and V (DV columns each, row r: token r / hkv, head r % hkv) that go into pages of 2^st_shift slots
+    const int32_t* st_slots;            // per token, < 0: not stored
+    const __nv_bfloat16 *st_k, *st_v;
+    int64_t st_k_stride, st_v_stride;
+    __nv_bfloat16 *st_kc, *st_vc;
+    int st_rows, st_shift;
+};
+
+// The copy of this CTA's share of the rows, a part at a time by whichever warp is free (a counter in shared memory deals them out): half a warp per row, all loads of a
+// part before its stores.  (A rotation by single rows, and loads under a condition, ran one row after the other: 283 us for 848 rows; one warp alone took 85.)
+struct FaCopy {
+    static constexpr int PAIRS = FA_COPY_PAIRS, ROWS = 2 * PAIRS;         // rows of a part
+    int end, begin, row, slot;            // of the share; first row of the part this warp has next (end: none), slot of this lane's row in it
+
+    __device__ __forceinline__ void next(const FaParams& p, int* counter, int lane) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(counter, 1);
+        row = min(begin + ROWS * __shfl_sync(0xffffffffu, i, 0), end);
+        slot = lane < ROWS && row + lane < end ? p.st_slots[(row + lane) / p.hkv] : -1;
+    }
+    __device__ __forceinline__ void start(const FaParams& p, int* counter, int lane) {
+        begin = (int)((int64_t)p.st_rows * blockIdx.x / gridDim.x);
+        end = (int)((int64_t)p.st_rows * (blockIdx.x + 1) / gridDim.x);
+        next(p, counter, lane);
+    }
+    __device__ __forceinline__ bool part(const FaParams& p, int* counter, int lane) {
+        if (row >= end) return false;
+        const int in = min(row + lane, end - 1);                         // past the end: a row of this share once more, stored nowhere
+        const int half = lane >> 4, col = (lane & 15) * 8;
+        const int tok = in / p.hkv, head = in - tok * p.hkv;
+        const int to = slot < 0 ? -1 : (((slot >> p.st_shift) * p.hkv + head) << p.st_shift) + (slot & ((1 << p.st_shift) - 1));
+        next(p, counter, lane);
+        uint4 k[PAIRS], v[PAIRS];
+        int dst[PAIRS];
+#pragma unroll
+        for (int j = 0; j < PAIRS; ++j) {
+            const int from = 2 * j + half;
+            dst[j] = __shfl_sync(0xffffffffu, to, from);
+            const int t = __shfl_sync(0xffffffffu, tok, from), h = __shfl_sync(0xffffffffu, head, from);
+            k[j] = *reinterpret_cast<const uint4*>(p.st_k + t * p.st_k_stride + h * DV + col);
+            v[j] = *reinterpret_cast<const uint4*>(p.st_v + t * p.st_v_stride + h * DV + col);
+        }
+#pragma unroll
+        for (int j = 0; j < PAIRS; ++j)
+            if (dst[j] >= 0) {
+                *reinterpret_cast<uint4*>(p.st_kc + (int64_t)dst[j] * DV + col) = k[j];
+                *reinterpret_cast<uint4*>(p.st_vc + (int64_t)dst[j] * DV + col) = v[j];
+            }
+        __syncwarp();
+        return true;
+    }
 };
 
 template <int DQK>
@@ -93,8 +147,8 @@ constexpr uint32_t B_QFULL = 0, B_KFULL = 2, B_VFULL = B_KFULL + NSLOT, B_S = B_
                    B_QEMPTY = B_VRAW + 1 /* from here on 2 arrivals each: the two MMA warps */, B_KEMPTY = B_QEMPTY + 2, B_VEMPTY = B_KEMPTY + NSLOT,
                    B_P = B_VEMPTY + NSLOT /* [tile][buffer]; from here on 128 arrivals each */, B_L = B_P + 4, B_OFREE = B_L + 2, B_VFIX = B_OFREE + 2,
                    B_COUNT = B_VFIX + 1;
-constexpr uint32_t BAR_TMEM = B_COUNT * 8, BAR_DEAD = BAR_TMEM + 4;      // tcgen05.alloc result; set when a wait gave up
-static_assert(BAR_DEAD + 4 <= 320, "barrier area");
+constexpr uint32_t BAR_TMEM = B_COUNT * 8, BAR_DEAD = BAR_TMEM + 4, BAR_COPY = BAR_DEAD + 4;      // tcgen05.alloc result; set when a wait gave up; parts dealt out
+static_assert(BAR_COPY + 4 <= 320, "barrier area");
 
 __device__ __forceinline__ void fa_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
@@ -205,8 +259,8 @@ struct FaSlot {
     }
 };
 
-// GENERAL: scores with a distance bias, or a scale that is not positive.
-template <int DQK, bool PAIR_HEADS, bool GENERAL>
+// GENERAL: scores with a distance bias, or a scale that is not positive.  STORE: warps 8-11, between items, and 15 scatter the step's K and V rows into their pages.
+template <int DQK, bool PAIR_HEADS, bool GENERAL, bool STORE>
 __global__ void __launch_bounds__(THREADS, 1)
 fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
           const __grid_constant__ CUtensorMap tm_k2, const __grid_constant__ FaParams p) {
@@ -220,6 +274,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
     auto fa_wait = [&](uint32_t b, uint32_t parity) { return bounded_wait(b, parity, dead, p.report); };
     auto lane_wait = [&](uint32_t b, uint32_t parity) { return bounded_wait_as<false>(b, parity, dead, p.report); };
     int4* list = reinterpret_cast<int4*>(smem + L::kOffList);
+    int* parts = reinterpret_cast<int*>(smem + L::kOffBar + BAR_COPY);
     float* lbuf = reinterpret_cast<float*>(smem + L::kOffL);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -227,6 +282,7 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
         for (uint32_t i = 0; i < B_COUNT; ++i) mbar_init(bar(i), i >= B_P ? 128 : i >= B_QEMPTY ? 2 : 1);
         mbar_fence_init();
         *reinterpret_cast<volatile uint32_t*>(smem + L::kOffBar + BAR_DEAD) = 0;
+        if (STORE) *reinterpret_cast<volatile int*>(smem + L::kOffBar + BAR_COPY) = 0;
     }
     if (warp == 12) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars + BAR_TMEM), "r"(512u) : "memory");
@@ -405,6 +461,8 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         uint32_t items[2] = {0, 0}, fixes = 0;
         FaSlot vs;
+        FaCopy copy;
+        if (STORE) copy.start(p, parts, lane);
         const bool wide = (reinterpret_cast<uintptr_t>(p.out) & 31) == 0 && (p.out_stride & 15) == 0;      // 32-byte stores: whole sectors
         for (int e = 0; e < n_items; ++e) {
             const FaItem it = fa_item<PAIR_HEADS>(p, list, e);
@@ -495,7 +553,9 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 fa_arrive(bar(B_OFREE + t));
                 ++items[t];
             }
+            if (STORE) copy.part(p, parts, lane);                        // while the next item's products run
         }
+        if (STORE) while (copy.part(p, parts, lane)) {}
     } else if (warp < 14) {
         // ---- products of one tile (all lanes walk and wait, one issues) -------------------------------------------------------
         const int t = warp - 12;
@@ -627,6 +687,10 @@ fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 if (L::kQBufs > 1 && j == ask && e + 1 < n_items && !load_q(e + 1)) goto leave;
             }
         }
+    } else if (STORE) {
+        FaCopy copy;
+        copy.start(p, parts, lane);
+        while (copy.part(p, parts, lane)) {}
     }
 leave:
     __syncwarp();
@@ -639,7 +703,7 @@ leave:
 
 // Launch; the caller has filled everything but hp / max_rb and built the maps (box of Q: 64 x 128, of K and V: 64 x box_rows or 64 x BN;
 // tk2 is only read with 192-wide heads).
-template <int DQK, bool PAIR_HEADS, bool GENERAL>
+template <int DQK, bool PAIR_HEADS, bool GENERAL, bool STORE = false>
 int fa_launch(FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tk2, int total_q, int max_seqlen_q,
               cudaStream_t stream) {
     constexpr int RT = PAIR_HEADS ? BM : 2 * BM;
@@ -648,7 +712,7 @@ int fa_launch(FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const C
     if (const int rc = b200wait::launch_word(&p.report); rc != B200_OK) return rc;
     if (p.hp >= 2048 || p.max_rb >= (1 << 20)) return B200_EUNSUPPORTED;
     static B200SmemOptIn optin;
-    B200_CUDA_CHECK((b200_ctx*)nullptr, optin.ensure(fa_kernel<DQK, PAIR_HEADS, GENERAL>, FaSmem<DQK>::kTotal));
+    B200_CUDA_CHECK((b200_ctx*)nullptr, optin.ensure(fa_kernel<DQK, PAIR_HEADS, GENERAL, STORE>, FaSmem<DQK>::kTotal));
     int dev = 0, sms = 0;
     B200_CUDA_CHECK((b200_ctx*)nullptr, cudaGetDevice(&dev));
     B200_CUDA_CHECK((b200_ctx*)nullptr, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -656,7 +720,7 @@ int fa_launch(FaParams& p, const CUtensorMap& tq, const CUtensorMap& tk, const C
     if (bound > (1ll << 30)) return B200_EUNSUPPORTED;
     int64_t grid = bound < sms ? bound : sms;
     if ((bound + grid - 1) / grid > ITEM_CAP) grid = (bound + ITEM_CAP - 1) / ITEM_CAP;
-    B200_LAUNCH((fa_kernel<DQK, PAIR_HEADS, GENERAL>), dim3((unsigned)grid), THREADS, (FaSmem<DQK>::kTotal), stream, tq, tk, tv, tk2, p);
+    B200_LAUNCH((fa_kernel<DQK, PAIR_HEADS, GENERAL, STORE>), dim3((unsigned)grid), THREADS, (FaSmem<DQK>::kTotal), stream, tq, tk, tv, tk2, p);
     return b200_launch_status(nullptr);
 }
 

@@ -9,7 +9,7 @@ int b200_prefill_fa_launch(b200_ctx* ctx, int layer, const void* q, int64_t q_st
                            const void* v, int64_t v_stride0, const int32_t* cu_q, const int32_t* cu_k,
                            const int32_t* block_tables, int bt_stride, void* out, int64_t out_stride0, int total_q,
                            int num_seqs, int max_seqlen_q, int num_q_heads, int num_kv_heads, float scale,
-                           cudaStream_t stream) {
+                           const int32_t* slot_mapping, int num_slots, cudaStream_t stream) {
     constexpr int D = B200_HEAD_DIM;
     CUtensorMap tq, tk, tv;
     if (!make_map(&tq, q, (uint64_t)num_q_heads * D, (uint64_t)total_q, (uint64_t)q_stride0, BM)) return B200_EUNSUPPORTED;
@@ -43,8 +43,24 @@ int b200_prefill_fa_launch(b200_ctx* ctx, int layer, const void* q, int64_t q_st
             !make_map(&tv, v, (uint64_t)num_kv_heads * D, (uint64_t)total_q, (uint64_t)v_stride0, BN))
             return B200_EUNSUPPORTED;
     }
+    if (slot_mapping) {                  // rows, and the layer's cache rows, are named by 32 bits
+        if (block_tables || scale <= 0.f || ctx->num_blocks * ctx->num_kv_heads * ctx->block_size >= (1ll << 31) || (int64_t)num_slots * num_kv_heads >= (1ll << 31) - 256)
+            return B200_EUNSUPPORTED;
+        p.st_slots = slot_mapping;
+        p.st_k = static_cast<const __nv_bfloat16*>(k);
+        p.st_v = static_cast<const __nv_bfloat16*>(v);
+        p.st_k_stride = k_stride0;
+        p.st_v_stride = v_stride0;
+        p.st_kc = ctx->k_layer(layer);
+        p.st_vc = ctx->v_layer(layer);
+        p.st_rows = num_slots * num_kv_heads;
+        p.st_shift = ctx->block_shift;
+    }
     // An even head group: the item's two tiles are two heads that share every K and V tile.  Else (groups of 1, 3, ..): 256 rows of one head.
     const bool pair = (num_q_heads / num_kv_heads) % 2 == 0;
+    if (slot_mapping)
+        return pair ? fa_launch<D, true, false, true>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream)
+                    : fa_launch<D, false, false, true>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream);
     if (scale > 0.f)
         return pair ? fa_launch<D, true, false>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream) : fa_launch<D, false, false>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream);
     return pair ? fa_launch<D, true, true>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream) : fa_launch<D, false, true>(p, tq, tk, tv, tk, total_q, max_seqlen_q, stream);

@@ -30,6 +30,7 @@ SIGNATURES = {
     "b200_decode_small_splits": (_i, [_vp, _i, _i, _i]),
     "b200_paged_prefill": (_i, [_vp, _i, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _vp, _i, _vp, _i64,
                                  _i, _i, _i, _i, _i, _i, _f, _vp]),
+    "b200_paged_prefill_store": (_i, [_vp, _i, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _i, _f, _vp]),
     "b200_rmsnorm": (_i, [_vp, _i64, _vp, _vp, _i64, _i, _i, _f, _vp]),
     "b200_add_rmsnorm": (_i, [_vp, _vp, _vp, _vp, _i, _i, _f, _vp]),
     "b200_qknorm_rope_store": (_i, [_vp, _i, _vp, _i64, _i, _i, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp]),

@@ -25,12 +25,16 @@ def store_kvcache(key: torch.Tensor, value: torch.Tensor, k_cache: torch.Tensor,
     ``k_cache`` / ``v_cache`` must be the layer views of the cache bound with ``ops.bind_kv_cache``;
     they are accepted for signature compatibility and checked, the library addresses the bound cache.
     """
+    _check_store(key, value, k_cache, slot_mapping)
+    ops.store_kv(layer_id, key, value, slot_mapping)
+
+
+def _check_store(key: torch.Tensor, value: torch.Tensor, k_cache: torch.Tensor, slot_mapping: torch.Tensor) -> None:
     n, num_heads, head_dim = key.shape
     assert key.stride(-1) == 1 and value.stride(-1) == 1
     assert key.stride(1) == head_dim and value.stride(1) == head_dim
     assert slot_mapping.numel() == n
     assert k_cache.dim() == 4 and k_cache.shape[1] == num_heads and k_cache.shape[3] == head_dim
-    ops.store_kv(layer_id, key, value, slot_mapping)
 
 
 class Attention(nn.Module):
@@ -51,6 +55,10 @@ class Attention(nn.Module):
         """
         ctx = get_context()
         have_cache = self.k_cache.numel() > 0 and self.v_cache.numel() > 0
+        if have_cache and not kv_stored and ctx.is_prefill and ctx.block_tables is None:
+            _check_store(k, v, self.k_cache, ctx.slot_mapping)
+            return ops.paged_prefill_store(self.layer_id, q, k, v, ctx.slot_mapping, ctx.cu_seqlens_q, ctx.cu_seqlens_k, ctx.max_seqlen_q, ctx.max_seqlen_k,
+                                           self.scale)
         if have_cache and not kv_stored:
             store_kvcache(k, v, self.k_cache, self.v_cache, ctx.slot_mapping, self.layer_id)
         if ctx.is_prefill:

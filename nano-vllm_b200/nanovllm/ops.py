@@ -134,6 +134,35 @@ def paged_prefill(layer: int, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q:
     return out
 
 
+def paged_prefill_store(layer: int, q, k, v, slot_mapping, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: int, max_seqlen_k: int, scale: float) -> torch.Tensor:
+    """``store_kv`` and ``paged_prefill`` of packed prompts: as one launch where the attention is long enough to hide the copies."""
+    t, hq, d = q.shape
+    if k.shape == v.shape and slot_mapping.numel() == k.shape[0] and prefill_hides_store(t, cu_seqlens_q.numel() - 1, hq, k.shape[1]):
+        for x, n in ((q, "q"), (k, "k"), (v, "v")):
+            _need(x, torch.bfloat16, n)
+        for x, n in ((slot_mapping, "slot_mapping"), (cu_seqlens_q, "cu_seqlens_q"), (cu_seqlens_k, "cu_seqlens_k")):
+            _need(x, torch.int32, n)
+        assert all(x.stride(2) == 1 and x.stride(1) == d for x in (q, k, v))
+        out = torch.empty((t, hq, d), dtype=q.dtype, device=q.device)
+        h = nat.handle()
+        rc = h.lib.b200_paged_prefill_store(h.ptr, layer, q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
+                                            slot_mapping.data_ptr(), slot_mapping.numel(), cu_seqlens_q.data_ptr(), cu_seqlens_k.data_ptr(), out.data_ptr(),
+                                            out.stride(0), t, cu_seqlens_q.numel() - 1, int(max_seqlen_q), hq, k.shape[1], scale, _stream())
+        if rc != -2:                                        # B200_EUNSUPPORTED
+            nat.check(rc, h.ptr)
+            return out
+        LAUNCHES[0] -= 1
+    store_kv(layer, k, v, slot_mapping)
+    return paged_prefill(layer, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, scale)
+
+
+def prefill_hides_store(total: int, seqs: int, heads: int, kv_heads: int) -> bool:
+    """Whether the attention of packed prompts is long enough to hide the copies of their K and V.  Many short prompts are not: their items are over before a part
+    is copied.  us (inside / two launches), 16 heads on 8: 28 x 561 84 / 107, 64 x 128 40 / 46, 64 x 64 25 / 30, 256 x 64 92 / 99; 8 on 8: 256 x 64 71 / 72,
+    256 x 32 61 / 60, 256 x 16 57 / 52; 32 on 8: 256 x 16 147 / 137, 512 x 32 285 / 277, 64 x 32 36 / 40."""
+    return total >= 64 * seqs or seqs <= 64
+
+
 # ---- fused ops around it ---------------------------------------------------------
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor | None = None) -> torch.Tensor:
     """x: contiguous [..., cols], or 2-D with unit inner stride (a column slice of a wider row)."""
