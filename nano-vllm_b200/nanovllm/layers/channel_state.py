@@ -87,7 +87,6 @@ class _ChannelStateMixer:
         self.in_cols = _pad8(at)
         self.w_in = torch.zeros(self.in_cols, self.width, dtype=self.dtype, device=self.device)
         self.second = {leaf[:-1] + "2": torch.zeros(cols, _pad8(new[leaf]), dtype=self.dtype, device=self.device) for leaf, cols in self.low_rank()}
-        self._second_t = {leaf: w.t() for leaf, w in self.second.items()}           # views
 
     def _cols(self, proj: torch.Tensor, leaf: str) -> torch.Tensor:
         a, rows = self.at[leaf]
@@ -100,7 +99,7 @@ class _ChannelStateMixer:
         t = proj[:, a:a + w.shape[1]]
         if f32 and self._mm_f32_out:
             try:
-                return torch.mm(t, self._second_t[leaf[:-1] + "2"], out_dtype=torch.float32)
+                return torch.mm(t, w.t(), out_dtype=torch.float32)
             except (RuntimeError, TypeError):
                 self._mm_f32_out = False
         y = F.linear(t, w)
