@@ -107,7 +107,7 @@ class Qwen3ForCausalLM:
         # the launches they replace, bit for bit
         fits = all(k % 512 == 0 and k <= 3072 and n % 16 == 0 for n, k in ((self.q_size + 2 * self.kv_size, self.hidden), (self.hidden, self.q_size),
                                                                            (self.inter, self.hidden), (self.hidden, self.inter)))
-        self.few_rows = 16 if mode == "auto" and self.tc_linear and tp_size == 1 and fits and max(tcc[3], tcc[5]) <= 8 else 0
+        self.few_rows = min(16, self.tc_max_rows) if mode == "auto" and self.tc_linear and tp_size == 1 and fits and max(tcc[3], tcc[5]) <= 8 else 0
         # B200_TAIL=mega: in decode steps of up to 256 rows on one GPU, everything between two attention kernels
         # (o_proj, add+norm, gate_up+SiluAndMul, down_proj, add+norm, the next layer's qkv_proj) is ONE persistent launch
         # (csrc/layer_tail.cu) instead of seven.  Measured 58-70 us per layer against 30 us for the chain (r02_layer_tail_microbench.json):
