@@ -236,7 +236,7 @@ class Qwen3ForCausalLM:
     def _attention(self, li: int, qkv: torch.Tensor, positions: torch.Tensor, ctx, before_attention=None, no_pdl: bool = False):
         """q/k-norm + RoPE + KV append + attention on the raw qkv projection (one or two launches) -> [t, q_size].
         ``before_attention`` runs right before the attention launch (cross-stream waits of the two-stream step);
-        ``no_pdl``: that launch carries no programmatic-dependent-launch attribute.  Decode steps only when either is used."""
+        ``no_pdl``: that launch carries no programmatic-dependent-launch attribute (decode steps only)."""
         import contextlib
         L, attn = self.layers[li], self.attn[li]
         hq, hkv, d, t = self.num_heads, self.num_kv_heads, self.head_dim, qkv.shape[0]
@@ -256,7 +256,8 @@ class Qwen3ForCausalLM:
             v = qkv[:, self.q_size + self.kv_size:].view(t, hkv, d)
             if before_attention is not None:
                 before_attention()
-                with plain:                                   # decode: the operator's decode branch, on this half's metadata
+            if no_pdl:                                        # decode: the operator's decode branch, on the metadata given
+                with plain:
                     o = ops.paged_decode(li, q, ctx.block_tables, ctx.context_lens, attn.scale)
             else:
                 o = attn(q, k, v, kv_stored=True)

@@ -64,3 +64,11 @@ def test_the_row_limit_of_the_own_products_holds_for_few_rows(most, monkeypatch)
     got, want, _, model = run(monkeypatch, {"B200_LINEAR_MAX_ROWS": str(most)})
     assert max(FewRowsOps.rows_seen, default=0) <= most
     close(got, want)
+
+
+@pytest.mark.parametrize("heads,fused_max", [(4, None), (4, 0), (8, None)])
+def test_attention_of_few_rows_starts_when_the_projection_has_ended(heads, fused_max, monkeypatch):
+    """Both forms of the attention behind it: without the early-launch attribute."""
+    got, want, fake, _ = run(monkeypatch, {}, fused_max, heads)
+    assert fake.calls["linear_rows"] > 0 and FewRowsOps.attention_pdl and not any(FewRowsOps.attention_pdl)
+    close(got, want)
