@@ -271,12 +271,12 @@ int b200m_channel_state(const void* x, int64_t stride, int q_off, int k_off, int
 
 /* The delta rule of b200m_channel_state over prompt portions in bf16, on the tensor cores (csrc/channel_delta.cu), for decays of at most one (rate[h]
  * never above zero).  dim <= 128, dim and vdim multiples of 8, x, decay_in, decay_bias, state and workspace 16-byte aligned, offsets and strides of
- * whole 16-byte pieces; else B200_EUNSUPPORTED.  max_q: at least the longest portion.  The workspace is at most 256 MiB (the answer to
- * sizes of 0), or one chunk of sixteen tokens of every sequence: longer steps are cut into several launch pairs. */
-size_t b200m_channel_delta_workspace_bytes(int num_seqs, int max_q, int num_heads);
+ * whole 16-byte pieces; else B200_EUNSUPPORTED.  The workspace's rows are a chunk of sixteen tokens of all heads; workspace_bytes is what a step of n tokens in
+ * num_seqs sequences has (n / 16 + num_seqs rows, whatever the lengths).  Any smaller number of whole rows will do: the step is then cut into several launch pairs. */
+size_t b200m_channel_delta_workspace_bytes(int n, int num_seqs, int num_heads);
 int b200m_channel_delta_prompts(const void* x, int64_t stride, int q_off, int k_off, int v_off, const void* write_in, int64_t write_stride,
                                 const float* decay_in, int64_t decay_stride, const float* rate, const float* decay_bias, float decay_sign, float* state,
-                                const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k, float* out, int n, int num_seqs, int max_q,
+                                const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k, float* out, int n, int num_seqs,
                                 int num_heads, int num_kv_heads, int dim, int vdim, float q_scale, void* workspace, size_t workspace_bytes,
                                 void* stream);
 

@@ -17,8 +17,9 @@
 // 2.4e-7 of their norm off, a key channel of the state 1e-7 to 1.8e-7 (median); the fp32-pipe form of recurrent_mix.cu 1e-7 to 1.9e-6 and 0.7e-7 to 1.8e-6.  (fp16 pairs, 22
 // bits, with half of the products: 1.2e-7 to 3.5e-7, and nothing left of a state below 2^-25 of one; both kernels together 357 us where these take 440.)
 //
-// Measured on a B200, 16 heads of 128 x 128, both kernels together against that form: 4 x 2048 tokens 465 us against 668, 1 x 4096 635 against
-// 1314, 16 x 1000 926 against 1126, 12 x 600 433 against 544, 16 x 64 73 against 87.
+// Measured on a B200, 16 heads of 128 x 128, both kernels together against that form: 4 x 2048 tokens 447 us against 669, 1 x 4096 634 against
+// 1314, 16 x 1000 872 against 1127, 12 x 600 408 against 544, 16 x 64 71 against 84, 1 x 2048 beside 511 single tokens 870 against 1130.  With the workspace laid out as
+// sequences x longest portion, and a launch pair for what of that fitted 256 MiB, that last step was 128 pairs of nearly empty grids and took 6.7 ms.
 #include "mma_common.cuh"
 #include "state_common.cuh"
 
@@ -74,6 +75,26 @@ __device__ __forceinline__ float cd_sum(uint64_t v) {
     const float2 f = cd_two(v);
     return f.x + f.y;
 }
+// Rows of the workspace (a row: a chunk, all heads).  Sequence s has those from here on, a place that needs no sum over the sequences in front of it:
+// ceil(l / 16) <= floor((q + l) / 16) - floor(q / 16) + 1, so n / 16 + sequences rows hold every step of n tokens, whatever its lengths.
+__device__ __forceinline__ int chunk_row(int q0, int s) { return q0 / CD_L + s; }
+// The sequence that a row is of (-1: none), 128 at a time by a whole warp
+__device__ __forceinline__ int row_sequence(const int32_t* __restrict__ cu_q, int num_seqs, int row, int lane) {
+    int upto = 0;
+    for (int s0 = 0; s0 < num_seqs; s0 += 128) {
+        int start[4], have = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int s = s0 + 32 * i + lane;
+            start[i] = s < num_seqs ? chunk_row(cu_q[s], s) : 0x7fffffff;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) have += __popc(__ballot_sync(0xffffffffu, start[i] <= row));
+        upto += have;
+        if (have < 128) break;
+    }
+    return upto - 1;
+}
 // a pair of floats -> three bf16 terms each: their roundings, the roundings of what these leave, and the rest.  3 x 8 bits: nothing is lost
 __device__ __forceinline__ void split3(uint64_t v, uint32_t& a, uint32_t& b, uint32_t& c) {
     const float2 f = cd_two(v);
@@ -90,7 +111,7 @@ __device__ __forceinline__ void split3(uint64_t v, uint32_t& a, uint32_t& b, uin
 // (weighted least squares, reweighted until the ripples are equal (Lawson); coefficients rounded one by one, the rest fitted again; the first of log1p is
 // one).  Off by 3.3e-8 of log1p(y) and 3e-9 of 2^f, before fp32's own rounding.  The exponent is reduced in two parts (Cody and Waite).  2^f is 1 + f (...), so
 // that a decay next to one is rounded once: the power unit's last bits add up over a sequence.  Over |x| <= 100 and rates of -1e-3 to -16 no further from
-// float64 than expf and log1pf (rate -400: 1.5 times), in half of their instructions.  Below 2^-126: zero.
+// float64 than expf and log1pf (rate -400: 1.5 times).  Below 2^-126: zero.
 __device__ __forceinline__ float decay_fit(float x, float rate) {
     constexpr float L[9] = {1.f, -0.49999648f, 0.3332133f, -0.24857217f, 0.19153848f, -0.13754188f, 0.07920883f, -0.0300683f, 0.0053654225f};
     constexpr float Q[6] = {0.6931472f, 0.24022648f, 0.0555036f, 0.009618506f, 0.0013390806f, 0.00015326463f};
@@ -133,7 +154,7 @@ __device__ __forceinline__ void mma_rest(float (&c)[4], const uint32_t (&a)[3][4
 // ---- first kernel: decays, A, B, T, W, Q ------------------------------------------------------------------------------------------------
 // A_ts and B_ts need the decays between s and t.  Pairs of tokens are taken by the largest of four levels (half blocks of 8, 4, 2, 1 tokens) whose middle
 // parts them: with the middle m, k_t and q_t take g_m ... g_t, k_s takes g_(s+1) ... g_(m-1), all at most one, and a level is one product of
-// [8 k rows, 8 q rows] with [8 k rows].  Bound by its instructions: 168 us for 8192 tokens of 16 heads (operands as fp16 pairs 137).
+// [8 k rows, 8 q rows] with [8 k rows].  Bound by its instructions: 161 us for 8192 tokens of 16 heads (operands as fp16 pairs 137).
 constexpr int CP_THREADS = 128;
 struct CpSmem {
     static constexpr int RAW_K = 0, RAW_Q = CD_L * CD_D * 2, A = 2 * RAW_Q, B = A + CD_L * CD_L * 4, T = B + CD_L * CD_L * 4,
@@ -192,13 +213,14 @@ __device__ __forceinline__ void level_factors(const uint64_t (&g)[CD_L / 2], con
 __global__ void __launch_bounds__(CP_THREADS, 4) channel_delta_prepare_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t stride, int q_off, int k_off, const __nv_bfloat16* __restrict__ write_in, int64_t write_stride,
     const float* __restrict__ decay_in, int64_t decay_stride, const float* __restrict__ rate, const float* __restrict__ bias, float sign,
-    const int32_t* __restrict__ cu_q, unsigned char* __restrict__ ws, int H, int G, int dim, int first, int chunks) {
+    const int32_t* __restrict__ cu_q, unsigned char* __restrict__ ws, int num_seqs, int H, int G, int dim, int first_row) {
     B200_PDL_SYNC();
     using SM = CpSmem;
     extern __shared__ __align__(128) unsigned char cp_smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t4 = lane & 3, s = blockIdx.y;
-    const int h = blockIdx.x % H, c = blockIdx.x / H;
-    const int q0 = cu_q[s], qlen = cu_q[s + 1] - q0, t0 = (first + c) * CD_L;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t4 = lane & 3;
+    const int h = blockIdx.x % H, row = first_row + blockIdx.x / H, s = row_sequence(cu_q, num_seqs, row, lane);
+    if (s < 0) return;
+    const int q0 = cu_q[s], qlen = cu_q[s + 1] - q0, t0 = (row - chunk_row(q0, s)) * CD_L;
     if (t0 >= qlen) return;
     const int len = min(CD_L, qlen - t0);
     const uint32_t sbase = smem_u32(cp_smem);
@@ -329,7 +351,7 @@ __global__ void __launch_bounds__(CP_THREADS, 4) channel_delta_prepare_kernel(
     __syncthreads();
     level_sums(2 >> (warp >> 1));
     __syncthreads();
-    unsigned char* wp = ws + (((int64_t)s * chunks + c) * H + h) * (int64_t)CW_BYTES;
+    unsigned char* wp = ws + (int64_t)blockIdx.x * CW_BYTES;
     if (warp == 0) {
         // a lane has a column of T.  Places above the diagonal stay zero; a row takes the entries up to its own token alone
         const int j = lane & (CD_L - 1);
@@ -495,24 +517,25 @@ __device__ __forceinline__ void cd_arrive(int id) { asm volatile("bar.arrive %0,
 
 // Eight consumer warps: warp 2 p + hf holds 16 value columns (p) and 64 of the channels (hf), so that two warps per scheduler hide each other's waits;
 // a pair adds its two halves of W S and of Q S through shared memory.  Two copying warps, two chunks ahead.  Bound by the consumers' chain per chunk:
-// 2.3 us of 156 products (fp16 pairs: 84 products, 1.67 us, of one warp per 16 columns and all channels 4.0).
+// 2.2 us of 156 products (fp16 pairs: 84 products, 1.67 us, of one warp per 16 columns and all channels 4.0).
 constexpr int CD_THREADS = 320;
 __global__ void __launch_bounds__(CD_THREADS, 1) channel_delta_chunks_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t stride, int v_off, const unsigned char* __restrict__ ws, float* __restrict__ state,
     const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q, const int32_t* __restrict__ cu_k, float* __restrict__ out, int H, int dim,
-    int vdim, float q_scale, int first, int chunks) {
+    int vdim, float q_scale, int first_row, int rows_here) {
     B200_PDL_SYNC();
     using SM = CdSmem;
     extern __shared__ __align__(128) unsigned char cd_smem[];
     const int h = blockIdx.x, s = blockIdx.y, col0 = blockIdx.z * CD_VC, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const SeqSpan sp = seq_span(cu_q, cu_k, nullptr, s);
-    const int nch = min(chunks, (sp.qlen + CD_L - 1) / CD_L - first);       // this launch's chunks
+    const int row = chunk_row(sp.q0, s), first = max(0, first_row - row);   // first of this launch's chunks
+    const int nch = min((sp.qlen + CD_L - 1) / CD_L, first_row + rows_here - row) - first;
     if (nch <= 0) return;
     const uint32_t sbase = smem_u32(cd_smem);
     const int row0 = sp.q0 + first * CD_L, rows = sp.qlen - first * CD_L;   // its tokens (and the later launches')
     if (warp >= 8) {
         const int pt = threadIdx.x & 63;
-        const unsigned char* wp = ws + ((int64_t)s * chunks * H + h) * (int64_t)CW_BYTES + pt * 16;
+        const unsigned char* wp = ws + ((int64_t)(row + first - first_row) * H + h) * CW_BYTES + pt * 16;
         const __nv_bfloat16* vp = x + (int64_t)row0 * stride + v_off + (int64_t)h * vdim + col0 + (pt & 7) * 8;
         const bool v_in = col0 + (pt & 7) * 8 < vdim;
         auto fetch = [&](int c) {
@@ -707,51 +730,45 @@ __global__ void __launch_bounds__(CD_THREADS, 1) channel_delta_chunks_kernel(
     }
 }
 
-// Chunks of every sequence that a launch pair handles: what a workspace of WS_BOUND bytes holds, but at least one
-constexpr int64_t WS_BOUND = 256ll << 20;
-int64_t chunks_per_launch(int num_seqs, int max_q, int num_heads) {
-    const int64_t all = ((int64_t)max_q + CD_L - 1) / CD_L, fit = WS_BOUND / ((int64_t)num_seqs * num_heads * CW_BYTES);
-    return all < fit ? all : fit > 0 ? fit : 1;
-}
-
 }  // namespace
 
-extern "C" size_t b200m_channel_delta_workspace_bytes(int num_seqs, int max_q, int num_heads) {
-    if (max_q <= 0 || num_seqs <= 0 || num_heads <= 0) return (size_t)WS_BOUND;
-    return (size_t)chunks_per_launch(num_seqs, max_q, num_heads) * num_seqs * (size_t)num_heads * CW_BYTES;
+extern "C" size_t b200m_channel_delta_workspace_bytes(int n, int num_seqs, int num_heads) {
+    if (n < 0 || num_seqs < 0 || num_heads <= 0) return 0;
+    return ((size_t)(n / CD_L) + (size_t)num_seqs) * (size_t)num_heads * CW_BYTES;
 }
 
 extern "C" int b200m_channel_delta_prompts(const void* x, int64_t stride, int q_off, int k_off, int v_off, const void* write_in, int64_t write_stride,
                                            const float* decay_in, int64_t decay_stride, const float* rate, const float* decay_bias, float decay_sign,
                                            float* state, const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k, float* out, int n,
-                                           int num_seqs, int max_q, int num_heads, int num_kv_heads, int dim, int vdim, float q_scale, void* workspace,
+                                           int num_seqs, int num_heads, int num_kv_heads, int dim, int vdim, float q_scale, void* workspace,
                                            size_t workspace_bytes, void* stream) {
     if (!x || !write_in || !decay_in || !state || !state_slots || !out || !rate || !decay_bias || !cu_q || !cu_k) return B200_EINVAL;
     if (num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads || dim <= 0 || vdim <= 0) return B200_EINVAL;
-    if (decay_stride < (int64_t)num_heads * dim || n < 0 || max_q < 0) return B200_EINVAL;
+    if (decay_stride < (int64_t)num_heads * dim || n < 0) return B200_EINVAL;
     if (dim > CD_D || dim % 8 || vdim % 8 || stride % 8 || q_off % 8 || k_off % 8 || v_off % 8 || decay_stride % 4) return B200_EUNSUPPORTED;
     for (const void* p : {x, static_cast<const void*>(decay_in), static_cast<const void*>(decay_bias), static_cast<const void*>(state),
                           static_cast<const void*>(workspace)})
         if (reinterpret_cast<uintptr_t>(p) % 16) return B200_EUNSUPPORTED;
-    if (num_seqs <= 0 || n == 0 || max_q == 0) return B200_OK;
+    if (num_seqs <= 0 || n == 0) return B200_OK;
     if (num_seqs > 65535 || decay_stride > (1 << 27) || (vdim + CD_VC - 1) / CD_VC > 65535) return B200_EUNSUPPORTED;
-    if (!workspace || workspace_bytes < b200m_channel_delta_workspace_bytes(num_seqs, max_q, num_heads)) return B200_EINVAL;
+    const int64_t all = (int64_t)(n / CD_L) + num_seqs, fit = (int64_t)(workspace_bytes / ((size_t)num_heads * CW_BYTES));
+    const int rows = (int)(all < fit ? all : fit);                                          // of a launch pair
+    if (!workspace || rows <= 0) return B200_EINVAL;
+    if ((int64_t)num_heads * rows > 0x7fffffff || all > 0x7fffffff - rows) return B200_EUNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
     unsigned char* ws = static_cast<unsigned char*>(workspace);
-    const int all = (max_q + CD_L - 1) / CD_L, chunks = (int)chunks_per_launch(num_seqs, max_q, num_heads);
-    const int64_t blocks = (int64_t)num_heads * chunks;
-    if (blocks > 0x7fffffff) return B200_EUNSUPPORTED;
     static B200SmemOptIn opt, opt_prepare;
     if (opt.ensure(channel_delta_chunks_kernel, CdSmem::BYTES) != cudaSuccess) return B200_ECUDA;
     if (opt_prepare.ensure(channel_delta_prepare_kernel, CpSmem::BYTES) != cudaSuccess) return B200_ECUDA;
-    for (int first = 0; first < all; first += chunks) {
-        B200_LAUNCH((channel_delta_prepare_kernel), dim3((unsigned)blocks, num_seqs), CP_THREADS, CpSmem::BYTES, st, xb, stride, q_off,
+    for (int first = 0; first < all; first += rows) {
+        const int here = (int)(all - first < rows ? all - first : rows);
+        B200_LAUNCH((channel_delta_prepare_kernel), (unsigned)(num_heads * here), CP_THREADS, CpSmem::BYTES, st, xb, stride, q_off,
                     k_off, static_cast<const __nv_bfloat16*>(write_in), write_stride, decay_in, decay_stride, rate, decay_bias, decay_sign, cu_q, ws,
-                    num_heads, num_kv_heads, dim, first, chunks);
+                    num_seqs, num_heads, num_kv_heads, dim, first);
         if (const int rc = b200_launch_status(nullptr); rc != B200_OK) return rc;
         B200_LAUNCH((channel_delta_chunks_kernel), dim3(num_heads, num_seqs, (vdim + CD_VC - 1) / CD_VC), CD_THREADS, CdSmem::BYTES, st, xb, stride, v_off,
-                    static_cast<const unsigned char*>(ws), state, state_slots, cu_q, cu_k, out, num_heads, dim, vdim, q_scale, first, chunks);
+                    static_cast<const unsigned char*>(ws), state, state_slots, cu_q, cu_k, out, num_heads, dim, vdim, q_scale, first, here);
         if (const int rc = b200_launch_status(nullptr); rc != B200_OK) return rc;
     }
     return B200_OK;

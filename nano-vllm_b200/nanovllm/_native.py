@@ -71,7 +71,7 @@ MIX_SIGNATURES = {
     "b200m_diag_scan": (_i, [_vp, _i64, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _i, _vp]),
     "b200m_gated_delta": (_i, [_vp, _i64, _i, _i, _i, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _vp]),
     "b200m_channel_delta_workspace_bytes": (_sz, [_i, _i, _i]),
-    "b200m_channel_delta_prompts": (_i, [_vp, _i64, _i, _i, _i, _vp, _i64, _vp, _i64, _vp, _vp, _f, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
+    "b200m_channel_delta_prompts": (_i, [_vp, _i64, _i, _i, _i, _vp, _i64, _vp, _i64, _vp, _vp, _f, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                                          _f, _vp, _sz, _vp]),
     "b200m_channel_state": (_i, [_vp, _i64, _i, _i, _i, _vp, _i64, _vp, _i64, _vp, _vp, _f, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                                  _i, _f, _i, _vp]),

@@ -248,8 +248,9 @@ class ModelRunner:
             for i, s in enumerate(seqs):
                 s.block_table = list(range(i * per, (i + 1) * per))
                 s.state_slot = i
-        # what a prompt step over long cached prefixes holds beside these activations counts as peak too
+        # what a prompt step over long cached prefixes, or of many sequences, holds beside these activations counts as peak too
         scratch = getattr(self.model, "prompt_scratch_bytes", lambda rows: 0)(cfg.max_num_seqs * cfg.max_model_len)
+        scratch += getattr(self.model, "step_scratch_bytes", lambda seqs: 0)(cfg.max_num_seqs)
         held = torch.empty(scratch, dtype=torch.uint8, device=self.device)
         self.run(seqs, True)
         del held

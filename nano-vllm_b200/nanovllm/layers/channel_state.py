@@ -188,6 +188,9 @@ class ChannelDeltaMixer(_ChannelStateMixer):
         super().unbind()
         self.conv_state = []
 
+    def step_scratch_bytes(self, seqs: int) -> int:
+        return mixops.delta_scratch_bytes(self.heads, seqs) if self.dtype != torch.float32 and 64 < self.dim <= 128 else 0
+
     def mix(self, h: torch.Tensor, positions, ctx, spans: mixops.StepSpans, inst: int = 0, out: torch.Tensor | None = None) -> torch.Tensor:
         """-> the output projection's operand [n, heads * vdim]."""
         Q = self.qk_cols

@@ -586,14 +586,28 @@ def gated_delta(x: torch.Tensor, q_off: int, k_off: int, v_off: int, ba: torch.T
     return out
 
 
-_DELTA_WS = [0, 0]             # workspace bytes of a chunk of one sequence and head, and the most that a step takes beyond one chunk
+DELTA_WORKSPACE = 1 << 30      # most bytes that a step of the chunked delta rule takes at a time; a longer step is cut into several launch pairs
 
 
 def delta_chunks(max_q: int, dim: int) -> bool:
-    """Whether a step's portions take the chunked form of the channel delta rule.  Its rows are 128 channels wide; a chunk is sixteen tokens: one
-    16-token portion 15 us against 16 (16 heads), sixteen of them 29 against 35 (8 heads 21 against 21), of 6 tokens 28 against 27 (8 heads 19
-    against 16); longer ones 1.2 to 3 times faster."""
+    """Whether the chunked form of the channel delta rule takes a step: its rows are 128 channels wide, a chunk is sixteen tokens."""
     return max_q >= 16 and 64 < dim <= 128
+
+
+def delta_pays(n: int, num_seqs: int, max_q: int, tiles: int) -> bool:
+    """Whether a step of n tokens in num_seqs portions, the longest of max_q, is faster in chunks than token by token (tiles: heads x 64-column tiles of the values).
+    Both forms' times in us, fitted to 90 steps of 1 to 512 portions and 16 or 32 tiles: the longest portion is a chain of 0.326 a token against 0.139; a portion and
+    tile cost 0.030 and 0.002 a token against 0.023 and 0.027 a chunk.  Chunks that a step has: of the longest portion, and at least one, or three quarters
+    of one more than its tokens fill, of each other.  10 us for the second launch.  No measured step takes the slower form by more than the runs differ; the other
+    way up to 17 us (1.34 times) are left.  us, 16 heads of 128 x 128, chunks against tokens: 1 x 64 20 / 25, 16 x 16 31 / 29, 16 x 64 71 / 84, 512 x 16 840 / 773, 128 x 128 891 / 1045,
+    4 x 2048 447 / 670, 1 x 2048 beside 511 single tokens 870 / 1130, 1 x 256 beside them 753 / 500, 1 x 8192 beside 100 x 20 1405 / 3422."""
+    chunks = max(num_seqs - 1, (n - max_q) / 16 + 0.75 * (num_seqs - 1)) + max_q / 16
+    return 0.187 * max_q + tiles * (0.0074 * num_seqs + 0.002 * n - 0.027 * chunks) >= 10
+
+
+def delta_scratch_bytes(heads: int, seqs: int) -> int:
+    """What a prompt step of ``seqs`` sequences holds for the chunked delta rule beyond a step of as many tokens in one (a workspace row a sequence at most)."""
+    return min(nat.load_mix().b200m_channel_delta_workspace_bytes(0, seqs, heads), DELTA_WORKSPACE)
 
 
 def channel_state(x: torch.Tensor, q_off: int, k_off: int, v_off: int, write: torch.Tensor | None, decay_in: torch.Tensor, rate: torch.Tensor,
@@ -604,7 +618,7 @@ def channel_state(x: torch.Tensor, q_off: int, k_off: int, v_off: int, write: to
     with unit-norm q and k; None: gated linear attention.  decay_in fp32 [n, heads * dim] is scratch (single-token steps
     form the decays in place first); state fp32 [slots, heads, vdim, dim] -> fp32 [n, heads, vdim].
     ``forgetting``: the caller's rates are never above zero, so that no decay is above one; bf16 portions under the delta rule then run on the
-    tensor cores (``delta_chunks``)."""
+    tensor cores where that is faster (``delta_pays``)."""
     n = x.shape[0]
     is32 = _is32(x)
     assert x.dim() == 2 and x.stride(1) == 1 and decay_in.dtype == torch.float32 and decay_in.stride(1) == 1 and decay_in.shape == (n, heads * dim)
@@ -613,21 +627,19 @@ def channel_state(x: torch.Tensor, q_off: int, k_off: int, v_off: int, write: to
     assert write is None or (write.shape == (n, heads) and write.stride(1) == 1)
     _same(is32, write)
     out = torch.empty(n, heads, vdim, dtype=torch.float32, device=x.device)
-    if forgetting and write is not None and not is32 and spans.cu_q is not None and delta_chunks(spans.max_q, dim):
+    if (forgetting and write is not None and not is32 and spans.cu_q is not None and delta_chunks(spans.max_q, dim)
+            and delta_pays(n, spans.num_seqs, spans.max_q, heads * -(-vdim // 64))):
         lib = nat.load_mix()
-        if not _DELTA_WS[0]:
-            _DELTA_WS[:] = lib.b200m_channel_delta_workspace_bytes(1, 1, 1), lib.b200m_channel_delta_workspace_bytes(0, 0, 0)
-        chunks, one = (spans.max_q + 15) >> 4, _DELTA_WS[0] * spans.num_seqs * heads
-        fit = max(1, min(chunks, _DELTA_WS[1] // one))      # chunks that a pair of launches takes
-        size = fit * one
+        need, row = lib.b200m_channel_delta_workspace_bytes(n, spans.num_seqs, heads), lib.b200m_channel_delta_workspace_bytes(0, 1, heads)
+        size = min(need, max(DELTA_WORKSPACE // row, 1) * row)
         ws = torch.empty(size, dtype=torch.uint8, device=x.device)
         rc = lib.b200m_channel_delta_prompts(
             x.data_ptr(), x.stride(0), q_off, k_off, v_off, write.data_ptr(), write.stride(0), decay_in.data_ptr(), decay_in.stride(0), rate.data_ptr(),
             decay_bias.data_ptr(), decay_sign, state.data_ptr(), state_slots.data_ptr(), spans.cu_q.data_ptr(), spans.cu_k.data_ptr(), out.data_ptr(), n,
-            spans.num_seqs, spans.max_q, heads, kv_heads, dim, vdim, q_scale, ws.data_ptr(), size, _stream())
+            spans.num_seqs, heads, kv_heads, dim, vdim, q_scale, ws.data_ptr(), size, _stream())
         if rc != -2:                                        # B200_EUNSUPPORTED: other alignments and odd sizes, below
             nat.check_mix(rc)
-            ops.LAUNCHES[0] += 2 * -(-chunks // fit) - 1
+            ops.LAUNCHES[0] += 2 * -(-need // size) - 1
             return out
         ops.LAUNCHES[0] -= 1
     if spans.cu_q is None or spans.max_q <= 4:

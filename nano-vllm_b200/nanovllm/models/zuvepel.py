@@ -149,6 +149,10 @@ class ZuvepelForCausalLM:
     def state_slot_bytes(self) -> int:
         return sum(b.branches.mixer.state_slot_bytes() * b.passes for b in self.blocks)
 
+    def step_scratch_bytes(self, seqs: int) -> int:
+        """What a prompt step of this many sequences holds beside the activations of one of as many tokens in few."""
+        return max((b.branches.mixer.step_scratch_bytes(seqs) for b in self.blocks if isinstance(b.branches.mixer, ChannelDeltaMixer)), default=0)
+
     def bind_cache(self, num_blocks: int, block_size: int, num_state_slots: int) -> None:
         self.block_size = block_size
         for b in self.blocks:
