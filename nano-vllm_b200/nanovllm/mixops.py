@@ -783,13 +783,30 @@ def moe_capacity(pairs: int, num_experts: int) -> int:
     return (pairs + num_experts * (bm - 1) + bm - 1) // bm * bm
 
 
+def router_kernel(n: int, outputs: int, K: int, is32: bool) -> bool:
+    """Whether the router's kernel forms the logits, or the library.  The kernel's tiles are 32 tokens by 40 outputs, and every 40 outputs read x again: it is the faster one
+    for up to 40 outputs, and for more while its tiles fit the SMs at once.  The library reads fp32, so bf16 rows pay a copy there.  us, kernel / library, K = 2048, bf16 (fp32):
+    8192 x 40 42 / 102 (43 / 55), 8192 x 80 83 / 129 (85 / 84), 8192 x 128 142 / 130 (159 / 84), 8192 x 256 251 / 203 (280 / 157), 2048 x 64 40 / 45 (41 / 35), 512 x 256 24 / 39 (27 / 35),
+    256 x 512 41 / 35 in fp32, 64 x 512 14 / 22 (14 / 19), 1 x 64 5.6 / 9.0 (5.6 / 6.7), 1 x 256 5.1 / 7.0 (4.8 / 4.4), 1 x 1000 12.8 / 7.7 (12.5 / 5.4).  One token: the library's
+    product of a vector; the kernel spreads K over eight CTAs at most."""
+    if n == 1:
+        return (outputs <= 64 and K <= 2048 or outputs <= 256 and K <= 1024) if is32 else outputs <= 40 or (outputs <= 512 and K <= 2048)
+    if n < 4 and outputs > 512:
+        return False
+    tiles = -(-n // 32) * -(-outputs // 40)
+    return outputs <= 40 or (tiles <= 100 if is32 else tiles <= 112 or outputs <= 80)
+
+
 def moe_logits(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """Router logits fp32 [n, outputs] = x w^T (+ bias); x [n, K] in the activation type, w [outputs, K] and bias fp32."""
     n, K = x.shape
     assert x.stride(1) == 1 and w.dtype == torch.float32 and w.is_contiguous() and w.shape[1] == K
     assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.shape == w.shape[:1])
+    is32 = _is32(x)
+    if not router_kernel(n, w.shape[0], K, bool(is32)):
+        return torch.nn.functional.linear(x.float(), w, bias)
     out = torch.empty(n, w.shape[0], dtype=torch.float32, device=x.device)
-    rc = nat.load_mix().b200m_moe_logits(x.data_ptr(), x.stride(0), w.data_ptr(), _p(bias), out.data_ptr(), n, w.shape[0], K, _is32(x), _stream())
+    rc = nat.load_mix().b200m_moe_logits(x.data_ptr(), x.stride(0), w.data_ptr(), _p(bias), out.data_ptr(), n, w.shape[0], K, is32, _stream())
     if rc == -2:                                            # B200_EUNSUPPORTED: odd sizes and alignments
         ops.LAUNCHES[0] -= 1
         return torch.nn.functional.linear(x.float(), w, bias)

@@ -24,3 +24,15 @@ def test_other_sizes_go_to_the_library():
     from nanovllm import mixops as mx
     x, w = torch.randn(5, 20, device="cuda"), torch.randn(3, 20, device="cuda")
     assert torch.allclose(mx.moe_logits(x, w), x @ w.t(), atol=1e-5)
+
+
+@pytest.mark.parametrize("n,E,own", [(40, 256, True), (4000, 256, False), (4000, 40, True)])
+def test_wide_routers_of_long_steps_are_the_librarys(n, E, own):
+    from nanovllm import mixops as mx, ops
+    g = torch.Generator(device="cuda").manual_seed(E)
+    x, w = torch.randn(n, 512, device="cuda", generator=g).bfloat16(), torch.randn(E, 512, device="cuda", generator=g)
+    before = ops.LAUNCHES[0]
+    got = mx.moe_logits(x, w)
+    assert ops.LAUNCHES[0] - before == int(own)
+    want = x.double() @ w.double().t()
+    assert (got - want).norm() <= 2e-6 * want.norm()
