@@ -39,9 +39,6 @@ constexpr int THREADS = 512;
 constexpr int ITEM_CAP = 96;            // items per CTA (more items: more CTAs)
 constexpr int LEVELS_CAP = 8192;        // row blocks per sequence that the longest-first order covers (its counters lie where Q will be)
 constexpr float LOG2E = 1.4426950408889634f;
-#ifndef FA_COPY_PAIRS
-#define FA_COPY_PAIRS 8
-#endif
 
 struct FaParams {
     const int32_t* cu_q;
@@ -82,7 +79,7 @@ struct FaParams {
 // The copy of this CTA's share of the rows, a part at a time by whichever warp is free (a counter in shared memory deals them out): half a warp per row, all loads of a
 // part before its stores.  (A rotation by single rows, and loads under a condition, ran one row after the other: 283 us for 848 rows; one warp alone took 85.)
 struct FaCopy {
-    static constexpr int PAIRS = FA_COPY_PAIRS, ROWS = 2 * PAIRS;         // rows of a part
+    static constexpr int PAIRS = 8, ROWS = 2 * PAIRS;         // rows of a part
     int end, begin, row, slot;            // of the share; first row of the part this warp has next (end: none), slot of this lane's row in it
 
     __device__ __forceinline__ void next(const FaParams& p, int* counter, int lane) {

@@ -129,6 +129,7 @@ struct DecayIn {
     const float* bias;        // CH: [H * dim], else [H]
     float sign;               // g = exp(rate_h * softplus(sign * (in + bias)))
 };
+__device__ __forceinline__ float decay_of(float a, float rate, float bias, float sign) { return expf(rate * softplus_(sign * (a + bias))); }
 
 template <typename T, int DPL, int LANES, int COLS, bool CH, bool DELTA>
 __global__ void __launch_bounds__(MS_THREADS) matrix_state_kernel(

@@ -3,7 +3,6 @@
 #include "mix_common.cuh"
 
 __device__ __forceinline__ float softplus_(float x) { return x > 20.f ? x : log1pf(expf(x)); }
-__device__ __forceinline__ float decay_of(float a, float rate, float bias, float sign) { return expf(rate * softplus_(sign * (a + bias))); }
 
 // What scalar linear attention does with a token: raw fp32 (or T) inputs -> (log decay, write weight).
 template <typename T>

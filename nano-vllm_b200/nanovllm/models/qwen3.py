@@ -8,8 +8,10 @@ inside them.  Per layer and per step this issues
     -> add_rmsnorm -> gate_up GEMM -> silu*mul -> down GEMM (+all-reduce)
 (for small decode batches the bracket and the attention are one kernel, b200_paged_decode_fused)
 
-GEMMs are library calls (cuBLAS through ``F.linear``, as in the reference, linear.py:51,73,153);
-everything else is one hand-written kernel from libb200attn.  Tensor parallelism shards heads and
+GEMMs of prompts and of large decode steps are library calls (cuBLAS through ``F.linear``, as in the reference,
+linear.py:51,73,153); decode steps of up to 128 rows have o_proj and down_proj on tcgen05 with split k (``ops.linear``), those
+of up to 16 rows all four projections as row-wise products with the norms and the activation inside (``ops.linear_rows``:
+four launches a layer around attention).  Everything else is one hand-written kernel from libb200attn.  Tensor parallelism shards heads and
 MLP columns exactly like the reference's *ParallelLinear classes (linear.py:54-156) and all-reduces
 after o_proj and down_proj only; the embedding table is replicated and the LM head stays
 vocab-sharded with a (max, argmax) combine instead of a logits gather (embed_head.py:56-66).
@@ -81,7 +83,8 @@ class Qwen3ForCausalLM:
         #   B200_LINEAR=auto (default): the two row-parallel projections (o_proj, down_proj) of decode steps of up to 128 rows
         #       run on tcgen05 with split-K 8 and the add+RMSNorm that follows consumes the fp32 partials in split order
         #       (csrc/linear_tc.cu): 4-21 % off the step at batch <= 128; at batch 256 and for the wide projections
-        #       (qkv, gate_up) the library GEMM is faster, so those stay cuBLAS, as under tensor parallelism;
+        #       (qkv, gate_up) of more than 16 rows the library GEMM is faster, so those stay cuBLAS, as under tensor parallelism;
+        #       steps of up to 16 rows: see few_rows below.  B200_LINEAR_MAX_ROWS: most rows of either;
         #   cublas: every projection through the library;  rows / tc: force the tcgen05 path for o/down / all four;
         #   gu: only gate_up + SiluAndMul on tcgen05 (one launch less per layer), the rest through the library.
         #   B200_LINEAR_CFG = "qkv_bn,gate_up_bn,o_bn,o_splits,down_bn,down_splits,pdl".

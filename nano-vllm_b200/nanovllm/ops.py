@@ -137,7 +137,7 @@ def paged_prefill(layer: int, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q:
 def paged_prefill_store(layer: int, q, k, v, slot_mapping, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: int, max_seqlen_k: int, scale: float) -> torch.Tensor:
     """``store_kv`` and ``paged_prefill`` of packed prompts: as one launch where the attention is long enough to hide the copies."""
     t, hq, d = q.shape
-    if k.shape == v.shape and slot_mapping.numel() == k.shape[0] and prefill_hides_store(t, cu_seqlens_q.numel() - 1, hq, k.shape[1]):
+    if k.shape == v.shape and slot_mapping.numel() == k.shape[0] and prefill_hides_store(t, cu_seqlens_q.numel() - 1):
         for x, n in ((q, "q"), (k, "k"), (v, "v")):
             _need(x, torch.bfloat16, n)
         for x, n in ((slot_mapping, "slot_mapping"), (cu_seqlens_q, "cu_seqlens_q"), (cu_seqlens_k, "cu_seqlens_k")):
@@ -156,10 +156,11 @@ def paged_prefill_store(layer: int, q, k, v, slot_mapping, cu_seqlens_q, cu_seql
     return paged_prefill(layer, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, scale)
 
 
-def prefill_hides_store(total: int, seqs: int, heads: int, kv_heads: int) -> bool:
+def prefill_hides_store(total: int, seqs: int) -> bool:
     """Whether the attention of packed prompts is long enough to hide the copies of their K and V.  Many short prompts are not: their items are over before a part
-    is copied.  us (inside / two launches), 16 heads on 8: 28 x 561 84 / 107, 64 x 128 40 / 46, 64 x 64 25 / 30, 256 x 64 92 / 99; 8 on 8: 256 x 64 71 / 72,
-    256 x 32 61 / 60, 256 x 16 57 / 52; 32 on 8: 256 x 16 147 / 137, 512 x 32 285 / 277, 64 x 32 36 / 40."""
+    is copied.  us (inside / two launches), 16 heads on 8: 28 x 561 84 / 107, 64 x 128 40 / 46, 64 x 64 25 / 30, 256 x 64 92 / 99; 8 on 8: 256 x 64 70 / 71,
+    256 x 32 61 / 60, 256 x 16 57 / 53; 32 on 8: 256 x 16 145 / 139, 512 x 32 310 / 275, 64 x 32 36 / 40; on one kv head, whose copies are an eighth: 8 heads 200 x 70 41 / 46, 28 x 561 42 / 47,
+    256 x 16 40 / 42, 16 heads 28 x 561 70 / 77, 32 heads 28 x 561 139 / 156, 256 x 16 138 / 134.  Up to 64 prompts, and 64 tokens of each: never slower, from 1 x 1 on."""
     return total >= 64 * seqs or seqs <= 64
 
 

@@ -1,6 +1,6 @@
 """Linear layers of at most 16 rows (csrc/linear_rows.cu) give bit for bit what the launches they replace give: the library's products and b200_linear's
-partials, the norm kernels and SiluAndMul.  One and two 8-row tiles, full and not, one CTA and clusters along k, one and two tiles of weights, rows that the norm holds
-in registers and reads twice, strided inputs."""
+partials, the norm kernels and SiluAndMul.  One and two 8-row tiles, full and not, one chain of sums and up to eight along k, one, two and four tiles of weights, rows that the
+norm holds in registers and reads twice, strided inputs."""
 import pytest
 import torch
 import torch.nn.functional as F
