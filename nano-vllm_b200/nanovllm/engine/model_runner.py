@@ -84,7 +84,7 @@ class ModelRunner:
         local = int(os.environ.get("LOCAL_RANK", rank))
         # Debug / CI knob: B200_TP_BACKEND=gloo with B200_TP_ONE_DEVICE=1 runs all tensor-parallel ranks on ONE GPU
         # (time-sliced processes, collectives through gloo, eager only): the sharding, the vocab-parallel sampling and
-        # the SPMD engine can then be checked on a single-GPU box.  Never the fast path: NCCL is the default.
+        # the SPMD engine can then be checked on a machine with one GPU.  Never the fast path: NCCL is the default.
         backend = os.environ.get("B200_TP_BACKEND", "nccl")
         if os.environ.get("B200_TP_ONE_DEVICE") == "1":
             local = 0

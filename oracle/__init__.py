@@ -19,6 +19,6 @@ Pinning status
   not vendored; installed here 2.8.3).  The reference holds no golden vectors
   for it => **parity unpinned** for the floating-point attention core; the
   oracle follows flash-attn's published semantics (mask alignment, paged
-  layout, fp32 softmax) and is additionally cross-checked on the GPU box
+  layout, fp32 softmax) and is additionally cross-checked on a GPU
   against the installed flash-attn binary when it is importable.
 """

@@ -2,8 +2,7 @@
 
     TORCH_COMPILE_DISABLE=1 python oracle/make_golden.py            # needs /root/reference
 
-The reference is Python, so it can be imported here (never on the GPU box: nothing at test time
-reads /root/reference).  What gets pinned:
+The reference is Python, so it can be imported here (nothing at test time reads it).  What gets pinned:
 
 1. hash_kat.json          BlockManager.compute_hash known answers          (block_manager.py:35-41)
 2. trace_<workload>.json  step-by-step digests of the reference Scheduler / BlockManager /
@@ -74,14 +73,14 @@ def workloads() -> dict:
     s5 = [(0.8, rnd.randint(16, 200), False) for _ in range(50)]
     out["eos64"] = dict(cfg=dict(max_num_seqs=16, max_num_batched_tokens=2048, kvcache_block_size=64,
                                  num_kvcache_blocks=60), prompts=p5, sps=s5, vocab=41, eos=7)
-    # BASELINE config 4's request mix at the bookkeeping level: 1024 requests against 512 running slots, so prefill
+    # a request mix at the bookkeeping level: 1024 requests against 512 running slots, so prefill
     # and decode steps interleave for the whole run; the cache is sized to force preemptions
     r6 = random.Random(4)
     p6 = [[r6.randint(0, 150000) for _ in range(r6.randint(50, 800))] for _ in range(1024)]
     s6 = [(0.7, r6.randint(10, 200), True) for _ in range(1024)]
     out["mixed1024"] = dict(cfg=dict(max_num_seqs=512, max_num_batched_tokens=16384, kvcache_block_size=256,
                                      num_kvcache_blocks=1100), prompts=p6, sps=s6, vocab=151936, eos=-1)
-    # BASELINE config 5's: 128 concurrent long-context requests (about 8k in, up to 1k out); every prompt is
+    # long contexts: 128 concurrent long-context requests (about 8k in, up to 1k out); every prompt is
     # longer than half the token budget, so prefill is chunked throughout, and blocks run out during decode
     r7 = random.Random(5)
     p7 = [[r7.randint(0, 150000) for _ in range(r7.randint(7000, 8192))] for _ in range(128)]

@@ -14,10 +14,11 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def record(name: str, payload: dict):
-    """Append measured parity numbers to gpurun_out/parity.jsonl so they can be read back after a GPU run."""
-    d = os.path.join(ROOT, "gpurun_out")
-    os.makedirs(d, exist_ok=True)
-    with open(os.path.join(d, "parity.jsonl"), "a") as f:
+    """Append measured parity numbers to the file that PARITY_LOG names, if it names one."""
+    path = os.environ.get("PARITY_LOG")
+    if not path:
+        return
+    with open(path, "a") as f:
         f.write(json.dumps(dict(test=name, **payload)) + "\n")
 
 

@@ -5,7 +5,7 @@ and the product both own the package name ``nanovllm``.
 
     python tests/ref_gpu_forward.py <model_dir> <script.json> <out.npz> [--dropin]
 
-With --dropin the same reference runs with INTEGRATION.md's option B applied (integration/b200_binding.py): only
+With --dropin the same reference runs with option B of the integration guide applied (integration/b200_binding.py): only
 Attention.forward and the cache allocation line change, every other module is the reference's own.
 
 What it does is what the reference's ModelRunner does in eager mode (engine/model_runner.py:17-48,103-121,195-220):

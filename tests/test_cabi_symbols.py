@@ -119,7 +119,7 @@ def test_ctypes_table_matches_header_prototypes():
 
 
 def test_integration_doc_binding_matches_table():
-    """The ctypes stub INTEGRATION.md shows a maintainer is the same binding the product uses."""
+    """The ctypes stub that the integration guide shows a maintainer is the same binding the product uses."""
     text = open(os.path.join(ROOT, "INTEGRATION.md")).read()
     text = re.sub(r"\n\s+(?=_)", " ", text)                       # join continued argtypes lines
     short = {"_vp": ctypes.c_void_p, "_i": ctypes.c_int, "_i64": ctypes.c_int64, "_f": ctypes.c_float, "_sz": ctypes.c_size_t}

@@ -1,11 +1,11 @@
 """Differential fuzzing of the host bookkeeping against the reference's own classes, where the reference is available.
 
-The committed golden traces (tests/golden/trace_*.json) pin seven hand-picked workloads.  In the build container the
+The committed golden traces (tests/golden/trace_*.json) pin seven hand-picked workloads.  Where its source is at hand the
 reference can also be executed directly, so this test draws a few hundred random small workloads (page sizes 2..256,
 tight caches that force preemption, shared prefixes, duplicates, EOS stops, tiny token budgets that force chunking),
 runs the REFERENCE's Scheduler / BlockManager / Sequence / prepare_* over them in a subprocess (both packages are called
 `nanovllm`, so they cannot share an interpreter) and requires the product to produce the same step-by-step digests.
-Skipped where /root/reference does not exist (e.g. on the GPU box) -- the golden traces cover that case.
+Skipped where the reference's source does not exist -- the golden traces cover that case.
 """
 import itertools
 import json

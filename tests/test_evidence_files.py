@@ -1,4 +1,4 @@
-"""The numbers DESIGN.md quotes are the ones in the committed evidence files (profiles/), and those files carry every key the
+"""The numbers that the design notes quote are the ones in the committed evidence files (profiles/), and those files carry every key the
 bench contract names.  No GPU: this only reads JSON / text that GPU runs left behind."""
 import json
 import os
@@ -26,7 +26,7 @@ def test_headline_bench_line_is_complete_and_consistent():
     assert d["cpu_baseline"]["kind"] in ("reference", "port") and d["cpu_baseline"]["cores"] >= 1
     assert not set(d["clocks"]["reasons"]) & {"hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown"}
     design = open(os.path.join(ROOT, "DESIGN.md")).read()
-    assert _fmt(d["value"]) in design and _fmt(d["e2e"]["value"]) in design, "DESIGN.md section 6 quotes another run"
+    assert _fmt(d["value"]) in design and _fmt(d["e2e"]["value"]) in design, "the design notes quote another run"
     assert f"{r['frac']:.3f}" in design
 
 

@@ -174,7 +174,7 @@ def test_engine_chunked_prefill_and_preemption(tiny_dir):
 
 
 def test_prefill_bench_size_rows_vs_oracle():
-    """BASELINE config-2 prefill shape (Hq16/Hkv8, prompts up to 1024 tokens, ~16k tokens per step): a few whole
+    """The serving benchmark's prefill shape (Hq16/Hkv8, prompts up to 1024 tokens, ~16k tokens per step): a few whole
     sequences against the oracle, the rest through a property -- every sequence's output is independent of its
     neighbours in the batch."""
     from nanovllm import ops
@@ -217,7 +217,7 @@ def test_engine_sampling_and_eos(tiny_dir):
 
 
 def test_decode_bench_shape_vs_oracle_rows():
-    """BASELINE config-2 decode shape (B=256, Hq16/Hkv8, page 256, context mix of bench step 0): sampled rows
+    """The serving benchmark's decode shape (B=256, Hq16/Hkv8, page 256, context mix of bench step 0): sampled rows
     against the oracle, and the checksum property that every row only depends on its own pages."""
     from nanovllm import ops
     from oracle.make_golden import workloads

@@ -12,8 +12,8 @@ Qwen3-0.6B dimensions (hidden 1024, 16/8 heads, vocab 151 936) with 256-token pa
 For every step this records the logits' relative L2 error of ref and of ours against truth and against each other,
 the worst element in bf16 roundings of the logit scale, and argmax agreement.  The bar: ours is no further from the
 fp32 truth than the reference's own GPU path is (x1.25 + 1e-3 slack), and every row whose fp32 argmax wins by more than
-8 bf16 roundings is decoded identically by all three.  The numbers land in gpurun_out/parity.jsonl; a copy of one
-run is committed under profiles/.
+8 bf16 roundings is decoded identically by all three.  PARITY_LOG collects the numbers; those of one
+run are committed under profiles/.
 """
 import json
 import os
@@ -143,7 +143,7 @@ def test_product_vs_reference_gpu_forward_vs_fp32_truth(layers, tmp_path):
 
 
 def test_reference_tree_with_only_the_operator_swapped(tmp_path):
-    """INTEGRATION.md option B, executed: the reference's own model (its linears, norms, RoPE, LM head; eager) with ONLY
+    """Option B of the integration guide, executed: the reference's own model (its linears, norms, RoPE, LM head; eager) with ONLY
     Attention.forward and the cache layout line changed to libb200attn.so (integration/b200_binding.py), against the
     unmodified reference (flash-attn + Triton store) on the same weights and the same serving script."""
     if not os.path.isdir(REF):

@@ -3,7 +3,7 @@ it (nanovllm/layers/attention.py:67-74: flash_attn_varlen_func for prefill, flas
 the same tensors, on the GPU.
 
 flash-attn is the reference's (unpinned, un-vendored) dependency; it cannot run on the CPU, so the CPU oracle restates
-its published semantics.  This file closes the loop on the GPU box, where the image ships flash-attn 2.8.x: it is used
+its published semantics.  This file closes the loop on a GPU, with flash-attn 2.8.x where it is installed: it is used
 here as a checker only.  Both pipelines keep S and the accumulator in fp32 and round P to bf16, but tile and order
 the sums differently, so the bar is the same as against the oracle: a few bf16 roundings of the output scale.
 The cache is stored in both layouts from the same logical pages: ours head-major [nblk, Hkv, bs, D], flash-attn's
@@ -22,7 +22,7 @@ pytestmark = pytest.mark.gpu
 
 
 def flash():
-    """Imported lazily (slow import; only needed on the GPU box); skip when the image has no flash-attn."""
+    """Imported lazily (slow import; only needed with a GPU); skip where flash-attn is missing."""
     return pytest.importorskip("flash_attn", reason="flash-attn (the reference's attention library) is not installed")
 
 

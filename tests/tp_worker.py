@@ -19,7 +19,7 @@ def main():
     import torch.distributed as dist
     rank, world, local = int(os.environ["RANK"]), int(os.environ["WORLD_SIZE"]), int(os.environ["LOCAL_RANK"])
     backend = os.environ.get("B200_TP_BACKEND", "nccl")
-    if os.environ.get("B200_TP_ONE_DEVICE") == "1":          # every rank on GPU 0 (single-GPU boxes; gloo collectives)
+    if os.environ.get("B200_TP_ONE_DEVICE") == "1":          # every rank on GPU 0 (machines with one GPU; gloo collectives)
         local = 0
     torch.cuda.set_device(local)
     if backend == "nccl":
