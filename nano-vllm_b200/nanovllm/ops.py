@@ -329,6 +329,9 @@ def linear_rows(x: torch.Tensor, w: torch.Tensor, norm_w: torch.Tensor | None = 
     _need(x, torch.bfloat16, "x"); _need(w, torch.bfloat16, "w")
     assert x.dim() == 2 and w.dim() == 2 and x.stride(1) == 1 and w.is_contiguous() and x.shape[1] == w.shape[1]
     assert add is None or (add.dtype == torch.bfloat16 and add.shape == x.shape and add.stride(1) == 1 and norm_w is not None)
+    if norm_w is not None:
+        _need(norm_w, torch.bfloat16, "norm_w")
+        assert norm_w.is_contiguous() and norm_w.numel() == x.shape[1]
     rows, k = x.shape
     n = w.shape[0] // 2 if silu else w.shape[0]
     out = torch.empty(rows, n, dtype=torch.bfloat16, device=x.device)

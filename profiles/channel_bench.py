@@ -106,6 +106,9 @@ def kernel_table(size: str, peaks: dict):
         x, wr, ba = rn(n, (2 * dg + sh) * d), rn(n, sh), torch.randn(n, 2 * sh, device=dev)
         add(f"channel_state, delta rule {label}", lambda: mixops.channel_state(x, 0, dg * d, 2 * dg * d, wr, z, rt, db, 1.0, state, slots, spn, sh, dg, d, d, d ** -0.5),
             n * ((2 * dg + sh) * d * 2 + sh * d * 8) + st_bytes, flops, "fma")
+        if q > 1:
+            add(f"channel_state, delta rule in chunks {label}", lambda: mixops.channel_state(x, 0, dg * d, 2 * dg * d, wr, z, rt, db, 1.0, state, slots, spn, sh, dg, d, d,
+                d ** -0.5, forgetting=True), n * ((2 * dg + sh) * d * 2 + sh * d * 8) + st_bytes, flops, "fma")
         add(f"gated_delta (musavik form) {label}", lambda: mixops.gated_delta(x, 0, dg * d, 2 * dg * d, ba, rt, hb0, state, slots, spn, sh, dg, d, d, d ** -0.5),
             n * ((2 * dg + sh) * d * 2 + sh * d * 4) + st_bytes, flops, "fma")
         xg = rn(n, 3 * sh * d)

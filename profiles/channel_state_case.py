@@ -1,4 +1,5 @@
-"""One small case of the channel-decay matrix-state kernels for an `ncu` capture: `python profiles/channel_state_case.py delta|gla prefill|decode`
+"""One small case of the fp32-pipe forms of the channel-decay matrix states for an `ncu` capture (what short portions and fp32 take; longer bf16 portions of
+the delta rule run in chunks: `tensor_core_case.py delta`): `python profiles/channel_state_case.py delta|gla prefill|decode`
 (16 heads, 128 x 128 states: a 4 x 1024-token prompt step, or a single-token step of 64 sequences)."""
 import os
 import sys

@@ -1,4 +1,4 @@
-"""Small cases of the tcgen05 kernels and the small-step decode kernel for `ncu` captures: `python profiles/tensor_core_case.py NAME`
+"""Small cases of the tensor-core kernels and of small steps for `ncu` captures: `python profiles/tensor_core_case.py NAME`
 
     prompt         fa_kernel: two prompts of 4096 tokens, 16 query over 8 kv heads
     window_prompt  fa_kernel: 4 x 2048 tokens over token-major cache rows, window 1024, distance bias
@@ -6,6 +6,10 @@
     experts        moe_rows_kernel: 8192 tokens x 4 of 32 experts, width 2048, feed-forward 768
     experts_few    moe_stream_kernel: the same of 64 tokens
     small_step     paged_decode_small_kernel: 4 rows of 1024 tokens, 16 over 8 heads
+    prompt_store   fa_kernel with the copies of K and V: 28 prompts of 561 tokens, 16 over 8 heads
+    rows           linear_rows_kernel: 4 rows, gate_up of Qwen3-0.6B with add + norm in front and SiluAndMul behind
+    router         moe_router_kernel: 8192 rows of 2048 columns, 40 outputs
+    delta          channel_delta kernels: 4 x 2048 tokens, 16 heads of 128 x 128 over 4 query/key heads
 """
 import os
 import sys
@@ -58,7 +62,32 @@ def small_step():
     return lambda: ops.paged_decode(0, q, bt, ctx, 128 ** -0.5)
 
 
-call = dict(prompt=prompt, window_prompt=window_prompt, latent=latent, experts=experts, experts_few=lambda: experts(64), small_step=small_step)[sys.argv[1]]()
+def prompt_store():
+    ops.bind_kv_cache(torch.zeros(ops.kv_cache_shape(1, 64, 8, 256, 128), device=dev).bfloat16())
+    q, k, v, slots = rnd(28 * 561, 16, 128), rnd(28 * 561, 8, 128), rnd(28 * 561, 8, 128), torch.arange(28 * 561, dtype=torch.int32, device=dev)
+    return lambda: ops.paged_prefill_store(0, q, k, v, slots, cu(28, 561), cu(28, 561), 561, 561, 128 ** -0.5)
+
+
+def rows():
+    x, add, norm, w = rnd(4, 1024), rnd(4, 1024), rnd(1024), rnd(6144, 1024)
+    return lambda: ops.linear_rows(x, w, norm, 1e-6, add, silu=True, pdl=True)[0]
+
+
+def router():
+    x, w = rnd(8192, 2048), torch.randn(40, 2048, device=dev)
+    return lambda: mixops.moe_logits(x, w)
+
+
+def delta():
+    S, q, H, G, d = 4, 2048, 16, 4, 128
+    x, write, z = rnd(S * q, (2 * G + H) * d), rnd(S * q, H), torch.randn(S * q, H * d, device=dev) - 4
+    rate, bias, state = -torch.linspace(1, 16, H, device=dev), torch.zeros(H * d, device=dev), torch.zeros(S, H, d, d, device=dev)
+    sp, slots = mixops.StepSpans(S, q, cu(S, q), cu(S, q), None), torch.arange(S, dtype=torch.int32, device=dev)
+    return lambda: mixops.channel_state(x, 0, G * d, 2 * G * d, write, z, rate, bias, 1.0, state, slots, sp, H, G, d, d, d ** -0.5, forgetting=True)
+
+
+call = dict(prompt=prompt, window_prompt=window_prompt, latent=latent, experts=experts, experts_few=lambda: experts(64), small_step=small_step,
+            prompt_store=prompt_store, rows=rows, router=router, delta=delta)[sys.argv[1]]()
 for _ in range(4):
     o = call()
 torch.cuda.synchronize()

@@ -61,3 +61,12 @@ def test_refused_sizes(ops):
     for rows, n, k, splits in [(17, 16, 512, 1), (1, 24, 512, 1), (1, 16, 544, 1), (1, 16, 512, 3), (1, 16, 1152, 9), (9, 16, 8192, 1)]:
         with pytest.raises(B200Error):
             ops.linear_rows(bf(rows, k).cuda(), bf(n, k).cuda(), splits=splits)
+
+
+def test_norm_weights_of_another_size_or_type_are_refused(ops):
+    """On the host: the kernel reads as many as x has columns."""
+    from nanovllm._native import B200Error
+    x, w = bf(4, 512).cuda(), bf(16, 512).cuda()
+    for norm_w in (bf(256).cuda(), bf(1024).cuda()[::2], bf(512).cuda().float(), bf(512)):
+        with pytest.raises((AssertionError, B200Error)):
+            ops.linear_rows(x, w, norm_w, 1e-6)
