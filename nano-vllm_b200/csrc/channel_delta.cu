@@ -13,9 +13,10 @@
 //
 // Precision: an operand of a product is fp32 in three bf16 terms (3 x 8 bits: nothing is lost) and six of the nine partial products are taken (the others are
 // below 2^-26), the largest ones apart and added outside the tensor cores, which cut sums off where the fp32 pipe rounds.  V is bf16 as it is.  S itself is fp32.
-// No scales: bf16 has fp32's range, so a state or a read-out that strong decays have made small keeps its bits.  Against float64 the results are 1.1e-7 to
-// 2.4e-7 of their norm off, a key channel of the state 1e-7 to 1.8e-7 (median); the fp32-pipe form of recurrent_mix.cu 1e-7 to 1.9e-6 and 0.7e-7 to 1.8e-6.  (fp16 pairs, 22
-// bits, with half of the products: 1.2e-7 to 3.5e-7, and nothing left of a state below 2^-25 of one; both kernels together 357 us where these take 440.)
+// No scales: bf16 has fp32's range, so a state or a read-out that strong decays have made small keeps its bits.  Against float64 the results are 0.9e-7 to 3.1e-7
+// of their norm off and the state 0.5e-7 to 3.7e-7, the fp32-pipe form of recurrent_mix.cu 1.0e-7 to 18.5e-7 and 0.8e-7 to 23e-7.  (That one is closer, 0.8e-7 for 1.0e-7,
+// where strong decays leave a state of a token or two: keys are rounded once more here.)  With fp16 pairs, 22 bits and half of the products, it was 1.2e-7 to 3.5e-7, and
+// nothing was left of a state below 2^-25 of one; both kernels together took 350 us where these take 447.
 //
 // Measured on a B200, 16 heads of 128 x 128, both kernels together against that form: 4 x 2048 tokens 447 us against 669, 1 x 4096 634 against
 // 1314, 16 x 1000 872 against 1127, 12 x 600 408 against 544, 16 x 64 71 against 84, 1 x 2048 beside 511 single tokens 870 against 1130.  With the workspace laid out as
@@ -154,7 +155,8 @@ __device__ __forceinline__ void mma_rest(float (&c)[4], const uint32_t (&a)[3][4
 // ---- first kernel: decays, A, B, T, W, Q ------------------------------------------------------------------------------------------------
 // A_ts and B_ts need the decays between s and t.  Pairs of tokens are taken by the largest of four levels (half blocks of 8, 4, 2, 1 tokens) whose middle
 // parts them: with the middle m, k_t and q_t take g_m ... g_t, k_s takes g_(s+1) ... g_(m-1), all at most one, and a level is one product of
-// [8 k rows, 8 q rows] with [8 k rows].  Bound by its instructions: 161 us for 8192 tokens of 16 heads (operands as fp16 pairs 137).
+// [8 k rows, 8 q rows] with [8 k rows].  Bound by its instructions (2880 a thread, 0.53 per cycle and scheduler): 161 us for
+// 8192 tokens of 16 heads (operands as fp16 pairs 137).
 constexpr int CP_THREADS = 128;
 struct CpSmem {
     static constexpr int RAW_K = 0, RAW_Q = CD_L * CD_D * 2, A = 2 * RAW_Q, B = A + CD_L * CD_L * 4, T = B + CD_L * CD_L * 4,
@@ -516,8 +518,8 @@ template <int COUNT>
 __device__ __forceinline__ void cd_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(COUNT) : "memory"); }
 
 // Eight consumer warps: warp 2 p + hf holds 16 value columns (p) and 64 of the channels (hf), so that two warps per scheduler hide each other's waits;
-// a pair adds its two halves of W S and of Q S through shared memory.  Two copying warps, two chunks ahead.  Bound by the consumers' chain per chunk:
-// 2.2 us of 156 products (fp16 pairs: 84 products, 1.67 us, of one warp per 16 columns and all channels 4.0).
+// a pair adds its two halves of W S and of Q S through shared memory.  Two copying warps, two chunks ahead.  Bound by the consumers' chain per chunk and
+// the tensor pipe (63 % busy): 2.2 us of 156 products (fp16 pairs: 84 products, 1.67 us, of one warp per 16 columns and all channels 4.0).
 constexpr int CD_THREADS = 320;
 __global__ void __launch_bounds__(CD_THREADS, 1) channel_delta_chunks_kernel(
     const __nv_bfloat16* __restrict__ x, int64_t stride, int v_off, const unsigned char* __restrict__ ws, float* __restrict__ state,
