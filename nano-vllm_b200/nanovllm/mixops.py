@@ -800,10 +800,11 @@ def router_kernel(n: int, outputs: int, K: int, is32: bool) -> bool:
 def moe_logits(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """Router logits fp32 [n, outputs] = x w^T (+ bias); x [n, K] in the activation type, w [outputs, K] and bias fp32."""
     n, K = x.shape
-    assert x.stride(1) == 1 and w.dtype == torch.float32 and w.is_contiguous() and w.shape[1] == K
-    assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.shape == w.shape[:1])
+    assert w.dtype == torch.float32 and w.shape[1] == K
+    assert bias is None or (bias.dtype == torch.float32 and bias.shape == w.shape[:1])
     is32 = _is32(x)
-    if not router_kernel(n, w.shape[0], K, bool(is32)):
+    plain = x.stride(1) == 1 and w.is_contiguous() and (bias is None or bias.is_contiguous())
+    if not plain or not router_kernel(n, w.shape[0], K, bool(is32)):
         return torch.nn.functional.linear(x.float(), w, bias)
     out = torch.empty(n, w.shape[0], dtype=torch.float32, device=x.device)
     rc = nat.load_mix().b200m_moe_logits(x.data_ptr(), x.stride(0), w.data_ptr(), _p(bias), out.data_ptr(), n, w.shape[0], K, is32, _stream())

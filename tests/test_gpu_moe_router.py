@@ -36,3 +36,14 @@ def test_wide_routers_of_long_steps_are_the_librarys(n, E, own):
     assert ops.LAUNCHES[0] - before == int(own)
     want = x.double() @ w.double().t()
     assert (got - want).norm() <= 2e-6 * want.norm()
+
+
+def test_other_strides_go_to_the_library():
+    """Rows, weights and biases that are views: what the library's product takes."""
+    from nanovllm import mixops as mx
+    g = torch.Generator(device="cuda").manual_seed(1)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, w, b = r(64, 30), r(64, 16), r(32)
+    want = x.double().t() @ w.double() + b.double()[::2]
+    for rows, weights, bias in ((x.t(), w.t().contiguous(), b[::2].contiguous()), (x.t().contiguous(), w.t(), b[::2].contiguous()), (x.t().contiguous(), w.t().contiguous(), b[::2])):
+        assert (mx.moe_logits(rows, weights, bias) - want).norm() <= 2e-6 * want.norm()
