@@ -272,6 +272,22 @@ int b200_add_rmsnorm_partials(const float* partials, int splits, void* residual,
 int b200_linear_rows(const void* x, int64_t x_stride0, const void* add, int64_t add_stride0, void* residual_out, const void* norm_w, float eps,
                      const void* w, void* out, int64_t out_stride0, int rows, int n, int k, int splits, int silu, int flags, void* stream);
 
+/* All layers of a decode step of at most 8 rows on one GPU, as ONE kernel (csrc/step_rows.cu): embedding, per layer qkv_proj, q/k-norm + RoPE + KV append + attention,
+ * o_proj, gate_up_proj + SiluAndMul, down_proj with the norms between, and the final norm (reference models/qwen3.py:146-175), with the bits of
+ * b200_embedding, b200_linear_rows, b200_paged_decode_fused and b200_add_rmsnorm.
+ *   weights: layers * 8 device pointers, per layer qkv [(hq + 2 hkv) * 128, hidden], o [hidden, hq * 128], gate_up [2 * inter, hidden] (gate rows, then up rows),
+ *   down [hidden, inter], the two layer norms' [hidden], q and k norms' [128]; all bf16, contiguous, 16-byte aligned; layer l uses cache layer l;
+ *   ids [rows] (outside the vocabulary: zeros); block_tables, context_lens, cos_sin as b200_paged_decode_fused; out [rows, hidden] bf16, contiguous;
+ *   workspace: b200_step_rows_workspace_bytes(...) bytes, 16-byte aligned, of this launch alone; its contents before and after mean nothing.
+ * b200_step_rows_workspace_bytes: 0 where the step is not this kernel's: at most 8 rows, 64 layers; hidden 512 or 1024; hq * 128 and inter multiples of 1024 up to 3072;
+ * one or two query heads per kv head; steps that b200_decode_small_splits takes.
+ * Launched cooperatively (one CTA per SM, all resident), after a memset node; graph-capturable.  Waits are bounded: see b200_wait_timeouts. */
+size_t b200_step_rows_workspace_bytes(const b200_ctx* ctx, int rows, int layers, int hidden, int inter, int num_q_heads, int bt_stride);
+int b200_step_rows(b200_ctx* ctx, const void* const* weights, int layers, const int64_t* ids, const void* embed, int64_t vocab,
+                   const void* final_norm, const float* cos_sin, float eps, const int32_t* block_tables, int bt_stride,
+                   const int32_t* context_lens, void* out, int rows, int hidden, int inter, int num_q_heads, float scale,
+                   void* workspace, size_t workspace_bytes, void* stream);
+
 /* The tail of a decoder layer for a decode-size batch on one GPU, as ONE persistent kernel (csrc/layer_tail.cu):
  *   o_proj -> residual add + RMSNorm -> gate_up_proj + SiluAndMul -> down_proj -> residual add + RMSNorm [-> next qkv_proj]
  * i.e. RowParallelLinear o_proj + RMSNorm.add_rms_forward + Qwen3MLP + the next layer's input_layernorm and

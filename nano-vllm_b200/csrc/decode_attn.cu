@@ -577,6 +577,8 @@ static bool use_mma_decode() {
     return v == 1;
 }
 
+bool b200_decode_forced_mma() { return use_mma_decode(); }
+
 static int decode_common(b200_ctx* ctx, int layer, const void* q, int64_t q_stride0, const int32_t* block_tables,
                          int bt_stride, const int32_t* context_lens, void* out, int64_t out_stride0, int batch,
                          int num_q_heads, float scale, void* workspace, size_t workspace_bytes, void* stream,

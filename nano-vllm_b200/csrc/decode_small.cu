@@ -7,15 +7,12 @@
 // share a long context exchange their partials through distributed shared memory.  No workspace, no atomics, one launch; the order of every
 // sum is fixed by the shape.
 //
-// Arithmetic as in decode_attn.cu: fp32 on the FMA pipe, half a warp per token, 16 lanes x 8 dims; FUSED takes the raw qkv projection
-// (q/k-norm, RoPE and the KV append happen here).  Wider head groups than GW heads take several CTAs per kv head (K and V then come from L2).
-#include "decode_common.cuh"
+// The walk over a context's chunks is decode_walk.cuh's; FUSED takes the raw qkv projection (q/k-norm, RoPE and the KV append happen here).  Wider head groups than GW heads take several CTAs per kv head (K and V then come from L2).
+#include "decode_walk.cuh"
 
 using namespace b200dec;
 
 namespace {
-
-constexpr int SW = 8;                              // warps per CTA
 
 __device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory"); }
 __device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
@@ -52,42 +49,16 @@ __global__ void __launch_bounds__(SW * 32, 1) paged_decode_small_kernel(const De
     int64_t row = c0 + warp < c1 ? row_of(c0 + warp) : 0;
     B200_PDL_WAIT();
 
-    auto load = [&](int ck, int64_t at, uint4 (&k)[8], uint4 (&v)[8]) {      // rows past the context: zeros, nothing is read
-        const int valid = old - ck * CHUNK;
-        const uint4* ks = reinterpret_cast<const uint4*>(p.k_layer + at * D) + j;
-        const uint4* vs = reinterpret_cast<const uint4*>(p.v_layer + at * D) + j;
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            const int t = 2 * it + hw;
-            k[it] = t < valid ? ks[t * (D / 8)] : make_uint4(0, 0, 0, 0);
-        }
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            const int t = 2 * it + hw;
-            v[it] = t < valid ? vs[t * (D / 8)] : make_uint4(0, 0, 0, 0);
-        }
+    const WalkLane wl(lane);
+    auto load = [&](int ck, int64_t at, uint4 (&k)[8], uint4 (&v)[8]) {
+        walk_load(wl, p.k_layer, at, old - ck * CHUNK, k);
+        walk_load(wl, p.v_layer, at, old - ck * CHUNK, v);
     };
     uint4 kr[8], vr[8];
     if (c0 + warp < c1) load(c0 + warp, row, kr, vr);
 
     // ---- queries ----
-    float qf[GW][8], qw[8], kw[8], cosr[8], sinr[8];
-    auto norm_rope = [&](float (&x)[8], const float (&w)[8]) {               // RMS norm -> bf16 -> NeoX rotation -> bf16, as qknorm_rope_store_kernel
-        float ss = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) ss = fmaf(x[e], x[e], ss);
-#pragma unroll
-        for (int o2 = 8; o2 > 0; o2 >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o2);
-        const float rstd = 1.0f / sqrtf(ss / (float)D + p.eps);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const float y = round_bf16(__fmul_rn(__fmul_rn(x[e], rstd), w[e]));
-            const float other = __shfl_xor_sync(0xffffffffu, y, 8);          // element d +- 64
-            const float r = (j < 8) ? __fsub_rn(__fmul_rn(y, cosr[e]), __fmul_rn(other, sinr[e]))
-                                    : __fadd_rn(__fmul_rn(y, cosr[e]), __fmul_rn(other, sinr[e]));
-            x[e] = round_bf16(r);
-        }
-    };
+    float qw[8], kw[8], cosr[8], sinr[8];
     const __nv_bfloat16* qrow = p.q + (int64_t)b * p.q_stride + j * 8;
     if (FUSED) {
         unpack8(*reinterpret_cast<const uint4*>(p.q_norm_w + j * 8), qw);
@@ -99,72 +70,19 @@ __global__ void __launch_bounds__(SW * 32, 1) paged_decode_small_kernel(const De
             sinr[e] = cs[64 + e];
         }
     }
-    float o[GW][8], m[GW], l[GW];
+    WalkState<GW> st;
 #pragma unroll
     for (int g = 0; g < GW; ++g) {
-        unpack8(*reinterpret_cast<const uint4*>(qrow + (head0 + g) * D), qf[g]);
-        if (FUSED) norm_rope(qf[g], qw);
-        m[g] = -INFINITY;
-        l[g] = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            qf[g][e] *= p.scale_log2;
-            o[g][e] = 0.f;
-        }
+        unpack8(*reinterpret_cast<const uint4*>(qrow + (head0 + g) * D), st.q[g]);
+        if (FUSED) walk_norm_rope(wl, st.q[g], qw, cosr, sinr, p.eps);
     }
-    // the score of token 2 * my_it + hw ends up in this lane (and its neighbour j ^ 1)
-    const int my_it = ((j >> 3) & 1) * 4 + ((j >> 2) & 1) * 2 + ((j >> 1) & 1);
+    st.begin(p.scale_log2);
 
 #pragma unroll 1
     for (int ck = c0 + warp; ck < c1; ck += SW) {
         uint4 kn[8], vn[8];
         if (ck + SW < c1) load(ck + SW, row_of(ck + SW), kn, vn);
-        float acc[GW][8];
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            float kf[8];
-            unpack8(kr[it], kf);
-#pragma unroll
-            for (int g = 0; g < GW; ++g) {
-                float a = qf[g][0] * kf[0];
-#pragma unroll
-                for (int e = 1; e < 8; ++e) a = fmaf(qf[g][e], kf[e], a);
-                acc[g][it] = a;
-            }
-        }
-        const bool ok = ck * CHUNK + 2 * my_it + hw < old;
-#pragma unroll
-        for (int g = 0; g < GW; ++g) {             // sum over the 16 dim slices, scattering tokens over lanes: 8 -> 4 -> 2 -> 1 values
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const float send = (j & 8) ? acc[g][x] : acc[g][x + 4], keep = (j & 8) ? acc[g][x + 4] : acc[g][x];
-                acc[g][x] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-            }
-#pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                const float send = (j & 4) ? acc[g][x] : acc[g][x + 2], keep = (j & 4) ? acc[g][x + 2] : acc[g][x];
-                acc[g][x] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-            }
-            const float send = (j & 2) ? acc[g][0] : acc[g][1], keep = (j & 2) ? acc[g][1] : acc[g][0];
-            float s = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s = ok ? s : -INFINITY;
-            const float m_new = fmaxf(m[g], warp_max(s));                    // a chunk holds at least one token
-            const float alpha = fast_exp2(m[g] - m_new), pv = fast_exp2(s - m_new);
-            m[g] = m_new;
-            l[g] = l[g] * alpha + ((j & 1) ? 0.f : pv);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[g][e] *= alpha;
-            // token 2 it + hw sits in lanes whose bits (8, 4, 2) spell it: fetch each weight from there
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const float w = __shfl_sync(0xffffffffu, pv, (lane & 16) | ((it & 4) << 1) | ((it & 2) << 1) | ((it & 1) << 1));
-                float vf[8];
-                unpack8(vr[it], vf);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) o[g][e] = fmaf(w, vf[e], o[g][e]);
-            }
-        }
+        st.chunk(wl, kr, vr, old - ck * CHUNK);
 #pragma unroll
         for (int it = 0; it < 8; ++it) {
             kr[it] = kn[it];
@@ -176,55 +94,22 @@ __global__ void __launch_bounds__(SW * 32, 1) paged_decode_small_kernel(const De
         const uint4 v_raw = *reinterpret_cast<const uint4*>(qrow + (p.hkv * G + p.hkv + kvh) * D);
         unpack8(*reinterpret_cast<const uint4*>(qrow + (p.hkv * G + kvh) * D), kn);
         unpack8(v_raw, vn);
-        norm_rope(kn, kw);
+        walk_norm_rope(wl, kn, kw, cosr, sinr, p.eps);
         if (hw == 0 && writer) {
             const int64_t at = (((int64_t)bt[old >> p.block_shift] * p.hkv + kvh) << p.block_shift) + (old & mask);
             *reinterpret_cast<uint4*>(p.k_layer_w + at * D + j * 8) = pack8(kn);
             *reinterpret_cast<uint4*>(p.v_layer_w + at * D + j * 8) = v_raw;
         }
-#pragma unroll
-        for (int g = 0; g < GW; ++g) {
-            float s = qf[g][0] * kn[0];
-#pragma unroll
-            for (int e = 1; e < 8; ++e) s = fmaf(qf[g][e], kn[e], s);
-#pragma unroll
-            for (int o2 = 8; o2 > 0; o2 >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o2);
-            const float m_new = fmaxf(m[g], s), alpha = fast_exp2(m[g] - m_new), pn = fast_exp2(s - m_new);
-            m[g] = m_new;
-            l[g] = l[g] * alpha + (lane == 0 ? pn : 0.f);
-            const float w = hw == 0 ? pn : 0.f;    // the halves' results are summed below
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[g][e] = fmaf(w, vn[e], o[g][e] * alpha);
-        }
+        st.own(wl, kn, vn);
     }
     // ---- the warps of this CTA meet ----
-#pragma unroll
-    for (int g = 0; g < GW; ++g) {
-        l[g] = warp_sum(l[g]);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[g][e] += __shfl_xor_sync(0xffffffffu, o[g][e], 16);
-        if (hw == 0) {
-            *reinterpret_cast<float4*>(&sh_o[warp][g][j * 8]) = make_float4(o[g][0], o[g][1], o[g][2], o[g][3]);
-            *reinterpret_cast<float4*>(&sh_o[warp][g][j * 8 + 4]) = make_float4(o[g][4], o[g][5], o[g][6], o[g][7]);
-        }
-        if (lane == 0) {
-            sh_ml[warp][g][0] = m[g];
-            sh_ml[warp][g][1] = l[g];
-        }
-    }
+    st.leave(wl, sh_o[warp], sh_ml[warp]);
     __syncthreads();
     auto store = [&](int g, int d, float v) { p.out[(int64_t)b * p.out_stride + (head0 + g) * D + d] = __float2bfloat16_rn(v); };
     for (int i = tid; i < GW * D; i += SW * 32) {
         const int g = i / D, d = i % D;
-        float M = -INFINITY, L = 0.f, a = 0.f;
-#pragma unroll
-        for (int w = 0; w < SW; ++w) M = fmaxf(M, sh_ml[w][g][0]);
-#pragma unroll
-        for (int w = 0; w < SW; ++w) {
-            const float f = sh_ml[w][g][0] == -INFINITY ? 0.f : fast_exp2(sh_ml[w][g][0] - M);
-            L = fmaf(f, sh_ml[w][g][1], L);
-            a = fmaf(f, sh_o[w][g][d], a);
-        }
+        float M, L, a;
+        walk_meet(sh_o, sh_ml, g, d, M, L, a);
         if (splits == 1) {
             store(g, d, L > 0.f ? a / L : 0.f);
         } else {

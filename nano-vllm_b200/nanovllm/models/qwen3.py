@@ -111,6 +111,8 @@ class Qwen3ForCausalLM:
         fits = all(k % 512 == 0 and k <= 3072 and n % 16 == 0 for n, k in ((self.q_size + 2 * self.kv_size, self.hidden), (self.hidden, self.q_size),
                                                                            (self.inter, self.hidden), (self.hidden, self.inter)))
         self.few_rows = min(16, self.tc_max_rows) if mode == "auto" and self.tc_linear and tp_size == 1 and fits and max(tcc[3], tcc[5]) <= 8 else 0
+        # ... or all layers as one kernel (csrc/step_rows.cu), where the step is its: again the same bits
+        self.one_kernel_step = self.few_rows > 0 and self.tc_cfg[3] == self.tc_cfg[5] == 8 and self.device.type == "cuda"
         # B200_TAIL=mega: in decode steps of up to 256 rows on one GPU, everything between two attention kernels
         # (o_proj, add+norm, gate_up+SiluAndMul, down_proj, add+norm, the next layer's qkv_proj) is ONE persistent launch
         # (csrc/layer_tail.cu) instead of seven.  Measured 58-70 us per layer against 30 us for the chain (r02_layer_tail_microbench.json):
@@ -375,8 +377,14 @@ class Qwen3ForCausalLM:
             return self._forward_dual(input_ids, positions, ctx)
         if self.mega_tail and not ctx.is_prefill and input_ids.shape[0] <= self.mega_rows and self.attn[0].k_cache.numel() > 0:
             return self._forward_mega(input_ids, positions, ctx)
+        few = not ctx.is_prefill and 0 < input_ids.shape[0] <= self.few_rows and self.attn[0].k_cache.numel() > 0
+        if few and self.one_kernel_step and input_ids.shape[0] <= self.fused_decode_max_batch:
+            out = ops.step_rows(input_ids, self.embed, [(L.qkv, L.o, L.gate_up, L.down, L.ln1, L.ln2, L.q_norm, L.k_norm) for L in self.layers], self.norm, eps,
+                                self.cos_sin, ctx.block_tables, ctx.context_lens, hq, self.attn[0].scale)
+            if out is not None:
+                return out
         h = ops.embedding(input_ids, self.embed)
-        if not ctx.is_prefill and 0 < h.shape[0] <= self.few_rows and self.attn[0].k_cache.numel() > 0:
+        if few:
             return self._forward_few_rows(h, positions, ctx)
         residual, in_peer = None, False
         cfg = self.tc_cfg

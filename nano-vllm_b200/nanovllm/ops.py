@@ -341,6 +341,36 @@ def linear_rows(x: torch.Tensor, w: torch.Tensor, norm_w: torch.Tensor | None = 
     return out, residual
 
 
+def step_rows(ids: torch.Tensor, embed: torch.Tensor, layers: list, final_norm: torch.Tensor, eps: float, cos_sin: torch.Tensor, block_tables: torch.Tensor,
+              context_lens: torch.Tensor, num_q_heads: int, scale: float) -> torch.Tensor | None:
+    """All layers of a decode step of at most 8 rows in one launch: token ids -> normed hidden states [rows, hidden], K and V appended to the cache's layers
+    0, 1, ...; ``layers``: per layer (qkv, o, gate_up, down, ln1, ln2, q_norm, k_norm).  None where the step is not the kernel's (csrc/step_rows.cu has the rule)."""
+    import ctypes
+    rows, hidden, inter, stride = ids.numel(), embed.shape[1], layers[0][3].shape[1], block_tables.stride(0)
+    h = nat.handle()
+    need = h.lib.b200_step_rows_workspace_bytes(h.ptr, rows, len(layers), hidden, inter, num_q_heads, stride)
+    if need == 0:
+        return None
+    _need(ids, torch.int64, "ids"); _need(block_tables, torch.int32, "block_tables"); _need(context_lens, torch.int32, "context_lens"); _need(cos_sin, torch.float32, "cos_sin")
+    q, qkv = num_q_heads * 128, (num_q_heads + 2 * h.kv.shape[3]) * 128
+    shapes = ((qkv, hidden), (hidden, q), (2 * inter, hidden), (hidden, inter), (hidden,), (hidden,), (128,), (128,))
+    for ws in (*layers, (embed, final_norm)):
+        for w in ws:
+            if w.dtype != torch.bfloat16 or not w.is_cuda or not w.is_contiguous() or w.data_ptr() & 15:
+                return None
+    if any(tuple(w.shape) != s for ws in layers for w, s in zip(ws, shapes)) or final_norm.numel() != hidden:
+        return None
+    assert ids.is_contiguous() and cos_sin.is_contiguous() and context_lens.is_contiguous() and block_tables.stride(1) == 1
+    assert block_tables.shape[0] >= rows and context_lens.numel() >= rows
+    ptrs = (ctypes.c_void_p * (8 * len(layers)))(*(w.data_ptr() for ws in layers for w in ws))
+    out = torch.empty(rows, hidden, dtype=torch.bfloat16, device=ids.device)
+    ws = torch.empty(need, dtype=torch.uint8, device=ids.device)
+    nat.check(h.lib.b200_step_rows(h.ptr, ptrs, len(layers), ids.data_ptr(), embed.data_ptr(), embed.shape[0], final_norm.data_ptr(), cos_sin.data_ptr(), eps,
+                                   block_tables.data_ptr(), stride, context_lens.data_ptr(), out.data_ptr(), rows, hidden, inter, num_q_heads, scale,
+                                   ws.data_ptr(), ws.numel(), _stream()), h.ptr)
+    return out
+
+
 def lm_head_sample(hidden: torch.Tensor, lm_head: torch.Tensor, temperatures: torch.Tensor | None, seed: int, step: int,
                    key_workspace: torch.Tensor, out: torch.Tensor | None = None, index_offset: int = 0,
                    out_keys: torch.Tensor | None = None, step_dev: torch.Tensor | None = None, block_n: int = 128,
