@@ -17,9 +17,20 @@ int b200m_moe_gemm_tc(const void* A, int64_t a_stride, const int32_t* sorted_row
 
 namespace {
 
+// A warp's best (value, index): the largest value, among equals the lowest index; lanes without one say NONE.  Values are no NaN; they are compared as whole numbers of the same
+// order (zeros of either sign as one), two reductions of the warp where ten shuffles and their comparisons were.  All lanes get both.
+constexpr int ROUTE_NONE = 0x7fffffff;
+__device__ __forceinline__ int route_best(float& v, int index) {
+    const uint32_t bits = __float_as_uint(v + 0.0f);                         // -0 + 0 = 0
+    const uint32_t key = index == ROUTE_NONE ? 0u : (bits & 0x80000000u) ? ~bits : bits | 0x80000000u;     // -inf: 0x007fffff, above NONE's
+    const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+    v = __uint_as_float((top & 0x80000000u) ? top & 0x7fffffffu : ~top);
+    return __reduce_min_sync(0xffffffffu, key == top ? (uint32_t)index : (uint32_t)ROUTE_NONE);
+}
+
 // One warp per token: lane l looks at experts l, l + 32, ...; the chosen ones are struck from a per-lane bit mask (so the kernel
-// serves up to 1024 experts), and every round ends in a warp arg-max that prefers the lower index among equal logits.  Lane 0's
-// result is broadcast before it is struck, so exactly the reported expert leaves the candidates whatever the logits hold (a NaN
+// serves up to 1024 experts), and every round ends in a warp arg-max that prefers the lower index among equal logits.  All lanes get the
+// result before it is struck, so exactly the reported expert leaves the candidates whatever the logits hold (a NaN
 // counts as minus infinity): the indices are always valid and distinct.
 __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict__ logits, int64_t ld, int n, int E, int top,
                                                         int32_t* __restrict__ idx, float* __restrict__ wgt) {
@@ -27,7 +38,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= n) return;
     const float* z = logits + (int64_t)t * ld;
-    constexpr int NONE = 0x7fffffff;
+    constexpr int NONE = ROUTE_NONE;
     uint32_t taken = 0;
     for (int k = 0; k < top; ++k) {
         int best = NONE;
@@ -40,17 +51,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
                 bv = v;
             }
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-            const int ob = __shfl_xor_sync(0xffffffffu, best, off);
-            if (ob != NONE && (best == NONE || ov > bv || (ov == bv && ob < best))) {
-                bv = ov;
-                best = ob;
-            }
-        }
-        best = __shfl_sync(0xffffffffu, best, 0);
-        bv = __shfl_sync(0xffffffffu, bv, 0);
+        best = route_best(bv, best);
         if (best == NONE) best = 0;                       // cannot happen while top <= E; keeps the index in range regardless
         if ((best & 31) == lane) taken |= 1u << (best >> 5);
         if (lane == 0) {
@@ -73,22 +74,25 @@ __global__ void __launch_bounds__(RG_WARPS * 32) moe_route_grouped_kernel(const 
                                                                           int num_real, int score_kind, int renorm, float scale,
                                                                           int32_t* __restrict__ idx, float* __restrict__ wgt) {
     B200_PDL_SYNC();
-    extern __shared__ float sh_route[];               // per warp: E plain scores, then E (at least as many as groups) group scores; after the group
+    extern __shared__ float sh_route[];               // per warp: E plain scores, E scores of choice, E (at least as many as groups) group scores; after the group
                                                       // choice 1 = open, 0 = closed.  Sized to E: 32 KB for the most experts left 28 warps on an SM
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * RG_WARPS + warp;
     if (t >= n) return;
     const float* z = logits + (int64_t)t * ld;
-    float* sc = sh_route + warp * 2 * E;
-    float* gs = sc + E;
-    constexpr int NONE = 0x7fffffff;
+    float *sc = sh_route + warp * 3 * E, *cs = sc + E, *gs = cs + E;
+    constexpr int NONE = ROUTE_NONE;
     if (score_kind == 0) {
         float mx = -INFINITY;
-        for (int e = lane; e < E; e += 32) mx = fmaxf(mx, z[e]);
+        for (int e = lane; e < E; e += 32) {
+            const float v = z[e];
+            sc[e] = v;
+            mx = fmaxf(mx, v);
+        }
         mx = warp_max(mx);
         float sum = 0.f;
         for (int e = lane; e < E; e += 32) {
-            const float p = expf(z[e] - mx);
+            const float p = expf(sc[e] - mx);
             sc[e] = p;
             sum += p;
         }
@@ -98,17 +102,17 @@ __global__ void __launch_bounds__(RG_WARPS * 32) moe_route_grouped_kernel(const 
     } else {
         for (int e = lane; e < E; e += 32) sc[e] = sigmoidf_(z[e]);
     }
+    for (int e = lane; e < E; e += 32) {              // what they are chosen by
+        const float c = sc[e] + (correction ? correction[e] : 0.f);
+        cs[e] = c == c ? c : -INFINITY;
+    }
     __syncwarp();
     const bool grouped = n_groups > 1 && keep < n_groups;
     const int gsize = grouped ? E / n_groups : E;
     if (grouped) {
         for (int gi = lane; gi < n_groups; gi += 32) {
             float best = -INFINITY;
-            for (int e = gi * gsize; e < (gi + 1) * gsize; ++e) {
-                float c = sc[e] + (correction ? correction[e] : 0.f);
-                if (!(c == c)) c = -INFINITY;
-                best = fmaxf(best, c);
-            }
+            for (int e = gi * gsize; e < (gi + 1) * gsize; ++e) best = fmaxf(best, cs[e]);
             gs[gi] = best;
         }
         __syncwarp();
@@ -123,47 +127,29 @@ __global__ void __launch_bounds__(RG_WARPS * 32) moe_route_grouped_kernel(const 
                     bv = v;
                 }
             }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-                const int ob = __shfl_xor_sync(0xffffffffu, best, off);
-                if (ob != NONE && (best == NONE || ov > bv || (ov == bv && ob < best))) {
-                    bv = ov;
-                    best = ob;
-                }
-            }
-            best = __shfl_sync(0xffffffffu, best, 0);
+            best = route_best(bv, best);
             if (best != NONE && (best & 31) == lane) open |= 1u << (best >> 5);
         }
         __syncwarp();
         for (int i = 0, gi = lane; gi < n_groups; ++i, gi += 32) gs[gi] = ((open >> i) & 1u) ? 1.f : 0.f;
         __syncwarp();
     }
-    uint32_t taken = 0;
+    uint32_t taken = 0;                               // chosen experts, and those of closed groups
+    if (grouped)
+        for (int i = 0, e = lane; e < E; ++i, e += 32) taken |= gs[e / gsize] == 0.f ? 1u << i : 0u;
     float wsum = 0.f;
     for (int k = 0; k < top; ++k) {
         int best = NONE;
         float bv = -INFINITY;
         for (int i = 0, e = lane; e < E; ++i, e += 32) {
             if ((taken >> i) & 1u) continue;
-            if (grouped && gs[e / gsize] == 0.f) continue;
-            float c = sc[e] + (correction ? correction[e] : 0.f);
-            if (!(c == c)) c = -INFINITY;
+            const float c = cs[e];
             if (best == NONE || c > bv) {
                 best = e;
                 bv = c;
             }
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-            const int ob = __shfl_xor_sync(0xffffffffu, best, off);
-            if (ob != NONE && (best == NONE || ov > bv || (ov == bv && ob < best))) {
-                bv = ov;
-                best = ob;
-            }
-        }
-        best = __shfl_sync(0xffffffffu, best, 0);
+        best = route_best(bv, best);
         if (best == NONE) best = 0;                   // only if fewer than `top` experts are open; keeps the index in range
         if ((best & 31) == lane) taken |= 1u << (best >> 5);
         const float w = sc[best];
@@ -627,7 +613,7 @@ extern "C" int b200m_moe_route_grouped(const float* logits, int64_t ld, int n, i
     if (score_kind < 0 || score_kind > 1) return B200_EINVAL;
     if (num_outputs > RG_MAX) return B200_EUNSUPPORTED;
     if (n == 0) return B200_OK;
-    B200_LAUNCH((moe_route_grouped_kernel), (n + RG_WARPS - 1) / RG_WARPS, RG_WARPS * 32, (size_t)RG_WARPS * 2 * num_outputs * sizeof(float), static_cast<cudaStream_t>(stream), logits, ld,
+    B200_LAUNCH((moe_route_grouped_kernel), (n + RG_WARPS - 1) / RG_WARPS, RG_WARPS * 32, (size_t)RG_WARPS * 3 * num_outputs * sizeof(float), static_cast<cudaStream_t>(stream), logits, ld,
                 n, num_outputs, top, correction, n_groups, keep, num_real, score_kind, renorm, scale, idx, wgt);
     return b200_launch_status(nullptr);
 }
