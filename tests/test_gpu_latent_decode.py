@@ -93,3 +93,24 @@ def test_pages_below_the_window_may_be_absent():
     for i, l in enumerate(lens):
         tables[i, :max(l - window, 0) // bs] = -1
     assert torch.equal(call(tables), want) and torch.isfinite(want).all()
+
+
+@pytest.mark.parametrize("rank,bs", [(512, 8), (512, 64), (256, 16), (512, 384)])
+def test_tile_edges_and_a_maximum_that_moves(rank, bs):
+    """Contexts around the 64-key tiles and over several turns of the rings; keys that grow with their position, so that the reference maximum moves in tile after tile.
+    Only the latents grow: the kernel has the rotated query in bf16, 2^-9 of it off, which times a rotated key 35 times as long (0.03 * 35 * sqrt(64) * 2^-9 = 0.016 of a score)
+    would show as 1.6 % of the weights."""
+    from nanovllm import mixops as mx
+    from nanovllm.layers.rotary_embedding import build_banded_cos_sin
+    H, rd, lens = 16, 64, [63, 64, 65, 127, 1, 705, 1409, 192]
+    n, nblk = len(lens), sum(-(-c // bs) for c in lens) + 1
+    tables, cache = make_tables(lens, bs, nblk, seed=70), bf(nblk * bs, rank + rd, seed=71)
+    for i, c in enumerate(lens):
+        p = torch.arange(c)
+        rows = tables[i][p // bs].long() * bs + p % bs
+        cache[rows, :rank] = (cache[rows, :rank].float() * (0.05 + p[:, None] / 40)).bfloat16()
+    q_lat, q_raw = bf(H, n, rank, seed=72).cuda(), bf(n, H, 128 + rd, seed=73).cuda()
+    cs = build_banded_cos_sin(rd, 4096, 1e4, None, "cuda")
+    args = (tables.cuda(), bs, mx.StepSpans(n, 1, None, None, torch.tensor(lens, dtype=torch.int32).cuda()), torch.linspace(-1, 1, H).cuda(), cs, 0.03)
+    want = mx.latent_attention(q_lat.float(), q_raw.float(), 128, cache.cuda().float(), *args)
+    assert_close_bf16(mx.latent_attention(q_lat, q_raw, 128, cache.cuda(), *args), want, f"{rank} {bs}", rel_l2=6e-3, ulps=3.0)
