@@ -13,7 +13,7 @@
 
 // moe_tc.cu: the grouped GEMM on tcgen05; B200_EUNSUPPORTED for shapes it does not take
 int b200m_moe_gemm_tc(const void* A, int64_t a_stride, const int32_t* sorted_rows, const int32_t* tile_expert, const int32_t* num_tiles, int max_tiles, const void* W, int N, int K,
-                      void* C, int out_f32, int act, int rows_per_expert, cudaStream_t stream);
+                      void* C, int out_f32, int act, int rows_per_expert, int early, cudaStream_t stream);
 
 namespace {
 
@@ -662,7 +662,7 @@ extern "C" int b200m_moe_gemm(const void* A, int64_t a_stride, const int32_t* so
     const bool tc = !is32 && (K % 8 == 0) && (a_stride % 8 == 0) && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) % 16 == 0);
     if (tc) {
         const int rc = gather ? B200_EUNSUPPORTED
-                              : b200m_moe_gemm_tc(A, a_stride, sorted_rows, tile_expert, num_tiles, max_tiles, W, N, K, C, out_f32, act, rows_per_expert, st);
+                              : b200m_moe_gemm_tc(A, a_stride, sorted_rows, tile_expert, num_tiles, max_tiles, W, N, K, C, out_f32, act, rows_per_expert, 0, st);
         if (rc != B200_EUNSUPPORTED) return rc;
         dim3 g2(act == 2 ? (n_out + MM_BN / 2 - 1) / (MM_BN / 2) : (N + MM_BN - 1) / MM_BN, max_tiles);
         using bf = __nv_bfloat16;

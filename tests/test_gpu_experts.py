@@ -138,3 +138,31 @@ def test_one_call_counts_as_its_steps_do(mx, N):
     assert (got - want).norm() <= 2e-5 * want.norm()
     cap = mx.moe_capacity(n * top, E)
     assert mx.nat.load_mix().b200m_moe_experts_workspace_bytes(n * top, E, width, N // 2) <= cap * 2 * (width + N // 2) + 12 * cap + 4096
+
+
+@pytest.mark.parametrize("act,N,K,width", [(1, 256, 64, 2048), (2, 2048, 64, 1024), (2, 512, 200, 2048), (1, 768, 264, 2176)])
+@pytest.mark.parametrize("n", [3, 160])
+def test_few_rows_over_several_turns(mx, n, act, N, K, width):
+    """One call for a few rows of many experts: more items than CTAs at a time, fewer steps of k than the ring has stages, tiles that end the grid's last turn anywhere; in turn with calls
+    of other routings, whose kernels begin while those of the call before are under way."""
+    E, top = 40, 2
+    g = torch.Generator(device="cuda").manual_seed(n + N)
+    inter = N // act
+    w_in = (torch.randn(E, N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    w_out = (torch.randn(E, width, inter, generator=g, device="cuda") * inter ** -0.5).to(torch.bfloat16)
+    calls = []
+    for turn in range(3):
+        idx = torch.stack([torch.randperm(E, generator=g, device="cuda")[:top] for _ in range(n)]).to(torch.int32)
+        h, wgt = torch.randn(n, K, generator=g, device="cuda").to(torch.bfloat16), torch.rand(n, top, generator=g, device="cuda")
+        calls.append((h, idx, wgt))
+    torch.cuda.synchronize()
+    got = [mx.moe_experts(h, idx, wgt, w_in, w_out, act, False) for h, idx, wgt in calls]
+    for (h, idx, wgt), y in zip(calls, got):
+        want = torch.zeros(n, width, device="cuda")
+        for k in range(top):
+            e = idx[:, k].long()
+            x = torch.einsum("tk,tnk->tn", h.float(), w_in[e].float())
+            x = torch.relu(x).square() if act == 1 else torch.nn.functional.silu(x[:, :inter]) * x[:, inter:]
+            want += wgt[:, k, None] * torch.einsum("ti,twi->tw", x.to(torch.bfloat16).float(), w_out[e].float())
+        # the activation is rounded to bf16 on both sides, of sums in another order: a few of its values differ by 2^-8
+        assert ((y - want).norm() / want.norm()).item() < 1e-3
