@@ -17,7 +17,7 @@
 //   * A warp's own chain of instructions is half of a link's time (31 % of the issue slots, nothing else busy), so they are counted: loads without branches, no spilled register (with 28 KB
 //     of L1 beside the ring each reload is a trip to L2: 500 bytes of them made the step 1.4 times as long).
 // Every sum has the order of the launches it replaces (linear_rows.cu, decode_small.cu): the results are theirs bit for bit.  Captured Qwen3-0.6B step, contexts of 100-1024
-// tokens, us, those launches / this kernel: 1 row 590 / 512, 2 rows 737 / 528, 4 rows 672 / 594, 8 rows 746 / 718; contexts of 16-64 tokens, 1 row 582 / 507.  16 rows took 979
+// tokens, us, those launches / this kernel: 1 row 590 / 494, 2 rows 737 / 512, 4 rows 672 / 576, 8 rows 746 / 698; contexts of 16-64 tokens, 1 row 582 / 489.  16 rows took 979
 // / 1160 (twice the exchange and the chunks of a warp one after the other), so they keep their launches.
 // CTAs wait for one another: launched cooperatively, one per SM.  Waits are bounded (wait_report.cuh).
 #include "decode_walk.cuh"
@@ -137,15 +137,18 @@ __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, uint32_t dea
     } while (!ok && !patience.over(SR_TESTS));
     return ok;
 }
-// N pairs of units per lane: pair i at at(i) where use(i), which is the same for all lanes (ALL: always).  One pair of the warp's is waited for first, by one lane, another one in each CTA:
-// all of them polled by everybody took the bandwidth of the L2 slices that hold them from the results themselves.
+// N pairs of units per lane: pair i at at(i) where use(i), which is the same for all lanes (ALL: always).  `one` >= 0: that pair of the warp's is waited for first, by one lane, another
+// one in each CTA; for what all 148 CTAs wait for (the norms' inputs) that is faster, everything else is asked for at once (first one pair everywhere: 1 row 512 us a step, 4
+// rows 594, 8 rows 717; nowhere 500, 578, 705; for the norms alone 494, 576, 698).
 template <int N, bool ALL, typename At, typename Use>
-__device__ __forceinline__ void get_pairs(uint32_t (&v)[N][2], At at, Use use, uint32_t tag, uint32_t dead, uint32_t* report, int first = 0) {
+__device__ __forceinline__ void get_pairs(uint32_t (&v)[N][2], At at, Use use, uint32_t tag, uint32_t dead, uint32_t* report, int one = -1) {
     Patience patience{dead, report};
     uint32_t a, b, bad;
-    const bool asks = (threadIdx.x & 31) == (blockIdx.x & 31);
-    do bad = get2_if(at(first), tag, a, b, asks);
-    while (__any_sync(0xffffffffu, bad) && !patience.over(SR_POLLS));
+    if (one >= 0) {
+        const bool asks = (threadIdx.x & 31) == (blockIdx.x & 31);
+        do bad = get2_if(at(one), tag, a, b, asks);
+        while (__any_sync(0xffffffffu, bad) && !patience.over(SR_POLLS));
+    }
     do {
         bad = 0;
 #pragma unroll
