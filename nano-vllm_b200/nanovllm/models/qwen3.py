@@ -11,7 +11,8 @@ inside them.  Per layer and per step this issues
 GEMMs of prompts and of large decode steps are library calls (cuBLAS through ``F.linear``, as in the reference,
 linear.py:51,73,153); decode steps of up to 128 rows have o_proj and down_proj on tcgen05 with split k (``ops.linear``), those
 of up to 16 rows all four projections as row-wise products with the norms and the activation inside (``ops.linear_rows``:
-four launches a layer around attention).  Everything else is one hand-written kernel from libb200attn.  Tensor parallelism shards heads and
+four launches a layer around attention), and steps of up to 8 rows are one launch over all layers where
+``ops.step_rows`` takes them.  Everything else is one hand-written kernel from libb200attn.  Tensor parallelism shards heads and
 MLP columns exactly like the reference's *ParallelLinear classes (linear.py:54-156) and all-reduces
 after o_proj and down_proj only; the embedding table is replicated and the LM head stays
 vocab-sharded with a (max, argmax) combine instead of a logits gather (embed_head.py:56-66).
