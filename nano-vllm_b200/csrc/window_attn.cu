@@ -364,13 +364,23 @@ __device__ __forceinline__ float wm_softcap(float v, float k, float cap2) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + wm_ex2(v * k)));
     return fmaf(-2.0f * cap2, r, cap2);
 }
+__device__ __forceinline__ void wm_mul2(float& a, float& b, float f) {       // both times f
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "+f"(a), "+f"(b)
+        : "f"(f));
+}
 __device__ __forceinline__ uint32_t wm_pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
 // KS (single-token steps with at most 16 query heads per key/value head): the CTA's 16 rows are shared by its four warps, each
-// of which takes 16 of a tile's 64 keys with its own running (max, sum, O); the four are merged through shared memory at the end.
+// of which takes 16 of a tile's 64 keys with its own running (max, sum, O); the four are merged through shared memory at the end.  Each warp copies its
+// own keys, both buffers ahead of the tile it is at, and waits for no other warp.  What bounds a CTA is the chain of a tile's instructions, memory only where
+// 350 CTAs and more run at once: 1.25 us per tile when a warp spent 650 instructions on it (cache addresses row by row, masks for rows that have no head,
+// rescaling O one by one) and met the others at two barriers; 400 now, 1.0 us.  16 over 8 heads of 128, a window of 2048, us of the layer: 64 sequences of
+// 1024-4096 tokens 127 -> 111 to 119 (two boxes), 16 of 100-4000 (split) 51.7 -> 47, 32 of 1000-4000 80 -> 68, 128 of 3000 218 -> 203, 8 of 500-8000 41 -> 39; the same
+// bits.  With the two barriers 118-121 (64), 75 (32); copies one tile ahead 112-117, 70.
 // PAD: dim <= DK and vdim <= DV (multiples of eight) elements are in memory, the rest of a tile's columns is zero.
 template <int DK, int DV, bool KS, bool QREG, int BN, bool PAD>
 __global__ void __launch_bounds__(128) window_attn_mma_kernel(
@@ -389,8 +399,10 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
     __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(wm_smem);       // [BM][KSTR]
     __nv_bfloat16* Ks = Qs + BM * KSTR;                                  // [2][64][KSTR]
     __nv_bfloat16* Vs = Ks + 2 * BN * KSTR;                           // [2][64][VSTR]
-    const int s = blockIdx.y, rep = H / G;
-    const int gz = blockIdx.z / splits, split = blockIdx.z - gz * splits;
+    // key-sharing: heads first, then splits, then sequences, so that the heads that read the same cache rows run at about the same time (heads last: 128
+    // sequences of 3000 tokens 220 us for 217, 56 of them 124 for 122, no difference where one wave holds all)
+    const int s = KS ? blockIdx.z : blockIdx.y, rep = H / G, bz = KS ? blockIdx.y : blockIdx.z;
+    const int split = KS ? bz / (G * vsets) : bz % splits, gz = KS ? bz % (G * vsets) : bz / splits;
     const int g = gz / vsets, vs = gz - g * vsets, vh = vsets > 1 ? vs : g;     // key head, value set, value head
     const int HV = H * vsets;
     const SeqSpan sp = seq_span(cu_q, cu_k, ctx_lens, s);
@@ -415,25 +427,59 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
     auto tile_of = [&](int u) { return u < n_keep ? u : t_lo + (u - n_keep); };
     const int32_t* bt = block_tables + (int64_t)s * bt_stride;
 
-    // a tile's rows: eight lanes copy one cache row (128 contiguous bytes per step), sixteen rows per pass.  The page numbers of a
-    // tile are looked up one tile ahead of its copies, so that the table read never stands between a warp and its next MMAs.
-    const int lr = tid >> 3, lc = tid & 7;
-    auto lookup = [&](int u, int (&pg)[BN / 16]) {
+    // a tile's rows: eight lanes copy one cache row (128 contiguous bytes per step), all threads sixteen rows per pass, or, key-sharing, each warp its own
+    // sixteen in four.  The page numbers of a tile are looked up one tile ahead of its copies, so that the table read never stands between a warp and its next MMAs.
+    constexpr int STEP = KS ? 4 : 16, PASSES = KS ? 4 : BN / 16;
+    const int lr = KS ? warp * 16 + (lane >> 3) : tid >> 3, lc = tid & 7;
+    // key-sharing and pages of a multiple of sixteen rows: a warp's rows lie in one page, one behind the other
+    const bool one_page = KS && bs_shift >= 4;
+    const uint32_t k_to = smem_u32(Ks + lr * KSTR + lc * 8), v_to = smem_u32(Vs + lr * VSTR + lc * 8);
+    auto lookup = [&](int u, int (&pg)[PASSES]) {
         const int t = tile_of(u);
+        if (one_page) {
+            const int j = t * BN + warp * 16;
+            pg[0] = u < u_hi && j < kmax ? bt[j >> bs_shift] : -1;
+            return;
+        }
 #pragma unroll
-        for (int p = 0; p < BN / 16; ++p) {
-            const int j = t * BN + p * 16 + lr;
+        for (int p = 0; p < PASSES; ++p) {
+            const int j = t * BN + p * STEP + lr;
             pg[p] = (u < u_hi && j < kmax) ? bt[bs_shift >= 0 ? j >> bs_shift : j / block_size] : -1;
         }
     };
-    auto load_tile = [&](int buf, int u, const int (&pg)[BN / 16]) {
+    auto load_tile = [&](int buf, int u, const int (&pg)[PASSES]) {
         const int j0 = tile_of(u) * BN;
         __nv_bfloat16* kd = Ks + buf * BN * KSTR;
         __nv_bfloat16* vd = Vs + buf * BN * VSTR;
         constexpr int KC = DK / 8, VC = DV / 8;
+        if (one_page) {
+            const int j = j0 + lr, left = pg[0] >= 0 ? kmax - j : 0;     // rows from this lane's first one on
+            const int64_t row = ((int64_t)max(pg[0], 0) << bs_shift) + (j & (block_size - 1));
+            const __nv_bfloat16* ks = cache + row * row_elems + g * dk + lc * 8;
+            const __nv_bfloat16* vs_ = cache + row * row_elems + v_off + vh * dv + lc * 8;
+            const uint32_t kb = k_to + buf * (BN * KSTR * 2), vb = v_to + buf * (BN * VSTR * 2);
 #pragma unroll
-        for (int p = 0; p < BN / 16; ++p) {
-            const int r = p * 16 + lr;
+            for (int p = 0; p < PASSES; ++p, ks += STEP * row_elems, vs_ += STEP * row_elems) {
+                const int nb = p * STEP < left ? 16 : 0;
+#pragma unroll
+                for (int c = 0; c < KC; c += 8) {
+                    if (KC % 8 && c + lc >= KC) break;
+                    const bool in = !PAD || (c + lc) * 8 < dk;
+                    wm_cp16(kb + (p * STEP * KSTR + c * 8) * 2, in ? ks + c * 8 : cache, in ? nb : 0);
+                }
+#pragma unroll
+                for (int c = 0; c < VC; c += 8) {
+                    if (VC % 8 && c + lc >= VC) break;
+                    const bool in = !PAD || (c + lc) * 8 < dv;
+                    wm_cp16(vb + (p * STEP * VSTR + c * 8) * 2, in ? vs_ + c * 8 : cache, in ? nb : 0);
+                }
+            }
+            wm_commit();
+            return;
+        }
+#pragma unroll
+        for (int p = 0; p < PASSES; ++p) {
+            const int r = p * STEP + lr;
             const int j = j0 + r;
             const bool ok = pg[p] >= 0;
             const int in_page = bs_shift >= 0 ? j & (block_size - 1) : j % block_size;
@@ -452,10 +498,18 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
         }
         wm_commit();
     };
-    int pg[BN / 16];
+    int pg[PASSES];
     lookup(u_lo, pg);
-    if (u_lo < u_hi) load_tile(0, u_lo, pg);
-    lookup(u_lo + 1, pg);
+    if constexpr (KS) {                                   // both buffers are on their way from the start
+        int second[PASSES];
+        lookup(u_lo + 1, second);
+        if (u_lo < u_hi) load_tile(0, u_lo, pg);
+        if (u_lo + 1 < u_hi) load_tile(1, u_lo + 1, second);
+        lookup(u_lo + 2, pg);
+    } else {
+        if (u_lo < u_hi) load_tile(0, u_lo, pg);
+        lookup(u_lo + 1, pg);
+    }
 
     // queries of this CTA's rows (plain loads; visible after the loop's first barrier)
     for (int e = tid; e < BM * (DK / 8); e += 128) {
@@ -488,7 +542,8 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
     const int wr0 = row0 + wrow, wr1 = min(nrows - 1, wr0 + 15);
     const int w_hi = wr0 < nrows ? first + wr1 / rep : -1;
     const int w_lo = rule.first_key(first + wr0 / rep);
-    const int f_hi = wr0 + 15 < nrows ? first + wr0 / rep : -1;
+    // (key-sharing: all rows are of one token, and what rows without a head sum up is not read)
+    const int f_hi = KS || wr0 + 15 < nrows ? first + wr0 / rep : -1;
     const int f_lo = rule.first_key(first + max(wr1, 0) / rep);
     const bool capped = rule.softcap > 0.f;
     const float scale2 = capped ? 1.0f : scale * WM_LOG2E;             // capped scores arrive scaled and in base-2 units
@@ -516,14 +571,14 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
 
     for (int u = u_lo; u < u_hi; ++u) {
         const int buf = (u - u_lo) & 1;
-        if (u + 1 < u_hi) {
+        if (!KS && u + 1 < u_hi) {
             load_tile(buf ^ 1, u + 1, pg);
             lookup(u + 2, pg);
-            wm_wait<1>();
-        } else {
-            wm_wait<0>();
         }
-        __syncthreads();
+        if (u + 1 < u_hi) wm_wait<1>();
+        else wm_wait<0>();
+        if constexpr (KS) __syncwarp();
+        else __syncthreads();
         const int j0 = tile_of(u) * BN + wkey;                        // first key this warp multiplies
         if (w_hi >= j0 && (w_lo < j0 + WK || j0 < keep_first)) {         // warp-uniform: some row of this warp sees some key of its share
             const __nv_bfloat16* kt = Ks + buf * BN * KSTR + wkey * KSTR;
@@ -563,7 +618,18 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
             }
             // scale, bias, mask; running maximum.  Inside the window of every row of the warp no mask is needed: two FMAs per score.
             float m_new[2] = {m_run[0], m_run[1]};
-            if (j0 + WK - 1 <= f_hi && j0 >= f_lo) {
+            if (KS && j0 + WK - 1 <= f_hi && j0 >= f_lo) {
+                const float d = (float)(pos_r[0] - j0 - 2 * t4);         // exact, and so is what is taken from it: the scores of the general form
+#pragma unroll
+                for (int n = 0; n < WK / 8; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int hh = e >> 1;
+                        const float v = fmaf(sc[n][e], scale2, -slope2[hh] * (d - (float)(n * 8 + (e & 1))));
+                        sc[n][e] = v;
+                        m_new[hh] = fmaxf(m_new[hh], v);
+                    }
+            } else if (!KS && j0 + WK - 1 <= f_hi && j0 >= f_lo) {
                 const float base0 = -slope2[0] * (float)(pos_r[0] - j0 - 2 * t4), base1 = -slope2[1] * (float)(pos_r[1] - j0 - 2 * t4);
 #pragma unroll
                 for (int n = 0; n < WK / 8; ++n)
@@ -606,12 +672,22 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
                     sc[n][e] = p;
                     l_run[e >> 1] += p;
                 }
+            if constexpr (KS) {
+                if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {          // a new maximum (with a distance bias in most tiles, without in few)
 #pragma unroll
-            for (int n = 0; n < DV / 8; ++n) {
-                o[n][0] *= alpha[0];
-                o[n][1] *= alpha[0];
-                o[n][2] *= alpha[1];
-                o[n][3] *= alpha[1];
+                    for (int n = 0; n < DV / 8; ++n) {
+                        wm_mul2(o[n][0], o[n][1], alpha[0]);
+                        wm_mul2(o[n][2], o[n][3], alpha[1]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int n = 0; n < DV / 8; ++n) {
+                    o[n][0] *= alpha[0];
+                    o[n][1] *= alpha[0];
+                    o[n][2] *= alpha[1];
+                    o[n][3] *= alpha[1];
+                }
             }
             // O += P V: P from the S fragments, V through transposing loads
             const uint32_t v_base = smem_u32(vt + ((lane & 7) + (((lane >> 3) & 1) << 3)) * VSTR + ((lane >> 4) << 3));
@@ -639,7 +715,16 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
                 }
             }
         }
-        __syncthreads();                                                 // the tile is consumed: its buffer may be refilled
+        // the tile is consumed: its buffer may be refilled (key-sharing: a warp's own part of it, by that warp)
+        if constexpr (KS) {
+            __syncwarp();
+            if (u + 2 < u_hi) {
+                load_tile(buf, u + 2, pg);
+                lookup(u + 3, pg);
+            }
+        } else {
+            __syncthreads();
+        }
     }
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
@@ -649,6 +734,7 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
     if constexpr (KS) {
         // merge the four warps' partials of the 16 rows through shared memory (the value buffers: all tiles are consumed)
         float* scr = reinterpret_cast<float*>(Vs);                       // [4][16][DV + 2]: max, sum, O
+        __syncthreads();
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
             float* pr = scr + ((size_t)warp * 16 + gq + 8 * hh) * (DV + 2);
@@ -775,7 +861,8 @@ int launch_window_mma_as(const void* q, int64_t q_stride, const void* cache, int
     int bs_shift = -1;
     if ((block_size & (block_size - 1)) == 0)
         for (bs_shift = 0; (1 << bs_shift) < block_size; ++bs_shift) {}
-    dim3 grid((max_q * (H / G) + BM - 1) / BM, num_seqs, G * vsets * splits);
+    const int shares = G * vsets * splits;
+    dim3 grid((max_q * (H / G) + BM - 1) / BM, KS ? shares : num_seqs, KS ? num_seqs : shares);
     bf* out16 = out_f32 ? nullptr : static_cast<bf*>(out);
     float* out32 = out_f32 ? static_cast<float*>(out) : nullptr;
     B200_LAUNCH((window_attn_mma_kernel<DK, DV, KS, QREG, BN, PAD>), grid, 128, smem, stream, static_cast<const bf*>(q), q_stride,
