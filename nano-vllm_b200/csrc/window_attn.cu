@@ -379,7 +379,7 @@ __device__ __forceinline__ uint32_t wm_pack(float lo, float hi) {
 // own keys, both buffers ahead of the tile it is at, and waits for no other warp.  What bounds a CTA is the chain of a tile's instructions, memory only where
 // 350 CTAs and more run at once: 1.25 us per tile when a warp spent 650 instructions on it (cache addresses row by row, masks for rows that have no head,
 // rescaling O one by one) and met the others at two barriers; 400 now, 1.0 us.  16 over 8 heads of 128, a window of 2048, us of the layer: 64 sequences of
-// 1024-4096 tokens 127 -> 111 to 119 (two boxes), 16 of 100-4000 (split) 51.7 -> 47, 32 of 1000-4000 80 -> 68, 128 of 3000 218 -> 203, 8 of 500-8000 41 -> 39; the same
+// 1024-4096 tokens 127 -> 111 to 119 (two boxes), 16 of 100-4000 (split) 51.5 -> 43.8, 32 of 1000-4000 80 -> 68, 128 of 3000 218 -> 203, 8 of 500-8000 41 -> 39; the same
 // bits.  With the two barriers 118-121 (64), 75 (32); copies one tile ahead 112-117, 70.
 // PAD: dim <= DK and vdim <= DV (multiples of eight) elements are in memory, the rest of a tile's columns is zero.
 template <int DK, int DV, bool KS, bool QREG, int BN, bool PAD>
@@ -429,25 +429,25 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
 
     // a tile's rows: eight lanes copy one cache row (128 contiguous bytes per step), all threads sixteen rows per pass, or, key-sharing, each warp its own
     // sixteen in four.  The page numbers of a tile are looked up one tile ahead of its copies, so that the table read never stands between a warp and its next MMAs.
-    constexpr int STEP = KS ? 4 : 16, PASSES = KS ? 4 : BN / 16;
+    constexpr int STEP = KS ? 4 : 16, PASSES = KS ? 4 : BN / 16, PAGES = KS ? 1 : PASSES;
     const int lr = KS ? warp * 16 + (lane >> 3) : tid >> 3, lc = tid & 7;
     // key-sharing and pages of a multiple of sixteen rows: a warp's rows lie in one page, one behind the other
     const bool one_page = KS && bs_shift >= 4;
     const uint32_t k_to = smem_u32(Ks + lr * KSTR + lc * 8), v_to = smem_u32(Vs + lr * VSTR + lc * 8);
-    auto lookup = [&](int u, int (&pg)[PASSES]) {
+    auto lookup = [&](int u, int (&pg)[PAGES]) {
         const int t = tile_of(u);
-        if (one_page) {
-            const int j = t * BN + warp * 16;
-            pg[0] = u < u_hi && j < kmax ? bt[j >> bs_shift] : -1;
-            return;
-        }
+        if constexpr (KS) {                               // the warp's page, or a lane's row's (lanes 16 and up: the same rows again)
+            const int j = t * BN + warp * 16 + (one_page ? 0 : lane & 15);
+            pg[0] = u < u_hi && j < kmax ? bt[bs_shift >= 0 ? j >> bs_shift : j / block_size] : -1;
+        } else {
 #pragma unroll
-        for (int p = 0; p < PASSES; ++p) {
-            const int j = t * BN + p * STEP + lr;
-            pg[p] = (u < u_hi && j < kmax) ? bt[bs_shift >= 0 ? j >> bs_shift : j / block_size] : -1;
+            for (int p = 0; p < PAGES; ++p) {
+                const int j = t * BN + p * STEP + lr;
+                pg[p] = (u < u_hi && j < kmax) ? bt[bs_shift >= 0 ? j >> bs_shift : j / block_size] : -1;
+            }
         }
     };
-    auto load_tile = [&](int buf, int u, const int (&pg)[PASSES]) {
+    auto load_tile = [&](int buf, int u, const int (&pg)[PAGES]) {
         const int j0 = tile_of(u) * BN;
         __nv_bfloat16* kd = Ks + buf * BN * KSTR;
         __nv_bfloat16* vd = Vs + buf * BN * VSTR;
@@ -477,13 +477,15 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
             wm_commit();
             return;
         }
-#pragma unroll
+        constexpr int UNROLL = KS ? 1 : PASSES;           // (key-sharing: small code, such pages are rare)
+#pragma unroll UNROLL
         for (int p = 0; p < PASSES; ++p) {
             const int r = p * STEP + lr;
             const int j = j0 + r;
-            const bool ok = pg[p] >= 0;
+            const int page = KS ? __shfl_sync(0xffffffffu, pg[0], r & 15) : pg[KS ? 0 : p];
+            const bool ok = page >= 0;
             const int in_page = bs_shift >= 0 ? j & (block_size - 1) : j % block_size;
-            const __nv_bfloat16* src = ok ? cache + ((int64_t)pg[p] * block_size + in_page) * row_elems : cache;
+            const __nv_bfloat16* src = ok ? cache + ((int64_t)page * block_size + in_page) * row_elems : cache;
             const int nb = ok ? 16 : 0;
 #pragma unroll
             for (int c = lc; c < KC; c += 8) {
@@ -498,13 +500,16 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
         }
         wm_commit();
     };
-    int pg[PASSES];
+    int pg[PAGES];
     lookup(u_lo, pg);
     if constexpr (KS) {                                   // both buffers are on their way from the start
-        int second[PASSES];
+        int second[PAGES];
         lookup(u_lo + 1, second);
-        if (u_lo < u_hi) load_tile(0, u_lo, pg);
-        if (u_lo + 1 < u_hi) load_tile(1, u_lo + 1, second);
+#pragma unroll 1
+        for (int b = 0; b < 2 && u_lo + b < u_hi; ++b) {
+            load_tile(b, u_lo + b, pg);
+            pg[0] = second[0];
+        }
         lookup(u_lo + 2, pg);
     } else {
         if (u_lo < u_hi) load_tile(0, u_lo, pg);
