@@ -2,6 +2,7 @@
 
     prompt         fa_kernel: two prompts of 4096 tokens, 16 query over 8 kv heads
     window_prompt  fa_kernel: 4 x 2048 tokens over token-major cache rows, window 1024, distance bias
+    window_step    window_attn_mma_kernel, key-sharing: 64 single tokens over 3072 rows, window 2048, 16 over 8 heads
     latent         latent_decode_kernel: 64 single tokens over 3072 cached rows of 512 + 64, 16 heads
     experts        moe_rows_kernel: 8192 tokens x 4 of 32 experts, width 2048, feed-forward 768
     experts_few    moe_stream_kernel: the same of 64 tokens
@@ -37,6 +38,13 @@ def window_prompt():
     q, cache = rnd(8192, 16 * 128), rnd(8192, 8 * 256)
     bt, sp = torch.arange(32, dtype=torch.int32, device=dev).view(4, 8), mixops.StepSpans(4, 2048, cu(4, 2048), cu(4, 2048), None)
     return lambda: mixops.window_attention(q, cache, bt, 256, sp, 16, 8, 128, 128, 0.088, distance_slopes(16, dev), 1024)
+
+
+def window_step():
+    q, cache = rnd(64, 16 * 128), rnd(64 * 3072, 8 * 256)
+    bt = torch.arange(64 * 12, dtype=torch.int32, device=dev).view(64, 12)
+    sp = mixops.StepSpans(64, 1, None, None, torch.full((64,), 3000, dtype=torch.int32, device=dev))
+    return lambda: mixops.window_attention(q, cache, bt, 256, sp, 16, 8, 128, 128, 0.088, distance_slopes(16, dev), 2048)
 
 
 def latent():
@@ -87,7 +95,7 @@ def delta():
 
 
 call = dict(prompt=prompt, window_prompt=window_prompt, latent=latent, experts=experts, experts_few=lambda: experts(64), small_step=small_step,
-            prompt_store=prompt_store, rows=rows, router=router, delta=delta)[sys.argv[1]]()
+            prompt_store=prompt_store, window_step=window_step, rows=rows, router=router, delta=delta)[sys.argv[1]]()
 for _ in range(4):
     o = call()
 torch.cuda.synchronize()
