@@ -217,7 +217,10 @@ __global__ void __launch_bounds__(S_THREADS, 2) moe_stream_kernel(const __grid_c
     const bool gated = p.act == 2;
     const int half = p.N >> 1, cols = gated ? 64 : 128, nblk = p.n_out / cols, ksteps = (p.K + 63) / 64;
     const int items = min(p.num_tiles[0], p.max_tiles) * nblk;
-    if ((int)blockIdx.x >= items) return;
+    if ((int)blockIdx.x >= items) {               // this grid ends behind the kernel in front also where no CTA has an item (no token with an expert of its own)
+        if (p.early) B200_PDL_WAIT();
+        return;
+    }
     if (tid == 0) {
         for (int i = 0; i < 2 * S_STAGES + 2; ++i) mbar_init(full + i * 8, 1);
         for (int i = 0; i < 2; ++i) mbar_init(acc_empty + i * 8, 128);

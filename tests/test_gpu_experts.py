@@ -166,3 +166,24 @@ def test_few_rows_over_several_turns(mx, n, act, N, K, width):
             want += wgt[:, k, None] * torch.einsum("ti,twi->tw", x.to(torch.bfloat16).float(), w_out[e].float())
         # the activation is rounded to bf16 on both sides, of sums in another order: a few of its values differ by 2^-8
         assert ((y - want).norm() / want.norm()).item() < 1e-3
+
+
+@pytest.mark.parametrize("act,N,K,width", [(1, 256, 64, 2048), (2, 2048, 64, 1024)])
+@pytest.mark.parametrize("n", [1, 64])
+def test_steps_whose_choices_are_all_identity_experts(mx, n, act, N, K, width):
+    """Without a row for any expert the products' CTAs have no item and leave at once, behind the kernel in front all the same: such steps in turn with ordinary ones, whose
+    workspace the allocator takes from the one just given back."""
+    E, top = 40, 2
+    g = torch.Generator(device="cuda").manual_seed(n + N)
+    inter = N // act
+    w_in = (torch.randn(E, N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    w_out = (torch.randn(E, width, inter, generator=g, device="cuda") * inter ** -0.5).to(torch.bfloat16)
+    h, wgt = torch.randn(n, K, generator=g, device="cuda").to(torch.bfloat16), torch.rand(n, top, generator=g, device="cuda")
+    idx = torch.stack([torch.randperm(E, generator=g, device="cuda")[:top] for _ in range(n)]).to(torch.int32)
+    none = torch.full_like(idx, -1)
+    want = mx.moe_experts(h, idx, wgt, w_in, w_out, act, False)
+    torch.cuda.synchronize()
+    for _ in range(4):
+        got = [mx.moe_experts(h, i, wgt, w_in, w_out, act, False) for i in (none, idx, none, none, idx)]
+        for y, i in zip(got, (none, idx, none, none, idx)):
+            assert torch.equal(y, want) if i is idx else not y.any()
