@@ -11,14 +11,14 @@
 //     barrier, no fence, no second trip for the data.  The buffers start as zeros.  Each is used again in every layer: whoever writes it has, through the
 //     chain of products, waited for everybody who read it the layer before (each reader publishes something afterwards that all of the next writers need; a CTA
 //     without tiles of the wide products reads no norms' inputs).  One way takes 0.36 us between two CTAs, 1.3-1.6 us as 148 of them ask for the same lines.
-//   * Keys and values of the cache do not depend on the step: they are on their way to L2 a layer ahead.  Contexts are cut over CTAs as in
-//     decode_small.cu; the first CTA of a context adds the parts up.
+//   * Keys and values of the cache do not depend on the step: a warp's first chunks are on their way to L2 a layer ahead, the others two chunks ahead.  Contexts are cut over
+//     CTAs as in decode_small.cu; the first CTA of a context adds the parts up.
 //   * The residual stream stays in shared memory, a copy per CTA: every CTA forms the norms for itself.
 //   * A warp's own chain of instructions is half of a link's time (31 % of the issue slots, nothing else busy), so they are counted: loads without branches, no spilled register (with 28 KB
 //     of L1 beside the ring each reload is a trip to L2: 500 bytes of them made the step 1.4 times as long).
 // Every sum has the order of the launches it replaces (linear_rows.cu, decode_small.cu): the results are theirs bit for bit.  Captured Qwen3-0.6B step, contexts of 100-1024
-// tokens, us, those launches / this kernel: 1 row 590 / 494, 2 rows 737 / 512, 4 rows 672 / 576, 8 rows 746 / 698; contexts of 16-64 tokens, 1 row 582 / 489.  16 rows took 979
-// / 1160 (twice the exchange and the chunks of a warp one after the other), so they keep their launches.
+// tokens, us, those launches / this kernel: 1 row 590 / 493, 2 rows 737 / 508, 4 rows 672 / 567, 8 rows 746 / 676; contexts of 16-64 tokens, 1 row 582 / 490.  16 rows took 979
+// / 1160 (twice the exchange and the chunks of a warp one after the other), so they keep their launches.  Long contexts: at sr_splits.
 // CTAs wait for one another: launched cooperatively, one per SM.  Waits are bounded (wait_report.cuh).
 #include "decode_walk.cuh"
 #include "tc_common.cuh"
@@ -40,7 +40,10 @@ constexpr int SR_HIDDEN = 1024;                    // widest residual stream
 constexpr int SR_K = 3 * SR_COLS;                  // widest input of o_proj and down_proj
 constexpr int SR_MAX_LAYERS = 64;
 constexpr int SR_MAX_CHUNKS = 128;                 // of one CTA's part of a context
-constexpr int SR_AHEAD = 4;                        // chunks a warp has on their way to L2 a layer ahead
+// Chunks a warp has on their way to L2, of the next layer and along its walk (there is no second pair of registers for the next chunk).  Four of the next layer and none along the walk
+// cost from the fifth chunk on what memory takes to answer (8 rows of 4096 tokens, without the LM head, us: 1260 for the launches' 1202); 4 and 4 1167, 4 and 2 1143, 4 and 6 1259, 2 and 2
+// 1110, asked for in front of the scores, and 1088 behind the values' loads.
+constexpr int SR_AHEAD = 2;
 
 constexpr int SR_SLOTS = 10;
 constexpr int SR_ROWS = 8;                         // one side of mma.sync
@@ -294,6 +297,12 @@ __global__ void __launch_bounds__(SR_THREADS, 1) step_rows_kernel(const __grid_c
     compute_sync();
     auto row_of = [&](int ck) -> int64_t { return (((int64_t)pages[ck - c0] * p.hkv + kvh) << p.block_shift) + (ck * CHUNK & mask); };   // first cache row of a chunk
     const int64_t own_row = attends && ctx > 0 ? (((int64_t)p.block_tables[(int64_t)b * p.bt_stride + (old >> p.block_shift)] * p.hkv + kvh) << p.block_shift) + (old & mask) : -1;
+    auto to_l2 = [&](const __nv_bfloat16* k_layer, const __nv_bfloat16* v_layer, int ck) {             // a chunk's 32 lines of 128 bytes of keys, and of values
+        const int64_t r = ck < c1 ? row_of(ck) : -1;
+        if (r < 0) return;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(k_layer + r * D + lane * 64));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(v_layer + r * D + lane * 64));
+    };
     auto load_chunk = [&](const __nv_bfloat16* layer, int ck, uint4 (&x)[8]) {
         const int64_t at = ck < c1 ? row_of(ck) : -1;                                  // behind the last chunk, or on an absent page: zeros
         walk_load(wl, layer, at, at < 0 ? 0 : old - ck * CHUNK, x);
@@ -519,6 +528,7 @@ __global__ void __launch_bounds__(SR_THREADS, 1) step_rows_kernel(const __grid_c
                 load_chunk(k_layer, ck + SW, kr);
                 st.values(wl, acc, vr, old - ck * CHUNK);
                 load_chunk(v_layer, ck + SW, vr);
+                to_l2(k_layer, v_layer, ck + SR_AHEAD * SW);
             }
             if (ctx > 0 && rank == p.splits - 1 && warp == SW - 1) {                   // the step's own token
                 float kn[8], vn[8];
@@ -575,15 +585,9 @@ __global__ void __launch_bounds__(SR_THREADS, 1) step_rows_kernel(const __grid_c
             narrow_tiles(second ? p.xa : p.xt, second ? inter : q_size, tag, second ? p.xd : p.xo);
         }
         if (second && attends && l + 1 < p.layers) {                                   // the next layer's keys and values, while the others finish this one
-                const int64_t at = (l + 1) * p.layer_elems;
+                const __nv_bfloat16 *k_next = p.k_base + (l + 1) * p.layer_elems, *v_next = p.v_base + (l + 1) * p.layer_elems;
 #pragma unroll 1
-                for (int i = 0, ck = c0 + warp; i < SR_AHEAD && ck < c1; ++i, ck += SW) {
-                    const int64_t r = row_of(ck);
-                    if (r < 0) continue;
-                    const int64_t line = at + r * D + lane * 64;                       // 32 lines of 128 bytes
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.k_base + line));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v_base + line));
-                }
+                for (int i = 0, ck = c0 + warp; i < SR_AHEAD && ck < c1; ++i, ck += SW) to_l2(k_next, v_next, ck);
         }
     }
 }
@@ -610,7 +614,10 @@ SrLayout sr_layout(int sm_count, int rows, int hidden, int inter, int hq, int hk
 }
 
 // Splits of a context, 0 where the step is not this kernel's.  What it takes: one CTA per (sequence, kv head) and split (decode_small.cu's rule, whose sums it repeats), at most a tile
-// of the wide products per warp and of the narrow ones per CTA, ring slots that are full.
+// of the wide products per warp and of the narrow ones per CTA, ring slots that are full.  Up to that rule's longest contexts this kernel is the faster one.  Captured Qwen3-0.6B step without
+// the LM head, tables of the widest such context, every row of the length named, us, launches / here: 1 row of 1024 tokens 577 / 460, 4096 678 / 600, 16384 1054 / 1032; 4 rows of 1024 673 / 554,
+// 4096 890 / 787, 8192 1184 / 1075; 8 rows of 1024 762 / 648, 2048 910 / 793, 4096 1201 / 1088; rows of a k-th of that each (least gain) 6 rows up to 4096 1073 / 1050.  Hidden 512 with 8 over 8
+// or 8 over 4 heads, 1024 with 24 over 12: 1.01 to 1.6 times at every length up to theirs.
 int sr_splits(const b200_ctx* ctx, int rows, int layers, int hidden, int inter, int hq, int bt_stride) {
     if (b200_decode_forced_mma()) return 0;
     if (!ctx->k_base || rows <= 0 || rows > SR_ROWS || layers <= 0 || layers > SR_MAX_LAYERS || layers > ctx->layers || hq <= 0 || ctx->num_kv_heads <= 0) return 0;

@@ -9,7 +9,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def build(monkeypatch, layers, hidden, inter, heads, kv_heads, pages, block):
+def build(monkeypatch, layers, hidden, inter, heads, kv_heads, pages, block, positions=4096):
     from nanovllm import ops
     from nanovllm.models.qwen3 import Qwen3ForCausalLM
     from nanovllm.utils.synthetic import PRESETS, hf_config_dict, random_weights
@@ -17,7 +17,7 @@ def build(monkeypatch, layers, hidden, inter, heads, kv_heads, pages, block):
         monkeypatch.delenv(name, raising=False)
     dims = dict(PRESETS["qwen3-0.6b"], num_hidden_layers=layers, hidden_size=hidden, intermediate_size=inter, num_attention_heads=heads, num_key_value_heads=kv_heads,
                 vocab_size=512)
-    model = Qwen3ForCausalLM(SimpleNamespace(**hf_config_dict(dims)), 0, 1, "cuda", max_position=4096)
+    model = Qwen3ForCausalLM(SimpleNamespace(**hf_config_dict(dims)), 0, 1, "cuda", max_position=positions)
     for name, w in random_weights(dims, seed=5).items():
         model.load_hf_tensor(name, w)
     start = torch.randn(ops.kv_cache_shape(layers, pages, kv_heads, block, 128), device="cuda", generator=torch.Generator(device="cuda").manual_seed(6)).bfloat16()
@@ -77,6 +77,38 @@ def test_same_bits_as_the_launches_replaced(hidden, inter, heads, kv_heads, bloc
             got = step(model, kv, start, lens, tables, ids, True, capture)
             assert calls and all(c is not None for c in calls)
             assert torch.isfinite(got[0]).all() and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), (rows, capture)
+
+
+@pytest.mark.parametrize("hidden,inter,heads,kv_heads", [(1024, 1024, 16, 8), (512, 1024, 8, 8), (1024, 1024, 24, 12)])
+@pytest.mark.parametrize("rows,block", [(1, 16), (1, 256), (2, 256), (3, 64), (4, 16), (8, 256)])
+def test_contexts_up_to_the_rules_upper_end(rows, block, hidden, inter, heads, kv_heads, monkeypatch):
+    """Tables of the widest context that a step of this kind may have, sixteen chunks of sixteen tokens a warp: contexts that fill them and that end around a turn of a CTA's warps, rows of
+    any length beside them.  One page more, and the step is the launches'."""
+    from nanovllm import ops
+    from nanovllm import _native as nat
+    splits = 1
+    while splits < 8 and rows * kv_heads * splits * 2 <= nat.handle().sm_count:
+        splits *= 2
+    most = 16 * 16 * 8 * splits
+    per = most // block
+    model, kv, start = build(monkeypatch, 2, hidden, inter, heads, kv_heads, rows * per, block, most)
+    calls = []
+    real = ops.step_rows
+    monkeypatch.setattr(ops, "step_rows", lambda *a: calls.append(real(*a)) or calls[-1])
+    ids = torch.arange(rows, device="cuda")
+    for turn, first in enumerate((most, most // 2 + 1, most // 8 * 3)):
+        lens = [[first, 5, most - 128, most // 16, 128 * splits + 1, most - 1, 1, most // 3][i] for i in range(rows)]
+        tables = torch.randperm(rows * per, generator=torch.Generator().manual_seed(turn)).view(rows, per)
+        for i, l in enumerate(lens):
+            tables[i, -(-l // block):] = -1                     # as the engine leaves them
+        want = step(model, kv, start, lens, tables.tolist(), ids, False)
+        del calls[:]
+        got = step(model, kv, start, lens, tables.tolist(), ids, True)
+        assert len(calls) == 1 and calls[0] is not None
+        assert torch.isfinite(got[0]).all() and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), lens
+    h = nat.handle()
+    need = lambda width: h.lib.b200_step_rows_workspace_bytes(h.ptr, rows, 2, hidden, inter, heads, width)
+    assert need(per) > 0 and need(per + 1) == 0
 
 
 @pytest.mark.parametrize("rows,hidden,inter,heads,kv_heads,per", [(9, 1024, 3072, 16, 8, 4), (1, 1536, 1024, 8, 4, 4), (4, 1024, 1536, 16, 8, 4), (4, 1024, 1024, 12, 6, 4),
