@@ -12,7 +12,7 @@
 //                      Two CTAs per SM walk the items with a ring each, so that the next item's weights are on their way while one's results are written; a CTA
 //                      per item, three per SM, left a short second turn (512 items on 444 places) and its ramp-up.  Weights do not depend on the kernel in front: the
 //                      first stages of them are asked for before it has ended (MoeParams.early).  Whole layer, us, before / after: 64 tokens 84.9 / 76.8, 256 90.4 / 82.1,
-//                      gated 64 109.4 / 103.4, 200 117.8 / 110.0.  More of them asked into L2 ahead of the ring made it slower (87, gated 110).
+//                      gated 64 108.5 / 100.1, 200 116.0 / 106.4, of width 1024 1 token 45.5 / 43.3, 64 57.2 / 53.8.  More of them asked into L2 ahead of the ring made it slower (87).
 //
 // Both read grouped rows: the experts' inputs are gathered (and weighted) by a copy in front.  Gathering them inside, four rows per TMA
 // gather instruction, took 383 us where the copy and the box loads take 23 + 158 (8192 tokens, width 2048, gate | up), and 89 us against 4.5 + 42 on 64 tokens.
@@ -344,8 +344,10 @@ __global__ void __launch_bounds__(S_THREADS, 2) moe_stream_kernel(const __grid_c
                 asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
                 for (int k = 0; k < 16; ++k) {
+                    const int at = low ? k : 16 + k;
+                    if (src[h * 32 + at] < 0) continue;       // no activation for rows without a pair, of a few tokens most of a tile's (width 1024, 1 token: 48.2 us the layer with it)
                     const float other = theirs[k];
-                    put(low ? k : 16 + k, siluf_(low ? v[k] : other) * (low ? other : v[16 + k]));
+                    put(at, siluf_(low ? v[k] : other) * (low ? other : v[16 + k]));
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
