@@ -380,7 +380,9 @@ __device__ __forceinline__ uint32_t wm_pack(float lo, float hi) {
 // 350 CTAs and more run at once: 1.25 us per tile when a warp spent 650 instructions on it (cache addresses row by row, masks for rows that have no head,
 // rescaling O one by one) and met the others at two barriers; 400 now, 1.0 us.  16 over 8 heads of 128, a window of 2048, us of the layer: 64 sequences of
 // 1024-4096 tokens 127 -> 111 to 119 (two boxes), 16 of 100-4000 (split) 51.5 -> 43.8, 32 of 1000-4000 80 -> 68, 128 of 3000 218 -> 203, 8 of 500-8000 41 -> 39; the same
-// bits.  With the two barriers 118-121 (64), 75 (32); copies one tile ahead 112-117, 70.
+// bits.  With the two barriers 118-121 (64), 75 (32); copies one tile ahead 112-117, 70.  The second tile's copies go out behind the queries: in front of them, steps of a few tiles waited
+// longer for their first one (50 of 500 tokens 40.1 us, 39.1 so; the former kernel 39.5).  Where memory is the bound of a single wave the two kernels are level: 44 / 46 / 48 / 50 / 52
+// sequences of 3000 tokens 85 / 88 / 90 / 95 / 98 us before, 82 / 90 / 92 / 93 / 95 here.
 // PAD: dim <= DK and vdim <= DV (multiples of eight) elements are in memory, the rest of a tile's columns is zero.
 template <int DK, int DV, bool KS, bool QREG, int BN, bool PAD>
 __global__ void __launch_bounds__(128) window_attn_mma_kernel(
@@ -502,19 +504,8 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
     };
     int pg[PAGES];
     lookup(u_lo, pg);
-    if constexpr (KS) {                                   // both buffers are on their way from the start
-        int second[PAGES];
-        lookup(u_lo + 1, second);
-#pragma unroll 1
-        for (int b = 0; b < 2 && u_lo + b < u_hi; ++b) {
-            load_tile(b, u_lo + b, pg);
-            pg[0] = second[0];
-        }
-        lookup(u_lo + 2, pg);
-    } else {
-        if (u_lo < u_hi) load_tile(0, u_lo, pg);
-        lookup(u_lo + 1, pg);
-    }
+    if (u_lo < u_hi) load_tile(0, u_lo, pg);
+    lookup(u_lo + 1, pg);
 
     // queries of this CTA's rows (plain loads; visible after the loop's first barrier)
     for (int e = tid; e < BM * (DK / 8); e += 128) {
@@ -554,6 +545,10 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
     const float scale2 = capped ? 1.0f : scale * WM_LOG2E;             // capped scores arrive scaled and in base-2 units
     const float cap2 = rule.softcap * WM_LOG2E, capk = capped ? 2.0f * WM_LOG2E * scale / rule.softcap : 0.f;
 
+    if constexpr (KS) {                                   // the second buffer, behind the queries, which every warp waits for first
+        if (u_lo + 1 < u_hi) load_tile(1, u_lo + 1, pg);
+        lookup(u_lo + 2, pg);
+    }
     __syncthreads();                                                     // the queries are staged: keep this warp's fragments in registers
     const uint32_t a_base = smem_u32(Qs + (wrow + (lane & 15)) * KSTR + ((lane >> 4) << 3));
     uint32_t qf[QREG ? DK / 16 : 1][4];
