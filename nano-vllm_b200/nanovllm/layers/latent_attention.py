@@ -98,6 +98,8 @@ class LatentAttention:
         q_lat = torch.bmm(q[:, :, :d].transpose(0, 1), self.w_uk)                       # [H, n, R]
         o_lat = mixops.latent_attention(q_lat, q, d, self.cache, ctx.block_tables, self.block_size, spans, self.sink,
                                         self.cos_sin, self.scale)
+        if torch.is_grad_enabled() and self.w_uv.requires_grad:                         # autograd takes no ``out``
+            return F.linear(torch.bmm(o_lat, self.w_uv.transpose(1, 2)).transpose(0, 1).reshape(n, H * self.vdim), self.w_o)
         o = torch.empty(n, H, self.vdim, dtype=h.dtype, device=h.device)                # the heads' products straight to their columns: no copy behind them
         torch.bmm(o_lat, self.w_uv.transpose(1, 2), out=o.transpose(0, 1))
         return F.linear(o.view(n, H * self.vdim), self.w_o)

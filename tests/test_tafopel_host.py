@@ -67,6 +67,31 @@ def test_shapes_beyond_the_kernels_are_refused_at_construction():
     SelectiveScanMixer(64, th.mamba(state=128)["mixer"], torch.float32, "cpu")
 
 
+@pytest.mark.parametrize("grad", [False, True])
+def test_single_token_latent_layer_takes_weights_that_require_grad(grad, monkeypatch):
+    """The last products behind the attention (its kernels have stand-ins here): each head's values in its own columns, where a program keeps the weights as parameters too, outside no_grad."""
+    from types import SimpleNamespace
+    from nanovllm.layers import latent_attention as la
+    m = th.latent()["mixer"]
+    layer = la.LatentAttention(64, m, 1e-5, torch.float32, "cpu", 16)
+    g = torch.Generator().manual_seed(3)
+    for name in ("w_down", "w_uq", "w_ukv", "w_o", "q_norm", "kv_norm"):
+        t = getattr(layer, name)
+        t.copy_(torch.randn(t.shape, generator=g))
+    o_lat = torch.randn(layer.heads, 5, layer.kv_rank, generator=g)
+    monkeypatch.setattr(la.mixops, "rmsnorm", lambda x, w, eps, cols=0: x[:, :cols].contiguous())
+    monkeypatch.setattr(la.mixops, "latent_store", lambda *a: None)
+    monkeypatch.setattr(la.mixops, "latent_expands", lambda *a: False)
+    monkeypatch.setattr(la.mixops, "latent_attention", lambda *a: o_lat)
+    w_uv, w_o = layer.w_uv.clone(), layer.w_o.clone()
+    if grad:
+        layer.w_uv, layer.w_o = torch.nn.Parameter(w_uv), torch.nn.Parameter(w_o)
+    ctx = SimpleNamespace(slot_mapping=None, block_tables=None)
+    y = layer.forward(torch.randn(5, 64, generator=g), None, ctx, None)
+    heads = [o_lat[h] @ w_uv[h].t() for h in range(layer.heads)]
+    assert torch.allclose(y, torch.cat(heads, 1) @ w_o.t(), rtol=1e-5, atol=1e-4) and y.requires_grad == grad
+
+
 def test_state_slots_follow_the_blocks():
     bm = BlockManager(6, 4, num_state_slots=2, prefix_cache=False)
     Sequence.block_size = 4
