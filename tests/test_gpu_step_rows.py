@@ -111,19 +111,28 @@ def test_contexts_up_to_the_rules_upper_end(rows, block, hidden, inter, heads, k
     assert need(per) > 0 and need(per + 1) == 0
 
 
-@pytest.mark.parametrize("rows,hidden,inter,heads,kv_heads,per", [(9, 1024, 3072, 16, 8, 4), (1, 1536, 1024, 8, 4, 4), (4, 1024, 1536, 16, 8, 4), (4, 1024, 1024, 12, 6, 4),
-                                                                 (4, 1024, 1024, 16, 4, 4), (8, 1024, 1024, 16, 8, 400)])
-def test_other_steps_keep_their_launches(rows, hidden, inter, heads, kv_heads, per, monkeypatch):
-    """More rows, other widths, wider head groups, contexts too long for the kernel: the step is taken by the others, whatever it is asked for."""
+@pytest.mark.parametrize("rows,hidden,inter,heads,kv_heads,per,asks", [(9, 1024, 3072, 16, 8, 4, True), (1, 1536, 1024, 8, 4, 4, True), (4, 1024, 1536, 16, 8, 4, True),
+                                                                      (4, 1024, 1024, 12, 6, 4, True), (4, 1024, 1024, 16, 4, 4, False), (8, 1024, 1024, 16, 8, 400, True)])
+def test_other_steps_keep_their_launches(rows, hidden, inter, heads, kv_heads, per, asks, monkeypatch):
+    """More rows, other widths, wider head groups (which the model itself keeps from asking), contexts too long for the kernel: it refuses the step, and the others take it."""
     from nanovllm import ops
+    from nanovllm import _native as nat
     model, kv, start = build(monkeypatch, 1, hidden, inter, heads, kv_heads, 16, 16)
     calls = []
     real = ops.step_rows
     monkeypatch.setattr(ops, "step_rows", lambda *a: calls.append(real(*a)) or calls[-1])
     ids = torch.arange(rows, device="cuda")
     lens, tables = [16] * rows, [[i] + [-1] * (per - 1) for i in range(rows)]
-    out, _ = step(model, kv, start, lens, tables, ids, True)
-    assert torch.isfinite(out).all() and all(c is None for c in calls)
+    want = step(model, kv, start, lens, tables, ids, False)
+    assert not calls
+    out, cache = step(model, kv, start, lens, tables, ids, True)
+    assert bool(calls) == asks and all(c is None for c in calls)
+    assert torch.isfinite(out).all() and torch.equal(out, want[0]) and torch.equal(cache, want[1])
+    h = nat.handle()
+    assert h.lib.b200_step_rows_workspace_bytes(h.ptr, rows, 1, hidden, inter, heads, per) == 0
+    L = model.layers[0]
+    assert real(ids, model.embed, [(L.qkv, L.o, L.gate_up, L.down, L.ln1, L.ln2, L.q_norm, L.k_norm)], model.norm, model.eps, model.cos_sin, i32(tables), i32(lens), heads,
+                model.attn[0].scale) is None
 
 
 def test_two_streams_have_a_workspace_each(monkeypatch):
