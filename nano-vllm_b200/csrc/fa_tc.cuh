@@ -21,8 +21,9 @@
 // most of it the softmax warps' instructions.  128-key blocks with one S per tile read less but put softmax, PV and QK of a tile in one
 // chain: 1950 cycles per 64 keys.  A quarter to a half of the exponentials by a polynomial on the multiply-add pipe shortened the step to
 // 1650 cycles and the time by nothing (the clock gave way).  Items are dealt out longest first (causal tiles late in a sequence see the
-// most keys), every other round from the far end, so CTAs finish together: 4 x 2048 tokens of latent attention 303 -> 285 us the layer, one prompt of 4096 239 -> 201, 3 of
-// 500-1500 behind 1000 others in a window 165 -> 148, packed prompts of 1000-4000 193 -> 177; what runs into the power limit gains a third of that.
+// most keys), every other round from the far end, so CTAs finish together.  One call at a time on a cool GPU, us of the layer: 4 x 2048 tokens of latent attention 303 -> 285, one
+// prompt of 4096 239 -> 201, 3 of 500-1500 behind 1000 others in a window 165 -> 148, packed prompts of 1000-4000 193 -> 177.  Back to back at the power limit's clock: 4 x 2048 of
+// latent attention 331 -> 317; windows (6 of 500-2200, 288 -> 282), 28 short packed prompts and long portions within 2 %, no more than runs of one side differ.
 #pragma once
 #include "tc_common.cuh"
 

@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
 
 constexpr int RG_MAX = 1024;       // experts (identity ones included) the grouped router serves
 constexpr int RG_WARPS = 4;
+static_assert(RG_WARPS * 3 * RG_MAX * sizeof(float) <= 48 * 1024, "a launch without the opt-in to more shared memory");
 
 // One warp per token.  s = softmax(z) over all `E` router outputs (score_kind 0) or sigmoid(z) (1); choice score c = s +
 // correction.  The E outputs form `n_groups` equal groups of neighbours; a group's score is its largest c, and only experts of
@@ -75,7 +76,8 @@ __global__ void __launch_bounds__(RG_WARPS * 32) moe_route_grouped_kernel(const 
                                                                           int32_t* __restrict__ idx, float* __restrict__ wgt) {
     B200_PDL_SYNC();
     extern __shared__ float sh_route[];               // per warp: E plain scores, E scores of choice, E (at least as many as groups) group scores; after the group
-                                                      // choice 1 = open, 0 = closed.  Sized to E: 32 KB for the most experts left 28 warps on an SM
+                                                      // choice 1 = open, 0 = closed.  Sized to E: 48 KB a CTA, 16 warps on an SM for the most experts (8192 tokens of 1024 outputs in 16 groups 87 us; two arrays,
+                                                      // 28 warps and a choice by shuffles 201)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * RG_WARPS + warp;
     if (t >= n) return;

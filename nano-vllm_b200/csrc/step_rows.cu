@@ -3,10 +3,11 @@
 //
 // What bounds such a step: its weights (31 MB a layer at hidden 1024) stream in 5 us, but a layer is a chain of five products that each need all of the one
 // before.  As five launches each link cost 4-5 us: launch, ramp-up, loads of x behind the dependency wait, drain.  Here every SM has one CTA for the
-// whole step, and a link is one exchange through L2 plus the products' own chain, 3-3.5 us in all:
+// whole step, and a link is one exchange through L2 plus the products' own chain, 3.1 us in all at 1 row and 3.4 at 4 (433 and 470 us for the 140 of 28 layers, contexts of 60 tokens):
 //   * Weights: a warp of each CTA copies the CTA's tiles of all layers, in the order of their use, into a ring in shared memory; it never waits for the exchanges, only for
 //     free slots.  A tile is 8 rows of W, the 8-column side of mma.sync; the rows of x are the other side.  (One tcgen05 tile is 128 rows: with so few the
-//     tensor rate is idle either way.)  A chain of 64 products takes 1600 cycles, which only another order of the sums could shorten.
+//     tensor rate is idle either way.)  A chain of 64 products takes 1600 cycles with one accumulator, the launches' order; two would
+//     be shorter and no less exact, with other roundings than theirs.
 //   * Exchange: a result travels as 8 bytes, two bf16 (or one fp32) and the layer's number + 1, stored and loaded whole; who needs it polls for the number.  No
 //     barrier, no fence, no second trip for the data.  The buffers start as zeros.  Each is used again in every layer: whoever writes it has, through the
 //     chain of products, waited for everybody who read it the layer before (each reader publishes something afterwards that all of the next writers need; a CTA
@@ -14,7 +15,7 @@
 //   * Keys and values of the cache do not depend on the step: a warp's first chunks are on their way to L2 a layer ahead, the others two chunks ahead.  Contexts are cut over
 //     CTAs as in decode_small.cu; the first CTA of a context adds the parts up.
 //   * The residual stream stays in shared memory, a copy per CTA: every CTA forms the norms for itself.
-//   * A warp's own chain of instructions is half of a link's time (31 % of the issue slots, nothing else busy), so they are counted: loads without branches, no spilled register (with 28 KB
+//   * A warp's own chain of instructions is half of a link's time (27 % of the issue slots at 4 rows of 1024 tokens, nothing else busy), so they are counted: loads without branches, no spilled register (with 28 KB
 //     of L1 beside the ring each reload is a trip to L2: 500 bytes of them made the step 1.4 times as long).
 // Every sum has the order of the launches it replaces (linear_rows.cu, decode_small.cu): the results are theirs bit for bit.  Captured Qwen3-0.6B step, contexts of 100-1024
 // tokens, us, those launches / this kernel: 1 row 590 / 493, 2 rows 737 / 508, 4 rows 672 / 567, 8 rows 746 / 676; contexts of 16-64 tokens, 1 row 582 / 490.  16 rows took 979

@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
     if (u_lo < u_hi) load_tile(0, u_lo, pg);
     lookup(u_lo + 1, pg);
 
-    // queries of this CTA's rows (plain loads; visible after the loop's first barrier)
+    // queries of this CTA's rows (plain loads; the __syncthreads before their fragments are loaded is the only barrier between the two: the key-sharing loop has none)
     for (int e = tid; e < BM * (DK / 8); e += 128) {
         const int r = e / (DK / 8), c = e - r * (DK / 8);
         const int rr = row0 + r;
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(
         lo_r[hh] = rule.first_key(first + i);
         slope2[hh] = (live[hh] && slopes) ? slopes[g * rep + (rr - i * rep)] * WM_LOG2E : 0.f;
     }
-    // keys any row of this warp sees: [w_lo, w_hi]; keys every row of this warp sees: [f_lo, f_hi] (empty unless all 16 rows are live)
+    // keys any row of this warp sees: [w_lo, w_hi]; keys every row of this warp sees: [f_lo, f_hi] (row tiles: empty unless all 16 rows are live)
     const int wr0 = row0 + wrow, wr1 = min(nrows - 1, wr0 + 15);
     const int w_hi = wr0 < nrows ? first + wr1 / rep : -1;
     const int w_lo = rule.first_key(first + wr0 / rep);
