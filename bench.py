@@ -131,7 +131,7 @@ def bench_config(world: int) -> dict:
 
 def ncu_traffic() -> tuple[float | None, str]:
     """dram__bytes_read.sum + dram__bytes_write.sum of ONE launch of the decode kernel at the batch-256 step, parsed from
-    the newest committed ncu summary under profiles/ (made by profiles/summarize_ncu.py); (None, why) if absent."""
+    the newest committed ncu summary under profiles/; (None, why) if absent."""
     import glob
     import re
     files = sorted(glob.glob(os.path.join(ROOT, "profiles", "r??_decode_kernel_ncu.txt")))
